@@ -69,6 +69,44 @@ def test_grouped_q4_gemm_matches_fp32(Nw, K, counts, out_dtype):
         r0 += n
 
 
+@pytest.mark.parametrize("F,K,counts", [(128, 128, [1, 0, 16, 17, 64, 65, 128, 129, 2]), (640, 2560, [3, 70, 1, 64, 300, 0, 20]),
+                                        (640, 256, [1] * 400 + [0] * 40 + [100] * 9)])      # the last: several units per block, both slot forms
+def test_grouped_q4_swiglu_matches_fp32(F, K, counts):
+    """Gate and up products with the activation in the epilogue: every row against silu(A @ gate^T) * (A @ up^T) in fp32 (bf16
+    output: half a unit in the last place, 2^-9, plus the fp32 sums); rows behind the last one untouched."""
+    import ctypes as C
+    from qwb200.models.quant import dequantize_q4, quantize_q4, to_engine_order
+    from qwb200.ops import lib as qlib
+    L = qlib.load(True)
+    g = torch.Generator(device="cuda").manual_seed(F + K)
+    E = len(counts)
+    W = torch.randn(E * 2 * F, K, generator=g, device="cuda") * 0.05
+    packed, scale = quantize_q4(W, scale_dtype=torch.bfloat16)
+    Wd = dequantize_q4(packed, scale).to(torch.bfloat16).float()
+    words = to_engine_order(packed).contiguous()
+    rows = sum(counts)
+    A = torch.randn(rows, K, generator=g, device="cuda").to(torch.bfloat16)
+    tiles, r0 = [], 0
+    for e, n in enumerate(counts):
+        tiles += [[r0 + t, min(128, n - t), e * 2 * F, 0] for t in range(0, n, 128)]
+        r0 += n
+    tiles += [[0, 0, 0, 0]] * 3
+    tt = torch.tensor(tiles, dtype=torch.int32, device="cuda")
+    out = torch.full((rows + 16, F + 8), 768.0, dtype=torch.bfloat16, device="cuda")
+    P = lambda t: C.c_void_p(t.data_ptr())
+    rc = L.qwk_gemm_q4_tc_swiglu(P(A), P(words), P(scale), P(out), P(tt), len(tiles), rows, E * 2 * F, F, K, K, F + 8,
+                                 C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    torch.cuda.synchronize()
+    assert torch.all(out[rows:].float() == 768.0) and torch.all(out[:, F:].float() == 768.0)
+    r0 = 0
+    for e, n in enumerate(counts):
+        a, w = A[r0:r0 + n].float(), Wd[e * 2 * F:(e + 1) * 2 * F].float()
+        ref = torch.nn.functional.silu(a @ w[:F].T) * (a @ w[F:].T)
+        assert torch.allclose(out[r0:r0 + n, :F].float(), ref, rtol=2 ** -8, atol=1e-3), e
+        r0 += n
+
+
 @pytest.mark.parametrize("T,N,K,ks", [(200, 324, 10240, 3), (128, 128, 256, 2), (77, 40, 640, 1)])
 def test_gemm_tc_split_k_partials_add_up(T, N, K, ks):
     """Split-K form: the partial products of the shares of K, added in order, equal the full product."""

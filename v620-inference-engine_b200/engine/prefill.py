@@ -82,7 +82,7 @@ class Prefiller:
             "scores": z((T, dm.model.d.score_cap), f32), "sel": z((T, c.idx_topk_blocks), i32), "sel_n": z((T,), i32),
             "rs": z((T, self.nrs_ld), f32), "pe": z((T, c.top_k), i32), "pw": z((T, c.top_k), f32),
             "sh_h": z((T, sc.sffn_l), bf), "sd": z((T, c.hidden), f32),
-            "xperm": z((Pn + 128, c.hidden), bf), "h13": z((Pn, 2 * c.ffn), bf), "h": z((Pn + 128, c.ffn), bf),
+            "xperm": z((Pn + 128, c.hidden), bf), "h": z((Pn + 128, c.ffn), bf),
             "y": z((Pn, c.hidden), f32),
             "ple_e": z((T, c.hidden), bf), "ple_kv": z((T, self.ple_ld), f32), "ple_send": z((T, 16), f32), "ple_red": z((T, 16), f32),
             "ple_gv": z((T, sc.xw), f32), "ple_nc": z((T, sc.xw), f32),
@@ -108,6 +108,7 @@ class Prefiller:
             if not self.q4_fused:
                 self.b["w13dq"] = z((sc.exp_l * 2 * c.ffn, c.hidden), bf)
                 self.b["w2dq"] = z((sc.exp_l * c.hidden, c.ffn), bf)
+                self.b["h13"] = z((Pn, 2 * c.ffn), bf)
         # ring of pinned staging buffers: a chunk's row tables are copied when the stream gets to them, which can be long after
         # the next chunk's tables are written on the host, so a buffer is refilled only once the copy that read it has run
         self.rows_ring = [torch.zeros(11 * T, dtype=torch.int32).pin_memory() for _ in range(3)]
@@ -457,10 +458,9 @@ class Prefiller:
         self._ck(L.qwk_moe_sort_T(_p(b["pe"]), T, k, E, 2 * F, H, self.max_tiles, _p(inv), _p(b["src_token"]), _p(t13), _p(t2),
                                   _p(b["bin"]), b["bin"].stride(0), H, _p(b["xperm"]), s), "moe_sort")
         if self.q4_fused:
-            # q4 words converted inside the GEMM's W-operand producer warps: no bf16 copy of the layer's experts
-            self._ck(L.qwk_gemm_q4_tc_grouped(_p(b["xperm"]), P(lw["w13"].data_ptr()), P(lw["s13"].data_ptr()), _p(b["h13"]),
-                                              _p(t13), self.max_tiles, Pn, E * 2 * F, 2 * F, H, H, 2 * F, 1, s), "experts13")
-            self._ck(L.qwk_swiglu_T(_p(b["h13"]), F, _p(b["h"]), Pn, s), "swiglu")
+            # q4 words converted inside the GEMM, the activation in its epilogue: no bf16 copy of the layer's experts
+            self._ck(L.qwk_gemm_q4_tc_swiglu(_p(b["xperm"]), P(lw["w13"].data_ptr()), P(lw["s13"].data_ptr()), _p(b["h"]),
+                                             _p(t13), self.max_tiles, Pn, E * 2 * F, F, H, H, F, s), "experts13")
             self._ck(L.qwk_gemm_q4_tc_grouped(_p(b["h"]), P(lw["w2"].data_ptr()), P(lw["s2"].data_ptr()), _p(b["y"]), _p(t2),
                                               self.max_tiles, Pn, E * H, H, F, F, H, 0, s), "experts2")
         else:

@@ -3,10 +3,10 @@
 // lm_head; role of the reference's rocBLAS call sites, src/kernels/gemm.hip:10-18).
 //
 // Persistent CTAs (two per SM) walk the 128 x 128 output tiles round-robin.  Warp roles:
-//   warp 0   : TMA producer - one thread issues cp.async.bulk.tensor loads (no multicast) of the
+//   warp 0   : TMA producer - one elected lane issues cp.async.bulk.tensor loads (no multicast) of the
 //              128 x 64 A tile and the 128 x 64 W tile of each k block into a 3-stage ring of
 //              128B-swizzled shared-memory tiles, completing on the stage's "full" mbarrier;
-//   warp 1   : allocates 256 TMEM columns (two accumulators), and one thread issues tcgen05.mma (M=128, N=128, K=16,
+//   warp 1   : allocates 256 TMEM columns (two accumulators), and issues tcgen05.mma (one elected lane; M=128, N=128, K=16,
 //              four per k block) reading both operands straight from shared memory through matrix descriptors;
 //              tcgen05.commit releases a stage ("empty" mbarrier) and, after a tile's last k block, signals that
 //              tile's accumulator ("done" mbarrier of the buffer);
@@ -19,9 +19,7 @@
 // an SM: 3 stages x 32 KB and 256 of the 512 TMEM columns each.
 // Every mbarrier wait is bounded; a wait that runs out records an error, the roles leave their loops and the
 // TMEM allocation is released before the kernel returns.
-#include <cuda.h>
-
-#include "stream.cuh"
+#include "tc.cuh"
 #include "tp.cuh"
 
 namespace qw {
@@ -43,34 +41,6 @@ constexpr int TC_STG_STAGES = 5;                 // k-block ring of the staged 1
 template <int BN, int ST, bool STG = false>
 constexpr int tc_smem_bytes() {
     return ST * tc_stage_bytes<BN>() + 1024 /*alignment*/ + 256 /*barriers*/ + (STG ? TC_EPI_WARPS * TC_STG_BYTES : 0);
-}
-
-__device__ __forceinline__ uint64_t make_sw128_desc(uint32_t saddr) {
-    // K-major operand tile, 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFF) >> 4);          // start address
-    d |= (uint64_t)1 << 16;                           // leading byte offset (unused with swizzle)
-    d |= (uint64_t)(1024 >> 4) << 32;                 // stride byte offset
-    d |= (uint64_t)1 << 46;                           // descriptor version (sm_100)
-    d |= (uint64_t)2 << 61;                           // SWIZZLE_128B
-    return d;
-}
-
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int c0, int c1, uint64_t *bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                 ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
-                 : "memory");
-}
-
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_c, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_c), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 struct GemmTcArgs {
@@ -243,18 +213,6 @@ __device__ __forceinline__ void send_piece(const GemmTcArgs &a, float *stg, int 
     }
 }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
 // The epilogue role of both kernels: warps `first_warp` .. `first_warp + n_warps - 1` (n_warps = 4: all 128 columns per warp;
 // 8: half of them), for every tile of this CTA in order.
 template <int BN = TC_BN, bool STG = false>
@@ -296,7 +254,7 @@ __device__ __forceinline__ void epilogue_role(const GemmTcArgs &a, uint32_t tmem
     }
 }
 
-// The MMA role of both kernels (one thread).
+// The MMA role of both kernels (one warp).
 template <int BN = TC_BN, int ST = TC_STAGES>
 __device__ __forceinline__ void mma_role(const GemmTcArgs &a, unsigned char *smem, uint32_t tmem, uint64_t *full, uint64_t *empty,
                                          uint64_t *done, uint64_t *acc_empty, int kblocks) {
@@ -308,21 +266,23 @@ __device__ __forceinline__ void mma_role(const GemmTcArgs &a, unsigned char *sme
         TileAt t;
         if (!tile_at<BN>(a, id, t)) continue;
         const int b = j & 1;
-        if (j >= 2 && !mbar_wait(acc_empty + b, (unsigned)((j >> 1) - 1) & 1u, a.err)) return;
+        if (j >= 2 && !mbar_wait_warp(acc_empty + b, (unsigned)((j >> 1) - 1) & 1u, a.err)) return;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         for (int kb = 0; kb < t.kbn; ++kb, ++it) {
             const unsigned s = it % ST;
-            if (!mbar_wait(full + s, (it / ST) & 1u, a.err)) return;
+            if (!mbar_wait_warp(full + s, (it / ST) & 1u, a.err)) return;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t sa = smem_u32(smem + s * tc_stage_bytes<BN>()), sb = sa + TC_A_BYTES;
+            if (elect_one()) {
 #pragma unroll
-            for (int k = 0; k < TC_BK / 16; ++k) {
-                const uint64_t da = make_sw128_desc(sa + k * 32), db = make_sw128_desc(sb + k * 32);
-                umma_bf16(tmem + (uint32_t)(b * BN), da, db, idesc, (kb | k) ? 1u : 0u);
+                for (int k = 0; k < TC_BK / 16; ++k) {
+                    const uint64_t da = make_sw128_desc(sa + k * 32), db = make_sw128_desc(sb + k * 32);
+                    umma_bf16(tmem + (uint32_t)(b * BN), da, db, idesc, (kb | k) ? 1u : 0u);
+                }
+                umma_commit(empty + s);          // the stage is free once these MMAs have read it
             }
-            umma_commit(empty + s);          // the stage is free once these MMAs have read it
         }
-        umma_commit(done + b);               // this tile's accumulator is complete
+        if (elect_one()) umma_commit(done + b);               // this tile's accumulator is complete
         ++j;
     }
 }
@@ -378,19 +338,19 @@ template <int BN, int ST, bool STG = false>
 __global__ void __launch_bounds__(320, (BN == TC_BN && !STG) ? 2 : 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA,
                                                          const __grid_constant__ CUtensorMap mapW, GemmTcArgs a) {
     extern __shared__ unsigned char raw[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const TcShared sh = tc_setup<BN, ST>(raw, warp, 1, 8);
     const int kblocks = (a.K + TC_BK - 1) / TC_BK;
     if (warp == 0) {
-        if (lane == 0) {
-            unsigned it = 0;
-            bool ok = tp_wait_thread(a.wait);
-            for (int id = blockIdx.x; id < a.total && ok; id += gridDim.x) {
-                TileAt t;
-                if (!tile_at<BN>(a, id, t)) continue;
-                for (int kb = 0; kb < t.kbn; ++kb, ++it) {
-                    const unsigned s = it % ST;
-                    if (it >= ST && !mbar_wait(sh.empty + s, (it / ST - 1) & 1u, a.err)) { ok = false; break; }
+        unsigned it = 0;
+        bool ok = __all_sync(0xffffffffu, tp_wait_thread(a.wait)) != 0;
+        for (int id = blockIdx.x; id < a.total && ok; id += gridDim.x) {
+            TileAt t;
+            if (!tile_at<BN>(a, id, t)) continue;
+            for (int kb = 0; kb < t.kbn; ++kb, ++it) {
+                const unsigned s = it % ST;
+                if (it >= ST && !mbar_wait_warp(sh.empty + s, (it / ST - 1) & 1u, a.err)) { ok = false; break; }
+                if (elect_one()) {
                     mbar_expect_tx(sh.full + s, tc_stage_bytes<BN>());
                     unsigned char *st = sh.smem + s * tc_stage_bytes<BN>();
                     tma_load_2d(st, &mapA, (t.kb0 + kb) * TC_BK, t.t0, sh.full + s);
@@ -399,7 +359,7 @@ __global__ void __launch_bounds__(320, (BN == TC_BN && !STG) ? 2 : 1) gemm_tc_ke
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) mma_role<BN, ST>(a, sh.smem, sh.tmem, sh.full, sh.empty, sh.done, sh.acc_empty, kblocks);
+        mma_role<BN, ST>(a, sh.smem, sh.tmem, sh.full, sh.empty, sh.done, sh.acc_empty, kblocks);
     } else {
         float *stg = nullptr;
         if constexpr (STG)
@@ -487,7 +447,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1) gemm_tc_pair
                                                                                         const __grid_constant__ CUtensorMap mapW,
                                                                                         GemmTcArgs a) {
     extern __shared__ unsigned char raw[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
     const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
@@ -516,14 +476,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1) gemm_tc_pair
     const uint32_t tmem = *tmem_slot;
     const int kblocks = (a.K + TC_BK - 1) / TC_BK;
     if (warp == 0) {
-        if (lane == 0) {
-            unsigned it = 0;
-            bool ok = tp_wait_thread(a.wait);
-            for (int id = cluster_id; id < a.total && ok; id += n_clusters) {
-                const PairTile t = pair_tile_at(a, id, rank);
-                for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                    const unsigned s = it % ST;
-                    if (it >= ST && !mbar_wait(empty + s, (it / ST - 1) & 1u, a.err)) { ok = false; break; }
+        unsigned it = 0;
+        bool ok = __all_sync(0xffffffffu, tp_wait_thread(a.wait)) != 0;
+        for (int id = cluster_id; id < a.total && ok; id += n_clusters) {
+            const PairTile t = pair_tile_at(a, id, rank);
+            for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                const unsigned s = it % ST;
+                if (it >= ST && !mbar_wait_warp(empty + s, (it / ST - 1) & 1u, a.err)) { ok = false; break; }
+                if (elect_one()) {
                     if (rank == 0) mbar_expect_tx(full + s, 2 * TC_PAIR_STAGE_BYTES);
                     const uint32_t bar = map_to_cta(smem_u32(full + s), 0);
                     unsigned char *st = smem + s * TC_PAIR_STAGE_BYTES;
@@ -533,7 +493,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1) gemm_tc_pair
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             // instruction descriptor: D fp32, A/B bf16, both K-major, N = 256, M = 256 (the pair's rows)
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TC_PAIR_BN >> 3) << 17) | ((uint32_t)(TC_PAIR_BM >> 4) << 24);
             int j = 0;
@@ -541,20 +501,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1) gemm_tc_pair
             bool ok = true;
             for (int id = cluster_id; id < a.total && ok; id += n_clusters) {
                 const int b = j & 1;
-                if (j >= 2 && !mbar_wait(acc_empty + b, (unsigned)((j >> 1) - 1) & 1u, a.err)) break;
+                if (j >= 2 && !mbar_wait_warp(acc_empty + b, (unsigned)((j >> 1) - 1) & 1u, a.err)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (int kb = 0; kb < kblocks; ++kb, ++it) {
                     const unsigned s = it % ST;
-                    if (!mbar_wait(full + s, (it / ST) & 1u, a.err)) { ok = false; break; }
+                    if (!mbar_wait_warp(full + s, (it / ST) & 1u, a.err)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t sa = smem_u32(smem + s * TC_PAIR_STAGE_BYTES), sb = sa + TC_A_BYTES;
+                    if (elect_one()) {
 #pragma unroll
-                    for (int k = 0; k < TC_BK / 16; ++k)
-                        umma_bf16_pair(tmem + (uint32_t)(b * TC_PAIR_BN), make_sw128_desc(sa + k * 32), make_sw128_desc(sb + k * 32), idesc,
-                                       (kb | k) ? 1u : 0u);
-                    umma_commit_pair(empty + s);
+                        for (int k = 0; k < TC_BK / 16; ++k)
+                            umma_bf16_pair(tmem + (uint32_t)(b * TC_PAIR_BN), make_sw128_desc(sa + k * 32), make_sw128_desc(sb + k * 32), idesc,
+                                           (kb | k) ? 1u : 0u);
+                        umma_commit_pair(empty + s);
+                    }
                 }
-                if (ok) umma_commit_pair(done + b);
+                if (ok && elect_one()) umma_commit_pair(done + b);
                 ++j;
             }
         }
@@ -606,192 +568,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1) gemm_tc_pair
     tp_signal(a.epi.sig);
 }
 
-// ------------------------------------------------------------------------------------------------------------------
-// Grouped GEMM with the weights in q4 (group 128, bf16 scales): the expert products of token-major prefill without a
-// bf16 copy of the layer's experts.  Same tile, pipeline and epilogue as gemm_tc_kernel; the W operand of a stage is
-// not loaded by TMA but produced by eight extra warps: two threads own row r of the 128 x 64 W tile, each fetches 4 q4
-// words (16 bytes) and the block's scale four k blocks ahead, converts them to four 16-byte bf16 chunks of the row with
-// packed bf16 arithmetic (the same values as the stand-alone dequantisation) and stores them where the 128-byte
-// swizzle puts them (chunk c of row r at chunk c ^ (r & 7)); a proxy fence makes the stores visible to the tensor
-// core's reads, and the thread arrives on the stage's "full" barrier (1 TMA arrival + 256 producer arrivals).  What
-// bounds the kernel is how fast the producer warps turn words into tiles (~150 instructions per thread and k block),
-// hence eight of them and two-wide arithmetic.
-// (Role of the reference's moe_gate_up_T / moe_down_T, src/kernels/moe_experts.hip:17-27.)
-// ------------------------------------------------------------------------------------------------------------------
-constexpr int Q4_AHEAD = 4;
-
-// grid: min(tiles, 2 x SMs) CTAs of 448 threads: warp 0 TMA (A), warp 1 MMA, warps 2-5 epilogue, warps 6-13 W producers.
-__global__ void __launch_bounds__(448, 2) gemm_tc_q4_kernel(const __grid_constant__ CUtensorMap mapA, GemmTcArgs a,
-                                                            const uint32_t *Wq, const bf16 *scale, long long w_rows) {
-    extern __shared__ unsigned char raw[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const TcShared sh = tc_setup(raw, warp, 1 + 256, 4);
-    const int kblocks = (a.K + TC_BK - 1) / TC_BK;
-    if (warp == 0) {
-        if (lane == 0) {
-            unsigned it = 0;
-            bool ok = true;
-            for (int id = blockIdx.x; id < a.total && ok; id += gridDim.x) {
-                TileAt t;
-                if (!tile_at(a, id, t)) continue;
-                for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                    const unsigned s = it % TC_STAGES;
-                    if (it >= TC_STAGES && !mbar_wait(sh.empty + s, (it / TC_STAGES - 1) & 1u, a.err)) { ok = false; break; }
-                    mbar_expect_tx(sh.full + s, TC_A_BYTES);
-                    tma_load_2d(sh.smem + s * TC_STAGE_BYTES, &mapA, kb * TC_BK, t.t0, sh.full + s);
-                }
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) mma_role(a, sh.smem, sh.tmem, sh.full, sh.empty, sh.done, sh.acc_empty, kblocks);
-    } else if (warp >= 6) {
-        // W producers: two threads per row of the tile, 32 k values (4 words, 4 chunks) each
-        const int p = threadIdx.x - 192, r = p >> 1, hf = p & 1;
-        const int wpr = a.K >> 3, spr = a.K >> 7;
-        const bf162 off2 = __floats2bfloat162_rn(136.f, 136.f);
-        unsigned it0 = 0;                        // k blocks of the tiles before this one
-        bool ok = true;
-        for (int id = blockIdx.x; id < a.total && ok; id += gridDim.x) {
-            TileAt t;
-            if (!tile_at(a, id, t)) continue;
-            const long long wrow = (long long)t.w0 + r;
-            const bool row_ok = t.n0 + r < a.N && wrow < w_rows;
-            const uint4 *src = reinterpret_cast<const uint4 *>(Wq + (row_ok ? wrow : 0) * wpr) + hf;
-            const unsigned short *sc_bits = reinterpret_cast<const unsigned short *>(scale + (row_ok ? wrow : 0) * spr);
-            uint4 ring[Q4_AHEAD];
-            unsigned short sring[Q4_AHEAD];      // the k block's scale travels with its words: no dependent load in the loop
-#pragma unroll
-            for (int i = 0; i < Q4_AHEAD; ++i) {
-                ring[i] = make_uint4(0u, 0u, 0u, 0u);
-                sring[i] = 0;
-                if (row_ok && i < kblocks) {
-                    ring[i] = __ldg(src + 2 * i);
-                    sring[i] = __ldg(sc_bits + (i >> 1));
-                }
-            }
-            for (int kb0 = 0; kb0 < kblocks && ok; kb0 += Q4_AHEAD) {
-#pragma unroll
-                for (int i = 0; i < Q4_AHEAD; ++i) {
-                    const int kb = kb0 + i;
-                    if (kb >= kblocks) break;
-                    const unsigned it = it0 + (unsigned)kb, s = it % TC_STAGES;
-                    const uint4 q = ring[i];
-                    // scale as a bf16 pair; (nibble - 8) is exact in bf16 and its product with a bf16 scale, rounded once to
-                    // bf16, equals the fp32 product rounded to bf16: the stand-alone conversion's values bit for bit
-                    const uint32_t sb = (uint32_t)sring[i] | ((uint32_t)sring[i] << 16);
-                    const bf162 sc2 = *reinterpret_cast<const bf162 *>(&sb);
-                    if (row_ok && kb + Q4_AHEAD < kblocks) {
-                        ring[i] = __ldg(src + 2 * (kb + Q4_AHEAD));
-                        sring[i] = __ldg(sc_bits + ((kb + Q4_AHEAD) >> 1));
-                    }
-                    if (it >= TC_STAGES && !mbar_wait(sh.empty + s, (it / TC_STAGES - 1) & 1u, a.err)) { ok = false; break; }
-                    unsigned char *dst = sh.smem + s * TC_STAGE_BYTES + TC_A_BYTES + r * 128;
-                    const uint32_t words[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        uint32_t o[4];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            uint32_t bits = ((words[c] >> (4 * j)) & 0x000F000Fu) | 0x43004300u;
-                            const bf162 v = __hmul2(__hsub2(*reinterpret_cast<bf162 *>(&bits), off2), sc2);
-                            o[j] = *reinterpret_cast<const uint32_t *>(&v);
-                        }
-                        *reinterpret_cast<uint4 *>(dst + (((hf * 4 + c) ^ (r & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-                    }
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                    mbar_arrive(sh.full + s);
-                }
-            }
-            it0 += (unsigned)kblocks;
-        }
-    } else {
-        epilogue_role(a, sh.tmem, sh.done, sh.acc_empty, warp, lane, 2, 4);
-    }
-    tc_teardown(sh, warp);
-}
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess) fn = (EncodeTiledFn)p;
-    }
-    return fn;
-}
-
-// 2-D bf16 row-major matrix [rows][cols] (row stride ld elements), box = 64 columns x box_rows rows, 128B swizzle.
-// A chunk issues ~800 of these for a few dozen distinct (address, shape) pairs - weights and the engine's fixed buffers -
-// so encoded maps are kept in a small direct-mapped table (per thread: the launchers run on the caller's thread) and an
-// encode is paid only on a miss.  A map depends on nothing but the key: the same address with the same shape encodes to
-// the same map whatever the memory holds.
-struct MapKey {
-    const void *base;
-    long long rows, cols, ld;
-    int box_rows, dev;
-    bool operator==(const MapKey &o) const {
-        return base == o.base && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && dev == o.dev;
-    }
-};
-struct MapSlot {
-    MapKey key;
-    CUtensorMap map;
-    bool used;
-};
-constexpr int MAP_SLOTS = 256;
-
-static bool make_map(CUtensorMap *m, const void *base, long long rows, long long cols, long long ld, int box_rows) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return false;
-    static thread_local MapSlot table[MAP_SLOTS] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const MapKey key{base, rows, cols, ld, box_rows, dev};
-    unsigned long long h = (unsigned long long)(uintptr_t)base * 0x9E3779B97F4A7C15ull;
-    h ^= (unsigned long long)rows * 0xC2B2AE3D27D4EB4Full + (unsigned long long)cols * 0x165667B19E3779F9ull + (unsigned long long)ld * 31 + box_rows;
-    MapSlot &slot = table[(h >> 40) % MAP_SLOTS];
-    if (slot.used && slot.key == key) {
-        *m = slot.map;
-        return true;
-    }
-    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    cuuint32_t box[2] = {(cuuint32_t)TC_BK, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    if (fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return false;
-    slot.key = key;
-    slot.map = *m;
-    slot.used = true;
-    return true;
-}
-
-// `per_sm` persistent CTAs per SM of the current device, or one CTA per tile when there are fewer tiles.
-static unsigned persistent_grid(int total, int per_sm = 2) {
-    static int sms[64] = {0};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) dev = 0;
-    if (!sms[dev]) {
-        int n = 0;
-        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-        sms[dev] = n;
-    }
-    const int cap = per_sm * sms[dev];
-    return (unsigned)(total < cap ? total : cap);
-}
-
 }  // namespace qw
 
 using namespace qw;
 
 // One-time (per device) opt-in to the kernels' dynamic shared memory.
-static bool configure_once(int which) {          // 0 dense 128-wide, 1 q4 grouped, 2 dense 256-wide, 3 / 4 the two with a staged epilogue, 5 / 6 the pair form
+static bool configure_once(int which) {          // 0 dense 128-wide, 2 dense 256-wide, 3 / 4 the two with a staged epilogue, 5 / 6 the pair form
     static bool done[7][64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -799,7 +581,6 @@ static bool configure_once(int which) {          // 0 dense 128-wide, 1 q4 group
     if (!done[which][dev]) {
         cudaError_t e;
         if (which == 0) e = cudaFuncSetAttribute(gemm_tc_kernel<TC_BN, TC_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
-        else if (which == 1) e = cudaFuncSetAttribute(gemm_tc_q4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
         else if (which == 2) e = cudaFuncSetAttribute(gemm_tc_kernel<TC_WIDE_BN, TC_WIDE_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                       tc_smem_bytes<TC_WIDE_BN, TC_WIDE_STAGES>());
         else if (which == 3) e = cudaFuncSetAttribute(gemm_tc_kernel<TC_BN, TC_STG_STAGES, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -960,25 +741,6 @@ QW_API int qwk_gemm_bf16_tc_grouped(const void *A, const void *W, void *C, const
     a.ksplit = 1; a.kb_per = 0; a.c_split = 0;
     if (!configure_once(0)) return -3;
     gemm_tc_kernel<TC_BN, TC_STAGES><<<persistent_grid(a.total), 320, TC_SMEM, s>>>(mA, mW, a);
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
-}
-
-// Grouped form with q4 weights: Wq uint32 [w_rows][K/8] (engine nibble order), scale bf16 [w_rows][K/128]; otherwise
-// as qwk_gemm_bf16_tc_grouped.  K a multiple of 128.
-QW_API int qwk_gemm_q4_tc_grouped(const void *A, const void *Wq, const void *scale, void *C, const void *tiles, int max_tiles,
-                                  int rows, long long w_rows, int Nw, int K, int lda, int ldc, int out_bf16, cudaStream_t s) {
-    if (rows <= 0 || max_tiles <= 0) return 0;
-    if ((K & 127) || (lda & 7) || ((uintptr_t)A & 15) || ((uintptr_t)Wq & 15)) return -1;
-    CUtensorMap mA;
-    if (!make_map(&mA, A, rows, K, lda, TC_BM)) return -3;
-    GemmTcArgs a{};
-    a.C32 = out_bf16 ? nullptr : (float *)C;
-    a.C16 = out_bf16 ? (bf16 *)C : nullptr;
-    a.T = rows; a.N = Nw; a.K = K; a.ldc = ldc; a.err = g_err_ptr; a.tiles = (const int4 *)tiles;
-    a.tiles_t = max_tiles; a.tiles_n = (Nw + TC_BN - 1) / TC_BN; a.total = a.tiles_t * a.tiles_n;
-    a.ksplit = 1; a.kb_per = 0; a.c_split = 0;
-    if (!configure_once(1)) return -3;
-    gemm_tc_q4_kernel<<<persistent_grid(a.total), 448, TC_SMEM, s>>>(mA, a, (const uint32_t *)Wq, (const bf16 *)scale, w_rows);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -26,7 +26,6 @@ int qwk_gemm_tc_pair_min_n(int min_n);
 int qwk_gemm_bf16_tc(const void *A, const void *W, void *C, int T, int N, int K, int lda, int ldw, int ldc, int out_bf16, cudaStream_t s);
 int qwk_gemm_bf16_tc_tp(void *tp_, const void *A, const void *W, void *C, int T, int N, int K, int lda, int ldw, int ldc, int out_bf16, int wait_kind, int epi_mode, int epi_kind, int ld_epi, cudaStream_t s);
 int qwk_gemm_bf16_tc_grouped(const void *A, const void *W, void *C, const void *tiles, int max_tiles, int rows, long long w_rows, int Nw, int K, int lda, int ldw, int ldc, int out_bf16, cudaStream_t s);
-int qwk_gemm_q4_tc_grouped(const void *A, const void *Wq, const void *scale, void *C, const void *tiles, int max_tiles, int rows, long long w_rows, int Nw, int K, int lda, int ldc, int out_bf16, cudaStream_t s);
 int qwk_gemm_bf16_tc_splitk(const void *A, const void *W, float *C, int T, int N, int K, int lda, int ldw, int ldc, int ksplit, long long c_split, cudaStream_t s);
 
 // gemv.cu
@@ -55,6 +54,10 @@ int qwk_moe_router(const void *Wrs, const void *x, float *rs, int nrs, int K, in
 int qwk_moe_route(const float *rs, int ld_rs, int M, int E, int top_k, int F, int e_first, int e_local, int *pair_expert, float *pair_w, void *sh_h, cudaStream_t s);
 int qwk_moe_gate_up_pair(const void *w13, const void *s13, const void *x, int ldx, const int *pair_expert, int M, int top_k, int F, int K, void *h, cudaStream_t s);
 int qwk_moe_down_combine(const void *w2, const void *s2, const void *h, const int *pair_expert, const float *pair_w, int M, int top_k, int F, int H, const void *shared_down, int ld_sd, const void *sh_h, int SF, float *out, int ldo, cudaStream_t s);
+
+// moe_tc.cu
+int qwk_gemm_q4_tc_grouped(const void *A, const void *Wq, const void *scale, void *C, const void *tiles, int max_tiles, int rows, long long w_rows, int Nw, int K, int lda, int ldc, int out_bf16, cudaStream_t s);
+int qwk_gemm_q4_tc_swiglu(const void *A, const void *Wq, const void *scale, void *C, const void *tiles, int max_tiles, int rows, long long w_rows, int F, int K, int lda, int ldc, cudaStream_t s);
 
 // mtp.cu
 int qwk_mtp_norm(const float *hidden, const int *tokens, const void *embed, int vocab, const float *nh1, const float *ne1, int H, int hc, float eps, void *hn, void *en, int M, cudaStream_t s);

@@ -415,16 +415,9 @@ struct Builder {
             const QwPrefillBufs &b = *c.b;
             const QwLayer &w = layer_of(c);
             const long long p0 = (long long)L.r0 * k;
-            PF_TRY(1, qwk_gemm_q4_tc_grouped(h_at(b.xperm, p0, H), w.w13, w.s13, h_at(b.h13, p0, 2 * F),
-                                             (char *)b.t13 + (long long)(l == 1) * b.max_tiles * 16, b.max_tiles, L.n * k, (long long)E * 2 * F, 2 * F, H, H,
-                                             2 * F, 1, L.s));
-        });
-        cur_cat = CAT_EXPERTS;
-        add([=](PCtx &c) {
-            const Lane &L = c.lane[l];
-            const QwPrefillBufs &b = *c.b;
-            const long long p0 = (long long)L.r0 * k;
-            PF_TRY(1, qwk_swiglu_T(h_at(b.h13, p0, 2 * F), F, h_at(b.h, p0, F), (long long)L.n * k, L.s));
+            PF_TRY(1, qwk_gemm_q4_tc_swiglu(h_at(b.xperm, p0, H), w.w13, w.s13, h_at(b.h, p0, F),
+                                            (char *)b.t13 + (long long)(l == 1) * b.max_tiles * 16, b.max_tiles, L.n * k, (long long)E * 2 * F, F, H, H,
+                                            F, L.s));
         });
         cur_cat = CAT_EXPERTS;
         add([=](PCtx &c) {

@@ -1,0 +1,142 @@
+// What the tensor-core (tcgen05) kernels share: operand descriptors, TMA tile loads, MMA issue and commit, accumulator reads,
+// tensor maps and the size of a persistent grid.
+#pragma once
+#include <cuda.h>
+
+#include "stream.cuh"
+
+namespace qw {
+
+__device__ __forceinline__ uint64_t make_sw128_desc(uint32_t saddr) {
+    // K-major operand tile, 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr & 0x3FFFF) >> 4);          // start address
+    d |= (uint64_t)1 << 16;                           // leading byte offset (unused with swizzle)
+    d |= (uint64_t)(1024 >> 4) << 32;                 // stride byte offset
+    d |= (uint64_t)1 << 46;                           // descriptor version (sm_100)
+    d |= (uint64_t)2 << 61;                           // SWIZZLE_128B
+    return d;
+}
+
+__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int c0, int c1, uint64_t *bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+                 ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(smem_u32(bar))
+                 : "memory");
+}
+
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_c, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_c), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit(uint64_t *bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// Roles that issue TMA loads and MMAs run as whole warps and elect the issuing lane at each group of instructions: tcgen05.mma
+// takes its descriptors from uniform registers, which the compiler can only keep across the loop when the branch is uniform for
+// the warp.  From a branch on one thread an MMA took 106 cycles to issue (83 with A in tensor memory) whatever its width;
+// elected, a 128 x 128 x 16 one takes 85 (68).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+// mbar_wait for a whole warp: one verdict for all lanes, so that the warp stays together when a wait runs out.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, unsigned parity, ErrorWord *err) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)) != 0;
+}
+
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
+                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+static EncodeTiledFn encode_fn() {
+    static EncodeTiledFn fn = nullptr;
+    if (!fn) {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess) fn = (EncodeTiledFn)p;
+    }
+    return fn;
+}
+
+// 2-D row-major matrix [rows][cols] (row stride ld elements) read in boxes of box_rows rows: bf16, 64 columns (128 bytes, 128B
+// swizzle), or bytes, 64 columns (64B swizzle).
+// A chunk issues ~800 of these for a few dozen distinct (address, shape) pairs - weights and the engine's fixed buffers -
+// so encoded maps are kept in a small direct-mapped table (per thread: the launchers run on the caller's thread) and an
+// encode is paid only on a miss.  A map depends on nothing but the key: the same address with the same shape encodes to
+// the same map whatever the memory holds.
+struct MapKey {
+    const void *base;
+    long long rows, cols, ld;
+    int box_rows, dev, bytes;
+    bool operator==(const MapKey &o) const {
+        return base == o.base && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && dev == o.dev && bytes == o.bytes;
+    }
+};
+struct MapSlot {
+    MapKey key;
+    CUtensorMap map;
+    bool used;
+};
+constexpr int MAP_SLOTS = 256;
+
+static bool make_map(CUtensorMap *m, const void *base, long long rows, long long cols, long long ld, int box_rows, bool bytes = false) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return false;
+    static thread_local MapSlot table[MAP_SLOTS] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const MapKey key{base, rows, cols, ld, box_rows, dev, bytes};
+    unsigned long long h = (unsigned long long)(uintptr_t)base * 0x9E3779B97F4A7C15ull;
+    h ^= (unsigned long long)rows * 0xC2B2AE3D27D4EB4Full + (unsigned long long)cols * 0x165667B19E3779F9ull + (unsigned long long)ld * 31 + box_rows * 2 + bytes;
+    MapSlot &slot = table[(h >> 40) % MAP_SLOTS];
+    if (slot.used && slot.key == key) {
+        *m = slot.map;
+        return true;
+    }
+    cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * (bytes ? 1 : 2)};
+    cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    if (fn(m, bytes ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+           bytes ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return false;
+    slot.key = key;
+    slot.map = *m;
+    slot.used = true;
+    return true;
+}
+
+// `per_sm` persistent CTAs per SM of the current device, or one CTA per tile when there are fewer tiles.
+static unsigned persistent_grid(int total, int per_sm = 2) {
+    static int sms[64] = {0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    if (!sms[dev]) {
+        int n = 0;
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+        sms[dev] = n;
+    }
+    const int cap = per_sm * sms[dev];
+    return (unsigned)(total < cap ? total : cap);
+}
+
+}  // namespace qw
