@@ -30,6 +30,30 @@ def test_attention_kernel_matches_fp32():
         assert rel(out, ref) < 1.5e-2, (L, rel(out, ref))
 
 
+@pytest.mark.parametrize("L,heads,size", [(1, 2, 1.0), (127, 1, 1.0), (128, 3, 1.0), (129, 2, 1.0), (256, 1, 1.0), (257, 2, 1.0),
+                                          (700, 5, 1.0), (520, 40, 1.0), (600, 2, 8.0), (300, 2, 40.0)])
+def test_attention_tile_edges_units_and_large_scores(L, heads, size):
+    """Key and query tiles with remainders, one and several units per block, and scores large enough that the running maximum
+    jumps between key tiles (late keys are made larger).  Against 64 bits; the kernel rounds the probabilities and the result
+    to bf16 (2^-9 each, relative to the row), so 1e-2 of the result's size bounds the error."""
+    import ctypes as C
+    from qwb200.ops import lib as qlib
+    L_ = qlib.load(True)
+    hd, D = 72, heads * 72
+    g = torch.Generator().manual_seed(L + heads)
+    qkv = torch.randn(L, 3 * D, generator=g)
+    qkv[:, D:2 * D] *= size * torch.linspace(0.2, 1.0, L)[:, None]
+    qkv = qkv.to(torch.bfloat16).cuda()
+    out = torch.full((L + 3, D), 7.0, dtype=torch.bfloat16, device="cuda")
+    s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert L_.qwk_vit_attention(C.c_void_p(qkv.data_ptr()), L, heads, C.c_void_p(out.data_ptr()), s) == 0
+    q, k, v = [t.double().view(L, heads, hd) for t in qkv.split(D, 1)]
+    att = torch.softmax(torch.einsum("qhd,khd->hqk", q, k) / math.sqrt(hd), -1)
+    ref = torch.einsum("hqk,khd->qhd", att, v).reshape(L, D)
+    assert rel(out[:L], ref) < 1e-2, rel(out[:L], ref)
+    assert torch.all(out[L:] == 7.0)
+
+
 def test_encoder_matches_reference_forward():
     from qwb200.vision import VisionConfig, VisionEncoder, synth_vision_weights, vision_reference
     cfg = VisionConfig(depth=3)

@@ -55,27 +55,11 @@ struct MgSlots {
     unsigned used[2], committed[2];
 };
 
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_c, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_c), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
 // Eight columns at a time: the packed pairs of two q4 words go out as they are formed, so no 32-register block is assembled.
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};"
                  ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(taddr)
                  : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr));
 }
 
 // The first used unit at or after `id` (steps of the grid); tl must hold the entry of `id` when id < total.
@@ -116,40 +100,6 @@ struct MgWalk {
         tl.z = __shfl_sync(0xffffffffu, tl.z, 0);
     }
 };
-
-// A wait that sleeps in hardware: most warps of this kernel wait most of the time, and what they would issue while polling is
-// taken from the converting warps.  Bounded by time (2 s) like every wait.
-__device__ __forceinline__ bool mg_try(uint64_t *bar, unsigned parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(20000u)
-        : "memory");
-    return ok != 0;
-}
-__device__ __noinline__ bool mg_wait_slow(uint64_t *bar, unsigned parity, ErrorWord *err) {
-    unsigned long long t0, t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
-    while (!mg_try(bar, parity)) {
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-        if (t - t0 > 2000000000ull) {
-            report(err, ERR_WAIT_TIMEOUT, __LINE__);
-            return false;
-        }
-        // another waiter already gave up: do not sit out the whole limit
-        if (err && *reinterpret_cast<volatile unsigned int *>(&err->code)) return false;
-    }
-    return true;
-}
-__device__ __forceinline__ bool mg_wait(uint64_t *bar, unsigned parity, ErrorWord *err) {
-    return mg_try(bar, parity) || mg_wait_slow(bar, parity, err);
-}
-__device__ __forceinline__ bool mg_wait_warp(uint64_t *bar, unsigned parity, ErrorWord *err) {
-    return __all_sync(0xffffffffu, mg_wait(bar, parity, err)) != 0;
-}
 
 template <bool SWIGLU>
 __global__ void __launch_bounds__(MG_THREADS, 1) moe_tc_kernel(const __grid_constant__ CUtensorMap mapX,
@@ -411,7 +361,7 @@ static int moe_tc_launch(MoeTcArgs &a, const void *A, const void *Wq, int rows, 
         done[dev] = true;
     }
     CUtensorMap mX, mW;
-    if (!make_map(&mX, A, rows, a.K, lda, 16) || !make_map(&mW, Wq, a.w_rows, a.K / 2, a.K / 2, 128, true)) return -3;
+    if (!make_map(&mX, A, rows, a.K, lda, 16) || !make_map(&mW, Wq, a.w_rows, a.K / 2, a.K / 2, 128, MAP_BYTES64)) return -3;
     a.err = g_err_ptr;
     a.mask = 0x000F000Fu;
     a.magic = 0x43004300u;

@@ -50,7 +50,57 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, unsigned parity, E
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)) != 0;
 }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_c, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_c), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
+// A wait that sleeps in hardware: where many warps of a block wait most of the time, what they would issue while polling is
+// taken from the working ones.  Bounded by time (2 s) like every wait.
+__device__ __forceinline__ bool mg_try(uint64_t *bar, unsigned parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(20000u)
+        : "memory");
+    return ok != 0;
+}
+static __device__ __noinline__ bool mg_wait_slow(uint64_t *bar, unsigned parity, ErrorWord *err) {
+    unsigned long long t0, t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    while (!mg_try(bar, parity)) {
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+        if (t - t0 > 2000000000ull) {
+            report(err, ERR_WAIT_TIMEOUT, __LINE__);
+            return false;
+        }
+        // another waiter already gave up: do not sit out the whole limit
+        if (err && *reinterpret_cast<volatile unsigned int *>(&err->code)) return false;
+    }
+    return true;
+}
+__device__ __forceinline__ bool mg_wait(uint64_t *bar, unsigned parity, ErrorWord *err) {
+    return mg_try(bar, parity) || mg_wait_slow(bar, parity, err);
+}
+__device__ __forceinline__ bool mg_wait_warp(uint64_t *bar, unsigned parity, ErrorWord *err) {
+    return __all_sync(0xffffffffu, mg_wait(bar, parity, err)) != 0;
+}
+
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr));
+}
+
+__device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
         "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
@@ -59,7 +109,17 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
           "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
           "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
         : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+    tmem_ld32_nowait(taddr, v);
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};"
+                 ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+                   "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(taddr)
+                 : "memory");
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
@@ -76,8 +136,10 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
-// 2-D row-major matrix [rows][cols] (row stride ld elements) read in boxes of box_rows rows: bf16, 64 columns (128 bytes, 128B
-// swizzle), or bytes, 64 columns (64B swizzle).
+// 2-D row-major matrix [rows][cols] (row stride ld elements) read in boxes of box_rows rows:
+enum MapKind { MAP_BF16 = 0,        // bf16, 64 columns, 128B swizzle
+               MAP_BYTES64 = 1,     // bytes, 64 columns, 64B swizzle
+               MAP_BF16_X8 = 2 };   // bf16, 8 columns (16 bytes), no swizzle
 // A chunk issues ~800 of these for a few dozen distinct (address, shape) pairs - weights and the engine's fixed buffers -
 // so encoded maps are kept in a small direct-mapped table (per thread: the launchers run on the caller's thread) and an
 // encode is paid only on a miss.  A map depends on nothing but the key: the same address with the same shape encodes to
@@ -85,9 +147,9 @@ static EncodeTiledFn encode_fn() {
 struct MapKey {
     const void *base;
     long long rows, cols, ld;
-    int box_rows, dev, bytes;
+    int box_rows, dev, kind;
     bool operator==(const MapKey &o) const {
-        return base == o.base && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && dev == o.dev && bytes == o.bytes;
+        return base == o.base && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && dev == o.dev && kind == o.kind;
     }
 };
 struct MapSlot {
@@ -97,26 +159,26 @@ struct MapSlot {
 };
 constexpr int MAP_SLOTS = 256;
 
-static bool make_map(CUtensorMap *m, const void *base, long long rows, long long cols, long long ld, int box_rows, bool bytes = false) {
+static bool make_map(CUtensorMap *m, const void *base, long long rows, long long cols, long long ld, int box_rows, MapKind kind = MAP_BF16) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
     static thread_local MapSlot table[MAP_SLOTS] = {};
     int dev = 0;
     cudaGetDevice(&dev);
-    const MapKey key{base, rows, cols, ld, box_rows, dev, bytes};
+    const MapKey key{base, rows, cols, ld, box_rows, dev, kind};
     unsigned long long h = (unsigned long long)(uintptr_t)base * 0x9E3779B97F4A7C15ull;
-    h ^= (unsigned long long)rows * 0xC2B2AE3D27D4EB4Full + (unsigned long long)cols * 0x165667B19E3779F9ull + (unsigned long long)ld * 31 + box_rows * 2 + bytes;
+    h ^= (unsigned long long)rows * 0xC2B2AE3D27D4EB4Full + (unsigned long long)cols * 0x165667B19E3779F9ull + (unsigned long long)ld * 31 + box_rows * 4 + kind;
     MapSlot &slot = table[(h >> 40) % MAP_SLOTS];
     if (slot.used && slot.key == key) {
         *m = slot.map;
         return true;
     }
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)ld * (bytes ? 1 : 2)};
-    cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
+    cuuint64_t strides[1] = {(cuuint64_t)ld * (kind == MAP_BYTES64 ? 1 : 2)};
+    cuuint32_t box[2] = {kind == MAP_BF16_X8 ? 8u : 64u, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
-    if (fn(m, bytes ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-           bytes ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    if (fn(m, kind == MAP_BYTES64 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+           kind == MAP_BYTES64 ? CU_TENSOR_MAP_SWIZZLE_64B : kind == MAP_BF16_X8 ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return false;
     slot.key = key;
     slot.map = *m;

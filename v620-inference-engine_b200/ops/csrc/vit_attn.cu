@@ -1,0 +1,280 @@
+// Attention of the vision tower on the 5th-generation tensor cores: non-causal, one image or video slice, head dim 72.
+// (Role of the reference's src/kernels/vision.hip attention.)
+//
+// A CTA takes 256 queries of one head as two tiles of 128 and walks the keys in tiles of 128.  Per tile S = Q K^T (128 x 128, fp32)
+// and O += P V accumulate in tensor memory; a thread of the tile's warp group owns one query row: it reads its 128 scores, keeps
+// the running reference maximum and sum in registers, and writes the probabilities back over the scores as bf16, where the second
+// product reads them as its A operand.  While one tile's scores are turned into probabilities the tensor core works for the other.
+//   warp 0       TMA: Q once per unit, K and V tiles of 128 rows, three stages each
+//   warp 1       MMAs: S0, S1, then per key tile PV0, next S0, PV1, next S1
+//   warps 4-11   softmax, one warp group per query tile
+// O is rescaled only when a row's maximum rises by more than 8 (in log2 units) above the reference the sums use: the probabilities
+// then stay below 256, which costs nothing in bf16 or fp32, and the rescaling pass over O is rare after the first tile.
+// Head dim 72 = 64 + 8: a row's first 64 values are a 128B-swizzled panel, the last 8 a panel of 16-byte rows whose partner (the
+// other 8 of an MMA's k = 16) is a zeroed block.  V is read as it lies (key-major): 64 + 64 columns, of which the second panel's
+// first 8 count; the rest belongs to other heads and lands in columns of O that nobody reads.
+// What bounds it: the exponentials (128 x 128 per tile at 16 a cycle and SM: 1024 cycles; MMAs 780), and 224 units on 148 SMs for
+// 3520 patches and 16 heads.  It replaces a flash kernel on mma.sync (16 queries a warp, each warp reading every K and V fragment
+// from shared memory), which took 444 us there; the tower as a whole went from 18.4 to 11.0 ms.
+#include "tc.cuh"
+
+namespace qw {
+
+constexpr int VT_D = 72, VT_STAGES = 3, VT_THREADS = 384;
+constexpr int VT_KA = 128 * 128, VT_KB = 128 * 16, VT_K = VT_KA + 2 * VT_KB;      // K (and Q) tile: wide panel, narrow panel, its zeros
+constexpr int VT_V = 2 * 128 * 128;
+constexpr int VT_SMEM = 2 * VT_K + VT_STAGES * (VT_K + VT_V) + 1024 + 512;
+
+struct VitAttnArgs {
+    int L, heads, qtiles;
+    bf16 *out;
+    float scale;             // log2(e) / sqrt(72)
+    ErrorWord *err;
+};
+
+// No-swizzle K-major operand: rows of 16 bytes, 8-row groups 128 bytes apart, the second k half `lbo` bytes further.
+__device__ __forceinline__ uint64_t make_plain_desc(uint32_t saddr, uint32_t lbo) {
+    return (uint64_t)((saddr & 0x3FFFF) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(128 >> 4) << 32) | ((uint64_t)1 << 46);
+}
+// 128B-swizzled operand that lies MN-major (rows of 64 MN values per k): 8-k groups 1024 bytes apart, the next 64 MN values `lbo` further.
+__device__ __forceinline__ uint64_t make_mn_desc(uint32_t saddr, uint32_t lbo) {
+    return (uint64_t)((saddr & 0x3FFFF) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+__global__ void __launch_bounds__(VT_THREADS, 1) vit_attn_tc_kernel(const __grid_constant__ CUtensorMap mapA,      // 64-column boxes of qkv
+                                                                    const __grid_constant__ CUtensorMap mapB,      // 8-column boxes
+                                                                    VitAttnArgs a) {
+    extern __shared__ unsigned char raw[];
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
+    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
+    // V stages first, then the wide panels, then the narrow ones: every swizzled panel starts on a multiple of 1024 bytes
+    unsigned char *sv = smem, *sq = sv + VT_STAGES * VT_V, *sk = sq + 2 * VT_K;
+    uint64_t *q_full = reinterpret_cast<uint64_t *>(sk + VT_STAGES * VT_K), *q_empty = q_full + 1;
+    uint64_t *k_full = q_empty + 1, *k_empty = k_full + VT_STAGES, *v_full = k_empty + VT_STAGES, *v_empty = v_full + VT_STAGES;
+    uint64_t *s_full = v_empty + VT_STAGES, *p_full = s_full + 2, *o_full = p_full + 2, *o_empty = o_full + 2;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(o_empty + 2);
+    if (threadIdx.x == 0) {
+        mbar_init(q_full, 1);
+        mbar_init(q_empty, 1);
+        for (int s = 0; s < VT_STAGES; ++s) { mbar_init(k_full + s, 1); mbar_init(k_empty + s, 1); mbar_init(v_full + s, 1); mbar_init(v_empty + s, 1); }
+        for (int t = 0; t < 2; ++t) { mbar_init(s_full + t, 1); mbar_init(p_full + t, 4); mbar_init(o_full + t, 1); mbar_init(o_empty + t, 4); }
+        mbar_fence_init();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    // the zero partners of the narrow panels (never written again)
+    for (int i = threadIdx.x; i < (2 + VT_STAGES) * (VT_KB / 16); i += VT_THREADS) {
+        const int tile = i / (VT_KB / 16), at = i % (VT_KB / 16);
+        *reinterpret_cast<uint4 *>(sq + tile * VT_K + VT_KA + VT_KB + at * 16) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tmem_slot;
+    const int units = a.qtiles * a.heads, ktiles = (a.L + 127) >> 7, D = a.heads * VT_D;
+    if (warp == 0) {
+        unsigned it = 0, u = 0;
+        bool ok = true;
+        for (int id = blockIdx.x; id < units && ok; id += gridDim.x, ++u) {
+            const int h = id / a.qtiles, q0 = (id % a.qtiles) * 256, col = h * VT_D;
+            if (u && !mg_wait_warp(q_empty, (u - 1) & 1u, a.err)) break;
+            if (elect_one()) {
+                mbar_expect_tx(q_full, 2 * (VT_KA + VT_KB));
+                for (int t = 0; t < 2; ++t) {
+                    tma_load_2d(sq + t * VT_K, &mapA, col, q0 + t * 128, q_full);
+                    tma_load_2d(sq + t * VT_K + VT_KA, &mapB, col + 64, q0 + t * 128, q_full);
+                }
+            }
+            for (int j = 0; j < ktiles; ++j, ++it) {
+                const unsigned s = it % VT_STAGES, ph = (it / VT_STAGES - 1) & 1u;
+                if (it >= VT_STAGES && !mg_wait_warp(k_empty + s, ph, a.err)) { ok = false; break; }
+                if (elect_one()) {
+                    mbar_expect_tx(k_full + s, VT_KA + VT_KB);
+                    tma_load_2d(sk + s * VT_K, &mapA, D + col, j * 128, k_full + s);
+                    tma_load_2d(sk + s * VT_K + VT_KA, &mapB, D + col + 64, j * 128, k_full + s);
+                }
+                if (it >= VT_STAGES && !mg_wait_warp(v_empty + s, ph, a.err)) { ok = false; break; }
+                if (elect_one()) {
+                    mbar_expect_tx(v_full + s, VT_V);
+                    tma_load_2d(sv + s * VT_V, &mapA, 2 * D + col, j * 128, v_full + s);
+                    tma_load_2d(sv + s * VT_V + VT_V / 2, &mapA, 2 * D + col + 64, j * 128, v_full + s);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // instruction descriptors: D fp32, A/B bf16, M = 128; S: N = 128, both K-major; O: N = 80, B MN-major
+        const uint32_t is = (1u << 4) | (1u << 7) | (1u << 10) | (16u << 17) | (8u << 24);
+        const uint32_t io = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) | (10u << 17) | (8u << 24);
+        unsigned it = 0, u = 0;
+        bool ok = true;
+        auto issue_s = [&](int t, unsigned st) {
+            const uint32_t q = smem_u32(sq + t * VT_K), k = smem_u32(sk + st * VT_K);
+            if (elect_one()) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) umma_bf16(tmem + t * 128u, make_sw128_desc(q + i * 32), make_sw128_desc(k + i * 32), is, i ? 1u : 0u);
+                umma_bf16(tmem + t * 128u, make_plain_desc(q + VT_KA, VT_KB), make_plain_desc(k + VT_KA, VT_KB), is, 1u);
+                umma_commit(s_full + t);
+                if (t) umma_commit(k_empty + st);
+            }
+        };
+        for (int id = blockIdx.x; id < units && ok; id += gridDim.x, ++u) {
+            if (!mg_wait_warp(q_full, u & 1u, a.err) || !mg_wait_warp(k_full + it % VT_STAGES, (it / VT_STAGES) & 1u, a.err)) break;
+            // the scores of a new unit overwrite probabilities that the last products of the old one read: same pipe, in order
+            issue_s(0, it % VT_STAGES);
+            issue_s(1, it % VT_STAGES);
+            if (ktiles == 1 && elect_one()) umma_commit(q_empty);
+            for (int j = 0; j < ktiles && ok; ++j, ++it) {
+                const unsigned s = it % VT_STAGES, sn = (it + 1) % VT_STAGES;
+                const bool more = j + 1 < ktiles;
+                if (more && !mg_wait_warp(k_full + sn, ((it + 1) / VT_STAGES) & 1u, a.err)) { ok = false; break; }
+                if (!mg_wait_warp(v_full + s, (it / VT_STAGES) & 1u, a.err)) { ok = false; break; }
+                for (int t = 0; t < 2; ++t) {
+                    if (j == 0 && u && !mg_wait_warp(o_empty + t, (u - 1) & 1u, a.err)) { ok = false; break; }
+                    if (!mg_wait_warp(p_full + t, it & 1u, a.err)) { ok = false; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t v = smem_u32(sv + s * VT_V);
+                    if (elect_one()) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            umma_bf16_ts(tmem + 256u + t * 80u, tmem + t * 128u + i * 8, make_mn_desc(v + i * 2048, VT_V / 2), io, (j | i) ? 1u : 0u);
+                        if (t) umma_commit(v_empty + s);
+                        if (!more) umma_commit(o_full + t);
+                    }
+                    if (more) issue_s(t, sn);
+                }
+                if (ok && j + 2 == ktiles && elect_one()) umma_commit(q_empty);      // the last scores of this unit are under way
+            }
+        }
+    } else if (warp >= 4) {
+        const int t = (warp - 4) >> 2, q = warp & 3;
+        const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16);
+        const uint32_t sbase = lane_base + t * 128u, obase = lane_base + 256u + t * 80u;
+        unsigned it = 0, u = 0;
+        bool ok = true;
+        for (int id = blockIdx.x; id < units && ok; id += gridDim.x, ++u) {
+            const int h = id / a.qtiles, row = (id % a.qtiles) * 256 + t * 128 + q * 32 + lane;
+            float ref = 0.f, sum = 0.f;
+            for (int j = 0; j < ktiles; ++j, ++it) {
+                if (!mg_wait_warp(s_full + t, it & 1u, a.err)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                uint32_t s[4][32];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) tmem_ld32_nowait(sbase + c * 32, s[c]);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (j + 1 == ktiles) {
+                    const int left = a.L - j * 128;
+#pragma unroll
+                    for (int c = 0; c < 128; ++c)
+                        if (c >= left) s[c >> 5][c & 31] = 0xff800000u;      // -inf
+                }
+                float m4[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) m4[c] = __uint_as_float(s[c][0]);
+#pragma unroll
+                for (int i = 1; i < 32; ++i)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) m4[c] = fmaxf(m4[c], __uint_as_float(s[c][i]));
+                const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * a.scale;
+                if (j == 0) {
+                    ref = mx;
+                } else if (__any_sync(0xffffffffu, mx > ref + 8.f)) {
+                    // every product issued before these scores is complete, this tile's last O among them
+                    const float nref = fmaxf(ref, mx), f = ex2(ref - nref);
+                    ref = nref;
+                    sum *= f;
+#pragma unroll 1
+                    for (int c = 0; c < 80; c += 16) {
+                        uint32_t o[16];
+                        tmem_ld16(obase + c, o);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
+                        tmem_st16(obase + c, o);
+                    }
+                }
+                float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    uint32_t p[16];
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        const float x0 = ex2(fmaf(__uint_as_float(s[c][2 * i]), a.scale, -ref)), x1 = ex2(fmaf(__uint_as_float(s[c][2 * i + 1]), a.scale, -ref));
+                        sum4[i & 3] += x0 + x1;
+                        p[i] = pack_bf16(x0, x1);
+                    }
+                    tmem_st16(sbase + c * 16, p);
+                }
+                sum += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(p_full + t);
+            }
+            if (!ok || !mg_wait_warp(o_full + t, u & 1u, a.err)) { ok = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const float r = 1.f / sum;
+            bf16 *o = a.out + (long long)row * D + h * VT_D;
+#pragma unroll
+            for (int c = 0; c < 80; c += 16) {
+                uint32_t v[16];
+                tmem_ld16(obase + c, v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (row >= a.L) continue;
+#pragma unroll
+                for (int i = 0; i < 16; i += 8) {
+                    if (c + i >= VT_D) continue;
+                    uint4 pk;
+                    pk.x = pack_bf16(__uint_as_float(v[i]) * r, __uint_as_float(v[i + 1]) * r);
+                    pk.y = pack_bf16(__uint_as_float(v[i + 2]) * r, __uint_as_float(v[i + 3]) * r);
+                    pk.z = pack_bf16(__uint_as_float(v[i + 4]) * r, __uint_as_float(v[i + 5]) * r);
+                    pk.w = pack_bf16(__uint_as_float(v[i + 6]) * r, __uint_as_float(v[i + 7]) * r);
+                    *reinterpret_cast<uint4 *>(o + c + i) = pk;
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(o_empty + t);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
+}  // namespace qw
+
+using namespace qw;
+
+// qkv [L][3 * heads * 72] bf16 (bias and rotary applied) -> out [L][heads * 72] bf16.  qkv and out 16-byte aligned.
+QW_API int qwk_vit_attention(const void *qkv, int L, int heads, void *out, cudaStream_t s) {
+    if (L <= 0) return 0;
+    if (((uintptr_t)qkv & 15) || ((uintptr_t)out & 15) || heads <= 0) return -1;
+    static bool done[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    if (!done[dev]) {
+        if (cudaFuncSetAttribute(vit_attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, VT_SMEM) != cudaSuccess) return -3;
+        done[dev] = true;
+    }
+    const long long ld = 3LL * heads * VT_D;
+    CUtensorMap mA, mB;
+    if (!make_map(&mA, qkv, L, ld, ld, 128) || !make_map(&mB, qkv, L, ld, ld, 128, MAP_BF16_X8)) return -3;
+    VitAttnArgs a{};
+    a.L = L; a.heads = heads; a.qtiles = (L + 255) / 256; a.out = (bf16 *)out; a.err = g_err_ptr;
+    a.scale = 1.4426950408889634f / sqrtf((float)VT_D);
+    vit_attn_tc_kernel<<<persistent_grid(a.qtiles * heads, 1), VT_THREADS, VT_SMEM, s>>>(mA, mB, a);
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
