@@ -119,8 +119,9 @@ int qwk_penalty_add(void *gen, void *seen, int V, const int *slots, const int *t
 
 // vision.cu
 int qwk_vit_embed(float *x, const float *y, const float *bias, const float *table, const int *idx, const float *wts, int L, int D, cudaStream_t s);
-int qwk_vit_layernorm(const float *x, const float *w, const float *b, int L, int D, float eps, void *out, cudaStream_t s);
-int qwk_vit_bias_rope(void *qkv, const float *bias, const int *pos_hw, int L, int heads, cudaStream_t s);
+int qwk_vit_layernorm(float *x, const float *y, const float *ybias, const float *w, const float *b, int L, int D, float eps, void *out, cudaStream_t s);
+int qwk_vit_rope_table(const int *pos_hw, int L, float *tab, cudaStream_t s);
+int qwk_vit_bias_rope(void *qkv, const float *bias, const float *tab, int L, int heads, cudaStream_t s);
 int qwk_vit_bias_gelu(void *y, const float *bias, int L, int D, int tanh_form, cudaStream_t s);
 int qwk_vit_residual_add(float *x, const float *y, const float *bias, int L, int D, int assign, cudaStream_t s);
 

@@ -2,7 +2,8 @@
 // gemm_tc.cu).  Residual stream fp32, GEMM operands bf16.
 //
 //   vit_embed          x = patch_gemm + bias + bilinear interpolation of the learned 48x48 position table
-//   vit_layernorm      bf16(LayerNorm(x) * w + b)
+//   vit_layernorm      bf16(LayerNorm(x) * w + b), after x += y + bias where a residual add precedes it
+//   vit_rope_table     cos | sin of every patch's 36 angles
 //   vit_bias_rope      qkv += bias, then 2-D rotary on q and k (pairs (t, t+36); first 18 frequencies by row,
 //                      last 18 by column)
 //   (attention: vit_attn.cu)
@@ -29,51 +30,139 @@ __global__ void __launch_bounds__(256) vit_embed_kernel(float *x, const float *y
     }
 }
 
-__global__ void __launch_bounds__(256) vit_layernorm_kernel(const float *x, const float *w, const float *b, int D, float eps,
-                                                            bf16 *out) {
-    __shared__ float scratch[32];
-    const int n = blockIdx.x;
-    const float *row = x + (long long)n * D;
+// A warp per row, the row in registers: with `y` the residual add x += y + ybias comes first and x is written back, so a block's
+// add and the next norm are one pass (at 3520 x 1152, 29 us as two kernels of one block per row and scalar accesses, 12 as one).
+constexpr int VLN_MAX = 12;      // float4 per lane: D <= 1536
+__device__ __forceinline__ float4 vit_ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__global__ void __launch_bounds__(128) vit_layernorm_kernel(float *x, const float *y, const float *ybias, const float *w, const float *b,
+                                                            int L, int D, float eps, bf16 *out) {
+    const int n = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (n >= L) return;
+    float *row = x + (long long)n * D;
+    float4 v[VLN_MAX];
     float s = 0.f;
-    for (int c = threadIdx.x; c < D; c += 256) s += row[c];
-    const float mean = block_sum<256>(s, scratch) / float(D);
-    float v = 0.f;
-    for (int c = threadIdx.x; c < D; c += 256) {
-        const float d = row[c] - mean;
-        v = fmaf(d, d, v);
+#pragma unroll
+    for (int i = 0; i < VLN_MAX; ++i) {
+        const int c = (i * 32 + lane) * 4;
+        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (c >= D) continue;
+        v[i] = vit_ld4(row + c);
+        if (y) {
+            const float4 a = vit_ld4(y + (long long)n * D + c), e = vit_ld4(ybias + c);
+            v[i].x += a.x + e.x; v[i].y += a.y + e.y; v[i].z += a.z + e.z; v[i].w += a.w + e.w;
+            *reinterpret_cast<float4 *>(row + c) = v[i];
+        }
+        s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
     }
-    const float rstd = rsqrtf(block_sum<256>(v, scratch) / float(D) + eps);
-    for (int c = threadIdx.x; c < D; c += 256) out[(long long)n * D + c] = __float2bfloat16((row[c] - mean) * rstd * w[c] + b[c]);
+    const float mean = warp_sum(s) / float(D);
+    float q = 0.f;
+#pragma unroll
+    for (int i = 0; i < VLN_MAX; ++i) {
+        if ((i * 32 + lane) * 4 >= D) continue;
+        v[i].x -= mean; v[i].y -= mean; v[i].z -= mean; v[i].w -= mean;
+        q = fmaf(v[i].x, v[i].x, q); q = fmaf(v[i].y, v[i].y, q); q = fmaf(v[i].z, v[i].z, q); q = fmaf(v[i].w, v[i].w, q);
+    }
+    const float rstd = rsqrtf(warp_sum(q) / float(D) + eps);
+#pragma unroll
+    for (int i = 0; i < VLN_MAX; ++i) {
+        const int c = (i * 32 + lane) * 4;
+        if (c >= D) continue;
+        const float4 ww = vit_ld4(w + c), bb = vit_ld4(b + c);
+        uint2 pk;
+        pk.x = pack_bf16(fmaf(v[i].x * rstd, ww.x, bb.x), fmaf(v[i].y * rstd, ww.y, bb.y));
+        pk.y = pack_bf16(fmaf(v[i].z * rstd, ww.z, bb.z), fmaf(v[i].w * rstd, ww.w, bb.w));
+        *reinterpret_cast<uint2 *>(out + (long long)n * D + c) = pk;
+    }
 }
 
-// one block per patch: bias on the whole row, rotary on q and k
-__global__ void __launch_bounds__(256) vit_bias_rope_kernel(bf16 *qkv, const float *bias, const int *pos_hw, int heads) {
-    const int n = blockIdx.x;
-    const int D = heads * VHD;
+// cos | sin of the 36 angles of every patch (first 18 by row, last 18 by column): [L][2][36], once per slice instead of once per
+// block, head and tensor.
+__global__ void __launch_bounds__(256) vit_rope_table_kernel(const int *pos_hw, int L, float *tab) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= L * VHALF) return;
+    const int n = i / VHALF, t = i - n * VHALF, f = t % VNF;
+    const float inv = exp2f(-2.f * float(f) / float(VHALF) * 13.287712379549449f);      // 10000^(-2f/36)
+    float sn, cs;
+    sincosf(float(pos_hw[n * 2 + (t < VNF ? 0 : 1)]) * inv, &sn, &cs);
+    tab[(long long)n * 2 * VHALF + t] = cs;
+    tab[(long long)n * 2 * VHALF + VHALF + t] = sn;
+}
+
+__device__ __forceinline__ void vit_unpack4(const bf16 *p, float (&v)[4]) {
+    const uint2 u = *reinterpret_cast<const uint2 *>(p);
+    v[0] = bf16_lo(u.x); v[1] = bf16_hi(u.x); v[2] = bf16_lo(u.y); v[3] = bf16_hi(u.y);
+}
+__device__ __forceinline__ void vit_pack4(bf16 *p, const float (&v)[4]) {
+    *reinterpret_cast<uint2 *>(p) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+}
+
+// One block per patch: bias on the whole row, rotary on q and k, four values (of each half of a head) per step.
+__global__ void __launch_bounds__(256) vit_bias_rope_kernel(bf16 *qkv, const float *bias, const float *tab, int heads) {
+    const int n = blockIdx.x, D = heads * VHD;
     bf16 *row = qkv + (long long)n * 3 * D;
-    for (int c = 2 * D + threadIdx.x; c < 3 * D; c += 256) row[c] = __float2bfloat16(__bfloat162float(row[c]) + bias[c]);
-    const float pr = float(pos_hw[n * 2]), pc = float(pos_hw[n * 2 + 1]);
-    for (int i = threadIdx.x; i < 2 * heads * VHALF; i += 256) {
-        const int t = i % VHALF, hh = i / VHALF;          // hh over q heads then k heads
-        const int f = t % VNF;
-        const float inv = exp2f(-2.f * float(f) / float(VHALF) * 13.287712379549449f);      // 10000^(-2f/36)
-        float sn, cs;
-        sincosf((t < VNF ? pr : pc) * inv, &sn, &cs);
-        const int base = hh * VHD;
-        const float a = __bfloat162float(row[base + t]) + bias[base + t];
-        const float b = __bfloat162float(row[base + t + VHALF]) + bias[base + t + VHALF];
-        row[base + t] = __float2bfloat16(a * cs - b * sn);
-        row[base + t + VHALF] = __float2bfloat16(b * cs + a * sn);
+    const float *cs = tab + (long long)n * 2 * VHALF, *sn = cs + VHALF;
+    const int rot = 2 * heads * (VHALF / 4), total = rot + D / 4;
+    for (int i = threadIdx.x; i < total; i += 256) {
+        float a[4];
+        if (i >= rot) {
+            const int c = 2 * D + (i - rot) * 4;
+            const float4 e = vit_ld4(bias + c);
+            vit_unpack4(row + c, a);
+            a[0] += e.x; a[1] += e.y; a[2] += e.z; a[3] += e.w;
+            vit_pack4(row + c, a);
+            continue;
+        }
+        const int hh = i / (VHALF / 4), t = (i - hh * (VHALF / 4)) * 4, c = hh * VHD + t;      // hh over q heads then k heads
+        const float4 ea = vit_ld4(bias + c), eb = vit_ld4(bias + c + VHALF), co = vit_ld4(cs + t), si = vit_ld4(sn + t);
+        float b[4], o[4], p[4];
+        vit_unpack4(row + c, a);
+        vit_unpack4(row + c + VHALF, b);
+        a[0] += ea.x; a[1] += ea.y; a[2] += ea.z; a[3] += ea.w;
+        b[0] += eb.x; b[1] += eb.y; b[2] += eb.z; b[3] += eb.w;
+        const float cc[4] = {co.x, co.y, co.z, co.w}, ss[4] = {si.x, si.y, si.z, si.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            o[k] = a[k] * cc[k] - b[k] * ss[k];
+            p[k] = b[k] * cc[k] + a[k] * ss[k];
+        }
+        vit_pack4(row + c, o);
+        vit_pack4(row + c + VHALF, p);
     }
 }
 
+// gelu, tanh form: 0.5 v (1 + tanh z) = v / (1 + exp(-2z)); erf form as written.
+__device__ __forceinline__ float vit_gelu(float v, int tanh_form) {
+    if (tanh_form) {
+        const float z = 0.7978845608028654f * (v + 0.044715f * v * v * v);
+        return __fdividef(v, 1.f + fminf(__expf(-2.f * z), 1e37f));
+    }
+    return 0.5f * v * (1.f + erff(v * 0.7071067811865476f));
+}
+constexpr int VG_ROWS = 8;
+// Eight columns per thread (their bias in registers) down eight rows: 16-byte accesses.  At 3520 x 4304 53 us with two-byte
+// accesses, a division per value and tanhf; 19 now.
+__global__ void __launch_bounds__(128) vit_bias_gelu8_kernel(bf16 *y, const float *bias, int L, int D, int tanh_form) {
+    const int c = (blockIdx.x * 128 + threadIdx.x) * 8;
+    if (c >= D) return;
+    float e[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) e[k] = bias[c + k];
+    const int n0 = blockIdx.y * VG_ROWS, n1 = min(L, n0 + VG_ROWS);
+#pragma unroll 4
+    for (int n = n0; n < n1; ++n) {
+        uint4 *p = reinterpret_cast<uint4 *>(y + (long long)n * D + c);
+        const uint4 u = *p;
+        const uint32_t in[4] = {u.x, u.y, u.z, u.w};
+        uint32_t o[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) o[k] = pack_bf16(vit_gelu(bf16_lo(in[k]) + e[2 * k], tanh_form), vit_gelu(bf16_hi(in[k]) + e[2 * k + 1], tanh_form));
+        *p = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+}
+// Any width.
 __global__ void vit_bias_gelu_kernel(bf16 *y, const float *bias, long long total, int D, int tanh_form) {
     const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const float v = __bfloat162float(y[i]) + bias[i % D];
-    const float g = tanh_form ? 0.5f * v * (1.f + tanhf(0.7978845608028654f * (v + 0.044715f * v * v * v)))
-                              : 0.5f * v * (1.f + erff(v * 0.7071067811865476f));
-    y[i] = __float2bfloat16(g);
+    if (i < total) y[i] = __float2bfloat16(vit_gelu(__bfloat162float(y[i]) + bias[i % D], tanh_form));
 }
 
 __global__ void vit_residual_add_kernel(float *x, const float *y, const float *bias, long long total, int D, int assign) {
@@ -95,20 +184,33 @@ QW_API int qwk_vit_embed(float *x, const float *y, const float *bias, const floa
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-QW_API int qwk_vit_layernorm(const float *x, const float *w, const float *b, int L, int D, float eps, void *out,
-                             cudaStream_t s) {
-    vit_layernorm_kernel<<<L, 256, 0, s>>>(x, w, b, D, eps, (bf16 *)out);
+// out = bf16(LayerNorm(x) * w + b); with y (null: none) x += y + ybias first.  D a multiple of 4, at most 1536; 16-byte aligned pointers.
+QW_API int qwk_vit_layernorm(float *x, const float *y, const float *ybias, const float *w, const float *b, int L, int D, float eps,
+                             void *out, cudaStream_t s) {
+    if ((D & 3) || D > VLN_MAX * 128) return -1;
+    vit_layernorm_kernel<<<(L + 3) / 4, 128, 0, s>>>(x, y, ybias, w, b, L, D, eps, (bf16 *)out);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-QW_API int qwk_vit_bias_rope(void *qkv, const float *bias, const int *pos_hw, int L, int heads, cudaStream_t s) {
-    vit_bias_rope_kernel<<<L, 256, 0, s>>>((bf16 *)qkv, bias, pos_hw, heads);
+// tab [L][2][36] fp32: cos | sin of every patch's rotary angles.
+QW_API int qwk_vit_rope_table(const int *pos_hw, int L, float *tab, cudaStream_t s) {
+    vit_rope_table_kernel<<<blocks_for((long long)L * VHALF), 256, 0, s>>>(pos_hw, L, tab);
+    return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+QW_API int qwk_vit_bias_rope(void *qkv, const float *bias, const float *tab, int L, int heads, cudaStream_t s) {
+    vit_bias_rope_kernel<<<L, 256, 0, s>>>((bf16 *)qkv, bias, tab, heads);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 QW_API int qwk_vit_bias_gelu(void *y, const float *bias, int L, int D, int tanh_form, cudaStream_t s) {
-    const long long total = (long long)L * D;
-    vit_bias_gelu_kernel<<<blocks_for(total), 256, 0, s>>>((bf16 *)y, bias, total, D, tanh_form);
+    if ((D & 7) == 0 && ((uintptr_t)y & 15) == 0) {
+        dim3 grid((D / 8 + 127) / 128, (L + VG_ROWS - 1) / VG_ROWS);
+        vit_bias_gelu8_kernel<<<grid, 128, 0, s>>>((bf16 *)y, bias, L, D, tanh_form);
+    } else {
+        const long long total = (long long)L * D;
+        vit_bias_gelu_kernel<<<blocks_for(total), 256, 0, s>>>((bf16 *)y, bias, total, D, tanh_form);
+    }
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -197,14 +197,17 @@ class VisionEncoder:
         D = c.dim
         self._gemm(pin, self.patch_w, y)
         self.check(lib.qwk_vit_embed(_p(x), _p(y), _p(self.patch_b), _p(self.table), _p(idx_d), _p(wts_d), L, D, s), "vit_embed")
+        tab = torch.empty(L, 2, c.head_dim // 2, device=self.dev)
+        self.check(lib.qwk_vit_rope_table(_p(pos_d), L, _p(tab), s), "vit_rope_table")
+        pend = (None, None)                     # the block output (and its bias) that the next norm adds to x
         for b in self.blocks:
-            self.check(lib.qwk_vit_layernorm(_p(x), _p(b["norm1.weight"]), _p(b["norm1.bias"]), L, D, C.c_float(c.eps), _p(xn), s), "vit_ln")
+            self.check(lib.qwk_vit_layernorm(_p(x), *pend, _p(b["norm1.weight"]), _p(b["norm1.bias"]), L, D, C.c_float(c.eps), _p(xn), s), "vit_ln")
             self._gemm(xn, b["attn.qkv.weight"], qkv)
-            self.check(lib.qwk_vit_bias_rope(_p(qkv), _p(b["attn.qkv.bias"]), _p(pos_d), L, c.heads, s), "vit_rope")
+            self.check(lib.qwk_vit_bias_rope(_p(qkv), _p(b["attn.qkv.bias"]), _p(tab), L, c.heads, s), "vit_rope")
             self.check(lib.qwk_vit_attention(_p(qkv), L, c.heads, _p(att), s), "vit_attention")
             self._gemm(att, b["attn.proj.weight"], y)
-            self.check(lib.qwk_vit_residual_add(_p(x), _p(y), _p(b["attn.proj.bias"]), L, D, 0, s), "vit_add")
-            self.check(lib.qwk_vit_layernorm(_p(x), _p(b["norm2.weight"]), _p(b["norm2.bias"]), L, D, C.c_float(c.eps), _p(xn), s), "vit_ln")
+            self.check(lib.qwk_vit_layernorm(_p(x), _p(y), _p(b["attn.proj.bias"]), _p(b["norm2.weight"]), _p(b["norm2.bias"]), L, D,
+                                             C.c_float(c.eps), _p(xn), s), "vit_ln")
             m = self.mlp[:L, :c.mlp]
             self._gemm(xn, b["mlp.linear_fc1.weight"], m)
             if m.is_contiguous():
@@ -214,9 +217,9 @@ class VisionEncoder:
                 self.check(lib.qwk_vit_bias_gelu(_p(mc), _p(b["mlp.linear_fc1.bias"]), L, c.mlp, 1, s), "vit_gelu")
                 m = mc
             self._gemm(m, b["mlp.linear_fc2.weight"], y)
-            self.check(lib.qwk_vit_residual_add(_p(x), _p(y), _p(b["mlp.linear_fc2.bias"]), L, D, 0, s), "vit_add")
+            pend = (_p(y), _p(b["mlp.linear_fc2.bias"]))
         T, DM = L // c.merge ** 2, D * c.merge ** 2
-        self.check(lib.qwk_vit_layernorm(_p(x), _p(self.m_nw), _p(self.m_nb), L, D, C.c_float(c.eps), _p(xn), s), "vit_ln")
+        self.check(lib.qwk_vit_layernorm(_p(x), *pend, _p(self.m_nw), _p(self.m_nb), L, D, C.c_float(c.eps), _p(xn), s), "vit_ln")
         h1 = torch.empty(T, DM, dtype=torch.bfloat16, device=self.dev)
         self._gemm(xn.view(T, DM), self.m_fc1, h1)
         self.check(lib.qwk_vit_bias_gelu(_p(h1), _p(self.m_fc1_b), T, DM, 0, s), "vit_gelu")
