@@ -260,3 +260,63 @@ def test_qsa_scores_tensor_core_form_matches_fp32(base, M):
             assert torch.all(scores[m, nb:] == -7.0)
             err = (scores[m, :nb] - want[m, :nb]).abs().max() / want[m, :nb].abs().max()
             assert err < 1e-3, (m, float(err))
+
+
+@pytest.mark.parametrize("M,V,pad", [(1, 248320, 0), (3, 1024, 0), (2, 7, 0), (5, 100, 1), (24, 4099, 1), (2, 31, 3)])
+def test_row_reduce_maximum_index_and_sum(M, V, pad):
+    """Rows shorter than the cluster's eight parts, rows that do not start on 16 bytes, ties (lowest index), a row of -inf with
+    one finite value and rows with NaN.  The sum of exponentials against 64 bits: __expf is good to 2 ulp + 2^-22 |x| and the
+    fp32 sum of positive terms to log2(V) ulp, 1e-5 covers both."""
+    from qwb200.ops import kernels as K_
+    g = torch.Generator(device="cuda").manual_seed(V)
+    full = torch.randn(M, V + pad, generator=g, device=_dev()) * 3
+    x = full[:, :V]
+    x[0, V // 2:] = x[0, : V // 2 + 1].max() if V > 1 else 0.0
+    if M > 1:
+        x[1] = -float("inf")
+        x[1, V - 1] = -2.5
+    val, idx, mx, sm = K_.row_reduce(x, idx0=11)
+    want, at = x.max(1)
+    assert torch.equal(val, want) and torch.equal(mx, want)
+    for m in range(M):
+        assert int(idx[m]) == 11 + int((x[m] == want[m]).nonzero()[0])
+        ref = torch.exp(x[m].double() - want[m].double()).sum()
+        assert abs(float(sm[m]) / float(ref) - 1) < 1e-5
+    x[0, V // 3] = float("nan")
+    assert torch.isnan(K_.row_reduce(x)[3][0])
+
+
+@pytest.mark.parametrize("M", [1, 5, 300])
+def test_ple_rows_through_decode_and_prefill_forms_agree(M):
+    """The n-gram layer's kernels with one row per block (M < 256) and eight: a run of M rows in one call equals the same rows one
+    call each, ring included (the same sums in the same order)."""
+    import ctypes as C
+    from qwb200.ops import lib as qlib
+    L = qlib.load(True)
+    hc, SH = 4, 320
+    xw, dev = hc * SH, _dev()
+    g = torch.Generator(device="cuda").manual_seed(M)
+    rn = lambda *s: torch.randn(*s, generator=g, device=dev)
+    kv, red, nc1, cw, X = rn(M, xw + SH), rn(M, 16).abs() + 0.1, rn(xw), rn(xw, 4), rn(M, xw)
+    ring0 = rn(2, 32, xw)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
+    P = lambda t: C.c_void_p(t.data_ptr())
+    s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    base = 40
+
+    def apply(rows, ring, Xr):
+        n = len(rows)
+        gv, nc = torch.empty(n, xw, device=dev), torch.empty(n, xw, device=dev)
+        k, r = kv[rows].contiguous(), red[rows].contiguous()
+        slot, pos, rs, rl = i32([1] * n), i32([base + i for i in rows]), i32([0] * n), i32([n] + [0] * (n - 1))
+        assert L.qwk_ple_apply(P(k), xw + SH, P(r), 16, P(nc1), P(cw), SH, hc, SH, 1e-6, 4, 3, P(gv), P(nc), P(ring), P(Xr), n, P(slot), P(pos),
+                               P(rs), P(rl), s) == 0
+    ring_a, Xa = ring0.clone(), X.clone()
+    apply(list(range(M)), ring_a, Xa)
+    ring_b, Xb = ring0.clone(), X.clone()
+    for i in range(M):
+        xi = Xb[i:i + 1].contiguous()
+        apply([i], ring_b, xi)
+        Xb[i] = xi[0]
+    torch.cuda.synchronize()
+    assert torch.equal(Xa, Xb) and torch.equal(ring_a, ring_b)

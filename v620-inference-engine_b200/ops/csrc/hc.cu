@@ -14,21 +14,20 @@
 
 namespace qw {
 
-// X[m][s][:] = embedding row of tokens[m] (this rank's columns) for every stream.
-__global__ void embed_rows_kernel(const int *tokens, const bf16 *table, int ld_table, int col0, int SH, int hc,
-                                  int vocab, float *X) {
-    const int m = blockIdx.x;
+// X[m][s][:] = embedding row of tokens[m] (this rank's columns) for every stream.  Four columns per thread, grid (M, ceil(SH / 1024)).
+__global__ void __launch_bounds__(256) embed_rows_kernel(const int *tokens, const bf16 *table, int ld_table, int col0, int SH, int hc,
+                                                         int vocab, float *X) {
+    const int m = blockIdx.x, c = (blockIdx.y * 256 + threadIdx.x) * 4;
     int t = tokens[m];
     QW_DCHECK(t >= 0 && t < vocab, 0x01000000u | (unsigned)(m & 0xffffff));          // token id outside the vocabulary (row m)
     if (t < 0 || t >= vocab) t = 0;
-    const bf16 *row = table + (long long)t * ld_table + col0;
-    for (int c = threadIdx.x; c < SH; c += blockDim.x) {
-        const float v = __bfloat162float(row[c]);
-        for (int s = 0; s < hc; ++s) X[((long long)m * hc + s) * SH + c] = v;
-    }
+    if (c >= SH) return;
+    const uint2 u = *reinterpret_cast<const uint2 *>(table + (long long)t * ld_table + col0 + c);
+    const float4 v = make_float4(bf16_lo(u.x), bf16_hi(u.x), bf16_lo(u.y), bf16_hi(u.y));
+    for (int s = 0; s < hc; ++s) *reinterpret_cast<float4 *>(X + ((long long)m * hc + s) * SH + c) = v;
 }
 
-// grid (M, hc).  pend may be null (no deferred combine).  y and ssq may be null (combine only).
+// Four columns per step.  grid (M, hc).  pend may be null (no deferred combine).  y and ssq may be null (combine only).
 __global__ void __launch_bounds__(256) hc_pre_kernel(float *X, const float *pend, int ld_pend, const float *inj, int ld_inj,
                                                      const float *w1 /* (1+w) [hc][SH] */, int SH, int hc, bf16 *y,
                                                      float *ssq, int ld_ssq) {
@@ -38,14 +37,19 @@ __global__ void __launch_bounds__(256) hc_pre_kernel(float *X, const float *pend
     float coef = 0.f;
     if (pend) coef = 2.f * sigmoidf_(inj[(long long)m * ld_inj + s] / float(hc));
     float acc = 0.f;
-    for (int c = threadIdx.x; c < SH; c += 256) {
-        float v = x[c];
+#pragma unroll 3
+    for (int c = threadIdx.x * 4; c < SH; c += 1024) {
+        float4 v = *reinterpret_cast<const float4 *>(x + c);
         if (pend) {
-            v = fmaf(pend[(long long)m * ld_pend + c], coef, v);
-            x[c] = v;
+            const float4 p = *reinterpret_cast<const float4 *>(pend + (long long)m * ld_pend + c);
+            v.x = fmaf(p.x, coef, v.x); v.y = fmaf(p.y, coef, v.y); v.z = fmaf(p.z, coef, v.z); v.w = fmaf(p.w, coef, v.w);
+            *reinterpret_cast<float4 *>(x + c) = v;
         }
-        if (y) y[((long long)m * hc + s) * SH + c] = __float2bfloat16(v * w1[s * SH + c]);
-        acc = fmaf(v, v, acc);
+        if (y) {
+            const float4 w = *reinterpret_cast<const float4 *>(w1 + s * SH + c);
+            *reinterpret_cast<uint2 *>(y + ((long long)m * hc + s) * SH + c) = make_uint2(pack_bf16(v.x * w.x, v.y * w.y), pack_bf16(v.z * w.z, v.w * w.w));
+        }
+        acc = fmaf(v.x, v.x, acc); acc = fmaf(v.y, v.y, acc); acc = fmaf(v.z, v.z, acc); acc = fmaf(v.w, v.w, acc);
     }
     if (ssq) {
         acc = block_sum<256>(acc, scratch);
@@ -355,12 +359,14 @@ QW_DCHECK_TU(hc)
 
 QW_API int qwk_embed_rows(const int *tokens, const void *table, int ld_table, int col0, int SH, int hc, int vocab,
                           float *X, int M, cudaStream_t s) {
-    embed_rows_kernel<<<M, 256, 0, s>>>(tokens, (const bf16 *)table, ld_table, col0, SH, hc, vocab, X);
+    if ((SH & 3) || (col0 & 3) || (ld_table & 3)) return -1;
+    embed_rows_kernel<<<dim3(M, (SH + 1023) / 1024), 256, 0, s>>>(tokens, (const bf16 *)table, ld_table, col0, SH, hc, vocab, X);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 QW_API int qwk_hc_pre(float *X, const float *pend, int ld_pend, const float *inj, int ld_inj, const float *w1, int SH,
                       int hc, void *y, float *ssq, int ld_ssq, int M, cudaStream_t s) {
+    if ((SH & 3) || (pend && (ld_pend & 3))) return -1;
     dim3 grid(M, hc);
     hc_pre_kernel<<<grid, 256, 0, s>>>(X, pend, ld_pend, inj, ld_inj, w1, SH, hc, (bf16 *)y, ssq, ld_ssq);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;

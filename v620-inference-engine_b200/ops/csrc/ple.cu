@@ -30,20 +30,52 @@ struct PleGatherArgs {
     long long *ids_out;          // optional [M][heads]
 };
 
-// grid (M, heads), 64 threads.
-__global__ void ple_gather_kernel(PleGatherArgs a) {
-    const int m = blockIdx.x, h = blockIdx.y;
+// Row id of head h for a token and its predecessors.
+__device__ __forceinline__ long long ple_row_id(const PleGatherArgs &a, int m, int h) {
     const int eos = c_ng.eos;
     const int t0 = a.ctx[m * 3], c1 = a.ctx[m * 3 + 1], c2 = a.ctx[m * 3 + 2];
-    const unsigned long long tok0 = (unsigned long long)t0;
     const int t1 = c1 >= 0 ? c1 : eos;
     const int t2 = (c2 >= 0 && t1 != eos) ? c2 : eos;
-    const int per = c_ng.heads / (c_ng.ngram - 1);
-    const int order = 2 + h / per;
-    unsigned long long mixed = tok0 * c_ng.mult[0] ^ (unsigned long long)t1 * c_ng.mult[1];
+    const int order = 2 + h / (c_ng.heads / (c_ng.ngram - 1));
+    unsigned long long mixed = (unsigned long long)t0 * c_ng.mult[0] ^ (unsigned long long)t1 * c_ng.mult[1];
     if (order >= 3) mixed ^= (unsigned long long)t2 * c_ng.mult[2];
-    long long id = (long long)(mixed % c_ng.sizes[h]) + c_ng.offsets[h];
-    id %= a.rows;                                   // scaled-down synthetic tables wrap
+    return ((long long)(mixed % c_ng.sizes[h]) + c_ng.offsets[h]) % a.rows;          // scaled-down synthetic tables wrap
+}
+
+// The byte layout in 16-byte pieces: half a warp per row (160 bytes: ten lanes), so a row crosses the host link as one or two
+// requests instead of byte loads.  M * heads rows, 16 per block.
+constexpr int PLE_G_ROWS = 16;
+__global__ void __launch_bounds__(256) ple_gather_f8_kernel(PleGatherArgs a, int total, int heads) {
+    const int i = blockIdx.x * PLE_G_ROWS + (threadIdx.x >> 4), lane = threadIdx.x & 15;
+    if (i >= total) return;
+    const int m = i / heads, h = i - m * heads;
+    const long long id = ple_row_id(a, m, h);
+    if (a.ids_out && lane == 0) a.ids_out[i] = id;
+    const unsigned char *bytes = (const unsigned char *)a.shards[id / a.rows_per_shard] + id % a.rows_per_shard * a.width;
+    if ((uintptr_t)bytes & 15) {                                     // a shard that does not start on 16 bytes
+        for (int j = lane; j < a.width; j += 16) a.e[(long long)i * a.width + j] = __float2bfloat16(c_f8_lut[bytes[j]]);
+        return;
+    }
+    const uint4 *row = reinterpret_cast<const uint4 *>(bytes);
+    uint4 *out = reinterpret_cast<uint4 *>(a.e + (long long)i * a.width);
+    for (int j = lane; j < a.width / 16; j += 16) {
+        const uint4 v = row[j];
+        const uint32_t b[4] = {v.x, v.y, v.z, v.w};
+        uint32_t o[8];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            o[2 * k] = pack_bf16(c_f8_lut[b[k] & 255u], c_f8_lut[(b[k] >> 8) & 255u]);
+            o[2 * k + 1] = pack_bf16(c_f8_lut[(b[k] >> 16) & 255u], c_f8_lut[b[k] >> 24]);
+        }
+        out[2 * j] = make_uint4(o[0], o[1], o[2], o[3]);
+        out[2 * j + 1] = make_uint4(o[4], o[5], o[6], o[7]);
+    }
+}
+
+// Every layout, element by element.  grid (M, heads), 64 threads.
+__global__ void ple_gather_kernel(PleGatherArgs a) {
+    const int m = blockIdx.x, h = blockIdx.y;
+    const long long id = ple_row_id(a, m, h);
     if (a.ids_out && threadIdx.x == 0) a.ids_out[m * c_ng.heads + h] = id;
     const long long sh = id / a.rows_per_shard, r = id % a.rows_per_shard;
     bf16 *out = a.e + ((long long)m * c_ng.heads + h) * a.width;
@@ -99,56 +131,78 @@ __global__ void __launch_bounds__(256) ple_stats_kernel(const float *kv, int ld_
     }
 }
 
-// grid (M, hc): gate, gated value gv and normalised conv input nc for the batch rows.
+__device__ __forceinline__ float4 ple_ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+
+// Gate, gated value gv and normalised conv input nc for the batch rows, four columns per thread.  grid (M, hc, ceil(SH / 1024)).
 __global__ void __launch_bounds__(256) ple_nc_kernel(const float *kv, int ld_kv, const float *red, int ld_red,
                                                      const float *nc1, int SH, int hc, int H, float eps, float *gv,
                                                      float *nc) {
-    const int m = blockIdx.x, s = blockIdx.y;
+    const int m = blockIdx.x, s = blockIdx.y, c = (blockIdx.z * 256 + threadIdx.x) * 4;
+    if (c >= SH) return;
     const float *r = red + (long long)m * ld_red;
     const float rk = rsqrtf(r[3 * s] / float(H) + eps), rq = rsqrtf(r[3 * s + 1] / float(H) + eps);
     const float gs = r[3 * s + 2] * rk * rq * rsqrtf(float(H));
     const float mag = sqrtf(fmaxf(fabsf(gs), 1e-6f));
     const float gate = sigmoidf_(gs < 0.f ? -mag : (gs > 0.f ? mag : 0.f));
     const float rn = rsqrtf(gate * gate * r[3 * hc] / float(H) + eps);
-    const float *v = kv + (long long)m * ld_kv + hc * SH;
-    for (int c = threadIdx.x; c < SH; c += 256) {
-        const float g = gate * v[c];
-        const long long o = ((long long)m * hc + s) * SH + c;
-        gv[o] = g;
-        nc[o] = g * rn * nc1[s * SH + c];
-    }
+    const float4 v = ple_ld4(kv + (long long)m * ld_kv + hc * SH + c), w = ple_ld4(nc1 + s * SH + c);
+    const float4 g = make_float4(gate * v.x, gate * v.y, gate * v.z, gate * v.w);
+    const long long o = ((long long)m * hc + s) * SH + c;
+    *reinterpret_cast<float4 *>(gv + o) = g;
+    *reinterpret_cast<float4 *>(nc + o) = make_float4(g.x * rn * w.x, g.y * rn * w.y, g.z * rn * w.z, g.w * rn * w.w);
 }
 
-// grid (M, hc): X += gv + silu(dilated conv of nc); taps at p-9, p-6, p-3, p from the batch or the ring.
+// X += gv + silu(dilated conv of nc); taps at p-9, p-6, p-3, p from the batch or the ring.  Four columns and `rows_per` rows per
+// thread: one row per block when there are few (a step of one row used four blocks and took 34 us, now 5), several with
+// the taps' weights in registers when there are many (4096 rows: 300 us, now 150).  grid (ceil(xw / 1024), ceil(M / rows_per)).
+constexpr int PLE_TAPS = 4;
 __global__ void __launch_bounds__(256) ple_conv_kernel(const float *gv, const float *nc, const float *ring, const float *cw,
-                                                       int SH, int hc, int taps, int dil, Rows rows, float *X) {
-    const int m = blockIdx.x, s = blockIdx.y;
-    const int slot = rows.slot[m], pos = rows.pos[m], rs = rows.run_start[m];
-    const int xw = hc * SH;
-    const float *rg = ring + (long long)slot * PLE_RING * xw;
-    for (int c = threadIdx.x; c < SH; c += 256) {
-        const int col = s * SH + c;
-        float acc = 0.f;
-        for (int k = 0; k < taps; ++k) {
-            const int back = (taps - 1 - k) * dil;
-            const int q = pos - back;
-            float v;
-            if (m - back >= rs) v = nc[(long long)(m - back) * xw + col];
-            else if (q >= 0) v = rg[(q % PLE_RING) * xw + col];
-            else v = 0.f;
-            acc = fmaf(cw[col * taps + k], v, acc);
+                                                       int xw, int dil, Rows rows, int rows_per, float *X) {
+    const int col = (blockIdx.x * 256 + threadIdx.x) * 4;
+    if (col >= xw) return;
+    float w[4][PLE_TAPS];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 t = ple_ld4(cw + (col + i) * PLE_TAPS);
+        w[i][0] = t.x; w[i][1] = t.y; w[i][2] = t.z; w[i][3] = t.w;
+    }
+    const int m1 = min(rows.M, (int)(blockIdx.y + 1) * rows_per);
+    for (int m = blockIdx.y * rows_per; m < m1; ++m) {
+        const int slot = rows.slot[m], pos = rows.pos[m], rs = rows.run_start[m];
+        const float *rg = ring + (long long)slot * PLE_RING * xw;
+        float4 v[PLE_TAPS];
+#pragma unroll
+        for (int k = 0; k < PLE_TAPS; ++k) {
+            const int back = (PLE_TAPS - 1 - k) * dil, q = pos - back;
+            if (m - back >= rs) v[k] = ple_ld4(nc + (long long)(m - back) * xw + col);
+            else if (q >= 0) v[k] = ple_ld4(rg + (q % PLE_RING) * xw + col);
+            else v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        X[(long long)m * xw + col] += gv[(long long)m * xw + col] + siluf_(acc);
+        float *xp = X + (long long)m * xw + col;
+        float4 x = ple_ld4(xp);
+        const float4 g = ple_ld4(gv + (long long)m * xw + col);
+        float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int k = 0; k < PLE_TAPS; ++k) {
+            a[0] = fmaf(w[0][k], v[k].x, a[0]); a[1] = fmaf(w[1][k], v[k].y, a[1]);
+            a[2] = fmaf(w[2][k], v[k].z, a[2]); a[3] = fmaf(w[3][k], v[k].w, a[3]);
+        }
+        x.x += g.x + siluf_(a[0]); x.y += g.y + siluf_(a[1]); x.z += g.z + siluf_(a[2]); x.w += g.w + siluf_(a[3]);
+        *reinterpret_cast<float4 *>(xp) = x;
     }
 }
 
-// grid (M, ceil(xw/256)): store the batch's nc rows in the ring (after ple_conv has read it).
-__global__ void ple_ring_kernel(const float *nc, float *ring, int xw, Rows rows) {
-    const int m = blockIdx.x, col = blockIdx.y * 256 + threadIdx.x;
+// Stores the batch's last nc rows of every run in the ring (after ple_conv has read it).  grid (ceil(M / rows_per), ceil(xw / 1024)).
+__global__ void __launch_bounds__(256) ple_ring_kernel(const float *nc, float *ring, int xw, Rows rows, int rows_per) {
+    const int col = (blockIdx.y * 256 + threadIdx.x) * 4;
     if (col >= xw) return;
-    const int rs = rows.run_start[m], len = rows.run_len[rs];
-    if ((m - rs) < len - PLE_RING) return;
-    ring[((long long)rows.slot[m] * PLE_RING + (rows.pos[m] % PLE_RING)) * xw + col] = nc[(long long)m * xw + col];
+    const int m1 = min(rows.M, (int)(blockIdx.x + 1) * rows_per);
+    for (int m = blockIdx.x * rows_per; m < m1; ++m) {
+        const int rs = rows.run_start[m], len = rows.run_len[rs];
+        if ((m - rs) < len - PLE_RING) continue;
+        *reinterpret_cast<float4 *>(ring + ((long long)rows.slot[m] * PLE_RING + (rows.pos[m] % PLE_RING)) * xw + col) =
+            ple_ld4(nc + (long long)m * xw + col);
+    }
 }
 
 }  // namespace qw
@@ -173,8 +227,13 @@ QW_API int qwk_ple_gather(const int *ctx, const void *const *shards, const void 
     PleGatherArgs a;
     a.ctx = ctx; a.shards = shards; a.scales = scales; a.rows_per_shard = rows_per_shard; a.rows = rows;
     a.layout = layout; a.width = width; a.e = (bf16 *)e; a.ids_out = ids_out;
-    dim3 grid(M, heads);
-    ple_gather_kernel<<<grid, 64, 0, s>>>(a);
+    if (layout == PLE_F8 && width % 16 == 0 && ((uintptr_t)e & 15) == 0) {
+        const int total = M * heads;
+        ple_gather_f8_kernel<<<(total + PLE_G_ROWS - 1) / PLE_G_ROWS, 256, 0, s>>>(a, total, heads);
+    } else {
+        dim3 grid(M, heads);
+        ple_gather_kernel<<<grid, 64, 0, s>>>(a);
+    }
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -189,11 +248,11 @@ QW_API int qwk_ple_apply(const float *kv, int ld_kv, const float *red, int ld_re
                          int SH, int hc, int H, float eps, int taps, int dil, float *gv, float *nc, float *ring,
                          float *X, int M, const int *slot, const int *pos, const int *run_start, const int *run_len,
                          cudaStream_t s) {
-    dim3 grid(M, hc);
+    if ((SH & 3) || (ld_kv & 3) || taps != PLE_TAPS) return -1;
     Rows rows{M, slot, pos, run_start, run_len};
-    ple_nc_kernel<<<grid, 256, 0, s>>>(kv, ld_kv, red, ld_red, nc1, SH, hc, H, eps, gv, nc);
-    ple_conv_kernel<<<grid, 256, 0, s>>>(gv, nc, ring, cw, SH, hc, taps, dil, rows, X);
-    dim3 g2(M, (hc * SH + 255) / 256);
-    ple_ring_kernel<<<g2, 256, 0, s>>>(nc, ring, hc * SH, rows);
+    const int xw = hc * SH, rows_per = M >= 256 ? 8 : 1, cb = (xw + 1023) / 1024, rb = (M + rows_per - 1) / rows_per;
+    ple_nc_kernel<<<dim3(M, hc, (SH + 1023) / 1024), 256, 0, s>>>(kv, ld_kv, red, ld_red, nc1, SH, hc, H, eps, gv, nc);
+    ple_conv_kernel<<<dim3(cb, rb), 256, 0, s>>>(gv, nc, ring, cw, xw, dil, rows, rows_per, X);
+    ple_ring_kernel<<<dim3(rb, cb), 256, 0, s>>>(nc, ring, xw, rows, rows_per);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
