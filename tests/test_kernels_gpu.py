@@ -320,3 +320,52 @@ def test_ple_rows_through_decode_and_prefill_forms_agree(M):
         Xb[i] = xi[0]
     torch.cuda.synchronize()
     assert torch.equal(Xa, Xb) and torch.equal(ring_a, ring_b)
+
+
+@pytest.mark.parametrize("SH,R,n_inj", [(2560, 320, 4), (2560, 320, 0), (256, 32, 4), (320, 40, 4), (88, 8, 4)])
+def test_mixer_rows_match_64_bits_and_do_not_depend_on_their_neighbours(SH, R, n_inj):
+    """Both mixer kernels at 1 to 32 rows (one and two passes of 16, a lone row in the second): against 64 bits on the same bf16
+    rows, and every row bit for bit what it is alone.  The down projection sums exact products in fp32 (K <= 2560: 1e-5 of the
+    result's size); the block input is rounded to bf16 once (2^-9 relative; half a percent of its size covers it)."""
+    import ctypes as C
+    from qwb200.ops import lib as qlib
+    L = qlib.load(True)
+    hc, eps, dev = 4, 1e-6, _dev()
+    down, M = R + n_inj, 32
+    ld = hc + hc * (R + 4)
+    g = torch.Generator(device="cuda").manual_seed(SH + R)
+    rn = lambda *s: torch.randn(*s, generator=g, device=dev)
+    X, pend, inj_prev, w1 = rn(M, hc, SH), rn(M, SH), rn(M, hc), 1 + 0.1 * rn(hc, SH)
+    Wd, Wu = (rn(down, hc, SH) * 0.05).to(torch.bfloat16), (rn(SH, hc, R) * 0.1).to(torch.bfloat16)
+    P = lambda t: C.c_void_p(t.data_ptr())
+    st = lambda: C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def both(rows, combine=True):
+        x, p, ip = X[rows].contiguous(), pend[rows].contiguous(), inj_prev[rows].contiguous()
+        n = len(rows)
+        xo, send, inj, out = torch.zeros_like(x), torch.zeros(n, ld, device=dev), torch.zeros(n, hc, device=dev), torch.zeros(n, SH + 8, dtype=torch.bfloat16, device=dev)
+        assert L.qwk_hc_down(P(x), P(xo) if combine else None, P(p) if combine else None, SH, P(ip), P(w1), P(Wd), P(send), ld, SH, hc, down, n, st()) == 0
+        xn = xo if combine else x
+        assert L.qwk_hc_up_mix(P(send), ld, P(Wu), P(xn), P(w1), SH, hc, R, n_inj, SH, C.c_float(eps), n, P(inj) if n_inj else None, hc,
+                               P(out), SH + 8, 8, st()) == 0
+        torch.cuda.synchronize()
+        return xn, send, inj, out
+    x, send, inj, out = both(list(range(M)))
+    x64 = X.double() + pend.double()[:, None] * (2 * torch.sigmoid(inj_prev.double() / hc))[..., None]
+    assert torch.allclose(x.double(), x64, rtol=1e-5, atol=1e-5)
+    y = (x * w1).to(torch.bfloat16).double()
+    part = torch.einsum("msc,jsc->msj", y, Wd.double())
+    got = send[:, hc:hc + hc * down].view(M, hc, down).double()
+    assert float((got - part).norm() / part.norm()) < 1e-5
+    r = torch.rsqrt(x.double().pow(2).mean(-1) + eps)
+    d = (r[..., None] * part).sum(1)
+    if n_inj:
+        assert float((inj.double() - d[:, R:]).norm() / d[:, R:].norm()) < 1e-5
+    u = torch.nn.functional.silu(d[:, :R] / hc)
+    gate = torch.sigmoid(torch.einsum("csr,mr->msc", Wu.double(), u))
+    want = (gate * y * r[..., None]).mean(1)
+    assert float((out[:, 8:].double() - want).norm() / want.norm()) < 5e-3 and torch.all(out[:, :8] == 0)
+    for rows in ([0], [31], list(range(1, 18)), list(range(24))):
+        x1, send1, inj1, out1 = both(rows)
+        assert torch.equal(x1, x[rows]) and torch.equal(send1, send[rows]) and torch.equal(inj1, inj[rows]) and torch.equal(out1, out[rows])
+    assert torch.equal(both([3], combine=False)[0][0], X[3])
