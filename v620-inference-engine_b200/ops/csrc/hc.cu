@@ -337,11 +337,6 @@ __device__ __forceinline__ void mma_rows(float (&c)[2][4], const uint4 &r, const
     mma_bf16(c[1], r.z, r8.z, r.w, r8.w, w.z, w.w);
 }
 
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
 constexpr int HM_THREADS = 512, HM_PAD = 32;      // padding of shared rows: their stride is 64 bytes off a multiple of 128
 constexpr int HD_CL = 8, HD_J = 8, HD_W = HM_THREADS / 32, HD_ROWS = 8, HD_CLUSTER_MIN = 4;
 // A CTA owns eight outputs j of one stream over all columns (its sixteen warps take every sixteenth chunk of 32).  The weights go

@@ -41,6 +41,12 @@ __device__ __forceinline__ uint32_t b_tile_addr(uint32_t x_base, unsigned row_st
     return x_base + (unsigned)rr * row_stride + (unsigned)(k0 + (((lane >> 3) & 1) << 3)) * 2u;
 }
 
+// 16 bytes global -> shared without a register in between.
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Fragment coordinates of the accumulator: c[0],c[1] -> (row = lane/4, n = 2*(lane%4) + {0,1}); c[2],c[3] -> row + 8.
 
 }  // namespace qw

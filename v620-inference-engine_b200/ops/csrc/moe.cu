@@ -309,9 +309,9 @@ __global__ void __launch_bounds__(256) moe_down_combine_kernel(const uint32_t *w
 using namespace qw;
 
 // Which form of the routed-expert kernels runs: bit 0 / 1 = gate-up / down on the tensor cores with direct loads,
-// bit 2 / 3 = gate-up / down on the tensor cores fed by bulk-async row copies (wins over bits 0 / 1), 0 = scalar kernels.
+// bit 2 / 3 = gate-up / down on the tensor cores fed by asynchronous copies (wins over bits 0 / 1), 0 = scalar kernels.
 // Default 12, measured inside the decode graph on the full model: scalar 5.37 ms per step, direct-load tensor-core forms
-// 5.37 / 5.7, bulk-copy-fed forms 4.85.  QW_MOE_MMA overrides at start-up, qwk_set_moe_mma at run time.
+// 5.37 / 5.7, copy-fed forms (then as bulk copies of rows) 4.85.  QW_MOE_MMA overrides at start-up, qwk_set_moe_mma at run time.
 static int g_moe_mma = -1;
 static int moe_mma_mask() {
     if (g_moe_mma < 0) {
@@ -374,20 +374,20 @@ QW_API int qwk_moe_gate_up_pair(const void *w13, const void *s13, const void *x,
     const SharedAct sa = take_shared_act();
     const int extra = sa.rs ? M : 0;          // one extra grid row per token for the shared expert's activation
     if ((moe_mma_mask() & 4) && (F & 15) == 0 && (K & 127) == 0) {
-        // bulk-copy-fed tensor-core form
+        // copy-fed tensor-core form
         const int ks = K >> 7;
-        const size_t smem = 128 + 2 * 16 * ((size_t)(K >> 1) + TM_PAD) + 2 * 16 * ks * 2 + 16 + (size_t)(K >> 3) * 16 + 16 * 2 * 16 * sizeof(float);
+        const size_t smem = 2 * 16 * ((size_t)(K >> 1) + TM_PAD) + 2 * 16 * ks * 2 + (size_t)(K >> 3) * 16 + CP_WARPS * 2 * 16 * sizeof(float);
         static bool attr[64] = {};
         int dev = 0;
         cudaGetDevice(&dev);
         if (dev < 0 || dev >= 64) dev = 0;
         if (!attr[dev]) {
-            cudaFuncSetAttribute(moe_gate_up_tma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+            cudaFuncSetAttribute(moe_gate_up_cp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
             attr[dev] = true;
         }
         if (smem <= 100 * 1024) {
-            cudaError_t e = launch_pdl(moe_gate_up_tma_kernel, dim3(F / 16, M * top_k + extra), dim3(512), smem, s, (const uint32_t *)w13,
-                                       (const bf16 *)s13, (const bf16 *)x, ldx, pair_expert, top_k, F, K, (bf16 *)h, g_err_ptr, sa, M * top_k);
+            cudaError_t e = launch_pdl(moe_gate_up_cp_kernel, dim3(F / 16, M * top_k + extra), dim3(CP_THREADS), smem, s, (const uint32_t *)w13,
+                                       (const bf16 *)s13, (const bf16 *)x, ldx, pair_expert, top_k, F, K, (bf16 *)h, sa, M * top_k);
             return e == cudaSuccess ? 0 : -2;
         }
     }
@@ -411,24 +411,23 @@ QW_API int qwk_moe_down_combine(const void *w2, const void *s2, const void *h, c
     if ((F & 127) || (SF & 7)) return -1;
     const FuseOut fo = take_fo();
     if ((moe_mma_mask() & 8) && (H & 15) == 0 && (F & 127) == 0 && (SF & 7) == 0 && (ld_sd & 7) == 0 && top_k <= 32) {
-        // bulk-copy-fed tensor-core form
+        // copy-fed tensor-core form
         const int ks = F >> 7;
-        const size_t smem = 128 + (size_t)top_k * 16 * ((F >> 1) + TM_PAD) + (shared_down ? 16 * ((size_t)SF * 2 + TM_PAD) : 0) +
-                            (size_t)top_k * (((16 * ks * 2) + 15) & ~15) + ((size_t)top_k * (F >> 3) + (SF >> 3)) * 16 + 16 * 16 * 4 + 32 * 4 + 32 * 4;
+        const size_t smem = (size_t)top_k * 16 * ((F >> 1) + TM_PAD) + (size_t)top_k * 32 * ks + ((size_t)top_k * (F >> 3) + (SF >> 3)) * 16 + CP_WARPS * 16 * 4 + 32 * 4 + 32 * 4;
         static bool attr = false;
         if (!attr) {
-            cudaFuncSetAttribute(moe_down_tma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
-            cudaFuncSetAttribute(moe_down_tma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
+            cudaFuncSetAttribute(moe_down_cp_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
+            cudaFuncSetAttribute(moe_down_cp_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
             attr = true;
         }
         if (smem <= 110 * 1024) {
             const dim3 g2(H / 16, M);
-            cudaError_t e = fo.mode ? launch_pdl(moe_down_tma_kernel<true>, g2, dim3(512), smem, s, (const uint32_t *)w2, (const bf16 *)s2,
+            cudaError_t e = fo.mode ? launch_pdl(moe_down_cp_kernel<true>, g2, dim3(CP_THREADS), smem, s, (const uint32_t *)w2, (const bf16 *)s2,
                                                  (const bf16 *)h, pair_expert, pair_w, top_k, F, H, (const bf16 *)shared_down, ld_sd,
-                                                 (const bf16 *)sh_h, SF, out, ldo, g_err_ptr, fo)
-                                    : launch_pdl(moe_down_tma_kernel<false>, g2, dim3(512), smem, s, (const uint32_t *)w2, (const bf16 *)s2,
+                                                 (const bf16 *)sh_h, SF, out, ldo, fo)
+                                    : launch_pdl(moe_down_cp_kernel<false>, g2, dim3(CP_THREADS), smem, s, (const uint32_t *)w2, (const bf16 *)s2,
                                                  (const bf16 *)h, pair_expert, pair_w, top_k, F, H, (const bf16 *)shared_down, ld_sd,
-                                                 (const bf16 *)sh_h, SF, out, ldo, g_err_ptr, fo);
+                                                 (const bf16 *)sh_h, SF, out, ldo, fo);
             return e == cudaSuccess ? 0 : -2;
         }
     }

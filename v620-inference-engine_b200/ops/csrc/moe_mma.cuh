@@ -26,7 +26,9 @@ namespace qw {
 
 // bf16 pair (exact integers -8..7) of nibble pair j of a q4 word in engine order
 __device__ __forceinline__ uint32_t q4_frag(uint32_t w, int j) {
-    uint32_t p = ((w >> (4 * j)) & 0x000F000Fu) | 0x43004300u;
+    uint32_t p;
+    // one three-input instruction: written as & and | with both constants known it becomes two
+    asm("{\n\t.reg .b32 m;\n\tmov.b32 m, 0x000F000F;\n\tlop3.b32 %0, %1, m, 0x43004300, 0xEA;\n\t}" : "=r"(p) : "r"(w >> (4 * j)));
     bf162 v = *reinterpret_cast<bf162 *>(&p);
     const bf162 off = __floats2bfloat162_rn(136.f, 136.f);
     v = __hsub2(v, off);
@@ -271,31 +273,45 @@ __global__ void __launch_bounds__(128) moe_down_mma_kernel(const uint32_t *w2, c
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// The same two products with the weights brought in by bulk-async (TMA, untiled) row copies into padded shared memory.
-// Direct 8-byte loads from sixteen rows at once touch one 32-byte sector per row per request, which HBM serves badly
-// (measured: 16 us for 17 MB); one bulk copy per weight row is fully coalesced, needs no registers while in flight, and
-// the operand words are then read from shared memory exactly as before (row stride padded by 32 bytes: the eight rows
-// of a request fall into disjoint bank groups).  One block per tile, every copy of the block issued at once, one
-// mbarrier; enough blocks are resident for the whole launch to be one wave.
+// The same two products with the weights brought to padded shared memory by cp.async (row stride 32 bytes more than the row: the
+// eight rows of a request fall into disjoint bank groups).  A tile's 16 rows are one piece of memory, so a warp's copies are
+// whole lines and need no register while in flight.  Direct 8-byte loads touch one 32-byte sector of sixteen rows per request,
+// and bulk copies of single rows (1,280 and 320 bytes) were bound by their number.  In a chain of their own, us for gate/up and
+// down with bulk copies and now: 1 row 10.4, 8.6 -> 8.4, 7.7; 8 rows 59, 38 -> 35, 28; 24 rows 172, 106 -> 96, 72.  What bounds
+// them now: the instructions of the conversion (three per two weights, beside 7 idle columns of every MMA) and, with few rows,
+// the chain routing -> weights -> sums.
+// Every column of the narrow operand holds the token: the result's column 0 is read, the others cost nothing.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int TM_PAD = 32;                 // bytes added to a weight row in shared memory
+constexpr int CP_WARPS = 8, CP_THREADS = CP_WARPS * 32;
 
-// grid (F / 16, pairs [+ M extra rows for the shared activation]), 512 threads.
-__global__ void __launch_bounds__(512) moe_gate_up_tma_kernel(const uint32_t *w13, const bf16 *s13, const bf16 *x, int ldx,
-                                                              const int *pair_expert, int top_k, int F, int K, bf16 *h, ErrorWord *err,
-                                                              SharedAct sa, int npairs) {
+// p / d for the small numbers of this file (p < 4096, d >= 1): a multiplication by 2^20 / d, rounded up.
+__device__ __forceinline__ int div_inv(int d) { return (1 << 20) / d + 1; }
+__device__ __forceinline__ int div_by(int p, int inv) { return (int)(((long long)p * inv) >> 20); }
+
+// One k group of 128 of 16 weight rows (at `w`, row stride srow) against the token's k group: c[0] is row r = lane / 4, c[2] row r + 8.
+__device__ __forceinline__ void q4_group(float (&c)[4], const unsigned char *w, int srow, const uint4 *x, int lane) {
+    const int r = lane >> 2, q = lane & 3;
+#pragma unroll
+    for (int ds = 0; ds < 2; ++ds) {
+        const int wi = ds * 8 + 2 * q;
+        const uint2 a0 = *reinterpret_cast<const uint2 *>(w + r * srow + wi * 4), a8 = *reinterpret_cast<const uint2 *>(w + (r + 8) * srow + wi * 4);
+        mma_q4_word(c, a0.x, a8.x, x[wi]);
+        mma_q4_word(c, a0.y, a8.y, x[wi + 1]);
+    }
+}
+
+// grid (F / 16, pairs [+ M extra rows for the shared activation]), 256 threads.
+__global__ void __launch_bounds__(CP_THREADS, 4) moe_gate_up_cp_kernel(const uint32_t *w13, const bf16 *s13, const bf16 *x, int ldx,
+                                                                       const int *pair_expert, int top_k, int F, int K, bf16 *h,
+                                                                       SharedAct sa, int npairs) {
     extern __shared__ __align__(128) unsigned char tm_smem[];
     const int rowb = K >> 1, srow = rowb + TM_PAD, ks = K >> 7, wpr = K >> 3;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(tm_smem);
-    unsigned char *wg = tm_smem + 128, *wu = wg + 16 * srow;
+    unsigned char *wg = tm_smem, *wu = wg + 16 * srow;
     bf16 *sg = reinterpret_cast<bf16 *>(wu + 16 * srow), *su = sg + 16 * ks;
-    uint4 *xs = reinterpret_cast<uint4 *>(reinterpret_cast<unsigned char *>(su + 16 * ks) + ((-(16 * ks * 4)) & 15));
-    float *red = reinterpret_cast<float *>(xs + wpr);          // [16 warps][2][16]
+    uint4 *xs = reinterpret_cast<uint4 *>(su + 16 * ks);       // 64 ks bytes of scales: 16-byte aligned
+    float *red = reinterpret_cast<float *>(xs + wpr);          // [8 warps][2][16]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid == 0) {
-        mbar_init(bar, 1);
-        mbar_fence_init();
-    }
     pdl_wait();
     pdl_trigger();
     if ((int)blockIdx.y >= npairs) {          // the extra rows of the grid: the shared expert's activation
@@ -307,45 +323,34 @@ __global__ void __launch_bounds__(512) moe_gate_up_tma_kernel(const uint32_t *w1
     if (e < 0) return;
     const int f0 = blockIdx.x * 16, m = p / top_k;
     const long long row_g = (long long)e * 2 * F + f0, row_u = row_g + F;
-    __syncthreads();                          // the barrier is initialised
-    if (warp == 0) {
-        if (lane == 0) mbar_expect_tx(bar, (unsigned)(32 * rowb + 2 * 16 * ks * 2));
-        __syncwarp();
-        if (lane < 16) bulk_g2s(wg + lane * srow, w13 + (row_g + lane) * wpr, (unsigned)rowb, bar);
-        else bulk_g2s(wu + (lane - 16) * srow, w13 + (row_u + lane - 16) * wpr, (unsigned)rowb, bar);
-        if (lane == 0) bulk_g2s(sg, s13 + row_g * ks, (unsigned)(16 * ks * 2), bar);
-        if (lane == 1) bulk_g2s(su, s13 + row_u * ks, (unsigned)(16 * ks * 2), bar);
+    {
+        // a matrix's 16 rows are one piece of memory: whole lines in thread order
+        const int ppr = rowb >> 4, inv = div_inv(ppr);
+        const unsigned char *g = reinterpret_cast<const unsigned char *>(w13 + row_g * wpr), *up = reinterpret_cast<const unsigned char *>(w13 + row_u * wpr);
+#pragma unroll 5
+        for (int i = tid; i < 16 * ppr; i += CP_THREADS) {
+            const int at = i * 16 + div_by(i, inv) * TM_PAD;
+            cp_async16(wg + at, g + i * 16);
+            cp_async16(wu + at, up + i * 16);
+        }
     }
-    const uint4 *xr = reinterpret_cast<const uint4 *>(x + (long long)m * ldx);
-    for (int i = tid; i < wpr; i += 512) xs[i] = __ldcg(xr + i);
+    for (int i = tid; i < 4 * ks; i += CP_THREADS)             // 16 rows' scales: 2 ks pieces of 16 bytes each
+        cp_async16(reinterpret_cast<unsigned char *>(sg) + i * 16,
+                   reinterpret_cast<const unsigned char *>(s13 + (i < 2 * ks ? row_g : row_u) * ks) + (i < 2 * ks ? i : i - 2 * ks) * 16);
+    for (int i = tid; i < wpr; i += CP_THREADS) cp_async16(xs + i, reinterpret_cast<const uint4 *>(x + (long long)m * ldx) + i);
+    cp_async_wait();
     __syncthreads();
-    const bool ok = mbar_wait(bar, 0u, err);
     const int r = lane >> 2, q = lane & 3;
     float ag = 0.f, ag8 = 0.f, au = 0.f, au8 = 0.f;
-    if (ok) {
-        for (int g = warp; g < ks; g += 16) {
-            float cg[4] = {0.f, 0.f, 0.f, 0.f}, cu[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int ds = 0; ds < 2; ++ds) {
-                const int wi = g * 16 + ds * 8 + 2 * q;
-                const uint2 a0 = *reinterpret_cast<const uint2 *>(wg + r * srow + wi * 4), a8 = *reinterpret_cast<const uint2 *>(wg + (r + 8) * srow + wi * 4);
-                const uint2 b0 = *reinterpret_cast<const uint2 *>(wu + r * srow + wi * 4), b8 = *reinterpret_cast<const uint2 *>(wu + (r + 8) * srow + wi * 4);
-                uint4 x0 = make_uint4(0u, 0u, 0u, 0u), x1 = x0;
-                if (r == 0) {                                               // column 0 of the narrow operand is the token
-                    x0 = xs[wi];
-                    x1 = xs[wi + 1];
-                }
-                mma_q4_word(cg, a0.x, a8.x, x0);
-                mma_q4_word(cg, a0.y, a8.y, x1);
-                mma_q4_word(cu, b0.x, b8.x, x0);
-                mma_q4_word(cu, b0.y, b8.y, x1);
-            }
-            if (q == 0) {
-                ag = fmaf(__bfloat162float(sg[r * ks + g]), cg[0], ag);
-                ag8 = fmaf(__bfloat162float(sg[(r + 8) * ks + g]), cg[2], ag8);
-                au = fmaf(__bfloat162float(su[r * ks + g]), cu[0], au);
-                au8 = fmaf(__bfloat162float(su[(r + 8) * ks + g]), cu[2], au8);
-            }
+    for (int g = warp; g < ks; g += CP_WARPS) {
+        float cg[4] = {0.f, 0.f, 0.f, 0.f}, cu[4] = {0.f, 0.f, 0.f, 0.f};
+        q4_group(cg, wg + g * 64, srow, xs + g * 16, lane);
+        q4_group(cu, wu + g * 64, srow, xs + g * 16, lane);
+        if (q == 0) {
+            ag = fmaf(__bfloat162float(sg[r * ks + g]), cg[0], ag);
+            ag8 = fmaf(__bfloat162float(sg[(r + 8) * ks + g]), cg[2], ag8);
+            au = fmaf(__bfloat162float(su[r * ks + g]), cu[0], au);
+            au8 = fmaf(__bfloat162float(su[(r + 8) * ks + g]), cu[2], au8);
         }
     }
     if (q == 0) {
@@ -353,48 +358,47 @@ __global__ void __launch_bounds__(512) moe_gate_up_tma_kernel(const uint32_t *w1
         red[(warp * 2 + 1) * 16 + r] = au; red[(warp * 2 + 1) * 16 + r + 8] = au8;
     }
     __syncthreads();
-    if (tid < 16) {
-        float gs = 0.f, us = 0.f;
+    if (tid < 32) {                           // lanes 0-15 gate, 16-31 up
+        float v = 0.f;
 #pragma unroll
-        for (int w = 0; w < 16; ++w) { gs += red[(w * 2) * 16 + tid]; us += red[(w * 2 + 1) * 16 + tid]; }
-        h[(long long)p * F + f0 + tid] = __float2bfloat16(siluf_(gs) * us);
+        for (int w = 0; w < CP_WARPS; ++w) v += red[w * 32 + tid];
+        const float up = __shfl_down_sync(0xffffffffu, v, 16);
+        if (tid < 16) h[(long long)p * F + f0 + tid] = __float2bfloat16(siluf_(v) * up);
     }
 }
 
-// grid (H / 16, M), 512 threads.  Shared memory: barrier(s) | top_k expert tiles [16][F/2 + pad] | shared tile
-// [16][SF*2 + pad] | scales [top_k][16][F/128] | h vectors | shared activation | reduction scratch.
+constexpr int DC_NS = 3;                   // quad-steps of the shared expert per warp that are fetched before the dependency wait
+// grid (H / 16, M), 256 threads.  Shared memory: top_k expert tiles [16][F/2 + pad] | scales [top_k][16][F/128] | h vectors |
+// shared activation | reduction scratch (64 KB at the model's shapes: three blocks per SM).
 template <bool FUSED>
-__global__ void __launch_bounds__(512) moe_down_tma_kernel(const uint32_t *w2, const bf16 *s2, const bf16 *h, const int *pair_expert,
-                                                           const float *pair_w, int top_k, int F, int H, const bf16 *shared_down,
-                                                           int ld_sd, const bf16 *sh_h, int SF, float *out, int ldo, ErrorWord *err,
-                                                           FuseOut fo) {
+__global__ void __launch_bounds__(CP_THREADS, 3) moe_down_cp_kernel(const uint32_t *w2, const bf16 *s2, const bf16 *h, const int *pair_expert,
+                                                                 const float *pair_w, int top_k, int F, int H, const bf16 *shared_down,
+                                                                 int ld_sd, const bf16 *sh_h, int SF, float *out, int ldo, FuseOut fo) {
     extern __shared__ __align__(128) unsigned char tm_smem[];
     const int rowb = F >> 1, srow = rowb + TM_PAD, ks = F >> 7, wpr = F >> 3;
-    const int srowb = SF * 2, ssrow = srowb + TM_PAD, sch = SF >> 3;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(tm_smem);              // [0] routed experts, [1] shared expert
-    unsigned char *we = tm_smem + 128;                                   // [top_k][16][srow]
-    unsigned char *wsd = we + (size_t)top_k * 16 * srow;                 // [16][ssrow]
-    bf16 *sc = reinterpret_cast<bf16 *>(wsd + (shared_down ? 16 * ssrow : 0));      // [top_k][16 * ks] (+ pad to 16 bytes per expert)
-    const int scb = ((16 * ks * 2) + 15) & ~15;                          // bytes of one expert's scales in shared memory
-    uint4 *hs = reinterpret_cast<uint4 *>(reinterpret_cast<unsigned char *>(sc) + (size_t)top_k * scb);      // [top_k][wpr]
+    const int sch = shared_down ? SF >> 3 : 0;                           // 16-byte pieces of a shared row
+    unsigned char *we = tm_smem;                                         // [top_k][16][srow]
+    bf16 *sc = reinterpret_cast<bf16 *>(we + (size_t)top_k * 16 * srow); // [top_k][16 * ks]: 32 ks bytes per expert
+    uint4 *hs = reinterpret_cast<uint4 *>(sc + (size_t)top_k * 16 * ks); // [top_k][wpr]
     uint4 *ss = hs + (size_t)top_k * wpr;                                // [sch]
-    float *red = reinterpret_cast<float *>(ss + sch);                    // [16 warps][16]
-    int *s_e = reinterpret_cast<int *>(red + 16 * 16);                   // [top_k]
+    float *red = reinterpret_cast<float *>(ss + sch);                    // [8 warps][16]
+    int *s_e = reinterpret_cast<int *>(red + CP_WARPS * 16);             // [top_k]
     float *s_w = reinterpret_cast<float *>(s_e + 32);                    // [top_k]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m = blockIdx.y, c0 = blockIdx.x * 16;
-    if (tid == 0) {
-        mbar_init(bar, 1);
-        mbar_init(bar + 1, 1);
-        mbar_fence_init();
-    }
-    __syncthreads();
-    // the shared expert's rows do not depend on the routing: their copies start before the wait for the router
-    if (shared_down && warp == 0) {
-        if (lane == 0) mbar_expect_tx(bar + 1, (unsigned)(16 * srowb));
-        __syncwarp();
-        if (lane < 16) bulk_g2s(wsd + lane * ssrow, shared_down + (long long)(c0 + lane) * ld_sd, (unsigned)srowb, bar + 1);
-    }
+    const int r = lane >> 2, q = lane & 3;
+    // the shared expert's rows do not depend on the routing: fetched, as operand words, before the wait for the router
+    const bf16 *sr = shared_down + (long long)(c0 + r) * ld_sd;
+    auto shared_words = [&](int st, uint4 &w0, uint4 &w8) {
+        const int pc = st * 4 + q;
+        w0 = w8 = make_uint4(0u, 0u, 0u, 0u);
+        if (pc >= sch) return;
+        w0 = __ldg(reinterpret_cast<const uint4 *>(sr) + pc);
+        w8 = __ldg(reinterpret_cast<const uint4 *>(sr + 8LL * ld_sd) + pc);
+    };
+    uint4 sw[DC_NS], sw8[DC_NS];
+#pragma unroll
+    for (int i = 0; i < DC_NS; ++i) shared_words(warp + CP_WARPS * i, sw[i], sw8[i]);
     pdl_wait();
     pdl_trigger();
     if (tid < top_k) {
@@ -402,79 +406,51 @@ __global__ void __launch_bounds__(512) moe_down_tma_kernel(const uint32_t *w2, c
         s_e[tid] = pair_expert[p];
         s_w[tid] = pair_w[p];
     }
+    for (int i = tid; i < top_k * wpr; i += CP_THREADS) cp_async16(hs + i, reinterpret_cast<const uint4 *>(h + (long long)m * top_k * F) + i);
+    for (int i = tid; i < sch; i += CP_THREADS) cp_async16(ss + i, reinterpret_cast<const uint4 *>(sh_h + (long long)m * SF) + i);
     __syncthreads();
-    // every warp issues the copies of its experts (one warp issuing all 170 of them took microseconds); the expected byte
-    // count is posted once by thread 0 - copies that complete earlier are accounted against it
-    if (tid == 0) {
-        int nloc = 0;
-        for (int j = 0; j < top_k; ++j) nloc += s_e[j] >= 0;
-        mbar_expect_tx(bar, (unsigned)(nloc * (16 * rowb + 16 * ks * 2)));
+    // an expert's 16 rows are one piece of memory; a thread keeps its places in the tile for all experts
+    const int ppr = rowb >> 4, inv_ppr = div_inv(ppr), inv_ks = div_inv(ks);
+    for (int i = tid; i < 16 * ppr; i += CP_THREADS) {
+        unsigned char *dst = we + i * 16 + div_by(i, inv_ppr) * TM_PAD;
+        const unsigned char *src = reinterpret_cast<const unsigned char *>(w2 + (long long)c0 * wpr) + i * 16;
+#pragma unroll 5
+        for (int j = 0; j < top_k; ++j) {
+            const int e = s_e[j];
+            if (e >= 0) cp_async16(dst + j * 16 * srow, src + (long long)e * H * rowb);
+        }
     }
-    for (int j = warp; j < top_k; j += 16) {
-        const int e = s_e[j];
-        if (e < 0) continue;
-        const long long row = (long long)e * H + c0;
-        if (lane < 16) bulk_g2s(we + ((size_t)j * 16 + lane) * srow, w2 + (row + lane) * wpr, (unsigned)rowb, bar);
-        if (lane == 16) bulk_g2s(reinterpret_cast<unsigned char *>(sc) + (size_t)j * scb, s2 + row * ks, (unsigned)(16 * ks * 2), bar);
+    for (int i = tid; i < top_k * 2 * ks; i += CP_THREADS) {
+        const int j = div_by(i >> 1, inv_ks), b = i - j * 2 * ks, e = s_e[j];
+        if (e >= 0) cp_async16(reinterpret_cast<unsigned char *>(sc) + i * 16, reinterpret_cast<const unsigned char *>(s2 + ((long long)e * H + c0) * ks) + b * 16);
+    }
+    cp_async_wait();
+    __syncthreads();
+    float a0 = 0.f, a8 = 0.f;
+    const int nitems = top_k * ks;
+    for (int it = warp; it < nitems; it += CP_WARPS) {
+        const int j = div_by(it, inv_ks), g = it - j * ks;
+        if (s_e[j] < 0) continue;                       // warp-uniform
+        float c[4] = {0.f, 0.f, 0.f, 0.f};
+        q4_group(c, we + (size_t)j * 16 * srow + g * 64, srow, hs + (size_t)j * wpr + g * 16, lane);
+        if (q == 0) {
+            const bf16 *sj = sc + (size_t)j * 16 * ks;
+            a0 = fmaf(__bfloat162float(sj[r * ks + g]) * s_w[j], c[0], a0);
+            a8 = fmaf(__bfloat162float(sj[(r + 8) * ks + g]) * s_w[j], c[2], a8);
+        }
     }
     {
-        // the activations: both loops' loads in flight together
-        const uint4 *hg = reinterpret_cast<const uint4 *>(h + (long long)m * top_k * F);
-        const int nh = top_k * wpr;
-        uint4 v0 = make_uint4(0u, 0u, 0u, 0u), v1 = v0, v2 = v0;
-        if (tid < nh) v0 = __ldcg(hg + tid);
-        if (tid + 512 < nh) v1 = __ldcg(hg + tid + 512);
-        if (shared_down && tid < sch) v2 = __ldcg(reinterpret_cast<const uint4 *>(sh_h + (long long)m * SF) + tid);
-        if (tid < nh) hs[tid] = v0;
-        if (tid + 512 < nh) hs[tid + 512] = v1;
-        for (int i = tid + 1024; i < nh; i += 512) hs[i] = __ldcg(hg + i);
-        if (shared_down) {
-            if (tid < sch) ss[tid] = v2;
-            for (int i = tid + 512; i < sch; i += 512) ss[i] = __ldcg(reinterpret_cast<const uint4 *>(sh_h + (long long)m * SF) + i);
-        }
-    }
-    __syncthreads();
-    const int r = lane >> 2, q = lane & 3;
-    float a0 = 0.f, a8 = 0.f;
-    bool ok = mbar_wait(bar, 0u, err);
-    if (ok) {
-        const int nitems = top_k * ks;
-        for (int it = warp; it < nitems; it += 16) {
-            const int j = it / ks, g = it - j * ks;
-            if (s_e[j] < 0) continue;                       // warp-uniform
-            const unsigned char *wj = we + (size_t)j * 16 * srow;
-            const uint4 *xj = hs + (size_t)j * wpr;
-            float c[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int ds = 0; ds < 2; ++ds) {
-                const int wi = g * 16 + ds * 8 + 2 * q;
-                const uint2 v0 = *reinterpret_cast<const uint2 *>(wj + r * srow + wi * 4), v8 = *reinterpret_cast<const uint2 *>(wj + (r + 8) * srow + wi * 4);
-                uint4 x0 = make_uint4(0u, 0u, 0u, 0u), x1 = x0;
-                if (r == 0) {
-                    x0 = xj[wi];
-                    x1 = xj[wi + 1];
-                }
-                mma_q4_word(c, v0.x, v8.x, x0);
-                mma_q4_word(c, v0.y, v8.y, x1);
-            }
-            if (q == 0) {
-                const bf16 *sj = reinterpret_cast<const bf16 *>(reinterpret_cast<const unsigned char *>(sc) + (size_t)j * scb);
-                a0 = fmaf(__bfloat162float(sj[r * ks + g]) * s_w[j], c[0], a0);
-                a8 = fmaf(__bfloat162float(sj[(r + 8) * ks + g]) * s_w[j], c[2], a8);
-            }
-        }
-    }
-    if (shared_down && mbar_wait(bar + 1, 0u, err)) {
         float c[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int st = warp; st * 4 < sch; st += 16) {         // quad-steps of four 16-byte pieces
-            const int pc = st * 4 + q;
-            uint4 w0 = make_uint4(0u, 0u, 0u, 0u), w8 = w0, xv = w0;
-            if (pc < sch) {
-                w0 = *reinterpret_cast<const uint4 *>(wsd + r * ssrow + pc * 16);
-                w8 = *reinterpret_cast<const uint4 *>(wsd + (r + 8) * ssrow + pc * 16);
-                if (r == 0) xv = ss[pc];
-            }
-            mma_bf16_chunk(c, w0, w8, xv);
+        auto shared_step = [&](int st, const uint4 &w0, const uint4 &w8) {
+            if (st * 4 >= sch) return;                  // warp-uniform
+            mma_bf16_chunk(c, w0, w8, st * 4 + q < sch ? ss[st * 4 + q] : make_uint4(0u, 0u, 0u, 0u));
+        };
+#pragma unroll
+        for (int i = 0; i < DC_NS; ++i) shared_step(warp + CP_WARPS * i, sw[i], sw8[i]);
+        for (int st = warp + CP_WARPS * DC_NS; st * 4 < sch; st += CP_WARPS) {
+            uint4 w0, w8;
+            shared_words(st, w0, w8);
+            shared_step(st, w0, w8);
         }
         a0 += c[0];
         a8 += c[2];
@@ -487,7 +463,7 @@ __global__ void __launch_bounds__(512) moe_down_tma_kernel(const uint32_t *w2, c
     if (tid < 16) {
         float v = 0.f;
 #pragma unroll
-        for (int w = 0; w < 16; ++w) v += red[w * 16 + tid];
+        for (int w = 0; w < CP_WARPS; ++w) v += red[w * 16 + tid];
         if (FUSED) fuse_put_col(fo, fuse_seq(fo), m, c0 + tid, __float_as_uint(v));      // fused reduce-scatter: to the column's owner
         else out[(long long)m * ldo + c0 + tid] = v;
     }
