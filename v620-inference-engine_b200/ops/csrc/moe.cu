@@ -16,23 +16,24 @@
 namespace qw {
 
 // Routing of row m from rs[m] = [ router logits (E) | shared gate logit | shared gate rows (F) | shared up rows (F) ].
-// One warp per row.
+// One warp per row; E <= 32 NI.
+template <int NI>
 __device__ __forceinline__ void route_row(const float *l, int E, int top_k, int e_first, int e_local, int *pair_expert,
                                           float *pair_w, int lane, int *stats) {
     // The ranking is done on the logits (the softmax is monotonic); only the chosen ones are exponentiated:
     // w_j = exp(l_j - l_top) / sum over the chosen.  Every lane keeps the best of its own elements cached, so a round
     // is one warp arg-max (5 shuffle steps) plus a rescan by the one lane that lost its best.
-    float v[32];     // E <= 1024
+    float v[NI];
     const int ni = (E + 31) >> 5;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
+    for (int i = 0; i < NI; ++i) {
         const int e = lane + 32 * i;
         v[i] = (i < ni && e < E) ? __ldcg(l + e) : -INFINITY;
     }
     float bv = -INFINITY;
     int bi = 0x7fffffff;
 #pragma unroll
-    for (int i = 0; i < 32; ++i)          // ascending index: strict > keeps the lowest index
+    for (int i = 0; i < NI; ++i)          // ascending index: strict > keeps the lowest index
         if (v[i] > bv) { bv = v[i]; bi = lane + 32 * i; }
     float topsum = 0.f, mine_w = 0.f, top0 = 0.f;
     int mine_e = -1;
@@ -53,7 +54,7 @@ __device__ __forceinline__ void route_row(const float *l, int E, int top_k, int 
             bv = -INFINITY;
             bi = 0x7fffffff;
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
+            for (int i = 0; i < NI; ++i) {
                 if (i == (wi >> 5)) v[i] = -INFINITY;
                 if (v[i] > bv) { bv = v[i]; bi = lane + 32 * i; }
             }
@@ -81,21 +82,33 @@ struct RouteArgs {
     int *stats;                                  // optional counter of local pairs (MoE balance statistics)
 };
 
-// `scratch`: 1056 floats of shared memory the caller does not need any more.
-__device__ __forceinline__ void route_all(const float *rs, int ld_rs, int M, const RouteArgs &r, float *scratch) {
+// Rows 0 .. M-1, a warp each.
+__device__ __forceinline__ void route_rows(const float *rs, int ld_rs, int M, const RouteArgs &r) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    float *s_log = scratch, *s_top = scratch + 1024;
-    for (int m = warp; m < M; m += nw)
-        route_row(rs + (long long)m * ld_rs, r.E, r.top_k, r.e_first, r.e_local, r.pair_expert + m * r.top_k,
-                  r.pair_w + m * r.top_k, lane, r.stats);
-    (void)s_log; (void)s_top;
-    if (r.sh_h) {
-        for (int i = threadIdx.x; i < M * r.F; i += blockDim.x) {
-            const int m = i / r.F, f = i % r.F;
-            const float *l = rs + (long long)m * ld_rs;
-            const float sg = sigmoidf_(__ldcg(l + r.E));
-            r.sh_h[i] = __float2bfloat16(siluf_(__ldcg(l + r.E + 1 + f)) * __ldcg(l + r.E + 1 + r.F + f) * sg);
+    for (int m = warp; m < M; m += nw) {
+        const float *l = rs + (long long)m * ld_rs;
+        if (r.E <= 512) route_row<16>(l, r.E, r.top_k, r.e_first, r.e_local, r.pair_expert + m * r.top_k, r.pair_w + m * r.top_k, lane, r.stats);
+        else route_row<32>(l, r.E, r.top_k, r.e_first, r.e_local, r.pair_expert + m * r.top_k, r.pair_w + m * r.top_k, lane, r.stats);
+    }
+}
+// The shared expert's activation of rows 0 .. M-1, elements i0, i0 + step, ...: four elements' loads in flight per thread.
+__device__ __forceinline__ void route_shared(const float *rs, int ld_rs, int M, const RouteArgs &r, int i0, int step) {
+    const int total = M * r.F;
+    for (int i = i0; i < total; i += 4 * step) {
+        float sg[4], g[4], u[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int e = i + k * step, m = e / r.F, f = e - m * r.F;
+            sg[k] = g[k] = u[k] = 0.f;
+            if (e >= total) continue;
+            const float *l = rs + (long long)m * ld_rs + r.E;
+            sg[k] = __ldcg(l);
+            g[k] = __ldcg(l + 1 + f);
+            u[k] = __ldcg(l + 1 + r.F + f);
         }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (i + k * step < total) r.sh_h[i + k * step] = __float2bfloat16(siluf_(g[k]) * u[k] * sigmoidf_(sg[k]));
     }
 }
 
@@ -115,7 +128,8 @@ __global__ void __launch_bounds__(SG_THREADS, 1) moe_router_kernel(SGemvArgs a, 
         if (threadIdx.x == 0) *r.ticket = 0u;
         return;
     }
-    route_all(a.y, a.ldy, a.M, r, reinterpret_cast<float *>(sg_smem + SG_HDR));      // the weight stages are free now
+    route_rows(a.y, a.ldy, a.M, r);
+    if (r.sh_h) route_shared(a.y, a.ldy, a.M, r, threadIdx.x, blockDim.x);
     if (threadIdx.x == 0) *r.ticket = 0u;
 }
 
@@ -148,19 +162,21 @@ static cudaError_t launch_router(SGemvArgs &a, const RouteArgs &r, cudaStream_t 
     return launch_router_nt<1>(a, r, smem1, grid, s);
 }
 
-// Stand-alone routing (tests, and callers that computed the logits elsewhere).  One block.
-// Each block routes 8 rows (a warp per row) and applies the shared activation to them.
+// Stand-alone routing (prefill, and callers that computed the logits elsewhere).  Eight rows per column of blocks: blockIdx.y == 0
+// routes them (a warp per row), the others share the activation of the shared expert, which as the tail of the routing block was
+// most of its time (20 rounds of loads one behind the other: 27 us at 6 rows, 35 at 100; now 6 and 8).
+constexpr int ROUTE_ROWS = 8, ROUTE_ACT_BLOCKS = 5;
 __global__ void __launch_bounds__(256) moe_route_kernel(const float *rs, int ld_rs, int M, RouteArgs r) {
     pdl_wait();
     pdl_trigger();
-    const int m0 = blockIdx.x * 8;
-    const int nm = min(8, M - m0);
+    const int m0 = blockIdx.x * ROUTE_ROWS, nm = min(ROUTE_ROWS, M - m0);
+    const float *l = rs + (long long)m0 * ld_rs;
     RouteArgs q = r;
     q.pair_expert += m0 * r.top_k;
     q.pair_w += m0 * r.top_k;
     if (q.sh_h) q.sh_h += (long long)m0 * r.F;
-    __shared__ float s_route[1056];
-    route_all(rs + (long long)m0 * ld_rs, ld_rs, nm, q, s_route);
+    if (blockIdx.y == 0) route_rows(l, ld_rs, nm, q);
+    else route_shared(l, ld_rs, nm, q, (blockIdx.y - 1) * 256 + threadIdx.x, ROUTE_ACT_BLOCKS * 256);
 }
 
 // 32 q4 values (one 16-byte load, engine order) dot 32 bf16 activations.
@@ -364,7 +380,7 @@ QW_API int qwk_moe_route(const float *rs, int ld_rs, int M, int E, int top_k, in
                          int *pair_expert, float *pair_w, void *sh_h, cudaStream_t s) {
     if (E > 1024 || top_k > 32) return -1;
     RouteArgs r = make_route(E, top_k, F, e_first, e_local, pair_expert, pair_w, sh_h, nullptr);
-    cudaError_t e = launch_pdl(moe_route_kernel, dim3((M + 7) / 8), dim3(256), 0, s, rs, ld_rs, M, r);
+    cudaError_t e = launch_pdl(moe_route_kernel, dim3((M + ROUTE_ROWS - 1) / ROUTE_ROWS, sh_h ? 1 + ROUTE_ACT_BLOCKS : 1), dim3(256), 0, s, rs, ld_rs, M, r);
     return e == cudaSuccess ? 0 : -2;
 }
 
