@@ -369,3 +369,51 @@ def test_mixer_rows_match_64_bits_and_do_not_depend_on_their_neighbours(SH, R, n
         x1, send1, inj1, out1 = both(rows)
         assert torch.equal(x1, x[rows]) and torch.equal(send1, send[rows]) and torch.equal(inj1, inj[rows]) and torch.equal(out1, out[rows])
     assert torch.equal(both([3], combine=False)[0][0], X[3])
+
+
+@pytest.mark.parametrize("N,K", [(1000, 2560), (160, 6144), (48, 1280), (33, 656)])
+def test_gemv_rows_are_the_same_bits_at_every_row_count(N, K):
+    """One, two and three tiles of eight rows per pass (three: 17 to 24 rows where they fit) and several passes: a row's sums do not
+    depend on how many rows share the step."""
+    from qwb200.ops import kernels as K_
+    g = torch.Generator(device="cuda").manual_seed(N)
+    W = (torch.randn(N, K, generator=g, device=_dev()) * 0.05).to(torch.bfloat16)
+    x = torch.randn(32, K, generator=g, device=_dev()).to(torch.bfloat16)
+    one = torch.cat([K_.gemv_bf16(W, x[i:i + 1]) for i in range(32)])
+    for M in (2, 8, 9, 16, 17, 20, 24, 25, 32):
+        assert torch.equal(K_.gemv_bf16(W, x[:M]), one[:M]), M
+    ref = x.double() @ W.double().T
+    assert float((one.double() - ref).norm() / ref.norm()) < 1e-5
+
+
+@pytest.mark.parametrize("M,base", [(33, 0), (100, 2), (41, 77)])
+def test_gdn_conv_of_a_prefill_chunk_matches_the_step_kernel(M, base):
+    """More than 32 rows take a warp per head; the same rows in pieces of at most 32 take the step kernel.  Same products; the norm of
+    a head is summed in another order (128 terms in fp32: 1e-6 relative)."""
+    import ctypes as C
+    from qwb200.ops import lib as qlib
+    L = qlib.load(True)
+    KL, VL, dev = 2, 6, _dev()
+    qkv = (2 * KL + VL) * 128
+    ld = qkv + VL * 128 + 2 * VL
+    g = torch.Generator(device="cuda").manual_seed(M)
+    rn = lambda *s: torch.randn(*s, generator=g, device=dev)
+    proj, cw, A, dt, ring0 = rn(M, ld), rn(qkv, 4) * 0.3, rn(VL), rn(VL), rn(2, 16, qkv)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)
+    P = lambda t: C.c_void_p(t.data_ptr())
+    s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def conv(pieces):
+        ring, out, at = ring0.clone(), [], 0
+        for n in pieces:
+            p, o, d, b = proj[at:at + n].contiguous(), torch.empty(n, qkv, device=dev), torch.empty(n, VL, device=dev), torch.empty(n, VL, device=dev)
+            rows = [i32([1] * n), i32([base + at + i for i in range(n)]), i32([0] * n), i32([n] + [0] * (n - 1))]
+            assert L.qwk_gdn_conv(P(p), ld, P(ring), P(cw), P(A), P(dt), KL, VL, n, *[P(r) for r in rows], P(o), P(d), P(b), C.c_float(1e-6), s) == 0
+            out.append((o, d, b))
+            torch.cuda.synchronize()
+            at += n
+        return [torch.cat(t) for t in zip(*out)] + [ring]
+    whole, parts = conv([M]), conv([20] * (M // 20) + ([M % 20] if M % 20 else []))
+    for x, y in zip(whole[:3], parts[:3]):
+        assert torch.allclose(x, y, rtol=1e-5, atol=1e-6)
+    assert torch.equal(whole[3], parts[3])
