@@ -121,7 +121,7 @@ struct EpiStore {
     }
 };
 
-// NT = activation-row tiles of 8 handled per pass (1 or 2).
+// NT = activation-row tiles of 8 handled per pass (1, 2 or 3).
 template <int NT, class XFill, class Epi>
 __device__ __forceinline__ void sgemv_core(const SGemvArgs &a, unsigned char *smem, const XFill &xfill, const Epi &epi) {
     uint64_t *full = reinterpret_cast<uint64_t *>(smem), *empty = full + 8;
@@ -240,6 +240,8 @@ static inline size_t sgemv_plan(SGemvArgs &a, int NT, int &grid, size_t extra = 
     const size_t Kb = (size_t)a.K * 2;
     int P = (int)((Kb + 2559) / 2560);
     while (a.K % (16 * P)) ++P;
+    // many activation rows leave room for short stages only; parts of a multiple of 128 keep every warp's k steps what they are
+    if (NT == 3 && a.K % (256 * P) == 0 && a.K / P % 128 == 0) P *= 2;
     a.P = P;
     if (a.nsplit < 1) a.nsplit = 1;
     const size_t stage = (size_t)SG_TILE * (Kb / P + ROW_PAD);
