@@ -26,6 +26,32 @@ def test_gemm_tc_matches_fp32(T, N, K, out_dtype):
     assert err < tol, err
 
 
+@pytest.mark.parametrize("T,N,K", [(1, 128, 512), (100, 2560, 6144), (100, 1793, 2560), (129, 324, 10240), (64, 100, 520), (200, 130, 4304),
+                                   (300, 2560, 1024), (128, 128, 4096),
+                                   # the line between the forms: 129-row and 256-row products in pairs, padded pairs, wide tiles
+                                   (129, 10240, 1152), (777, 4304, 512), (257, 16480, 128)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_gemm_tc_split_and_padded_forms_match_64_bits(T, N, K, out_dtype):
+    """Few tiles shared by clusters of 2, 4 and 8 CTAs (k blocks that do not divide evenly, ragged rows and columns) and the padded
+    pair and wide forms: fp32 sums of exact products (1e-5 of the result's size for K <= 10240; bf16 output 2^-9 more), twice the
+    same bits, and nothing outside the result written."""
+    from qwb200.ops import kernels as K_
+    g = torch.Generator(device="cuda").manual_seed(T + N + K)
+    A = torch.randn(T, K, generator=g, device="cuda").to(torch.bfloat16)
+    W = (torch.randn(N, K, generator=g, device="cuda") * 0.05).to(torch.bfloat16)
+    ldc = (N + 7) // 8 * 8 + 8
+    out = torch.full((T + 2, ldc), 768.0, dtype=out_dtype, device="cuda")
+    K_.gemm_bf16_tc(A, W, out=out[:T, :N])
+    again = torch.empty_like(out)
+    K_.gemm_bf16_tc(A, W, out=again[:T, :N])
+    torch.cuda.synchronize()
+    ref = A.double() @ W.double().T
+    assert torch.all(out[:, N:].float() == 768.0) and torch.all(out[T:].float() == 768.0)
+    assert torch.equal(out[:T, :N], again[:T, :N])
+    err = float((out[:T, :N].double() - ref).norm() / ref.norm())
+    assert err < (1e-5 if out_dtype == torch.float32 else 2 ** -8), err
+
+
 @pytest.mark.parametrize("Nw,K,counts", [(256, 256, [5, 0, 130, 128, 1, 300]), (1280, 2560, [80, 200, 0, 33]),
                                          (2560, 640, [77, 129, 64])])
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])

@@ -22,6 +22,8 @@
 #include "tc.cuh"
 #include "tp.cuh"
 
+#include <cooperative_groups.h>
+
 namespace qw {
 
 constexpr int TC_BM = 128, TC_BN = 128, TC_BK = 64, TC_STAGES = 3;
@@ -371,6 +373,118 @@ __global__ void __launch_bounds__(320, (BN == TC_BN && !STG) ? 2 : 1) gemm_tc_ke
 }
 
 // ------------------------------------------------------------------------------------------------------------------
+// The split form, for products with few output tiles: a cluster of KS CTAs shares one 128 x 128 tile, each over its part of the k
+// blocks.  A k block takes a CTA 0.3 us however few CTAs run, so 20 tiles of 96 k blocks took 29 us on 20 SMs.  When all
+// accumulators are complete, CTA c owns the columns [c * 128 / KS, ...): the others write theirs into its (now free) pipeline
+// stages, and it adds the parts in rank order - the sum does not depend on timing - and stores.
+// grid KS x tiles, 320 threads: warp 0 TMA, warp 1 MMA, warps 2-9 epilogue.
+// ------------------------------------------------------------------------------------------------------------------
+constexpr int TC_KS_STAGES = 5;
+template <int KS>
+__global__ void __launch_bounds__(320, 1) gemm_tc_ksplit_kernel(const __grid_constant__ CUtensorMap mapA,
+                                                                const __grid_constant__ CUtensorMap mapW, GemmTcArgs a) {
+    namespace cg = cooperative_groups;
+    constexpr int QC = TC_BN / KS;                                    // columns of a CTA's share of the tile
+    constexpr int PART = TC_BM * QC * 4, CH = QC / 4;                 // one part in shared memory; 16-byte chunks of its row
+    static_assert((KS - 1) * PART <= TC_KS_STAGES * TC_STAGE_BYTES, "the parts fit into the stages");
+    extern __shared__ unsigned char raw[];
+    const cg::cluster_group cl = cg::this_cluster();
+    const int warp = uniform_warp(), lane = threadIdx.x & 31, rank = blockIdx.x % KS;
+    const TcShared sh = tc_setup<TC_BN, TC_KS_STAGES>(raw, warp, 1, 8);
+    TileAt t;
+    tile_at(a, blockIdx.x / KS, t);
+    const int per = (t.kbn + KS - 1) / KS, k0 = min(t.kbn, rank * per), k1 = min(t.kbn, k0 + per);
+    if (warp == 0) {
+        for (int kb = k0; kb < k1; ++kb) {
+            const unsigned it = (unsigned)(kb - k0), s = it % TC_KS_STAGES;
+            if (it >= TC_KS_STAGES && !mbar_wait_warp(sh.empty + s, (it / TC_KS_STAGES - 1) & 1u, a.err)) break;
+            if (elect_one()) {
+                mbar_expect_tx(sh.full + s, TC_STAGE_BYTES);
+                unsigned char *st = sh.smem + s * TC_STAGE_BYTES;
+                tma_load_2d(st, &mapA, (t.kb0 + kb) * TC_BK, t.t0, sh.full + s);
+                tma_load_2d(st + TC_A_BYTES, &mapW, (t.kb0 + kb) * TC_BK, t.w0, sh.full + s);
+            }
+        }
+    } else if (warp == 1) {
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TC_BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
+        bool ok = true;
+        for (int kb = k0; kb < k1; ++kb) {
+            const unsigned it = (unsigned)(kb - k0), s = it % TC_KS_STAGES;
+            if (!mbar_wait_warp(sh.full + s, (it / TC_KS_STAGES) & 1u, a.err)) { ok = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t sa = smem_u32(sh.smem + s * TC_STAGE_BYTES), sb = sa + TC_A_BYTES;
+            if (elect_one()) {
+#pragma unroll
+                for (int k = 0; k < TC_BK / 16; ++k)
+                    umma_bf16(sh.tmem, make_sw128_desc(sa + k * 32), make_sw128_desc(sb + k * 32), idesc, (it | k) ? 1u : 0u);
+                umma_commit(sh.empty + s);
+            }
+        }
+        if (ok && k1 > k0 && elect_one()) umma_commit(sh.done);
+    } else if (k1 > k0) {
+        mbar_wait(sh.done, 0u, a.err);
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    }
+    __syncwarp();
+    cl.sync();                                                        // every accumulator is complete, every stage free
+    const int q = warp & 3, hf = warp >= 6 ? 1 : 0;                   // epilogue warps: 32 rows, every other share
+    if (warp >= 2 && k1 > k0) {
+        for (int c = hf; c < KS; c += 2) {
+            if (c == rank) continue;
+            unsigned char *dst = cl.map_shared_rank(sh.smem, c) + (rank < c ? rank : rank - 1) * PART + (q * 32 + lane) * QC * 4;
+#pragma unroll
+            for (int x = 0; x < QC; x += 16) {
+                uint32_t v[16];
+                tmem_ld16(sh.tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(c * QC + x), v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                for (int j = 0; j < 4; ++j)                           // chunk k of a row at chunk k ^ (row & (CH - 1)): no bank conflicts
+                    *reinterpret_cast<uint4 *>(dst + (((x / 4 + j) ^ (lane & (CH - 1))) << 4)) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            }
+        }
+    }
+    cl.sync();
+    if (warp >= 2) {
+        const int parts = (t.kbn + per - 1) / per;                    // ranks past these had no k blocks
+        const int row = t.t0 + q * 32 + lane;
+#pragma unroll
+        for (int x = hf * 16; x < QC; x += 32) {
+            uint32_t own[16];
+            tmem_ld16(sh.tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(rank * QC + x), own);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            float sum[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) sum[j] = 0.f;
+            for (int r = 0; r < parts; ++r) {
+                const unsigned char *src = sh.smem + (r < rank ? r : r - 1) * PART + (q * 32 + lane) * QC * 4;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    float4 v;
+                    if (r == rank) v = make_float4(__uint_as_float(own[4 * j]), __uint_as_float(own[4 * j + 1]), __uint_as_float(own[4 * j + 2]), __uint_as_float(own[4 * j + 3]));
+                    else v = *reinterpret_cast<const float4 *>(src + (((x / 4 + j) ^ (lane & (CH - 1))) << 4));
+                    sum[4 * j] += v.x; sum[4 * j + 1] += v.y; sum[4 * j + 2] += v.z; sum[4 * j + 3] += v.w;
+                }
+            }
+            const int col = t.n0 + rank * QC + x;
+            if (row >= a.T || col >= a.N) continue;
+            const long long at = t.c_off + (long long)row * a.ldc + col;
+            if (a.C32 && col + 16 <= a.N && ((a.ldc | col) & 3) == 0 && (t.c_off & 3) == 0) {
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4 *>(a.C32 + at + j) = make_float4(sum[j], sum[j + 1], sum[j + 2], sum[j + 3]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    if (col + j >= a.N) break;
+                    if (a.C32) a.C32[at + j] = sum[j];
+                    else a.C16[at + j] = __float2bfloat16(sum[j]);
+                }
+            }
+        }
+    }
+    tc_teardown(sh, warp);
+}
+
+// ------------------------------------------------------------------------------------------------------------------
 // The pair form of the dense kernel: two CTAs of a cluster (two neighbouring SMs) compute one 256 x 256 output tile with
 // tcgen05.mma.cta_group::2.  Each CTA loads its own 128 rows of A and ONE HALF of the tile's W rows (128 of 256) per k
 // block - 32 KB for 128 x 256 x 64 multiply-adds per SM, where the single-CTA forms need 48 KB (128 x 256 tile) or 64 KB
@@ -601,17 +715,71 @@ static int g_wide_min_n = 1024;          // products at least this wide use the 
 static int g_pair_min_n = 1024;          // products at least this wide (and 256 rows tall) use CTA pairs (0: never)
 static int g_stage_local = 1;            // 1: fp32 output of the wide and pair forms also leaves through the staging buffers
 
+// How many CTAs share a tile: of products of up to 256 rows, whose `tiles` tiles per 128 rows leave most SMs idle (1: none; every
+// CTA keeps at least four k blocks).  The number, and with it the order of a result's sum, does not depend on the rows below that
+// line, so that a short chunk and its halves give the same rows.
+constexpr int TC_KS_ROWS = 256;
+static int ksplit_of(int T, long long tiles, int kblocks) {
+    int ks = 1;
+    while (T <= TC_KS_ROWS && ks < 8 && tiles * ks * 2 <= NUM_SMS && kblocks >= 8 * ks) ks *= 2;
+    return ks;
+}
+template <int KS>
+static int launch_ksplit_of(const CUtensorMap &mA, const CUtensorMap &mW, GemmTcArgs &a, cudaStream_t s) {
+    constexpr int smem = tc_smem_bytes<TC_BN, TC_KS_STAGES>();
+    static bool done[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    if (!done[dev]) {
+        if (cudaFuncSetAttribute(gemm_tc_ksplit_kernel<KS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -3;
+        done[dev] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(a.total * KS));
+    cfg.blockDim = dim3(320);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = KS;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, gemm_tc_ksplit_kernel<KS>, mA, mW, a) == cudaSuccess ? 0 : -2;
+}
+static int launch_ksplit(int ks, const CUtensorMap &mA, const CUtensorMap &mW, GemmTcArgs &a, cudaStream_t s) {
+    if (ks == 2) return launch_ksplit_of<2>(mA, mW, a, s);
+    if (ks == 4) return launch_ksplit_of<4>(mA, mW, a, s);
+    return launch_ksplit_of<8>(mA, mW, a, s);
+}
+
 static int gemm_plain(GemmTcArgs &a, const void *A, const void *W, void *C, int T, int N, int K, int lda, int ldw, int ldc,
                       int out_bf16, cudaStream_t s) {
     if ((K & 7) || (lda & 7) || (ldw & 7) || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return -1;
-    // wide tiles pay when there are enough of them to fill the SMs and the last column tile is not mostly padding
     const int tiles_t = (T + TC_BM - 1) / TC_BM;
-    const bool wide = g_wide_min_n > 0 && N >= g_wide_min_n && (N % TC_WIDE_BN == 0 || N % TC_WIDE_BN > TC_BN) &&
-                      tiles_t * ((N + TC_WIDE_BN - 1) / TC_WIDE_BN) >= NUM_SMS / 2;
-    // pairs pay when the padding of the 256 x 256 tiles stays under ~6 % of the work and there are tiles for every pair of SMs
-    const long long pad_t = (long long)((T + TC_PAIR_BM - 1) / TC_PAIR_BM) * TC_PAIR_BM, pad_n = (long long)((N + TC_PAIR_BN - 1) / TC_PAIR_BN) * TC_PAIR_BN;
-    const bool pair = g_pair_min_n > 0 && N >= g_pair_min_n && T >= TC_PAIR_BM && pad_t * pad_n * 100 <= (long long)T * N * 106 &&
-                      (pad_t / TC_PAIR_BM) * (pad_n / TC_PAIR_BN) >= NUM_SMS / 4;
+    const int ks = a.epi.mode == 0 && !a.wait.flags && T <= TC_KS_ROWS ? ksplit_of(T, (N + TC_BN - 1) / TC_BN, (K + TC_BK - 1) / TC_BK) : 1;
+    if (ks > 1) {
+        CUtensorMap mA, mW;
+        if (!make_map(&mA, A, T, K, lda, TC_BM) || !make_map(&mW, W, N, K, ldw, TC_BN)) return -3;
+        a.C32 = out_bf16 ? nullptr : (float *)C;
+        a.C16 = out_bf16 ? (bf16 *)C : nullptr;
+        a.T = T; a.N = N; a.K = K; a.ldc = ldc; a.err = g_err_ptr; a.tiles = nullptr;
+        a.tiles_t = tiles_t; a.tiles_n = (N + TC_BN - 1) / TC_BN; a.total = a.tiles_t * a.tiles_n;
+        a.ksplit = 1; a.kb_per = 0; a.c_split = 0;
+        return launch_ksplit(ks, mA, mW, a, s);
+    }
+    // The form with the least time by what its tiles cost per 64 k values, measured in us: a 256 x 256 tile of a pair of SMs 0.45 (waves
+    // over 74 pairs), a 128 x 256 tile of an SM 0.55, a 128 x 128 tile 0.31 (bound by the 32 KB it loads; two share an SM and
+    // take twice that).  777 x 16480 x 2560: single CTAs 86 us, pairs (a third of their tiles' area padding) 73; 520 x 12800 x
+    // 2560: wide 44, pairs 54 (a third wave for 2 of 150 tiles).  A last column tile that is mostly padding rules the wide form out.
+    auto waves = [](long long tiles, int at_once) { return (double)((tiles + at_once - 1) / at_once); };
+    const long long n_one = (long long)tiles_t * ((N + TC_BN - 1) / TC_BN), n_wide = (long long)tiles_t * ((N + TC_WIDE_BN - 1) / TC_WIDE_BN);
+    const long long n_pair = (long long)((T + TC_PAIR_BM - 1) / TC_PAIR_BM) * ((N + TC_PAIR_BN - 1) / TC_PAIR_BN);
+    const double c_one = 0.31 * waves(n_one, NUM_SMS), c_wide = 0.55 * waves(n_wide, NUM_SMS), c_pair = 0.45 * waves(n_pair, NUM_SMS / 2);
+    const bool wide_ok = g_wide_min_n > 0 && N >= g_wide_min_n && (N % TC_WIDE_BN == 0 || N % TC_WIDE_BN > TC_BN);
+    const bool pair = g_pair_min_n > 0 && N >= g_pair_min_n && T > TC_BM && c_pair < c_one && (!wide_ok || c_pair < c_wide);
+    const bool wide = !pair && wide_ok && n_wide >= NUM_SMS / 2 && c_wide < c_one;
     if (pair) {
         CUtensorMap mA, mW;
         if (!make_map(&mA, A, T, K, lda, TC_BM) || !make_map(&mW, W, N, K, ldw, TC_PAIR_BN / 2)) return -3;
@@ -763,6 +931,8 @@ QW_API int qwk_gemm_bf16_tc_splitk(const void *A, const void *W, float *C, int T
     if (a.ksplit != ksplit) return -1;
     a.c_split = c_split;
     a.total = a.tiles_t * a.tiles_n * a.ksplit;
+    const int ks = ksplit_of(T, (long long)a.tiles_n * a.ksplit, a.kb_per);
+    if (ks > 1) return launch_ksplit(ks, mA, mW, a, s);
     if (!configure_once(0)) return -3;
     gemm_tc_kernel<TC_BN, TC_STAGES><<<persistent_grid(a.total), 320, TC_SMEM, s>>>(mA, mW, a);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
