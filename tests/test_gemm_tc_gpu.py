@@ -227,3 +227,25 @@ def test_gemm_tc_pair_form_matches_fp32(pair_form, T, N, K, out_dtype):
 
 def test_gemm_tc_pair_form_reduce_scatter_on_emulated_ranks(pair_form):
     test_gemm_tc_reduce_scatter_epilogue_on_emulated_ranks(1024, 2048, 256)
+
+
+@pytest.mark.parametrize("T,SH,R", [(1, 32, 32), (100, 2560, 320), (129, 264, 40), (1500, 2560, 320), (300, 8, 320)])
+def test_mixer_up_projection_with_the_mean_in_its_epilogue(T, SH, R):
+    """Gate product, sigmoid, weighted mean over the streams in one kernel, against 64 bits (bf16 output: 2^-9, and fp32 logits) and
+    with guard columns and rows."""
+    import ctypes as C
+    from qwb200.ops import lib as qlib
+    L = qlib.load(True)
+    g = torch.Generator(device="cuda").manual_seed(T + SH)
+    u = torch.randn(T, R, generator=g, device="cuda").to(torch.bfloat16)
+    W = (torch.randn(4 * SH, R, generator=g, device="cuda") * 0.1).to(torch.bfloat16)
+    xn = torch.randn(T, 4, SH, generator=g, device="cuda").to(torch.bfloat16)
+    out = torch.full((T + 2, SH + 8), 768.0, dtype=torch.bfloat16, device="cuda")
+    P = lambda t: C.c_void_p(t.data_ptr())
+    rc = L.qwk_gemm_mix_tc(P(u), P(W), P(xn), SH, P(out), SH + 8, T, R, R, R, C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    torch.cuda.synchronize()
+    gate = torch.sigmoid((u.double() @ W.double().T).view(T, SH, 4).permute(0, 2, 1))
+    ref = (gate * xn.double()).mean(1)
+    assert torch.all(out[T:].float() == 768.0) and torch.all(out[:, SH:].float() == 768.0)
+    assert float((out[:T, :SH].double() - ref).norm() / ref.norm()) < 2 ** -8

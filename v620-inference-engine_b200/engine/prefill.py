@@ -73,7 +73,7 @@ class Prefiller:
         one = not self.tp
         self.b = {
             "X": z((T, c.hc, sc.sh), f32), "xn": z((T, c.hc * sc.sh), bf), "d": z((self.hc_ksplit, T, self.hc_ld), f32) if one else None,
-            "u": z((T, c.hc_rank), bf), "inj_a": z((T, c.hc), f32), "inj_b": z((T, c.hc), f32), "g": z((T, c.hc * sc.sh), f32),
+            "u": z((T, c.hc_rank), bf), "inj_a": z((T, c.hc), f32), "inj_b": z((T, c.hc), f32), "g": None if one else z((T, c.hc * sc.sh), f32),
             "bin": z((T, c.hidden), bf) if one else None,
             "proj": z((T, self.proj_ld), f32), "o": z((T, self.o_ld), bf),
             "out_a": z((T, c.hidden), f32) if one else None, "out_b": z((T, c.hidden if one else sc.sh), f32),
@@ -292,8 +292,8 @@ class Prefiller:
                                            self.hc_ld, ks, self.T * self.hc_ld, s), "hc_down")
         self._ck(L.qwk_hc_mid_T(_p(b["d"]), self.hc_ld, c.hc_rank, n_inj, c.hc, _p(b["u"]), _p(inj_out), T, ks,
                                 self.T * self.hc_ld, s), "hc_mid")
-        self.gemm(b["u"][:T], hc["Wu"].data_ptr(), c.hch, c.hc_rank, b["g"][:T])
-        self._ck(L.qwk_hc_mix_T(_p(b["g"]), _p(b["xn"]), sc.sh, _p(b["bin"]), c.hidden, T, s), "hc_mix")
+        self._ck(L.qwk_gemm_mix_tc(_p(b["u"]), P(hc["Wu"].data_ptr()), _p(b["xn"]), sc.sh, _p(b["bin"]), c.hidden, T, c.hc_rank,
+                                   c.hc_rank, c.hc_rank, s), "hc_mix")
 
     # ---- one chunk, scheduled from Python (one GPU, one lane)
     @torch.no_grad()

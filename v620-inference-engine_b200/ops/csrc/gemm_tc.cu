@@ -61,6 +61,10 @@ struct GemmTcArgs {
     // epilogue sends fp32 tiles to other ranks' receive buffers instead of (mode != 0) storing them to C
     TpWait wait;
     TpEpilogue epi;
+    // mixer form: output columns 4 c + s are the gate logits of stream s of column c; the epilogue turns them into the block
+    // input C16[row][c] = mean over s of sigmoid(logit) * mix_xn[row][s][c] (rows of 4 * mix_cols) and no logit is stored
+    const bf16 *mix_xn;
+    int mix_cols;
 };
 
 struct TileAt {
@@ -99,9 +103,34 @@ __device__ __forceinline__ bool tile_at(const GemmTcArgs &a, int id, TileAt &t) 
     return true;
 }
 
+// Sigmoid for the mixer epilogue, which is what bounds that product: 2 ulp instead of 1 (a division instruction sequence of a dozen
+// less per value), under a rounding of the result to bf16.
+__device__ __forceinline__ float mix_gate(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+
 // One 32-column piece of an accumulator row -> C.
 __device__ __forceinline__ void store_piece(const GemmTcArgs &a, long long c_off, int row, int col0, const uint32_t (&v)[32]) {
     const int nmax = a.N - col0;
+    if (a.mix_xn) {
+        if (nmax < 32) return;                          // mix_cols is a multiple of 8: pieces are whole
+        const bf16 *x = a.mix_xn + (long long)row * 4 * a.mix_cols + (col0 >> 2);
+        uint4 xv[4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) xv[s] = __ldg(reinterpret_cast<const uint4 *>(x + (long long)s * a.mix_cols));
+        uint32_t o[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {                   // columns 2 j, 2 j + 1 of the piece
+            float lo = 0.f, hi = 0.f;
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                const uint32_t w = j == 0 ? xv[s].x : j == 1 ? xv[s].y : j == 2 ? xv[s].z : xv[s].w;
+                lo = fmaf(mix_gate(__uint_as_float(v[8 * j + s])), bf16_lo(w), lo);
+                hi = fmaf(mix_gate(__uint_as_float(v[8 * j + 4 + s])), bf16_hi(w), hi);
+            }
+            o[j] = pack_bf16(lo * 0.25f, hi * 0.25f);
+        }
+        *reinterpret_cast<uint4 *>(a.C16 + (long long)row * a.ldc + (col0 >> 2)) = make_uint4(o[0], o[1], o[2], o[3]);
+        return;
+    }
     if (a.epi.mode) {
         // fp32 pieces to the receive buffers: every rank's (parts of an all-reduce) or the column owner's (reduce-scatter)
         const int owner = a.epi.mode == 2 ? col0 / a.epi.cols_per_rank : 0;
@@ -758,7 +787,7 @@ static int gemm_plain(GemmTcArgs &a, const void *A, const void *W, void *C, int 
                       int out_bf16, cudaStream_t s) {
     if ((K & 7) || (lda & 7) || (ldw & 7) || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return -1;
     const int tiles_t = (T + TC_BM - 1) / TC_BM;
-    const int ks = a.epi.mode == 0 && !a.wait.flags && T <= TC_KS_ROWS ? ksplit_of(T, (N + TC_BN - 1) / TC_BN, (K + TC_BK - 1) / TC_BK) : 1;
+    const int ks = a.epi.mode == 0 && !a.wait.flags && !a.mix_xn && T <= TC_KS_ROWS ? ksplit_of(T, (N + TC_BN - 1) / TC_BN, (K + TC_BK - 1) / TC_BK) : 1;
     if (ks > 1) {
         CUtensorMap mA, mW;
         if (!make_map(&mA, A, T, K, lda, TC_BM) || !make_map(&mW, W, N, K, ldw, TC_BN)) return -3;
@@ -778,7 +807,7 @@ static int gemm_plain(GemmTcArgs &a, const void *A, const void *W, void *C, int 
     const long long n_pair = (long long)((T + TC_PAIR_BM - 1) / TC_PAIR_BM) * ((N + TC_PAIR_BN - 1) / TC_PAIR_BN);
     const double c_one = 0.31 * waves(n_one, NUM_SMS), c_wide = 0.55 * waves(n_wide, NUM_SMS), c_pair = 0.45 * waves(n_pair, NUM_SMS / 2);
     const bool wide_ok = g_wide_min_n > 0 && N >= g_wide_min_n && (N % TC_WIDE_BN == 0 || N % TC_WIDE_BN > TC_BN);
-    const bool pair = g_pair_min_n > 0 && N >= g_pair_min_n && T > TC_BM && c_pair < c_one && (!wide_ok || c_pair < c_wide);
+    const bool pair = g_pair_min_n > 0 && N >= g_pair_min_n && T > TC_BM && !a.mix_xn && c_pair < c_one && (!wide_ok || c_pair < c_wide);
     const bool wide = !pair && wide_ok && n_wide >= NUM_SMS / 2 && c_wide < c_one;
     if (pair) {
         CUtensorMap mA, mW;
@@ -888,6 +917,20 @@ QW_API int qwk_gemm_bf16_tc_tp(void *tp_, const void *A, const void *W, void *C,
         a.epi.sig = tp_make_signal(tp, epi_kind, 1);
     }
     return gemm_plain(a, A, W, C, T, N, K, lda, ldw, ldc, out_bf16, s);
+}
+
+// The mixer's up projection with the block input formed in the epilogue: A bf16 [T][lda] (the activated low-rank vector), W bf16
+// [4 SH][ldw] (row 4 c + s: gate of stream s, column c), xn bf16 [T][4][SH]; out bf16 [T][ld_out]: mean over the streams of
+// sigmoid(A . W^T) * xn.  The logits (fp32, 4 SH a row) are never stored: as a product and a kernel that read them back
+// 118 us at 4096 x 2560 and 41 at 1021, here 76 and 28 (wide tiles; in pairs 79 and 29).  SH a multiple of 8.
+QW_API int qwk_gemm_mix_tc(const void *A, const void *W, const void *xn, int SH, void *out, int ld_out, int T, int K, int lda, int ldw,
+                           cudaStream_t s) {
+    if (T <= 0) return 0;
+    if ((SH & 7) || (ld_out & 7) || ((uintptr_t)xn & 15) || ((uintptr_t)out & 15)) return -1;
+    GemmTcArgs a{};
+    a.mix_xn = (const bf16 *)xn;
+    a.mix_cols = SH;
+    return gemm_plain(a, A, W, out, T, 4 * SH, K, lda, ldw, ld_out, 1, s);
 }
 
 // Grouped form for expert-sorted rows: A bf16 [rows][lda] holds the rows of group after group, W bf16

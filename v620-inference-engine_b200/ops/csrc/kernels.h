@@ -25,6 +25,7 @@ int qwk_gemm_tc_stage_local(int on);
 int qwk_gemm_tc_pair_min_n(int min_n);
 int qwk_gemm_bf16_tc(const void *A, const void *W, void *C, int T, int N, int K, int lda, int ldw, int ldc, int out_bf16, cudaStream_t s);
 int qwk_gemm_bf16_tc_tp(void *tp_, const void *A, const void *W, void *C, int T, int N, int K, int lda, int ldw, int ldc, int out_bf16, int wait_kind, int epi_mode, int epi_kind, int ld_epi, cudaStream_t s);
+int qwk_gemm_mix_tc(const void *A, const void *W, const void *xn, int SH, void *out, int ld_out, int T, int K, int lda, int ldw, cudaStream_t s);
 int qwk_gemm_bf16_tc_grouped(const void *A, const void *W, void *C, const void *tiles, int max_tiles, int rows, long long w_rows, int Nw, int K, int lda, int ldw, int ldc, int out_bf16, cudaStream_t s);
 int qwk_gemm_bf16_tc_splitk(const void *A, const void *W, float *C, int T, int N, int K, int lda, int ldw, int ldc, int ksplit, long long c_split, cudaStream_t s);
 
@@ -78,7 +79,6 @@ int qwk_ple_apply(const float *kv, int ld_kv, const float *red, int ld_red, cons
 // prefill.cu
 int qwk_hc_prenorm_T(float *X, const float *pend, int ld_pend, const float *inj, const float *w1, int SH, int hc, float eps, void *xn, int T, cudaStream_t s);
 int qwk_hc_mid_T(const float *d, int ld_d, int R, int n_inj, int hc, void *u, float *inj, int T, int nsplit, long long split_stride, cudaStream_t s);
-int qwk_hc_mix_T(const float *g, const void *xn, int SH, void *bin, int ld_bin, int T, cudaStream_t s);
 int qwk_q4_dequant(const void *w, const void *scale, long long rows, int K, void *out, cudaStream_t s);
 int qwk_swiglu_T(const void *h13, int F, void *h, long long P, cudaStream_t s);
 int qwk_moe_combine_T(const float *y, int ld_y, const int *inv, const float *pair_w, int top_k, const float *shared, int H, float *out, int T, cudaStream_t s);

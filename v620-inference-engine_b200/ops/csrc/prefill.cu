@@ -66,26 +66,6 @@ __global__ void hc_mid_T_kernel(const float *d, int ld_d, int R, int n_inj, int 
     else inj[t * n_inj + (j - R)] = v;
 }
 
-// g [T][SH*hc] fp32 with columns ordered (c, s); bin[t][c] = mean_s sigmoid(g[t][c][s]) * xn[t][s][c].  hc == 4, SH even,
-// ld_bin even.  One thread per two neighbouring columns.
-__global__ void hc_mix_T_kernel(const float *g, const bf16 *xn, int SH, bf16 *bin, int ld_bin, long long total2) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total2) return;
-    const int h2 = SH >> 1;
-    const long long t = i / h2;
-    const int c = (int)(i - t * h2) * 2;
-    const float4 g0 = *reinterpret_cast<const float4 *>(g + (t * SH + c) * 4);
-    const float4 g1 = *reinterpret_cast<const float4 *>(g + (t * SH + c + 1) * 4);
-    const bf16 *x = xn + t * 4 * SH + c;
-    const float2 x0 = __bfloat1622float2(*reinterpret_cast<const bf162 *>(x));
-    const float2 x1 = __bfloat1622float2(*reinterpret_cast<const bf162 *>(x + SH));
-    const float2 x2 = __bfloat1622float2(*reinterpret_cast<const bf162 *>(x + 2 * SH));
-    const float2 x3 = __bfloat1622float2(*reinterpret_cast<const bf162 *>(x + 3 * SH));
-    const float v0 = sigmoidf_(g0.x) * x0.x + sigmoidf_(g0.y) * x1.x + sigmoidf_(g0.z) * x2.x + sigmoidf_(g0.w) * x3.x;
-    const float v1 = sigmoidf_(g1.x) * x0.y + sigmoidf_(g1.y) * x1.y + sigmoidf_(g1.z) * x2.y + sigmoidf_(g1.w) * x3.y;
-    *reinterpret_cast<bf162 *>(bin + t * ld_bin + c) = __floats2bfloat162_rn(v0 * 0.25f, v1 * 0.25f);
-}
-
 // q4 (engine order) rows -> bf16 rows.  One thread per word (8 values).
 __global__ void q4_dequant_kernel(const uint32_t *w, const bf16 *scale, int K, bf16 *out, long long words) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -217,12 +197,6 @@ QW_API int qwk_hc_mid_T(const float *d, int ld_d, int R, int n_inj, int hc, void
     const long long total = (long long)T * (R + n_inj);
     hc_mid_T_kernel<<<blocks_for(total, 256), 256, 0, s>>>(d, ld_d, R, n_inj, hc, (bf16 *)u, inj, total, nsplit < 1 ? 1 : nsplit,
                                                            split_stride);
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
-}
-QW_API int qwk_hc_mix_T(const float *g, const void *xn, int SH, void *bin, int ld_bin, int T, cudaStream_t s) {
-    if ((SH & 1) || (ld_bin & 1)) return -1;
-    const long long total = (long long)T * (SH >> 1);
-    hc_mix_T_kernel<<<blocks_for(total, 256), 256, 0, s>>>(g, (const bf16 *)xn, SH, (bf16 *)bin, ld_bin, total);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 QW_API int qwk_q4_dequant(const void *w, const void *scale, long long rows, int K, void *out, cudaStream_t s) {

@@ -157,13 +157,7 @@ struct Builder {
             add([=](PCtx &c) {
                 const Lane &L = c.lane[l];
                 const QwPrefillBufs &b = *c.b;
-                PF_TRY(1, qwk_gemm_bf16_tc(h_at(b.u, L.r0, R), hc_of(c).Wu, f_at(b.g, L.r0, hc * SH), L.n, hc * SH, R, R, R, hc * SH, 0, L.s));
-            });
-            cur_cat = CAT_GLUE_MIX;
-            add([=](PCtx &c) {
-                const Lane &L = c.lane[l];
-                const QwPrefillBufs &b = *c.b;
-                PF_TRY(1, qwk_hc_mix_T(f_at(b.g, L.r0, hc * SH), h_at(b.xn, L.r0, hc * SH), SH, h_at(b.bin, L.r0, H), H, L.n, L.s));
+                PF_TRY(1, qwk_gemm_mix_tc(h_at(b.u, L.r0, R), hc_of(c).Wu, h_at(b.xn, L.r0, hc * SH), SH, h_at(b.bin, L.r0, H), H, L.n, R, R, R, L.s));
             });
             return;
         }
