@@ -1,0 +1,44 @@
+"""Rules that the kernels' sources keep and that no run can show to be broken without harm: read from the text, on the CPU."""
+import glob
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "v620-inference-engine_b200", "ops", "csrc")
+
+
+def _text(path):
+    """Source without comments."""
+    return re.sub(r"//[^\n]*|/\*.*?\*/", "", open(path).read(), flags=re.S)
+
+
+def _kernels(path):
+    """(name, body) of every kernel of a file; a body ends where its braces do."""
+    t = _text(path)
+    for m in re.finditer(r"__global__[^;{]*?(\w+)\(", t):
+        at = depth = t.index("{", t.index(")", m.end()))
+        end, depth = at, 0
+        while True:
+            depth += {"{": 1, "}": -1}.get(t[end], 0)
+            end += 1
+            if depth == 0:
+                break
+        yield m.group(1), t[at:end]
+
+
+def _sources():
+    return sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh")))
+
+
+def test_a_cluster_meets_before_one_block_reaches_into_another():
+    """Shared memory of another block of the cluster may be used only when that block has begun to run."""
+    seen = 0
+    for path in _sources():
+        for name, body in _kernels(path):
+            first = body.find("map_shared_rank")
+            if first < 0:
+                continue
+            seen += 1
+            handle = re.search(r"(\w+)\s*=\s*cg::this_cluster\(\)|cg::cluster_group (\w+)", body)
+            sync = body.find(next(g for g in handle.groups() if g) + ".sync()")
+            assert 0 <= sync < first, (os.path.basename(path), name)
+    assert seen >= 3

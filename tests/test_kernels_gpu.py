@@ -417,3 +417,13 @@ def test_gdn_conv_of_a_prefill_chunk_matches_the_step_kernel(M, base):
     for x, y in zip(whole[:3], parts[:3]):
         assert torch.allclose(x, y, rtol=1e-5, atol=1e-6)
     assert torch.equal(whole[3], parts[3])
+
+
+def test_row_reduce_many_short_rows():
+    """Thousands of clusters in flight whose blocks have next to nothing to do before they hand over their parts."""
+    from qwb200.ops import kernels as K_
+    x = torch.randn(6000, 5, generator=torch.Generator(device="cuda").manual_seed(3), device=_dev())
+    for _ in range(5):
+        val, idx, mx, sm = K_.row_reduce(x)
+        assert torch.equal(val, x.max(1).values) and torch.equal(idx.long(), x.argmax(1)) and torch.equal(mx, val)
+        assert torch.allclose(torch.log(sm.double()) + mx.double(), torch.logsumexp(x.double(), 1), atol=1e-5)

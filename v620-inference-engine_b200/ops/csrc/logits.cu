@@ -20,8 +20,9 @@ __global__ void __cluster_dims__(RR_CTAS, 1, 1) __launch_bounds__(RR_THREADS) ro
     __shared__ int si[32];
     __shared__ float part_max[RR_CTAS], part_sum[RR_CTAS];          // rank 0's: every CTA's (max, sum, index)
     __shared__ int part_idx[RR_CTAS];
-    pdl_wait();
     cg::cluster_group cl = cg::this_cluster();
+    cl.sync();          // every CTA of the cluster runs: rank 0's memory may be written (before the wait for the logits, which is longer)
+    pdl_wait();
     const int m = blockIdx.y, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float *l = logits + (long long)m * ld;
     const int per = ((V + RR_CTAS - 1) / RR_CTAS + 3) & ~3, c0 = blockIdx.x * per, c1 = min(V, c0 + per);
