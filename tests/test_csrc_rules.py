@@ -42,3 +42,20 @@ def test_a_cluster_meets_before_one_block_reaches_into_another():
             sync = body.find(next(g for g in handle.groups() if g) + ".sync()")
             assert 0 <= sync < first, (os.path.basename(path), name)
     assert seen >= 3
+
+
+def test_waits_before_warp_wide_instructions_are_voted_on():
+    """Lanes come out of a polling loop one by one and may even disagree on its outcome; every wait is one verdict for the warp, and
+    tensor memory is read only after the warp has come together."""
+    for path in _sources():
+        t = _text(path)
+        calls = re.findall(r"\b(?:mbar_wait|mg_wait)\((?!uint64_t)", t)
+        inside = re.findall(r"__all_sync\(0xffffffffu, (?:mbar_wait|mg_wait)\(", t)
+        assert len(calls) == len(inside), os.path.basename(path)
+        for fn in re.findall(r"__device__ __forceinline__ void tmem_ld\w+\(uint32_t taddr[^{]*\{([^}]*)", t):
+            assert fn.lstrip().startswith(("__syncwarp();", "tmem_ld")), os.path.basename(path)
+    # no lane skips to the next warp-wide load by itself: a lane's row or column only guards its stores
+    for name in ("moe_tc.cu", "vit_attn.cu", "gemm_tc.cu"):
+        t = _text(os.path.join(CSRC, name))
+        for m in re.finditer(r"tcgen05\.wait::ld\.sync\.aligned[^\n]*\n([^\n]*)", t):
+            assert not re.search(r"if \((?:row|col)\b.*\) continue;", m.group(1)), (name, m.group(1))

@@ -257,7 +257,7 @@ __device__ __forceinline__ void epilogue_role(const GemmTcArgs &a, uint32_t tmem
         TileAt t;
         if (!tile_at<BN>(a, id, t)) continue;
         const int b = j & 1;
-        if (!mbar_wait(done + b, (unsigned)(j >> 1) & 1u, a.err)) return;
+        if (!mbar_wait_warp(done + b, (unsigned)(j >> 1) & 1u, a.err)) return;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int row = t.t0 + q * 32 + lane;
         const bool row_ok = row < a.T && q * 32 + lane < t.rows_valid;
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(320, 1) gemm_tc_ksplit_kernel(const __grid_con
         }
         if (ok && k1 > k0 && elect_one()) umma_commit(sh.done);
     } else if (k1 > k0) {
-        mbar_wait(sh.done, 0u, a.err);
+        mbar_wait_warp(sh.done, 0u, a.err);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
     __syncwarp();
@@ -673,7 +673,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1) gemm_tc_pair
         for (int id = cluster_id; id < a.total; id += n_clusters) {
             const PairTile t = pair_tile_at(a, id, rank);
             const int b = j & 1;
-            if (!mbar_wait(done + b, (unsigned)(j >> 1) & 1u, a.err)) break;
+            if (!mbar_wait_warp(done + b, (unsigned)(j >> 1) & 1u, a.err)) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const int row = t.t0 + q * 32 + lane;
             const bool row_ok = row < a.T;

@@ -56,6 +56,7 @@ struct MgSlots {
 };
 
 // Eight columns at a time: the packed pairs of two q4 words go out as they are formed, so no 32-register block is assembled.
+// The caller has just voted on a wait: its warp is whole.
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0,%1,%2,%3,%4,%5,%6,%7};"
                  ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(taddr)
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) moe_tc_kernel(const __grid_cons
                     const uint32_t sc_bits = (uint32_t)ring[i] * 0x10001u;
                     const bf162 sc2 = *reinterpret_cast<const bf162 *>(&sc_bits);
                     if (kb + 2 * MG_AHEAD < kblocks) ring[i] = __ldg(sp + kb + 2 * MG_AHEAD);
-                    if (!mg_wait(full + ws, w_phase, a.err)) { ok = false; break; }
+                    if (!mg_wait_warp(full + ws, w_phase, a.err)) { ok = false; break; }
                     uint32_t words[16];
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
@@ -260,7 +261,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) moe_tc_kernel(const __grid_cons
                                 const bf162 v = __hmul2(__hsub2(*reinterpret_cast<bf162 *>(&bits), off2), sc2);
                                 o[c][j] = *reinterpret_cast<const uint32_t *>(&v);
                             }
-                        if (n && !mg_wait(a_empty2 + half, (n - 1) & 1u, a.err)) { ok = false; break; }
+                        if (n && !mg_wait_warp(a_empty2 + half, (n - 1) & 1u, a.err)) { ok = false; break; }
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                         for (int c = 0; c < 4; ++c) tmem_st8(lane_base + half * 64 + c * 8, o[c]);
@@ -288,7 +289,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) moe_tc_kernel(const __grid_cons
             const int rows = w.tl.y, N = (rows + 15) & ~15;
             const bool big = N > 64;
             const int s = big ? 0 : sl.next;
-            if (!mg_wait(done + s, sl.committed[s] & 1u, a.err)) { ok = false; break; }
+            if (!mg_wait_warp(done + s, sl.committed[s] & 1u, a.err)) { ok = false; break; }
             ++sl.committed[s];
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t d0 = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(s * 128), d1 = d0 + (big ? 128u : 64u);
@@ -301,11 +302,11 @@ __global__ void __launch_bounds__(MG_THREADS, 1) moe_tc_kernel(const __grid_cons
                 const int n = rows - c0;                 // rows of this piece that exist (16 or more: all)
                 const long long at = (long long)(w.tl.x + c0) * a.ldc + col;
                 if (SWIGLU) {
-                    if (col >= a.Nw) continue;
                     bf16 *p = a.C16 + at;
+                    const int nc = col < a.Nw ? n : 0;
 #pragma unroll
                     for (int j = 0; j < 16; ++j, p += a.ldc)
-                        if (j < n) *p = __float2bfloat16(siluf_(__uint_as_float(u[j])) * __uint_as_float(v[j]));
+                        if (j < nc) *p = __float2bfloat16(siluf_(__uint_as_float(u[j])) * __uint_as_float(v[j]));
                 } else if (a.C32 && n >= 16 && col + 128 < a.Nw) {
                     float *p = a.C32 + at;
 #pragma unroll

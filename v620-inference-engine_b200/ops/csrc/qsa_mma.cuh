@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(128, 3) qsa_attend_mma_kernel(QsaAttendArgs a,
         for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
     float mx0 = -INFINITY, mx1 = -INFINITY, l0 = 0.f, l1 = 0.f;
     for (int tile = 0; tile < ntiles; ++tile) {
-        mbar_wait(kbar, (unsigned)tile & 1u, g_err);        // this tile's K rows have landed (bounded; a time-out is recorded)
+        mbar_wait_warp(kbar, (unsigned)tile & 1u, g_err);        // this tile's K rows have landed (bounded; a time-out is recorded)
         // ---- S = Q K^T for this warp's 16 tokens
         float s[2][4];
 #pragma unroll
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(128, 3) qsa_attend_mma_kernel(QsaAttendArgs a,
             acc[n][2] *= c1; acc[n][3] *= c1;
         }
         __syncthreads();         // P visible
-        mbar_wait(vbar, (unsigned)tile & 1u, g_err);        // this tile's V rows have landed
+        mbar_wait_warp(vbar, (unsigned)tile & 1u, g_err);        // this tile's V rows have landed
         // ---- O += P V for this warp's 64 output dims
         {
             const int mid = lane >> 3;

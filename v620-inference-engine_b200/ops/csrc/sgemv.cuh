@@ -154,7 +154,7 @@ __device__ __forceinline__ void sgemv_core(const SGemvArgs &a, unsigned char *sm
         // ---- producer warp: lane r copies row r of each stage
         for (int q = 0; q < total; ++q) {
             const int s = q % a.nstage;
-            if (q >= a.nstage && !mbar_wait(empty + s, (unsigned)(q / a.nstage - 1) & 1u, a.err)) break;
+            if (q >= a.nstage && !mbar_wait_warp(empty + s, (unsigned)(q / a.nstage - 1) & 1u, a.err)) break;
             const int kp = q % a.P, i = (q / a.P) % cnt;
             const int it = (int)blockIdx.x + i * (int)gridDim.x;
             const int split = it / tps, row0 = (it - split * tps) * SG_TILE;
@@ -193,7 +193,7 @@ __device__ __forceinline__ void sgemv_core(const SGemvArgs &a, unsigned char *sm
             for (int t = 0; t < NT; ++t) c[t][0] = c[t][1] = c[t][2] = c[t][3] = 0.f;
             for (int kp = 0; kp < a.P; ++kp, ++q) {
                 const int s = q % a.nstage;
-                ok = mbar_wait(full + s, (unsigned)(q / a.nstage) & 1u, a.err);
+                ok = mbar_wait_warp(full + s, (unsigned)(q / a.nstage) & 1u, a.err);
                 if (!ok) break;
                 const uint32_t tb = st_base + (unsigned)s * stage_bytes;
                 for (int st = warp; st < steps; st += 8) {

@@ -54,5 +54,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, unsigned parity, ErrorW
     report(err, ERR_WAIT_TIMEOUT, __LINE__);
     return false;
 }
+// The same for a whole warp: one verdict for all lanes.  Lanes leave the polling loop one by one, and a wait may run out in some of
+// them only; the vote brings them together again before an instruction that needs the warp whole (tcgen05.ld / st, ldmatrix, mma).
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, unsigned parity, ErrorWord *err) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)) != 0;
+}
 
 }  // namespace qw

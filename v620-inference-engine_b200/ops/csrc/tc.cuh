@@ -45,10 +45,6 @@ __device__ __forceinline__ bool elect_one() {
     return p != 0;
 }
 __device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
-// mbar_wait for a whole warp: one verdict for all lanes, so that the warp stays together when a wait runs out.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, unsigned parity, ErrorWord *err) {
-    return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)) != 0;
-}
 
 __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_c, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -88,11 +84,14 @@ static __device__ __noinline__ bool mg_wait_slow(uint64_t *bar, unsigned parity,
 __device__ __forceinline__ bool mg_wait(uint64_t *bar, unsigned parity, ErrorWord *err) {
     return mg_try(bar, parity) || mg_wait_slow(bar, parity, err);
 }
+// One verdict for all lanes (see mbar_wait_warp).
 __device__ __forceinline__ bool mg_wait_warp(uint64_t *bar, unsigned parity, ErrorWord *err) {
     return __all_sync(0xffffffffu, mg_wait(bar, parity, err)) != 0;
 }
 
+// Loads and stores of tensor memory need the warp whole; lanes may have parted at a store that only some of them do.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    __syncwarp();
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
@@ -101,6 +100,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 }
 
 __device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t (&v)[32]) {
+    __syncwarp();
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
         "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
@@ -116,6 +116,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
 }
 
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    __syncwarp();
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};"
                  ::"r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
                    "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(taddr)

@@ -228,10 +228,9 @@ __global__ void __launch_bounds__(VT_THREADS, 1) vit_attn_tc_kernel(const __grid
                 uint32_t v[16];
                 tmem_ld16(obase + c, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (row >= a.L) continue;
 #pragma unroll
                 for (int i = 0; i < 16; i += 8) {
-                    if (c + i >= VT_D) continue;
+                    if (c + i >= VT_D || row >= a.L) continue;
                     uint4 pk;
                     pk.x = pack_bf16(__uint_as_float(v[i]) * r, __uint_as_float(v[i + 1]) * r);
                     pk.y = pack_bf16(__uint_as_float(v[i + 2]) * r, __uint_as_float(v[i + 3]) * r);
