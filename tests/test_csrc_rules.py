@@ -3,6 +3,8 @@ import glob
 import os
 import re
 
+import pytest
+
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "v620-inference-engine_b200", "ops", "csrc")
 
 
@@ -59,3 +61,9 @@ def test_waits_before_warp_wide_instructions_are_voted_on():
         t = _text(os.path.join(CSRC, name))
         for m in re.finditer(r"tcgen05\.wait::ld\.sync\.aligned[^\n]*\n([^\n]*)", t):
             assert not re.search(r"if \((?:row|col)\b.*\) continue;", m.group(1)), (name, m.group(1))
+
+
+@pytest.mark.parametrize("name", ["gemm_tc.cu"])
+def test_divisions_are_rounded_like_any_other_operation(name):
+    """Sigmoids and the like that were formed with a correctly rounded division stay so."""
+    assert "__fdividef" not in _text(os.path.join(CSRC, name))

@@ -103,10 +103,6 @@ __device__ __forceinline__ bool tile_at(const GemmTcArgs &a, int id, TileAt &t) 
     return true;
 }
 
-// Sigmoid for the mixer epilogue, which is what bounds that product: 2 ulp instead of 1 (a division instruction sequence of a dozen
-// less per value), under a rounding of the result to bf16.
-__device__ __forceinline__ float mix_gate(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
-
 // One 32-column piece of an accumulator row -> C.
 __device__ __forceinline__ void store_piece(const GemmTcArgs &a, long long c_off, int row, int col0, const uint32_t (&v)[32]) {
     const int nmax = a.N - col0;
@@ -123,8 +119,8 @@ __device__ __forceinline__ void store_piece(const GemmTcArgs &a, long long c_off
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
                 const uint32_t w = j == 0 ? xv[s].x : j == 1 ? xv[s].y : j == 2 ? xv[s].z : xv[s].w;
-                lo = fmaf(mix_gate(__uint_as_float(v[8 * j + s])), bf16_lo(w), lo);
-                hi = fmaf(mix_gate(__uint_as_float(v[8 * j + 4 + s])), bf16_hi(w), hi);
+                lo = fmaf(sigmoidf_(__uint_as_float(v[8 * j + s])), bf16_lo(w), lo);
+                hi = fmaf(sigmoidf_(__uint_as_float(v[8 * j + 4 + s])), bf16_hi(w), hi);
             }
             o[j] = pack_bf16(lo * 0.25f, hi * 0.25f);
         }
