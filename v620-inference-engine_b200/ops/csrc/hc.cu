@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(HM_THREADS, 2) hc_up_mma_kernel(const float *r
                 if (m >= n) break;
                 const float4 r = *reinterpret_cast<const float4 *>(rs[m]);
                 const float d = fmaf(r.w, v[b][3], fmaf(r.z, v[b][2], fmaf(r.y, v[b][1], r.x * v[b][0])));
-                const float t = d * (1.f / float(hc)), f = __fdividef(t, 1.f + __expf(-t));
+                const float f = siluf_(d * (1.f / float(hc)));
                 const bf16 hi = __float2bfloat16(f);
                 const float r1 = f - __bfloat162float(hi);
                 const bf16 mid = __float2bfloat16(r1);
