@@ -63,7 +63,7 @@ def test_waits_before_warp_wide_instructions_are_voted_on():
             assert not re.search(r"if \((?:row|col)\b.*\) continue;", m.group(1)), (name, m.group(1))
 
 
-@pytest.mark.parametrize("name", ["gemm_tc.cu", "hc.cu"])
+@pytest.mark.parametrize("name", sorted(os.path.basename(p) for p in _sources()))
 def test_divisions_are_rounded_like_any_other_operation(name):
     """Sigmoids and the like that were formed with a correctly rounded division stay so."""
     assert "__fdividef" not in _text(os.path.join(CSRC, name))
