@@ -54,6 +54,29 @@ def test_attention_tile_edges_units_and_large_scores(L, heads, size):
     assert torch.all(out[L:] == 7.0)
 
 
+@pytest.mark.parametrize("L", [129, 200, 520])
+def test_attention_rows_whose_first_scores_are_all_minus_infinity(L):
+    """Scores of the first key tile overflow to -inf: those keys get no weight, and the rest of the row counts as always."""
+    import ctypes as C
+    from qwb200.ops import lib as qlib
+    hd, heads = 72, 2
+    D = heads * hd
+    g = torch.Generator().manual_seed(L)
+    qkv = torch.randn(L, 3 * D, generator=g)
+    qkv[:, 0] = 3e38
+    qkv[:, D] = 0.0
+    qkv[:128, D] = -3e38
+    qkv = qkv.to(torch.bfloat16).cuda()
+    out = torch.empty(L, D, dtype=torch.bfloat16, device="cuda")
+    assert qlib.load(True).qwk_vit_attention(C.c_void_p(qkv.data_ptr()), L, heads, C.c_void_p(out.data_ptr()),
+                                             C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    q, k, v = [t.double().view(L, heads, hd) for t in qkv.split(D, 1)]
+    s = torch.einsum("qhd,khd->hqk", q, k) / math.sqrt(hd)
+    att = torch.softmax(s.float().double(), -1)
+    ref = torch.einsum("hqk,khd->qhd", att, v).reshape(L, D)
+    assert rel(out, ref) < 1e-2, rel(out, ref)
+
+
 def test_encoder_matches_reference_forward():
     from qwb200.vision import VisionConfig, VisionEncoder, synth_vision_weights, vision_reference
     cfg = VisionConfig(depth=3)

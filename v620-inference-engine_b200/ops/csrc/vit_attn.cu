@@ -41,12 +41,6 @@ __device__ __forceinline__ uint64_t make_mn_desc(uint32_t saddr, uint32_t lbo) {
     return (uint64_t)((saddr & 0x3FFFF) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
 __global__ void __launch_bounds__(VT_THREADS, 1) vit_attn_tc_kernel(const __grid_constant__ CUtensorMap mapA,      // 64-column boxes of qkv
                                                                     const __grid_constant__ CUtensorMap mapB,      // 8-column boxes
                                                                     VitAttnArgs a) {
@@ -185,10 +179,10 @@ __global__ void __launch_bounds__(VT_THREADS, 1) vit_attn_tc_kernel(const __grid
                     for (int c = 0; c < 4; ++c) m4[c] = fmaxf(m4[c], __uint_as_float(s[c][i]));
                 const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * a.scale;
                 if (j == 0) {
-                    ref = mx;
+                    ref = fmaxf(mx, -1e30f);      // a row whose first scores are all -inf keeps a finite reference
                 } else if (__any_sync(0xffffffffu, mx > ref + 8.f)) {
                     // every product issued before these scores is complete, this tile's last O among them
-                    const float nref = fmaxf(ref, mx), f = ex2(ref - nref);
+                    const float nref = fmaxf(ref, mx), f = exp2f(ref - nref);
                     ref = nref;
                     sum *= f;
 #pragma unroll 1
@@ -207,7 +201,7 @@ __global__ void __launch_bounds__(VT_THREADS, 1) vit_attn_tc_kernel(const __grid
                     uint32_t p[16];
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
-                        const float x0 = ex2(fmaf(__uint_as_float(s[c][2 * i]), a.scale, -ref)), x1 = ex2(fmaf(__uint_as_float(s[c][2 * i + 1]), a.scale, -ref));
+                        const float x0 = exp2f(fmaf(__uint_as_float(s[c][2 * i]), a.scale, -ref)), x1 = exp2f(fmaf(__uint_as_float(s[c][2 * i + 1]), a.scale, -ref));
                         sum4[i & 3] += x0 + x1;
                         p[i] = pack_bf16(x0, x1);
                     }
