@@ -129,6 +129,39 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
     return *reinterpret_cast<uint32_t *>(&h);
 }
 
+// V neighbouring columns of a row: V = 4 as one access (16-byte aligned floats, 8-byte aligned bf16), V = 1 for any width and address.
+template <int V>
+__device__ __forceinline__ void ld_cols(const float *p, float (&v)[V]) {
+    if constexpr (V == 4) {
+        const float4 t = *reinterpret_cast<const float4 *>(p);
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+        v[0] = *p;
+    }
+}
+template <int V>
+__device__ __forceinline__ void ld_cols(const bf16 *p, float (&v)[V]) {
+    if constexpr (V == 4) {
+        const uint2 t = *reinterpret_cast<const uint2 *>(p);
+        v[0] = bf16_lo(t.x); v[1] = bf16_hi(t.x); v[2] = bf16_lo(t.y); v[3] = bf16_hi(t.y);
+    } else {
+        v[0] = __bfloat162float(*p);
+    }
+}
+template <int V>
+__device__ __forceinline__ void st_cols(float *p, const float (&v)[V]) {
+    if constexpr (V == 4) *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+    else *p = v[0];
+}
+template <int V>
+__device__ __forceinline__ void st_cols(bf16 *p, const float (&v)[V]) {
+    if constexpr (V == 4) *reinterpret_cast<uint2 *>(p) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
+    else *p = __float2bfloat16(v[0]);
+}
+// host side: do all of these start on 16 bytes (null does)
+template <typename... P>
+inline bool aligned16(const P *...p) { return ((reinterpret_cast<uintptr_t>(p) | ...) & 15) == 0; }
+
 // Streaming 16-byte load that does not allocate in L1 (weights are read once).
 __device__ __forceinline__ uint4 ld_stream(const void *p) {
     uint4 v;

@@ -17,17 +17,18 @@
 
 namespace qw {
 
-// X[m][s][:] = embedding row of tokens[m] (this rank's columns) for every stream.  Four columns per thread, grid (M, ceil(SH / 1024)).
+// X[m][s][:] = embedding row of tokens[m] (this rank's columns) for every stream.  V columns per thread, grid (M, ceil(SH / 256 V)).
+template <int V>
 __global__ void __launch_bounds__(256) embed_rows_kernel(const int *tokens, const bf16 *table, int ld_table, int col0, int SH, int hc,
                                                          int vocab, float *X) {
-    const int m = blockIdx.x, c = (blockIdx.y * 256 + threadIdx.x) * 4;
+    const int m = blockIdx.x, c = (blockIdx.y * 256 + threadIdx.x) * V;
     int t = tokens[m];
     QW_DCHECK(t >= 0 && t < vocab, 0x01000000u | (unsigned)(m & 0xffffff));          // token id outside the vocabulary (row m)
     if (t < 0 || t >= vocab) t = 0;
     if (c >= SH) return;
-    const uint2 u = *reinterpret_cast<const uint2 *>(table + (long long)t * ld_table + col0 + c);
-    const float4 v = make_float4(bf16_lo(u.x), bf16_hi(u.x), bf16_lo(u.y), bf16_hi(u.y));
-    for (int s = 0; s < hc; ++s) *reinterpret_cast<float4 *>(X + ((long long)m * hc + s) * SH + c) = v;
+    float v[V];
+    ld_cols<V>(table + (long long)t * ld_table + col0 + c, v);
+    for (int s = 0; s < hc; ++s) st_cols<V>(X + ((long long)m * hc + s) * SH + c, v);
 }
 
 // Four columns per step.  grid (M, hc).  pend may be null (no deferred combine).  y and ssq may be null (combine only).
@@ -604,8 +605,10 @@ QW_DCHECK_TU(hc)
 
 QW_API int qwk_embed_rows(const int *tokens, const void *table, int ld_table, int col0, int SH, int hc, int vocab,
                           float *X, int M, cudaStream_t s) {
-    if ((SH & 3) || (col0 & 3) || (ld_table & 3)) return -1;
-    embed_rows_kernel<<<dim3(M, (SH + 1023) / 1024), 256, 0, s>>>(tokens, (const bf16 *)table, ld_table, col0, SH, hc, vocab, X);
+    if (((SH | col0 | ld_table) & 3) == 0 && aligned16(table, X))
+        embed_rows_kernel<4><<<dim3(M, (SH + 1023) / 1024), 256, 0, s>>>(tokens, (const bf16 *)table, ld_table, col0, SH, hc, vocab, X);
+    else
+        embed_rows_kernel<1><<<dim3(M, (SH + 255) / 256), 256, 0, s>>>(tokens, (const bf16 *)table, ld_table, col0, SH, hc, vocab, X);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
