@@ -47,3 +47,18 @@ def test_embedding_rows_of_any_width_and_address(SH, col0, ld, off):
     X = shifted(torch.zeros(M, hc, SH, device=DEV), off)
     assert _lib().qwk_embed_rows(P(tok), P(table), ld, col0, SH, hc, vocab, P(X), M, S()) == 0
     assert torch.equal(X, table[tok.long(), col0:col0 + SH].float().unsqueeze(1).expand(M, hc, SH))
+
+
+@pytest.mark.parametrize("SH,ld,off", [(64, 64, 0), (63, 64, 0), (64, 65, 0), (64, 64, 1), (1030, 1031, 2)])
+@pytest.mark.parametrize("pending", [True, False])
+def test_deferred_combine_of_any_width_and_address(SH, ld, off, pending):
+    """X += pending * gate, its bf16 rows and sums of squares, against 64 bits (fp32 sums of up to 1,030 squares: 1e-6; bf16 rows 2^-8)."""
+    M, hc = 5, 4
+    rn = gen(SH + ld)
+    X, pend, inj, w1 = (shifted(t, off) for t in (rn(M, hc, SH), rn(M, ld), rn(M, hc), 1 + 0.1 * rn(hc, SH)))
+    y, ssq = shifted(torch.zeros(M, hc, SH, dtype=torch.bfloat16, device=DEV), off), torch.zeros(M, hc, device=DEV)
+    want = X.double() + (pend[:, None, :SH].double() * (2 * torch.sigmoid(inj.double() / hc))[..., None] if pending else 0)
+    assert _lib().qwk_hc_pre(P(X), P(pend) if pending else None, ld, P(inj), hc, P(w1), SH, hc, P(y), P(ssq), hc, M, S()) == 0
+    assert torch.allclose(X.double(), want, rtol=1e-6, atol=1e-6)
+    assert torch.allclose(y.double(), X.double() * w1.double(), rtol=2 ** -8, atol=1e-30)
+    assert torch.allclose(ssq.double(), X.double().pow(2).sum(-1), rtol=1e-6)

@@ -31,7 +31,8 @@ __global__ void __launch_bounds__(256) embed_rows_kernel(const int *tokens, cons
     for (int s = 0; s < hc; ++s) st_cols<V>(X + ((long long)m * hc + s) * SH + c, v);
 }
 
-// Four columns per step.  grid (M, hc).  pend may be null (no deferred combine).  y and ssq may be null (combine only).
+// V columns per thread and step.  grid (M, hc).  pend may be null (no deferred combine).  y and ssq may be null (combine only).
+template <int V>
 __global__ void __launch_bounds__(256) hc_pre_kernel(float *X, const float *pend, int ld_pend, const float *inj, int ld_inj,
                                                      const float *w1 /* (1+w) [hc][SH] */, int SH, int hc, bf16 *y,
                                                      float *ssq, int ld_ssq) {
@@ -42,18 +43,25 @@ __global__ void __launch_bounds__(256) hc_pre_kernel(float *X, const float *pend
     if (pend) coef = 2.f * sigmoidf_(inj[(long long)m * ld_inj + s] / float(hc));
     float acc = 0.f;
 #pragma unroll 3
-    for (int c = threadIdx.x * 4; c < SH; c += 1024) {
-        float4 v = *reinterpret_cast<const float4 *>(x + c);
+    for (int c = threadIdx.x * V; c < SH; c += 256 * V) {
+        float v[V];
+        ld_cols<V>(x + c, v);
         if (pend) {
-            const float4 p = *reinterpret_cast<const float4 *>(pend + (long long)m * ld_pend + c);
-            v.x = fmaf(p.x, coef, v.x); v.y = fmaf(p.y, coef, v.y); v.z = fmaf(p.z, coef, v.z); v.w = fmaf(p.w, coef, v.w);
-            *reinterpret_cast<float4 *>(x + c) = v;
+            float p[V];
+            ld_cols<V>(pend + (long long)m * ld_pend + c, p);
+#pragma unroll
+            for (int k = 0; k < V; ++k) v[k] = fmaf(p[k], coef, v[k]);
+            st_cols<V>(x + c, v);
         }
         if (y) {
-            const float4 w = *reinterpret_cast<const float4 *>(w1 + s * SH + c);
-            *reinterpret_cast<uint2 *>(y + ((long long)m * hc + s) * SH + c) = make_uint2(pack_bf16(v.x * w.x, v.y * w.y), pack_bf16(v.z * w.z, v.w * w.w));
+            float w[V];
+            ld_cols<V>(w1 + s * SH + c, w);
+#pragma unroll
+            for (int k = 0; k < V; ++k) w[k] *= v[k];
+            st_cols<V>(y + ((long long)m * hc + s) * SH + c, w);
         }
-        acc = fmaf(v.x, v.x, acc); acc = fmaf(v.y, v.y, acc); acc = fmaf(v.z, v.z, acc); acc = fmaf(v.w, v.w, acc);
+#pragma unroll
+        for (int k = 0; k < V; ++k) acc = fmaf(v[k], v[k], acc);
     }
     if (ssq) {
         acc = block_sum<256>(acc, scratch);
@@ -614,9 +622,11 @@ QW_API int qwk_embed_rows(const int *tokens, const void *table, int ld_table, in
 
 QW_API int qwk_hc_pre(float *X, const float *pend, int ld_pend, const float *inj, int ld_inj, const float *w1, int SH,
                       int hc, void *y, float *ssq, int ld_ssq, int M, cudaStream_t s) {
-    if ((SH & 3) || (pend && (ld_pend & 3))) return -1;
     dim3 grid(M, hc);
-    hc_pre_kernel<<<grid, 256, 0, s>>>(X, pend, ld_pend, inj, ld_inj, w1, SH, hc, (bf16 *)y, ssq, ld_ssq);
+    if ((SH & 3) == 0 && (!pend || (ld_pend & 3) == 0) && aligned16(X, pend, y ? w1 : nullptr, (bf16 *)y))
+        hc_pre_kernel<4><<<grid, 256, 0, s>>>(X, pend, ld_pend, inj, ld_inj, w1, SH, hc, (bf16 *)y, ssq, ld_ssq);
+    else
+        hc_pre_kernel<1><<<grid, 256, 0, s>>>(X, pend, ld_pend, inj, ld_inj, w1, SH, hc, (bf16 *)y, ssq, ld_ssq);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
