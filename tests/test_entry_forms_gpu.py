@@ -62,3 +62,18 @@ def test_deferred_combine_of_any_width_and_address(SH, ld, off, pending):
     assert torch.allclose(X.double(), want, rtol=1e-6, atol=1e-6)
     assert torch.allclose(y.double(), X.double() * w1.double(), rtol=2 ** -8, atol=1e-30)
     assert torch.allclose(ssq.double(), X.double().pow(2).sum(-1), rtol=1e-6)
+
+
+@pytest.mark.parametrize("H,hc,off", [(64, 4, 0), (63, 4, 0), (63, 1, 0), (61, 3, 0), (64, 4, 1), (1537, 3, 0)])
+def test_mtp_norm_of_any_width_and_address(H, hc, off):
+    """Both norms against 64 bits (one rounding to bf16: 2^-8, and the fp32 sum of squares)."""
+    M, vocab, eps = 3, 20, 1e-6
+    rn = gen(H)
+    hidden, nh, ne = shifted(rn(M, hc, H), off), shifted(1 + 0.1 * rn(hc * H), off), 1 + 0.1 * rn(H)
+    embed, tok = rn(vocab, H).to(torch.bfloat16), i32([3, 19, 0])
+    hn, en = shifted(torch.zeros(M, hc, H, dtype=torch.bfloat16, device=DEV), off), torch.zeros(M, H, dtype=torch.bfloat16, device=DEV)
+    assert _lib().qwk_mtp_norm(P(hidden), P(tok), P(embed), vocab, P(nh), P(ne), H, hc, C.c_float(eps), P(hn), P(en), M, S()) == 0
+    h, e = hidden.double().view(M, -1), embed[tok.long()].double()
+    h = h * torch.rsqrt(h.pow(2).mean(1, keepdim=True) + eps) * nh.double()
+    e = e * torch.rsqrt(e.pow(2).mean(1, keepdim=True) + eps) * ne.double()
+    assert torch.allclose(hn.double().view(M, -1), h, rtol=2 ** -8, atol=1e-30) and torch.allclose(en.double(), e, rtol=2 ** -8, atol=1e-30)

@@ -6,9 +6,10 @@
 
 namespace qw {
 
-// grid M, 256 threads.  hidden [M][hc][H] fp32 -> hn bf16 [(m*hc + s)][H] = hidden * rsqrt(mean over all) * nh1;
-// en bf16 [m][H] = gemma_norm(embed[token m]) with ne1 = 1 + w.
+// grid M.  hidden [M][hc][H] fp32 -> hn bf16 [(m*hc + s)][H] = hidden * rsqrt(mean over all) * nh1;
+// en bf16 [m][H] = gemma_norm(embed[token m]) with ne1 = 1 + w.  V columns per thread and step.
 constexpr int MN_THREADS = 1024;      // a row of 10,240 values is 2.5 pieces of four per thread (with 256 threads and scalar loads 29 us a row, now 7)
+template <int V>
 __global__ void __launch_bounds__(MN_THREADS) mtp_norm_kernel(const float *hidden, const int *tokens, const bf16 *embed, int vocab,
                                                               const float *nh1, const float *ne1, int H, int hc, float eps, bf16 *hn,
                                                               bf16 *en) {
@@ -22,9 +23,11 @@ __global__ void __launch_bounds__(MN_THREADS) mtp_norm_kernel(const float *hidde
     const float *x = hidden + (long long)m * n;
     float ss = 0.f, es = 0.f;
 #pragma unroll 3
-    for (int i = threadIdx.x * 4; i < n; i += MN_THREADS * 4) {
-        const float4 v = *reinterpret_cast<const float4 *>(x + i);
-        ss = fmaf(v.x, v.x, ss); ss = fmaf(v.y, v.y, ss); ss = fmaf(v.z, v.z, ss); ss = fmaf(v.w, v.w, ss);
+    for (int i = threadIdx.x * V; i < n; i += MN_THREADS * V) {
+        float v[V];
+        ld_cols<V>(x + i, v);
+#pragma unroll
+        for (int k = 0; k < V; ++k) ss = fmaf(v[k], v[k], ss);
     }
     for (int i = threadIdx.x; i < H; i += MN_THREADS) {
         const float v = __bfloat162float(e[i]);
@@ -34,9 +37,13 @@ __global__ void __launch_bounds__(MN_THREADS) mtp_norm_kernel(const float *hidde
     es = block_sum<MN_THREADS>(es, scratch);
     const float r = rsqrtf(ss / float(n) + eps), re = rsqrtf(es / float(H) + eps);
 #pragma unroll 3
-    for (int i = threadIdx.x * 4; i < n; i += MN_THREADS * 4) {
-        const float4 v = *reinterpret_cast<const float4 *>(x + i), w = *reinterpret_cast<const float4 *>(nh1 + i);
-        *reinterpret_cast<uint2 *>(hn + (long long)m * n + i) = make_uint2(pack_bf16(v.x * r * w.x, v.y * r * w.y), pack_bf16(v.z * r * w.z, v.w * r * w.w));
+    for (int i = threadIdx.x * V; i < n; i += MN_THREADS * V) {
+        float v[V], w[V];
+        ld_cols<V>(x + i, v);
+        ld_cols<V>(nh1 + i, w);
+#pragma unroll
+        for (int k = 0; k < V; ++k) v[k] = v[k] * r * w[k];
+        st_cols<V>(hn + (long long)m * n + i, v);
     }
     for (int i = threadIdx.x; i < H; i += MN_THREADS) en[(long long)m * H + i] = __float2bfloat16(__bfloat162float(e[i]) * re * ne1[i]);
 }
@@ -58,8 +65,8 @@ using namespace qw;
 
 QW_API int qwk_mtp_norm(const float *hidden, const int *tokens, const void *embed, int vocab, const float *nh1, const float *ne1,
                         int H, int hc, float eps, void *hn, void *en, int M, cudaStream_t s) {
-    if (H & 3) return -1;
-    return launch_pdl(mtp_norm_kernel, dim3(M), dim3(MN_THREADS), 0, s, hidden, tokens, (const bf16 *)embed, vocab, nh1, ne1, H, hc, eps,
+    const bool vec = (hc * H & 3) == 0 && aligned16(hidden, nh1, (bf16 *)hn);
+    return launch_pdl(vec ? mtp_norm_kernel<4> : mtp_norm_kernel<1>, dim3(M), dim3(MN_THREADS), 0, s, hidden, tokens, (const bf16 *)embed, vocab, nh1, ne1, H, hc, eps,
                       (bf16 *)hn, (bf16 *)en) == cudaSuccess ? 0 : -2;
 }
 QW_API int qwk_mtp_add(const float *fh, const float *fe, int H, int hc, float *X, int M, cudaStream_t s) {
