@@ -77,3 +77,45 @@ def test_mtp_norm_of_any_width_and_address(H, hc, off):
     h = h * torch.rsqrt(h.pow(2).mean(1, keepdim=True) + eps) * nh.double()
     e = e * torch.rsqrt(e.pow(2).mean(1, keepdim=True) + eps) * ne.double()
     assert torch.allclose(hn.double().view(M, -1), h, rtol=2 ** -8, atol=1e-30) and torch.allclose(en.double(), e, rtol=2 ** -8, atol=1e-30)
+
+
+@pytest.mark.parametrize("SH,pad,taps,off,M", [(32, 0, 4, 0, 20), (32, 0, 4, 0, 300), (31, 0, 4, 0, 20), (32, 1, 4, 0, 20), (32, 0, 3, 0, 20),
+                                               (32, 0, 5, 0, 300), (33, 3, 2, 0, 7), (32, 0, 4, 1, 20), (32, 0, 1, 2, 5)])
+def test_ngram_layer_of_any_width_taps_and_address(SH, pad, taps, off, M):
+    """Gate, dilated convolution over two runs of rows and their slots' rings, ring update: against the same formulas in 64 bits
+    (fp32 throughout: 2e-5 of a value covers a dozen roundings)."""
+    hc, H, eps, dil, RING = 4, 128, 1e-6, 3, 32
+    xw = hc * SH
+    rn = gen(SH * taps + M)
+    kv, red, nc1, cw, X, ring = (shifted(t, off) for t in (rn(M, xw + SH + pad), rn(M, 16).abs() + 0.1, rn(xw), rn(xw, taps), rn(M, xw), rn(2, RING, xw)))
+    first = M // 3
+    runs = [(0, 0, first, 5), (1, first, M - first, 40)]                    # slot, first row, rows, position
+    slot, pos, rs, rl = [], [], [], [0] * M
+    for sl, r0, n, p0 in runs:
+        slot += [sl] * n
+        pos += [p0 + i for i in range(n)]
+        rs += [r0] * n
+        rl[r0] = n
+    old, x0 = ring.double().clone(), X.double().clone()
+    gv, nc = shifted(torch.zeros(M, xw, device=DEV), off), shifted(torch.zeros(M, xw, device=DEV), off)
+    t = [i32(v) for v in (slot, pos, rs, rl)]
+    assert _lib().qwk_ple_apply(P(kv), xw + SH + pad, P(red), 16, P(nc1), P(cw), SH, hc, H, C.c_float(eps), taps, dil, P(gv), P(nc), P(ring), P(X), M,
+                                *[P(v) for v in t], S()) == 0
+    r = red.double()[:, :3 * hc].view(M, hc, 3)
+    gs = r[..., 2] * torch.rsqrt(r[..., 0] / H + eps) * torch.rsqrt(r[..., 1] / H + eps) / H ** 0.5
+    gate = torch.sigmoid(torch.sign(gs) * gs.abs().clamp_min(1e-6).sqrt())
+    rnorm = torch.rsqrt(gate ** 2 * red.double()[:, 3 * hc:3 * hc + 1] / H + eps)
+    g = gate[..., None] * kv.double()[:, None, xw:xw + SH]
+    n = (g * rnorm[..., None]).view(M, xw) * nc1.double()
+    conv = torch.zeros(M, xw, dtype=torch.float64, device=DEV)
+    for m in range(M):
+        for k in range(taps):
+            back = (taps - 1 - k) * dil
+            q = pos[m] - back
+            v = n[m - back] if m - back >= rs[m] else old[slot[m], q % RING] if q >= 0 else 0.0
+            conv[m] += cw.double()[:, k] * v
+    assert torch.allclose(X.double(), x0 + g.reshape(M, xw) + torch.nn.functional.silu(conv), rtol=2e-5, atol=2e-5)
+    for m in range(M):
+        if m - rs[m] >= rl[rs[m]] - RING:
+            old[slot[m], pos[m] % RING] = n[m]
+    assert torch.allclose(ring.double(), old, rtol=2e-5, atol=2e-5)

@@ -133,11 +133,12 @@ __global__ void __launch_bounds__(256) ple_stats_kernel(const float *kv, int ld_
 
 __device__ __forceinline__ float4 ple_ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
 
-// Gate, gated value gv and normalised conv input nc for the batch rows, four columns per thread.  grid (M, hc, ceil(SH / 1024)).
+// Gate, gated value gv and normalised conv input nc for the batch rows, V columns per thread.  grid (M, hc, ceil(SH / 256 V)).
+template <int V>
 __global__ void __launch_bounds__(256) ple_nc_kernel(const float *kv, int ld_kv, const float *red, int ld_red,
                                                      const float *nc1, int SH, int hc, int H, float eps, float *gv,
                                                      float *nc) {
-    const int m = blockIdx.x, s = blockIdx.y, c = (blockIdx.z * 256 + threadIdx.x) * 4;
+    const int m = blockIdx.x, s = blockIdx.y, c = (blockIdx.z * 256 + threadIdx.x) * V;
     if (c >= SH) return;
     const float *r = red + (long long)m * ld_red;
     const float rk = rsqrtf(r[3 * s] / float(H) + eps), rq = rsqrtf(r[3 * s + 1] / float(H) + eps);
@@ -145,20 +146,26 @@ __global__ void __launch_bounds__(256) ple_nc_kernel(const float *kv, int ld_kv,
     const float mag = sqrtf(fmaxf(fabsf(gs), 1e-6f));
     const float gate = sigmoidf_(gs < 0.f ? -mag : (gs > 0.f ? mag : 0.f));
     const float rn = rsqrtf(gate * gate * r[3 * hc] / float(H) + eps);
-    const float4 v = ple_ld4(kv + (long long)m * ld_kv + hc * SH + c), w = ple_ld4(nc1 + s * SH + c);
-    const float4 g = make_float4(gate * v.x, gate * v.y, gate * v.z, gate * v.w);
+    float g[V], w[V];
+    ld_cols<V>(kv + (long long)m * ld_kv + hc * SH + c, g);
+    ld_cols<V>(nc1 + s * SH + c, w);
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+        g[k] *= gate;
+        w[k] = g[k] * rn * w[k];
+    }
     const long long o = ((long long)m * hc + s) * SH + c;
-    *reinterpret_cast<float4 *>(gv + o) = g;
-    *reinterpret_cast<float4 *>(nc + o) = make_float4(g.x * rn * w.x, g.y * rn * w.y, g.z * rn * w.z, g.w * rn * w.w);
+    st_cols<V>(gv + o, g);
+    st_cols<V>(nc + o, w);
 }
 
 // X += gv + silu(dilated conv of nc); taps at p-9, p-6, p-3, p from the batch or the ring.  Four columns and `rows_per` rows per
 // thread: one row per block when there are few (a step of one row used four blocks and took 34 us, now 5), several with
-// the taps' weights in registers when there are many (4096 rows: 300 us, now 150).  grid (ceil(xw / 1024), ceil(M / rows_per)).
+// the taps' weights in registers when there are many (4096 rows: 300 us, now 150).  grid (ceil(M / rows_per), ceil(xw / 1024)).
 constexpr int PLE_TAPS = 4;
 __global__ void __launch_bounds__(256) ple_conv_kernel(const float *gv, const float *nc, const float *ring, const float *cw,
                                                        int xw, int dil, Rows rows, int rows_per, float *X) {
-    const int col = (blockIdx.x * 256 + threadIdx.x) * 4;
+    const int col = (blockIdx.y * 256 + threadIdx.x) * 4;
     if (col >= xw) return;
     float w[4][PLE_TAPS];
 #pragma unroll
@@ -166,8 +173,8 @@ __global__ void __launch_bounds__(256) ple_conv_kernel(const float *gv, const fl
         const float4 t = ple_ld4(cw + (col + i) * PLE_TAPS);
         w[i][0] = t.x; w[i][1] = t.y; w[i][2] = t.z; w[i][3] = t.w;
     }
-    const int m1 = min(rows.M, (int)(blockIdx.y + 1) * rows_per);
-    for (int m = blockIdx.y * rows_per; m < m1; ++m) {
+    const int m1 = min(rows.M, (int)(blockIdx.x + 1) * rows_per);
+    for (int m = blockIdx.x * rows_per; m < m1; ++m) {
         const int slot = rows.slot[m], pos = rows.pos[m], rs = rows.run_start[m];
         const float *rg = ring + (long long)slot * PLE_RING * xw;
         float4 v[PLE_TAPS];
@@ -192,16 +199,34 @@ __global__ void __launch_bounds__(256) ple_conv_kernel(const float *gv, const fl
     }
 }
 
-// Stores the batch's last nc rows of every run in the ring (after ple_conv has read it).  grid (ceil(M / rows_per), ceil(xw / 1024)).
+// The same for any number of taps, width and address: a row and a column per thread.  grid (M, ceil(xw / 256)).
+__global__ void __launch_bounds__(256) ple_conv_any_kernel(const float *gv, const float *nc, const float *ring, const float *cw,
+                                                           int xw, int taps, int dil, Rows rows, float *X) {
+    const int m = blockIdx.x, col = blockIdx.y * 256 + threadIdx.x;
+    if (col >= xw) return;
+    const int slot = rows.slot[m], pos = rows.pos[m], rs = rows.run_start[m];
+    const float *rg = ring + (long long)slot * PLE_RING * xw;
+    float acc = 0.f;
+    for (int k = 0; k < taps; ++k) {
+        const int back = (taps - 1 - k) * dil, q = pos - back;
+        const float v = m - back >= rs ? nc[(long long)(m - back) * xw + col] : q >= 0 ? rg[(q % PLE_RING) * xw + col] : 0.f;
+        acc = fmaf(cw[col * taps + k], v, acc);
+    }
+    X[(long long)m * xw + col] += gv[(long long)m * xw + col] + siluf_(acc);
+}
+
+// Stores the batch's last nc rows of every run in the ring (after ple_conv has read it).  grid (ceil(M / rows_per), ceil(xw / 256 V)).
+template <int V>
 __global__ void __launch_bounds__(256) ple_ring_kernel(const float *nc, float *ring, int xw, Rows rows, int rows_per) {
-    const int col = (blockIdx.y * 256 + threadIdx.x) * 4;
+    const int col = (blockIdx.y * 256 + threadIdx.x) * V;
     if (col >= xw) return;
     const int m1 = min(rows.M, (int)(blockIdx.x + 1) * rows_per);
     for (int m = blockIdx.x * rows_per; m < m1; ++m) {
         const int rs = rows.run_start[m], len = rows.run_len[rs];
         if ((m - rs) < len - PLE_RING) continue;
-        *reinterpret_cast<float4 *>(ring + ((long long)rows.slot[m] * PLE_RING + (rows.pos[m] % PLE_RING)) * xw + col) =
-            ple_ld4(nc + (long long)m * xw + col);
+        float v[V];
+        ld_cols<V>(nc + (long long)m * xw + col, v);
+        st_cols<V>(ring + ((long long)rows.slot[m] * PLE_RING + (rows.pos[m] % PLE_RING)) * xw + col, v);
     }
 }
 
@@ -248,11 +273,18 @@ QW_API int qwk_ple_apply(const float *kv, int ld_kv, const float *red, int ld_re
                          int SH, int hc, int H, float eps, int taps, int dil, float *gv, float *nc, float *ring,
                          float *X, int M, const int *slot, const int *pos, const int *run_start, const int *run_len,
                          cudaStream_t s) {
-    if ((SH & 3) || (ld_kv & 3) || taps != PLE_TAPS) return -1;
     Rows rows{M, slot, pos, run_start, run_len};
-    const int xw = hc * SH, rows_per = M >= 256 ? 8 : 1, cb = (xw + 1023) / 1024, rb = (M + rows_per - 1) / rows_per;
-    ple_nc_kernel<<<dim3(M, hc, (SH + 1023) / 1024), 256, 0, s>>>(kv, ld_kv, red, ld_red, nc1, SH, hc, H, eps, gv, nc);
-    ple_conv_kernel<<<dim3(cb, rb), 256, 0, s>>>(gv, nc, ring, cw, xw, dil, rows, rows_per, X);
-    ple_ring_kernel<<<dim3(rb, cb), 256, 0, s>>>(nc, ring, xw, rows, rows_per);
+    const int xw = hc * SH;
+    if (((SH | ld_kv) & 3) == 0 && taps == PLE_TAPS && aligned16(kv, nc1, cw, gv, nc, ring, X)) {
+        const int rows_per = M >= 256 ? 8 : 1, cb = (xw + 1023) / 1024, rb = (M + rows_per - 1) / rows_per;
+        ple_nc_kernel<4><<<dim3(M, hc, (SH + 1023) / 1024), 256, 0, s>>>(kv, ld_kv, red, ld_red, nc1, SH, hc, H, eps, gv, nc);
+        ple_conv_kernel<<<dim3(rb, cb), 256, 0, s>>>(gv, nc, ring, cw, xw, dil, rows, rows_per, X);
+        ple_ring_kernel<4><<<dim3(rb, cb), 256, 0, s>>>(nc, ring, xw, rows, rows_per);
+    } else {
+        const int cb = (xw + 255) / 256;
+        ple_nc_kernel<1><<<dim3(M, hc, (SH + 255) / 256), 256, 0, s>>>(kv, ld_kv, red, ld_red, nc1, SH, hc, H, eps, gv, nc);
+        ple_conv_any_kernel<<<dim3(M, cb), 256, 0, s>>>(gv, nc, ring, cw, xw, taps, dil, rows, X);
+        ple_ring_kernel<1><<<dim3(M, cb), 256, 0, s>>>(nc, ring, xw, rows, 1);
+    }
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
