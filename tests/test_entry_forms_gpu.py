@@ -119,3 +119,24 @@ def test_ngram_layer_of_any_width_taps_and_address(SH, pad, taps, off, M):
         if m - rs[m] >= rl[rs[m]] - RING:
             old[slot[m], pos[m] % RING] = n[m]
     assert torch.allclose(ring.double(), old, rtol=2e-5, atol=2e-5)
+
+
+@pytest.mark.parametrize("pad,off", [(0, 0), (1, 0), (3, 0), (0, 1), (2, 3)])
+def test_chunked_scan_takes_projections_of_any_stride_and_address(pad, off):
+    """The output norm reads the gate z from the projection rows: the same bits wherever these rows start."""
+    KL, VL, M = 1, 2, 70
+    qkv_l = (2 * KL + VL) * 128
+    ld0 = (qkv_l + VL * 128 + 2 * VL + 3) // 4 * 4
+    rn = gen(5)
+    qkv, beta, decay, proj0, S0, nw = rn(M, qkv_l) * 0.1, torch.sigmoid(rn(M, VL)), torch.sigmoid(rn(M, VL) + 3), rn(M, ld0), rn(1, VL, 128, 128) * 0.1, 1 + 0.1 * rn(128)
+    need = 64 * 1024 * 1024
+
+    def scan(pad, off):
+        proj = shifted(torch.cat([proj0, torch.zeros(M, pad, device=DEV)], 1), off)
+        st, o, scratch = S0.clone(), torch.zeros(M, VL * 128, dtype=torch.bfloat16, device=DEV), torch.zeros(need // 4, device=DEV)
+        assert _lib().qwk_gdn_scan_chunked(P(qkv), P(decay), P(beta), P(proj), ld0 + pad, P(st), P(shifted(nw, off)), KL, VL, M, P(i32([0] * M)), P(scratch), P(o),
+                                           C.c_float(1e-6), S()) == 0
+        torch.cuda.synchronize()
+        return st, o
+    want, got = scan(0, 0), scan(pad, off)
+    assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1]) and float(got[1].float().abs().max()) > 0

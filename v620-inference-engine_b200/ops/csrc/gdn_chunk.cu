@@ -387,13 +387,22 @@ __global__ void __launch_bounds__(256) gdn_chunk_apply_kernel(GdnChunkArgs a) {
 // 3. gated RMS norm over each head's 128 outputs
 // ------------------------------------------------------------------------------------------------
 // A warp per (row, head), four values per lane (a block of 128 with two meetings per head and row took 121 us at 4096 x 48, this 44).
+template <bool VEC>
 __global__ void __launch_bounds__(256) gdn_chunk_norm_kernel(GdnChunkArgs a) {
     const long long i = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (i >= (long long)a.M * a.VL) return;
     const int m = (int)(i / a.VL), h = (int)(i - (long long)m * a.VL), c = (threadIdx.x & 31) * 4;
     const int qkv_l = (2 * a.KL + a.VL) * CD;
-    const float4 o = *reinterpret_cast<const float4 *>(a.Oraw + i * CD + c), w = *reinterpret_cast<const float4 *>(a.norm_w + c);
-    const float4 z = *reinterpret_cast<const float4 *>(a.proj + (long long)m * a.ld_proj + qkv_l + h * CD + c);
+    const float4 o = *reinterpret_cast<const float4 *>(a.Oraw + i * CD + c);
+    const float *wp = a.norm_w + c, *zp = a.proj + (long long)m * a.ld_proj + qkv_l + h * CD + c;
+    float4 w, z;
+    if (VEC) {
+        w = *reinterpret_cast<const float4 *>(wp);
+        z = *reinterpret_cast<const float4 *>(zp);
+    } else {                                                     // rows of the projection that do not start on 16 bytes
+        w = make_float4(wp[0], wp[1], wp[2], wp[3]);
+        z = make_float4(zp[0], zp[1], zp[2], zp[3]);
+    }
     const float r = rsqrtf(warp_sum(fmaf(o.x, o.x, o.y * o.y) + fmaf(o.z, o.z, o.w * o.w)) / float(CD) + a.eps);
     *reinterpret_cast<uint2 *>(a.o + i * CD + c) =
         make_uint2(pack_bf16(o.x * r * w.x * sigmoidf_(z.x), o.y * r * w.y * sigmoidf_(z.y)), pack_bf16(o.z * r * w.z * sigmoidf_(z.z), o.w * r * w.w * sigmoidf_(z.w)));
@@ -409,7 +418,7 @@ using namespace qw;
 QW_API int qwk_gdn_scan_chunked(const float *qkv, const float *decay, const float *beta, const float *proj, int ld_proj,
                                 float *S, const float *norm_w, int KL, int VL, int M, const int *slot, float *scratch,
                                 void *o, float eps, cudaStream_t s) {
-    if (M < 1 || KL < 1 || VL % KL != 0 || (ld_proj & 3)) return -1;
+    if (M < 1 || KL < 1 || VL % KL != 0) return -1;
     static bool attr_done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -436,6 +445,8 @@ QW_API int qwk_gdn_scan_chunked(const float *qkv, const float *decay, const floa
     if (VL >= 32) gdn_chunk_apply_kernel<64><<<dim3(2, VL), 256, apply_smem<64>(), s>>>(a);
     else if (VL >= 16) gdn_chunk_apply_kernel<32><<<dim3(4, VL), 256, apply_smem<32>(), s>>>(a);
     else gdn_chunk_apply_kernel<16><<<dim3(8, VL), 256, apply_smem<16>(), s>>>(a);
-    gdn_chunk_norm_kernel<<<(unsigned)(((long long)M * VL + 7) / 8), 256, 0, s>>>(a);
+    const unsigned blocks = (unsigned)(((long long)M * VL + 7) / 8);
+    if ((ld_proj & 3) == 0 && aligned16(proj, norm_w)) gdn_chunk_norm_kernel<true><<<blocks, 256, 0, s>>>(a);
+    else gdn_chunk_norm_kernel<false><<<blocks, 256, 0, s>>>(a);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
