@@ -140,3 +140,40 @@ def test_chunked_scan_takes_projections_of_any_stride_and_address(pad, off):
         return st, o
     want, got = scan(0, 0), scan(pad, off)
     assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1]) and float(got[1].float().abs().max()) > 0
+
+
+@pytest.mark.parametrize("runs", [[(0, 40, 3)], [(1, 13, 0), (0, 27, 6)], [(0, 1, 20), (1, 8, 2), (2, 30, 50)], [(2, 33, 1), (0, 33, 0), (1, 2, 9)]])
+@pytest.mark.parametrize("off,pad", [(0, 0), (1, 0), (0, 1)])
+def test_gdn_conv_of_many_rows_in_several_runs(runs, off, pad):
+    """More than 32 rows: every run's taps come from its own rows and its own slot's ring, wherever the run begins within a block's
+    eight rows.  Against 64 bits (four products, silu and a norm of 128 in fp32: 1e-5)."""
+    KL, VL, RING = 1, 2, 16
+    qkv_l = (2 * KL + VL) * 128
+    ld = qkv_l + VL * 128 + 2 * VL + pad
+    M = sum(n for _, n, _ in runs)
+    rn = gen(M + off)
+    proj, cw, ring = shifted(rn(M, ld), off), shifted(rn(qkv_l, 4) * 0.3, off), shifted(rn(3, RING, qkv_l), off)
+    A, dt = rn(VL), rn(VL)
+    slot, pos, rs, rl = [], [], [], [0] * M
+    for sl, n, p0 in runs:
+        rl[len(slot)] = n
+        rs += [len(slot)] * n
+        slot += [sl] * n
+        pos += [p0 + i for i in range(n)]
+    old = ring.double().clone()
+    qkv, dec, beta = torch.zeros(M, qkv_l, device=DEV), torch.zeros(M, VL, device=DEV), torch.zeros(M, VL, device=DEV)
+    t = [i32(v) for v in (slot, pos, rs, rl)]
+    assert _lib().qwk_gdn_conv(P(proj), ld, P(ring), P(cw), P(A), P(dt), KL, VL, M, *[P(v) for v in t], P(qkv), P(dec), P(beta), C.c_float(1e-6), S()) == 0
+    p, want = proj.double(), torch.zeros(M, qkv_l, dtype=torch.float64, device=DEV)
+    for m in range(M):
+        for k in range(4):
+            back, q = 3 - k, pos[m] - 3 + k
+            want[m] += cw.double()[:, k] * (p[m - back, :qkv_l] if m - back >= rs[m] else old[slot[m], q % RING] if q >= 0 else 0.0)
+    want = torch.nn.functional.silu(want).view(M, -1, 128)
+    norm = torch.rsqrt(want.pow(2).sum(-1, keepdim=True) + 1e-6)
+    want[:, :KL] *= norm[:, :KL] / 128 ** 0.5
+    want[:, KL:2 * KL] *= norm[:, KL:2 * KL]
+    assert torch.allclose(qkv.double(), want.view(M, -1), rtol=1e-5, atol=1e-6)
+    z = p[:, qkv_l + VL * 128:]
+    assert torch.allclose(beta.double(), torch.sigmoid(z[:, :VL]), rtol=1e-5, atol=1e-6)
+    assert torch.allclose(dec.double(), torch.exp(-torch.exp(A.double()) * torch.nn.functional.softplus(z[:, VL:2 * VL] + dt.double())), rtol=1e-5, atol=1e-6)

@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(128) gdn_conv_kernel(GdnConvArgs a) {
     }
 }
 
-// The same for a prefill chunk (more than MAX_ROWS rows: one run of one slot, row 0 its first): a warp per head and 8 rows, four
+// The same for a prefill chunk (more than MAX_ROWS rows; long runs, though nothing depends on it): a warp per head and 8 rows, four
 // channels per lane, so a head's norm is five shuffles instead of two meetings of a block per row and four rows' loads are in
 // flight.  4096 rows, 80 heads: 180 us with the kernel above, 95 here.  The last row of blocks forms decay
 // and beta.  grid (ceil(M / 8), ceil((2 KL + VL) / 4) + 1), 128 threads.
@@ -97,28 +97,31 @@ __global__ void __launch_bounds__(128) gdn_conv_prefill_kernel(GdnConvArgs a) {
         return;
     }
     if (head >= 2 * a.KL + a.VL) return;
-    const int pos0 = a.rows.pos[0];
-    const float *ring = a.ring + (long long)a.rows.slot[0] * GDN_RING * qkv_l + c;
     float tap[4][4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         const float4 t = *reinterpret_cast<const float4 *>(a.cw + (c + j) * 4);
         tap[j][0] = t.x; tap[j][1] = t.y; tap[j][2] = t.z; tap[j][3] = t.w;
     }
-    auto row_at = [&](int m) {               // pre-conv row m of the chunk; before it the ring, before the sequence zero
-        if (m >= 0) return *reinterpret_cast<const float4 *>(a.proj + (long long)m * a.ld_proj + c);
-        const int q = pos0 + m;
-        return q >= 0 ? *reinterpret_cast<const float4 *>(ring + (q % GDN_RING) * qkv_l) : make_float4(0.f, 0.f, 0.f, 0.f);
+    auto proj_at = [&](int m) { return *reinterpret_cast<const float4 *>(a.proj + (long long)m * a.ld_proj + c); };
+    auto back_from = [&](int m, int back) {  // pre-conv row `back` rows before m: of m's run, before it the slot's ring, before the sequence zero
+        if (m - back >= a.rows.run_start[m]) return proj_at(m - back);
+        const int q = a.rows.pos[m] - back;
+        return q >= 0 ? *reinterpret_cast<const float4 *>(a.ring + ((long long)a.rows.slot[m] * GDN_RING + q % GDN_RING) * qkv_l + c)
+                      : make_float4(0.f, 0.f, 0.f, 0.f);
     };
-    float4 w0 = row_at(m0 - 3), w1 = row_at(m0 - 2), w2 = row_at(m0 - 1);
+    float4 w0 = back_from(m0, 3), w1 = back_from(m0, 2), w2 = back_from(m0, 1);
     for (int mb = m0; mb < m1; mb += 4) {
         float4 cur[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) cur[k] = mb + k < m1 ? row_at(mb + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < 4; ++k) cur[k] = mb + k < m1 ? proj_at(mb + k) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int m = mb + k;
             if (m >= m1) break;
+            if (m > m0 && a.rows.run_start[m] == m) {          // a run begins inside these rows
+                w0 = back_from(m, 3); w1 = back_from(m, 2); w2 = back_from(m, 1);
+            }
             float4 v;
             v.x = siluf_(fmaf(tap[0][3], cur[k].x, fmaf(tap[0][2], w2.x, fmaf(tap[0][1], w1.x, tap[0][0] * w0.x))));
             v.y = siluf_(fmaf(tap[1][3], cur[k].y, fmaf(tap[1][2], w2.y, fmaf(tap[1][1], w1.y, tap[1][0] * w0.y))));
@@ -381,7 +384,7 @@ QW_API int qwk_gdn_conv(const float *proj, int ld_proj, float *ring, const float
     a.KL = KL; a.VL = VL; a.rows = Rows{M, slot, pos, run_start, run_len};
     a.qkv = qkv; a.decay = decay; a.beta = beta; a.eps = eps;
     if (VL > 128) return -1;
-    if (M > MAX_ROWS && (ld_proj & 3) == 0 && ((uintptr_t)proj & 15) == 0) {
+    if (M > MAX_ROWS && (ld_proj & 3) == 0 && aligned16(proj, ring, cw, qkv)) {
         gdn_conv_prefill_kernel<<<dim3((M + CONVP_ROWS - 1) / CONVP_ROWS, (2 * KL + VL + 3) / 4 + 1), 128, 0, s>>>(a);
     } else {
         dim3 grid((M + CONV_ROWS - 1) / CONV_ROWS, 2 * KL + VL);
