@@ -177,3 +177,18 @@ def test_gdn_conv_of_many_rows_in_several_runs(runs, off, pad):
     z = p[:, qkv_l + VL * 128:]
     assert torch.allclose(beta.double(), torch.sigmoid(z[:, :VL]), rtol=1e-5, atol=1e-6)
     assert torch.allclose(dec.double(), torch.exp(-torch.exp(A.double()) * torch.nn.functional.softplus(z[:, VL:2 * VL] + dt.double())), rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("D,off", [(1152, 0), (1153, 0), (1536, 0), (1540, 0), (2050, 0), (72, 1), (1152, 2)])
+@pytest.mark.parametrize("add", [True, False])
+def test_vision_norm_of_any_width_and_address(D, off, add):
+    """x += y + bias, then the norm in bf16 (2^-8 of a value, and fp32 sums under a mean of near 0: 1e-5), against 64 bits."""
+    L, eps = 9, 1e-6
+    rn = gen(D)
+    x, y, yb, w, b = (shifted(t, off) for t in (rn(L, D), rn(L, D), rn(D), 1 + 0.1 * rn(D), rn(D)))
+    out = shifted(torch.zeros(L, D, dtype=torch.bfloat16, device=DEV), off)
+    want = x.double() + (y.double() + yb.double() if add else 0)
+    assert _lib().qwk_vit_layernorm(P(x), P(y) if add else None, P(yb) if add else None, P(w), P(b), L, D, C.c_float(eps), P(out), S()) == 0
+    assert torch.allclose(x.double(), want, rtol=1e-6, atol=1e-6)
+    ref = torch.nn.functional.layer_norm(x.double(), (D,), w.double(), b.double(), eps)
+    assert torch.allclose(out.double(), ref, rtol=2 ** -8, atol=1e-5)

@@ -75,6 +75,24 @@ __global__ void __launch_bounds__(128) vit_layernorm_kernel(float *x, const floa
     }
 }
 
+// The same for any width and address: a block per row.
+__global__ void __launch_bounds__(256) vit_layernorm_any_kernel(float *x, const float *y, const float *ybias, const float *w, const float *b,
+                                                                int D, float eps, bf16 *out) {
+    __shared__ float scratch[32];
+    float *row = x + (long long)blockIdx.x * D;
+    const float *add = y ? y + (long long)blockIdx.x * D : nullptr;
+    float s = 0.f;
+    for (int c = threadIdx.x; c < D; c += 256) {
+        if (y) row[c] += add[c] + ybias[c];
+        s += row[c];
+    }
+    const float mean = block_sum<256>(s, scratch) / float(D);
+    float q = 0.f;
+    for (int c = threadIdx.x; c < D; c += 256) q = fmaf(row[c] - mean, row[c] - mean, q);
+    const float rstd = rsqrtf(block_sum<256>(q, scratch) / float(D) + eps);
+    for (int c = threadIdx.x; c < D; c += 256) out[(long long)blockIdx.x * D + c] = __float2bfloat16((row[c] - mean) * rstd * w[c] + b[c]);
+}
+
 // cos | sin of the 36 angles of every patch (first 18 by row, last 18 by column): [L][2][36], once per slice instead of once per
 // block, head and tensor.
 __global__ void __launch_bounds__(256) vit_rope_table_kernel(const int *pos_hw, int L, float *tab) {
@@ -180,11 +198,13 @@ QW_API int qwk_vit_embed(float *x, const float *y, const float *bias, const floa
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-// out = bf16(LayerNorm(x) * w + b); with y (null: none) x += y + ybias first.  D a multiple of 4, at most 1536; 16-byte aligned pointers.
+// out = bf16(LayerNorm(x) * w + b); with y (null: none) x += y + ybias first.
 QW_API int qwk_vit_layernorm(float *x, const float *y, const float *ybias, const float *w, const float *b, int L, int D, float eps,
                              void *out, cudaStream_t s) {
-    if ((D & 3) || D > VLN_MAX * 128) return -1;
-    vit_layernorm_kernel<<<(L + 3) / 4, 128, 0, s>>>(x, y, ybias, w, b, L, D, eps, (bf16 *)out);
+    if ((D & 3) == 0 && D <= VLN_MAX * 128 && aligned16(x, y, y ? ybias : nullptr, w, b, (float *)out))
+        vit_layernorm_kernel<<<(L + 3) / 4, 128, 0, s>>>(x, y, ybias, w, b, L, D, eps, (bf16 *)out);
+    else
+        vit_layernorm_any_kernel<<<L, 256, 0, s>>>(x, y, ybias, w, b, D, eps, (bf16 *)out);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
