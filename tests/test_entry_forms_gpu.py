@@ -192,3 +192,27 @@ def test_vision_norm_of_any_width_and_address(D, off, add):
     assert torch.allclose(x.double(), want, rtol=1e-6, atol=1e-6)
     ref = torch.nn.functional.layer_norm(x.double(), (D,), w.double(), b.double(), eps)
     assert torch.allclose(out.double(), ref, rtol=2 ** -8, atol=1e-5)
+
+
+@pytest.mark.parametrize("heads,off", [(2, 0), (2, 1), (16, 4), (1, 2)])
+def test_vision_rotary_at_any_address(heads, off):
+    """The same bits from aligned and shifted rows, and against 64 bits (one rounding to bf16, relative to the pair's size)."""
+    L, hd = 11, 72
+    D = heads * hd
+    rn = gen(heads)
+    q0, bias, pos = rn(L, 3 * D).to(torch.bfloat16), rn(3 * D), torch.stack([torch.arange(L), torch.arange(L) % 4], 1).to(torch.int32).to(DEV)
+
+    def rope(off):
+        qkv, tab = shifted(q0, off), shifted(torch.zeros(L, 2, 36, device=DEV), off)
+        assert _lib().qwk_vit_rope_table(P(pos), L, P(tab), S()) == 0
+        assert _lib().qwk_vit_bias_rope(P(qkv), P(shifted(bias, off)), P(tab), L, heads, S()) == 0
+        return qkv
+    got = rope(off)
+    assert torch.equal(got, rope(0))
+    v = (q0.double() + bias.double()).view(L, 3, heads, 2, 36)
+    ang = torch.cat([pos[:, :1].double(), pos[:, 1:].double()], 1).repeat_interleave(18, 1) * (10000.0 ** (-2.0 * torch.arange(18, device=DEV).double() / 36)).repeat(2)
+    c, s = ang.cos()[:, None, None], ang.sin()[:, None, None]
+    a, b = v[:, :2, :, 0], v[:, :2, :, 1]
+    want = v.clone()
+    want[:, :2, :, 0], want[:, :2, :, 1] = a * c - b * s, b * c + a * s
+    assert torch.allclose(got.double().view(L, 3, heads, 2, 36), want, rtol=2 ** -8, atol=2e-5)

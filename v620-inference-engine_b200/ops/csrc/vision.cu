@@ -106,45 +106,42 @@ __global__ void __launch_bounds__(256) vit_rope_table_kernel(const int *pos_hw, 
     tab[(long long)n * 2 * VHALF + VHALF + t] = sn;
 }
 
-__device__ __forceinline__ void vit_unpack4(const bf16 *p, float (&v)[4]) {
-    const uint2 u = *reinterpret_cast<const uint2 *>(p);
-    v[0] = bf16_lo(u.x); v[1] = bf16_hi(u.x); v[2] = bf16_lo(u.y); v[3] = bf16_hi(u.y);
-}
-__device__ __forceinline__ void vit_pack4(bf16 *p, const float (&v)[4]) {
-    *reinterpret_cast<uint2 *>(p) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
-}
-
-// One block per patch: bias on the whole row, rotary on q and k, four values (of each half of a head) per step.
+// One block per patch: bias on the whole row, rotary on q and k, V values (of each half of a head) per step: four, or one where a
+// pointer does not allow it.
+template <int V>
 __global__ void __launch_bounds__(256) vit_bias_rope_kernel(bf16 *qkv, const float *bias, const float *tab, int heads) {
     const int n = blockIdx.x, D = heads * VHD;
     bf16 *row = qkv + (long long)n * 3 * D;
     const float *cs = tab + (long long)n * 2 * VHALF, *sn = cs + VHALF;
-    const int rot = 2 * heads * (VHALF / 4), total = rot + D / 4;
+    const int rot = 2 * heads * (VHALF / V), total = rot + D / V;
     for (int i = threadIdx.x; i < total; i += 256) {
-        float a[4];
+        float a[V], e[V];
         if (i >= rot) {
-            const int c = 2 * D + (i - rot) * 4;
-            const float4 e = vit_ld4(bias + c);
-            vit_unpack4(row + c, a);
-            a[0] += e.x; a[1] += e.y; a[2] += e.z; a[3] += e.w;
-            vit_pack4(row + c, a);
+            const int c = 2 * D + (i - rot) * V;
+            ld_cols<V>(row + c, a);
+            ld_cols<V>(bias + c, e);
+#pragma unroll
+            for (int k = 0; k < V; ++k) a[k] += e[k];
+            st_cols<V>(row + c, a);
             continue;
         }
-        const int hh = i / (VHALF / 4), t = (i - hh * (VHALF / 4)) * 4, c = hh * VHD + t;      // hh over q heads then k heads
-        const float4 ea = vit_ld4(bias + c), eb = vit_ld4(bias + c + VHALF), co = vit_ld4(cs + t), si = vit_ld4(sn + t);
-        float b[4], o[4], p[4];
-        vit_unpack4(row + c, a);
-        vit_unpack4(row + c + VHALF, b);
-        a[0] += ea.x; a[1] += ea.y; a[2] += ea.z; a[3] += ea.w;
-        b[0] += eb.x; b[1] += eb.y; b[2] += eb.z; b[3] += eb.w;
-        const float cc[4] = {co.x, co.y, co.z, co.w}, ss[4] = {si.x, si.y, si.z, si.w};
+        const int hh = i / (VHALF / V), t = (i - hh * (VHALF / V)) * V, c = hh * VHD + t;      // hh over q heads then k heads
+        float b[V], f[V], co[V], si[V], o[V], p[V];
+        ld_cols<V>(row + c, a);
+        ld_cols<V>(row + c + VHALF, b);
+        ld_cols<V>(bias + c, e);
+        ld_cols<V>(bias + c + VHALF, f);
+        ld_cols<V>(cs + t, co);
+        ld_cols<V>(sn + t, si);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            o[k] = a[k] * cc[k] - b[k] * ss[k];
-            p[k] = b[k] * cc[k] + a[k] * ss[k];
+        for (int k = 0; k < V; ++k) {
+            a[k] += e[k];
+            b[k] += f[k];
+            o[k] = a[k] * co[k] - b[k] * si[k];
+            p[k] = b[k] * co[k] + a[k] * si[k];
         }
-        vit_pack4(row + c, o);
-        vit_pack4(row + c + VHALF, p);
+        st_cols<V>(row + c, o);
+        st_cols<V>(row + c + VHALF, p);
     }
 }
 
@@ -215,7 +212,8 @@ QW_API int qwk_vit_rope_table(const int *pos_hw, int L, float *tab, cudaStream_t
 }
 
 QW_API int qwk_vit_bias_rope(void *qkv, const float *bias, const float *tab, int L, int heads, cudaStream_t s) {
-    vit_bias_rope_kernel<<<L, 256, 0, s>>>((bf16 *)qkv, bias, tab, heads);
+    if (aligned16((bf16 *)qkv, bias, tab)) vit_bias_rope_kernel<4><<<L, 256, 0, s>>>((bf16 *)qkv, bias, tab, heads);
+    else vit_bias_rope_kernel<1><<<L, 256, 0, s>>>((bf16 *)qkv, bias, tab, heads);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
