@@ -216,3 +216,13 @@ def test_vision_rotary_at_any_address(heads, off):
     want = v.clone()
     want[:, :2, :, 0], want[:, :2, :, 1] = a * c - b * s, b * c + a * s
     assert torch.allclose(got.double().view(L, 3, heads, 2, 36), want, rtol=2 ** -8, atol=2e-5)
+
+
+def test_vision_gelu_of_more_rows_than_a_grid_is_high():
+    """600,000 rows of eight columns."""
+    L, D = 600_000, 8
+    rn = gen(1)
+    y, bias = rn(L, D).to(torch.bfloat16), rn(D)
+    want = torch.nn.functional.gelu(y.float() + bias, approximate="tanh")
+    assert _lib().qwk_vit_bias_gelu(P(y), P(bias), L, D, 1, S()) == 0
+    assert torch.allclose(y.float(), want, rtol=2 ** -8, atol=1e-6)

@@ -153,12 +153,12 @@ constexpr int VG_ROWS = 8;
 // Eight columns per thread (their bias in registers) down eight rows: 16-byte accesses.  At 3520 x 4304 53 us with two-byte
 // accesses, a division per value for its column; 19 now.
 __global__ void __launch_bounds__(128) vit_bias_gelu8_kernel(bf16 *y, const float *bias, int L, int D, int tanh_form) {
-    const int c = (blockIdx.x * 128 + threadIdx.x) * 8;
+    const int c = (blockIdx.y * 128 + threadIdx.x) * 8;
     if (c >= D) return;
     float e[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) e[k] = bias[c + k];
-    const int n0 = blockIdx.y * VG_ROWS, n1 = min(L, n0 + VG_ROWS);
+    const int n0 = blockIdx.x * VG_ROWS, n1 = min(L, n0 + VG_ROWS);
 #pragma unroll 4
     for (int n = n0; n < n1; ++n) {
         uint4 *p = reinterpret_cast<uint4 *>(y + (long long)n * D + c);
@@ -219,7 +219,7 @@ QW_API int qwk_vit_bias_rope(void *qkv, const float *bias, const float *tab, int
 
 QW_API int qwk_vit_bias_gelu(void *y, const float *bias, int L, int D, int tanh_form, cudaStream_t s) {
     if ((D & 7) == 0 && ((uintptr_t)y & 15) == 0) {
-        dim3 grid((D / 8 + 127) / 128, (L + VG_ROWS - 1) / VG_ROWS);
+        dim3 grid((L + VG_ROWS - 1) / VG_ROWS, (D / 8 + 127) / 128);
         vit_bias_gelu8_kernel<<<grid, 128, 0, s>>>((bf16 *)y, bias, L, D, tanh_form);
     } else {
         const long long total = (long long)L * D;
