@@ -226,3 +226,11 @@ def test_vision_gelu_of_more_rows_than_a_grid_is_high():
     want = torch.nn.functional.gelu(y.float() + bias, approximate="tanh")
     assert _lib().qwk_vit_bias_gelu(P(y), P(bias), L, D, 1, S()) == 0
     assert torch.allclose(y.float(), want, rtol=2 ** -8, atol=1e-6)
+
+
+def test_logits_reduction_of_more_rows_than_a_grid_is_high():
+    from qwb200.ops import kernels as K
+    x = gen(2)(70_000, 9)
+    val, idx, mx, sm = K.row_reduce(x)
+    assert torch.equal(val, x.max(1).values) and torch.equal(idx.long(), x.argmax(1))
+    assert torch.allclose(torch.log(sm) + mx, torch.logsumexp(x, 1), atol=1e-5)

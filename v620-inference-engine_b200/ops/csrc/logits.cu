@@ -9,7 +9,7 @@ namespace qw {
 
 // A row is reduced by a cluster of eight CTAs, each with an eighth of the columns: its own maximum first, the sum of exponentials
 // around it from a second pass (L1 / L2), and rank 0 puts the eight parts together.  One CTA per row took 32 us for 248,320
-// logits (one SM's loads in flight); eight take 7.  grid (8, M), 512 threads.  out_val[m], out_idx[m] (index offset by idx0); lse
+// logits (one SM's loads in flight); eight take 7.  grid 8 M, 512 threads.  out_val[m], out_idx[m] (index offset by idx0); lse
 // parts: out_max[m], out_sum[m].
 constexpr int RR_CTAS = 8, RR_THREADS = 512;
 __global__ void __cluster_dims__(RR_CTAS, 1, 1) __launch_bounds__(RR_THREADS) row_reduce_kernel(const float *logits, int ld, int V, int idx0,
@@ -23,9 +23,9 @@ __global__ void __cluster_dims__(RR_CTAS, 1, 1) __launch_bounds__(RR_THREADS) ro
     cg::cluster_group cl = cg::this_cluster();
     cl.sync();          // every CTA of the cluster runs: rank 0's memory may be written (before the wait for the logits, which is longer)
     pdl_wait();
-    const int m = blockIdx.y, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int m = blockIdx.x / RR_CTAS, rank = blockIdx.x % RR_CTAS, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const float *l = logits + (long long)m * ld;
-    const int per = ((V + RR_CTAS - 1) / RR_CTAS + 3) & ~3, c0 = blockIdx.x * per, c1 = min(V, c0 + per);
+    const int per = ((V + RR_CTAS - 1) / RR_CTAS + 3) & ~3, c0 = rank * per, c1 = min(V, c0 + per);
     const bool vec = ((uintptr_t)l & 15) == 0;
     float bv = -INFINITY;
     int bi = 0x7fffffff;
@@ -70,12 +70,12 @@ __global__ void __cluster_dims__(RR_CTAS, 1, 1) __launch_bounds__(RR_THREADS) ro
         z = block_sum<RR_THREADS>(z, scratch);
     }
     if (threadIdx.x == 0) {
-        *cl.map_shared_rank(&part_max[blockIdx.x], 0) = mx;
-        *cl.map_shared_rank(&part_idx[blockIdx.x], 0) = si[0];
-        *cl.map_shared_rank(&part_sum[blockIdx.x], 0) = z;
+        *cl.map_shared_rank(&part_max[rank], 0) = mx;
+        *cl.map_shared_rank(&part_idx[rank], 0) = si[0];
+        *cl.map_shared_rank(&part_sum[rank], 0) = z;
     }
     cl.sync();
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (rank == 0 && threadIdx.x == 0) {
         float M = part_max[0];
         int at = part_idx[0];
         for (int r = 1; r < RR_CTAS; ++r)                            // ranks hold ascending columns: a later equal one does not win
@@ -167,7 +167,7 @@ QW_API int qwk_advance_rows(int *tokens, int *pos, int *ctx3, const int *next, i
 QW_API int qwk_row_reduce(const float *logits, int ld, int V, int idx0, int M, float *out_val, int *out_idx,
                           float *out_max, float *out_sum, cudaStream_t s) {
     if (M <= 0) return 0;
-    return launch_pdl(row_reduce_kernel, dim3(RR_CTAS, M), dim3(RR_THREADS), 0, s, logits, ld, V, idx0, out_val, out_idx, out_max, out_sum) ==
+    return launch_pdl(row_reduce_kernel, dim3((unsigned)(RR_CTAS * (long long)M)), dim3(RR_THREADS), 0, s, logits, ld, V, idx0, out_val, out_idx, out_max, out_sum) ==
                    cudaSuccess ? 0 : -2;
 }
 
