@@ -234,3 +234,33 @@ def test_logits_reduction_of_more_rows_than_a_grid_is_high():
     val, idx, mx, sm = K.row_reduce(x)
     assert torch.equal(val, x.max(1).values) and torch.equal(idx.long(), x.argmax(1))
     assert torch.allclose(torch.log(sm) + mx, torch.logsumexp(x, 1), atol=1e-5)
+
+
+@pytest.mark.parametrize("SH,R,n_inj,M", [(6400, 8, 4, 1), (6400, 8, 4, 9), (10240, 16, 0, 3), (32, 320, 300, 5), (32, 64, 500, 1)])
+def test_mixers_with_long_rows_and_with_many_inject_rows(SH, R, n_inj, M):
+    """Rows that leave no room for the tensor-core form's operands, and more low-rank and inject rows than a block has threads, against
+    64 bits (fp32 sums of up to 10,240 exact products: 1e-5 of the result's size; the block input is rounded to bf16 once)."""
+    L, hc, eps, H = _lib(), 4, 1e-6, SH
+    down = R + n_inj
+    ld = (hc + hc * down + 3) // 4 * 4
+    rn = gen(SH + M)
+    X, pend, ip, w1 = rn(M, hc, SH), rn(M, SH), rn(M, hc), 1 + 0.1 * rn(hc, SH)
+    Wd, Wu = (rn(down, hc, SH) * 0.05).to(torch.bfloat16), (rn(SH, hc, R) * 0.1).to(torch.bfloat16)
+    xo, send = torch.zeros_like(X), torch.zeros(M, ld, device=DEV)
+    assert L.qwk_hc_down(P(X), P(xo), P(pend), SH, P(ip), P(w1), P(Wd), P(send), ld, SH, hc, down, M, S()) == 0
+    x = X.double() + pend.double()[:, None] * (2 * torch.sigmoid(ip.double() / hc))[..., None]
+    assert torch.allclose(xo.double(), x, rtol=1e-5, atol=1e-5)
+    y = (xo * w1).to(torch.bfloat16).double()
+    part = torch.einsum("msc,jsc->msj", y, Wd.double())
+    got = send[:, hc:hc + hc * down].view(M, hc, down).double()
+    assert float((got - part).norm() / part.norm()) < 1e-5
+    assert torch.allclose(send[:, :hc].double(), xo.double().pow(2).sum(-1), rtol=1e-5)
+    inj, out = torch.zeros(M, max(n_inj, 1), device=DEV), torch.zeros(M, SH, dtype=torch.bfloat16, device=DEV)
+    assert L.qwk_hc_up_mix(P(send), ld, P(Wu), P(xo), P(w1), SH, hc, R, n_inj, H, C.c_float(eps), M, P(inj) if n_inj else None, max(n_inj, 1), P(out), SH, 0, S()) == 0
+    r = torch.rsqrt(xo.double().pow(2).mean(-1) + eps)
+    d = (r[..., None] * part).sum(1)
+    if n_inj:
+        assert float((inj.double() - d[:, R:]).norm() / d[:, R:].norm()) < 1e-5
+    gate = torch.sigmoid(torch.einsum("csr,mr->msc", Wu.double(), torch.nn.functional.silu(d[:, :R] / hc)))
+    want = (gate * y * r[..., None]).mean(1)
+    assert float((out.double() - want).norm() / want.norm()) < 5e-3

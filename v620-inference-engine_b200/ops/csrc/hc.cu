@@ -72,10 +72,11 @@ __global__ void __launch_bounds__(256) hc_pre_kernel(float *X, const float *pend
 constexpr int UP_ROWS = 4;     // rows per block of the fused hc_up_mix
 constexpr int UP_MAXI = 5;     // 16-byte weight pieces per lane: covers mixer ranks up to 320
 
-// The form with the collectives inside (several ranks): waits for the all-reduce of the down projection, sends the all-gather.
+// FUSED: the form with the collectives inside (several ranks): waits for the all-reduce of the down projection, sends the all-gather.
+// Otherwise: without them, for more low-rank and inject rows than hc_up_mma_kernel has threads.
 // grid (ceil(SH/8), ceil(M/UPR)), 256 threads.  hc must be 4 (one 8-lane group per stream).
 // y[s][c] = bf16(X[s][c] * w1[s][c]) is recomputed here exactly as hc_down_kernel computed it.
-template <int UPR>
+template <bool FUSED, int UPR>
 __global__ void __launch_bounds__(256, 3) hc_up_mix_kernel(const float *red, int ld_red, const bf16 *Wu /* [SH][hc][R] */,
                                                         const float *X, const float *w1, int SH, int hc, int R, int hc_down,
                                                         float inv_H, float eps, int M, float *inj, int ld_inj, bf16 *bin,
@@ -109,13 +110,17 @@ __global__ void __launch_bounds__(256, 3) hc_up_mix_kernel(const float *red, int
         for (int mm = 0; mm < UPR; ++mm)
             xw[mm] = (c < SH && mm < nrow) ? __ldcg(X + ((long long)(m0 + mm) * hc + s) * SH + c) * w1v : 0.f;
     }
-    // the reduced vector: the ranks' words added in rank order, staged once per block into shared memory, with every
+    // the reduced vector (FUSED: the ranks' words added in rank order), staged once per block into shared memory, with every
     // thread's loads in flight together
     float *reds = rs + UPR * hc;       // [UPR][ld_red]
-    const unsigned int seq_in = fuse_seq(fi);
+    if constexpr (!FUSED) {
+        const int used = hc + hc * hc_down;
+        for (int i = threadIdx.x; i < nrow * used; i += 256) reds[i / used * ld_red + i % used] = __ldcg(red + (long long)(m0 + i / used) * ld_red + i % used);
+    }
+    const unsigned int seq_in = FUSED ? fuse_seq(fi) : 0u;
     // what this mixer's down projection wrote of each row (an even count), as pairs of words; a thread has
     // the loads of two pairs from four ranks in flight at once
-    const int npair = (hc + hc * hc_down) >> 1, total = nrow * npair;
+    const int npair = (hc + hc * hc_down) >> 1, total = FUSED ? nrow * npair : 0;
     for (int p0 = threadIdx.x; p0 < total; p0 += 512) {
         const int p1 = p0 + 256;
         const bool two = p1 < total;
@@ -147,7 +152,7 @@ __global__ void __launch_bounds__(256, 3) hc_up_mix_kernel(const float *red, int
     }
     __syncthreads();
     if (c >= SH) return;
-    const unsigned int seq_out = fuse_seq(fo);
+    const unsigned int seq_out = FUSED ? fuse_seq(fo) : 0u;
     float acc[UPR];
 #pragma unroll
     for (int mm = 0; mm < UPR; ++mm) acc[mm] = 0.f;
@@ -182,7 +187,8 @@ __global__ void __launch_bounds__(256, 3) hc_up_mix_kernel(const float *red, int
         v += __shfl_xor_sync(0xffffffffu, v, 16);
         if (lane == 0 && mm < nrow) {
             const bf16 o = __float2bfloat16(v / float(hc));
-            fuse_put_all(fo, seq_out, m0 + mm, c, (unsigned int)__bfloat16_as_ushort(o));      // fused all-gather
+            if (FUSED) fuse_put_all(fo, seq_out, m0 + mm, c, (unsigned int)__bfloat16_as_ushort(o));      // fused all-gather
+            else bin[(long long)(m0 + mm) * ld_bin + bin_col0 + c] = o;
         }
     }
 }
@@ -214,7 +220,8 @@ struct HcDownArgs {
     FuseOut fo;             // fused all-reduce of `send`
 };
 
-// The form with the collectives inside (several ranks).
+// FUSED: the form with the collectives inside (several ranks).  Otherwise: without them, for rows that hc_down_mma_kernel has no room for.
+template <bool FUSED>
 __global__ void __launch_bounds__(256, 3) hc_down_kernel(HcDownArgs a) {
     extern __shared__ __align__(16) unsigned char smraw[];
     bf16 *ybuf = reinterpret_cast<bf16 *>(smraw);          // [8][SH]
@@ -240,8 +247,9 @@ __global__ void __launch_bounds__(256, 3) hc_down_kernel(HcDownArgs a) {
     pf_issue(a.pf);
     pdl_wait();
     pdl_trigger();
-    const unsigned int seq_in = a.fi.active ? fuse_seq(a.fi) : 0u;
-    const unsigned int seq_out = fuse_seq(a.fo);
+    const bool scattered = FUSED && a.fi.active;
+    const unsigned int seq_in = scattered ? fuse_seq(a.fi) : 0u;
+    const unsigned int seq_out = FUSED ? fuse_seq(a.fo) : 0u;
     for (int r = 0; r < nrow; ++r) {           // the whole block builds each row slice: short dependent chains
         const int m = m0 + r;
         const float *xin = a.Xin + ((long long)m * a.hc + s) * a.SH;
@@ -257,7 +265,7 @@ __global__ void __launch_bounds__(256, 3) hc_down_kernel(HcDownArgs a) {
                 if (c < a.SH) {
                     xv[q] = __ldcg(reinterpret_cast<const float4 *>(xin + c));
                     wv[q] = __ldg(reinterpret_cast<const float4 *>(a.w1 + s * a.SH + c));
-                    if (a.pend && !a.fi.active) pv[q] = __ldcg(reinterpret_cast<const float4 *>(a.pend + (long long)m * a.ld_pend + c));
+                    if (a.pend && !scattered) pv[q] = __ldcg(reinterpret_cast<const float4 *>(a.pend + (long long)m * a.ld_pend + c));
                 }
             }
 #pragma unroll
@@ -267,7 +275,7 @@ __global__ void __launch_bounds__(256, 3) hc_down_kernel(HcDownArgs a) {
                     float4 v = xv[q];
                     if (a.pend) {
                         // fused reduce-scatter: the ranks' parts of the block output, added in rank order
-                        const float4 p = a.fi.active ? fuse_sum4(a.fi, seq_in, (long long)m * a.ld_pend + c) : pv[q];
+                        const float4 p = scattered ? fuse_sum4(a.fi, seq_in, (long long)m * a.ld_pend + c) : pv[q];
                         v.x = fmaf(p.x, coef, v.x); v.y = fmaf(p.y, coef, v.y);
                         v.z = fmaf(p.z, coef, v.z); v.w = fmaf(p.w, coef, v.w);
                         if (blockIdx.x == 0) *reinterpret_cast<float4 *>(a.Xout + ((long long)m * a.hc + s) * a.SH + c) = v;
@@ -283,7 +291,8 @@ __global__ void __launch_bounds__(256, 3) hc_down_kernel(HcDownArgs a) {
         if (blockIdx.x == 0) {                 // block-uniform: only these blocks need the sum of squares
             ss = block_sum<256>(ss, scratch);
             if (threadIdx.x == 0) {
-                fuse_put_all(a.fo, seq_out, m, s, __float_as_uint(ss));      // fused all-reduce
+                if (FUSED) fuse_put_all(a.fo, seq_out, m, s, __float_as_uint(ss));      // fused all-reduce
+                else a.send[(long long)m * a.ld_send + s] = ss;
             }
         }
     }
@@ -330,7 +339,10 @@ __global__ void __launch_bounds__(256, 3) hc_down_kernel(HcDownArgs a) {
     if (kw == 0 && lane == 0 && j < a.down) {
 #pragma unroll
         for (int m = 0; m < 8; ++m)
-            if (m < nrow) fuse_put_all(a.fo, seq_out, m0 + m, a.hc + s * a.down + j, __float_as_uint(acc[m]));
+            if (m < nrow) {
+                if (FUSED) fuse_put_all(a.fo, seq_out, m0 + m, a.hc + s * a.down + j, __float_as_uint(acc[m]));
+                else a.send[(long long)(m0 + m) * a.ld_send + a.hc + s * a.down + j] = acc[m];
+            }
     }
 }
 
@@ -637,7 +649,8 @@ static void hc_configure() {
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
     if (!attr_set[dev]) {
-        cudaFuncSetAttribute(hc_down_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+        cudaFuncSetAttribute(hc_down_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+        cudaFuncSetAttribute(hc_down_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
         cudaFuncSetAttribute(hc_down_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         cudaFuncSetAttribute(hc_up_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
         cudaFuncSetAttribute(hc_up_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
@@ -649,11 +662,11 @@ static void hc_configure() {
 QW_API int qwk_hc_up_mix(const float *red, int ld_red, const void *Wu, const float *X, const float *w1, int SH, int hc,
                          int R, int n_inj, int H, float eps, int M, float *inj, int ld_inj, void *bin, int ld_bin,
                          int bin_col0, cudaStream_t s) {
-    if (hc != 4 || (R & 7) || R > 8 * 8 * UP_MAXI || R + n_inj > HM_THREADS) return -1;
+    if (hc != 4 || (R & 7) || R > 8 * 8 * UP_MAXI) return -1;
     const FuseIn fi = take_fi();
     const FuseOut fo = take_fo();
     if ((fi.active != 0) != (fo.mode != 0)) return -1;          // the fused mixer both receives and sends
-    if (!fi.active) {
+    if (!fi.active && R + n_inj <= HM_THREADS) {
         hc_configure();
         const size_t smem = sizeof(bf16) * (3 * HM_ROWS + 4 * HU_COLS) * (((R + 31) & ~31) + HU_PAD);
         const int blocks = (SH + HU_COLS - 1) / HU_COLS;
@@ -667,7 +680,7 @@ QW_API int qwk_hc_up_mix(const float *red, int ld_red, const void *Wu, const flo
     dim3 grid((SH + 7) / 8, (M + UP_ROWS - 1) / UP_ROWS);
     const size_t smem = sizeof(float) * ((size_t)UP_ROWS * R + UP_ROWS * hc + (size_t)UP_ROWS * ld_red);
     if (smem > 48 * 1024) return -1;
-    return launch_pdl(hc_up_mix_kernel<UP_ROWS>, grid, dim3(256), smem, s, red, ld_red, (const bf16 *)Wu, X, w1, SH, hc, R, R + n_inj,
+    return launch_pdl(fi.active ? hc_up_mix_kernel<true, UP_ROWS> : hc_up_mix_kernel<false, UP_ROWS>, grid, dim3(256), smem, s, red, ld_red, (const bf16 *)Wu, X, w1, SH, hc, R, R + n_inj,
                       1.f / float(H), eps, M, inj, ld_inj, (bf16 *)bin, ld_bin, bin_col0, take_pf(), fi, fo) == cudaSuccess ? 0 : -2;
 }
 
@@ -682,10 +695,10 @@ QW_API int qwk_hc_down(const float *Xin, float *Xout, const float *pend, int ld_
     a.fi = take_fi(); a.fo = take_fo();
     if (a.fi.active && !a.fo.mode) return -1;          // a fused down projection always sends its all-reduce
     hc_configure();
-    if (!a.fo.mode) {
+    // room for eight weight rows and eight rows of the step, whatever M is: a row's sums do not depend on the rows beside it
+    if (!a.fo.mode && sizeof(bf16) * (HD_J + HD_ROWS) * (SH + HM_PAD) <= 200 * 1024) {
         const int tiles = (down + HD_J - 1) / HD_J;
         const size_t smem = sizeof(bf16) * (size_t)(HD_J + (M < HD_ROWS ? M : HD_ROWS)) * (SH + HM_PAD);
-        if (smem > 200 * 1024) return -1;
         if (M < HD_CLUSTER_MIN) return launch_pdl(hc_down_mma_kernel<false>, dim3(tiles, hc), dim3(HM_THREADS), smem, s, a) == cudaSuccess ? 0 : -2;
         return launch_pdl_cluster(hc_down_mma_kernel<true>, HD_CL, dim3((tiles + HD_CL - 1) / HD_CL * HD_CL, hc), dim3(HM_THREADS), smem, s, a) ==
                        cudaSuccess ? 0 : -2;
@@ -698,5 +711,5 @@ QW_API int qwk_hc_down(const float *Xin, float *Xout, const float *pend, int ld_
     const int rpb = 8 / a.wpr;
     dim3 grid((down + rpb - 1) / rpb, hc, (M + 7) / 8);
     const size_t smem = (size_t)8 * SH * sizeof(bf16);
-    return launch_pdl(hc_down_kernel, grid, dim3(256), smem, s, a) == cudaSuccess ? 0 : -2;
+    return launch_pdl(a.fo.mode ? hc_down_kernel<true> : hc_down_kernel<false>, grid, dim3(256), smem, s, a) == cudaSuccess ? 0 : -2;
 }
