@@ -68,6 +68,7 @@ int qwk_mtp_add(const float *fh, const float *fe, int H, int hc, float *X, int M
 int qwk_p2p_allreduce(const void *p2p, unsigned int k, const float *src, float *dst, int rows, int n, cudaStream_t s);
 int qwk_p2p_reduce_scatter(const void *p2p, unsigned int k, const float *src, float *dst, int rows, int n, cudaStream_t s);
 int qwk_p2p_allgather(const void *p2p, unsigned int k, int kind, long long off, int rows, int n, int elem, cudaStream_t s);
+int qwk_fuse_next(const void *p2p, int in_kind, unsigned int in_k, int in_n, int out_kind, unsigned int out_k, int out_mode, int out_n);
 int qwk_p2p_bump_base(const void *p2p, unsigned int by, cudaStream_t s);
 
 // ple.cu

@@ -197,6 +197,15 @@ QW_API int qwk_p2p_allgather(const void *p2p, unsigned int k, int kind, long lon
     return launch_pdl(p2p_exchange_kernel, dim3(p->ranks + 1), dim3(256), 0, s, a, 1) == cudaSuccess ? 0 : -2;
 }
 
+// What the next launch of this thread's stream of calls fuses, as the step's schedule sets it: it receives collective in_k of kind in_kind
+// (negative: nothing) and sends out_k of out_kind (out_mode 1: to every rank, 2: columns to their owner).  For tests of single kernels.
+QW_API int qwk_fuse_next(const void *p2p, int in_kind, unsigned int in_k, int in_n, int out_kind, unsigned int out_k, int out_mode, int out_n) {
+    if (!p2p || in_kind > 2 || out_kind > 2) return -1;
+    g_fi = in_kind < 0 ? FuseIn{} : make_fuse_in(p2p, in_kind, in_k, in_n);
+    g_fo = out_kind < 0 ? FuseOut{} : make_fuse_out(p2p, out_kind, out_k, out_mode, out_n);
+    return 0;
+}
+
 QW_API int qwk_p2p_bump_base(const void *p2p, unsigned int by, cudaStream_t s) {
     const QwP2P *p = (const QwP2P *)p2p;
     return launch_pdl(bump_base_kernel, dim3(1), dim3(32), 0, s, p->base, by) == cudaSuccess ? 0 : -2;
