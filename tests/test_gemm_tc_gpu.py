@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("T,N,K", [(128, 128, 64), (128, 128, 256), (256, 384, 2560), (200, 324, 2560), (4096, 512, 2560),
                                    (77, 130, 328),
-                                   # wide enough (N >= 1024, >= 74 tiles) for the 128 x 256 tile form, with ragged edges
+                                   # products that run in CTA pairs, with ragged edges
                                    (1024, 2560, 320), (2000, 1536, 640), (4096, 1200, 128), (1111, 10240, 64)])
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
 def test_gemm_tc_matches_fp32(T, N, K, out_dtype):
@@ -28,12 +28,12 @@ def test_gemm_tc_matches_fp32(T, N, K, out_dtype):
 
 @pytest.mark.parametrize("T,N,K", [(1, 128, 512), (100, 2560, 6144), (100, 1793, 2560), (129, 324, 10240), (64, 100, 520), (200, 130, 4304),
                                    (300, 2560, 1024), (128, 128, 4096),
-                                   # the line between the forms: 129-row and 256-row products in pairs, padded pairs, wide tiles
+                                   # the line between the forms: 129-row and 257-row products in pairs, padded pairs
                                    (129, 10240, 1152), (777, 4304, 512), (257, 16480, 128)])
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
 def test_gemm_tc_split_and_padded_forms_match_64_bits(T, N, K, out_dtype):
     """Few tiles shared by clusters of 2, 4 and 8 CTAs (k blocks that do not divide evenly, ragged rows and columns) and the padded
-    pair and wide forms: fp32 sums of exact products (1e-5 of the result's size for K <= 10240; bf16 output 2^-9 more), twice the
+    pair form: fp32 sums of exact products (1e-5 of the result's size for K <= 10240; bf16 output 2^-9 more), twice the
     same bits, and nothing outside the result written."""
     from qwb200.ops import kernels as K_
     g = torch.Generator(device="cuda").manual_seed(T + N + K)
@@ -249,3 +249,94 @@ def test_mixer_up_projection_with_the_mean_in_its_epilogue(T, SH, R):
     ref = (gate * xn.double()).mean(1)
     assert torch.all(out[T:].float() == 768.0) and torch.all(out[:, SH:].float() == 768.0)
     assert float((out[:T, :SH].double() - ref).norm() / ref.norm()) < 2 ** -8
+
+
+def _against_64_bits(T, N, K, out_dtype):
+    """fp32 sums of exact products (1e-5 of the result's size for K <= 2560; bf16 output 2^-9 more), and nothing outside the result."""
+    from qwb200.ops import kernels as K_
+    g = torch.Generator(device="cuda").manual_seed(T + N + K + 2)
+    A = torch.randn(T, K, generator=g, device="cuda").to(torch.bfloat16)
+    W = (torch.randn(N, K, generator=g, device="cuda") * 0.05).to(torch.bfloat16)
+    out = torch.full((T + 2, (N + 7) // 8 * 8 + 8), 768.0, dtype=out_dtype, device="cuda")
+    K_.gemm_bf16_tc(A, W, out=out[:T, :N])
+    ref = A.double() @ W.double().T
+    assert torch.all(out[:, N:].float() == 768.0) and torch.all(out[T:].float() == 768.0)
+    assert float((out[:T, :N].double() - ref).norm() / ref.norm()) < (1e-5 if out_dtype == torch.float32 else 2 ** -8)
+
+
+@pytest.mark.parametrize("T,N,K", [(520, 12800, 2560), (640, 12700, 72), (777, 10200, 320), (300, 10190, 136)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("stage", [1, 0])
+def test_gemm_tc_wide_tiles_match_64_bits(T, N, K, out_dtype, stage):
+    """128 x 256 tiles, with the fp32 output through the staging buffers and straight from registers, ragged rows and columns."""
+    from qwb200.ops import lib as qlib
+    L = qlib.load(True)
+    assert L.qwk_gemm_tc_form(T, N, K, 0) == 1
+    old = L.qwk_gemm_tc_stage_local(stage)
+    try:
+        _against_64_bits(T, N, K, out_dtype)
+    finally:
+        L.qwk_gemm_tc_stage_local(old)
+
+
+@pytest.mark.parametrize("T,SH,R,form", [(300, 2560, 320, 1), (3001, 2560, 320, 1), (520, 3200, 40, 1), (1021, 2560, 320, 0)])
+def test_mixer_up_projection_in_both_tile_forms(T, SH, R, form):
+    from qwb200.ops import lib as qlib
+    assert qlib.load(True).qwk_gemm_tc_form(T, 4 * SH, R, 1) == form
+    test_mixer_up_projection_with_the_mean_in_its_epilogue(T, SH, R)
+
+
+@pytest.fixture
+def only_pairs():
+    """Every product of more than 128 rows and at least 256 columns that is not split runs in CTA pairs."""
+    import ctypes as C
+    from qwb200.ops import lib as qlib
+    L = qlib.load(True)
+    old = L.qwk_gemm_tc_pair_min_n(-256)
+    word = torch.zeros(2, dtype=torch.int32, device="cuda")
+    L.qwk_set_error_word(C.c_void_p(word.data_ptr()))
+    yield word
+    torch.cuda.synchronize()
+    L.qwk_set_error_word(None)
+    L.qwk_gemm_tc_pair_min_n(old)
+
+
+@pytest.mark.parametrize("T,N,K", [(256, 256, 64), (512, 512, 256), (300, 700, 192), (1111, 1536, 128), (129, 300, 72), (257, 257, 320)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_gemm_tc_pairs_of_small_and_ragged_products_match_64_bits(only_pairs, T, N, K, out_dtype):
+    from qwb200.ops import lib as qlib
+    assert qlib.load(True).qwk_gemm_tc_form(T, N, K, 0) == 2
+    _against_64_bits(T, N, K, out_dtype)
+    assert only_pairs.tolist() == [0, 0]
+
+
+@pytest.mark.parametrize("T,N,K", [(1024, 2048, 256), (300, 512, 128), (129, 256, 64)])
+def test_gemm_tc_pair_form_reduce_scatter_with_ragged_rows(only_pairs, T, N, K):
+    test_gemm_tc_reduce_scatter_epilogue_on_emulated_ranks(T, N, K)
+
+
+def test_gemm_tc_wide_form_reduce_scatter():
+    from qwb200.ops import lib as qlib
+    assert qlib.load(True).qwk_gemm_tc_form(520, 12800, 64, 0) == 1
+    test_gemm_tc_reduce_scatter_epilogue_on_emulated_ranks(520, 12800, 64)
+
+
+@pytest.mark.parametrize("N,K", [(2560, 6144), (1793, 2560), (324, 4304), (12800, 640)])
+def test_gemm_tc_rows_keep_their_bits_on_each_side_of_the_split_line(N, K):
+    """Up to 256 rows, and from 257 on through single, wide and paired tiles: a row's result does not depend on the rows beside it.  Where
+    few tiles are split over clusters the two sides differ by the rounding of the sum: each is within 1e-5 of 64 bits."""
+    from qwb200.ops import kernels as K_, lib as qlib
+    L = qlib.load(True)
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    A = torch.randn(4096, K, generator=g, device="cuda").to(torch.bfloat16)
+    W = (torch.randn(N, K, generator=g, device="cuda") * 0.05).to(torch.bfloat16)
+    whole, head = K_.gemm_bf16_tc(A, W), K_.gemm_bf16_tc(A[:256], W)
+    tail = K_.gemm_bf16_tc(A[4096 - 256:], W)
+    for T in (1, 33, 100, 128, 129, 200):
+        assert torch.equal(K_.gemm_bf16_tc(A[:T], W), head[:T]) and torch.equal(K_.gemm_bf16_tc(A[4096 - T:], W), tail[256 - T:]), T
+    for T in (257, 520, 777, 1021, 2048):
+        assert torch.equal(K_.gemm_bf16_tc(A[:T], W), whole[:T]) and torch.equal(K_.gemm_bf16_tc(A[4096 - T:], W), whole[4096 - T:]), T
+    if L.qwk_gemm_tc_form(256, N, K, 0) != 3:
+        assert torch.equal(head, whole[:256])
+    else:
+        assert float((head - whole[:256]).double().norm() / head.double().norm()) < 2e-5

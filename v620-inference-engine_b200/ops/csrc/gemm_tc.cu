@@ -516,10 +516,10 @@ __global__ void __launch_bounds__(320, 1) gemm_tc_ksplit_kernel(const __grid_con
 // (two 128 x 128 tiles) for the same math: those stop at what an SM can pull out of L2 (~64 bytes per cycle), this one
 // does not.  The tensor cores of both SMs read both CTAs' shared memory; each SM accumulates its 128 rows x 256 columns
 // in its own tensor memory (two accumulators = all 512 columns).
-//   producer (warp 0, one thread, both CTAs): waits for its own "empty" barrier of the stage, loads its A tile and its W
+//   producer (warp 0, one elected lane, both CTAs): waits for its own "empty" barrier of the stage, loads its A tile and its W
 //       half with cp.async.bulk.tensor.cta_group::2 (no multicast), both completing on the LEADER's "full" barrier, on
 //       which the leader's producer has announced the 64 KB of the pair;
-//   MMA (warp 1, one thread, leader CTA only): four cta_group::2 MMAs per k block; tcgen05.commit (to both CTAs of the
+//   MMA (warp 1, one elected lane, leader CTA only): four cta_group::2 MMAs per k block; tcgen05.commit (to both CTAs of the
 //       pair) frees the stage in both CTAs and, after a tile's last k block, publishes the accumulator to both CTAs'
 //       epilogue warps;
 //   epilogue (warps 2-9, both CTAs): as in the single-CTA kernel, on the CTA's own 128 rows; hands the accumulator back
@@ -736,13 +736,14 @@ static bool configure_once(int which) {          // 0 dense 128-wide, 2 dense 25
     return true;
 }
 
-static int g_wide_min_n = 1024;          // products at least this wide use the 128 x 256 tile form (0: never)
-static int g_pair_min_n = 1024;          // products at least this wide (and 256 rows tall) use CTA pairs (0: never)
+static int g_wide_min_n = 1024;          // products at least this wide may use the 128 x 256 tile form (0: never)
+static int g_pair_min_n = 1024;          // products at least this wide and of more than 128 rows may use CTA pairs (0: never, negative: always)
 static int g_stage_local = 1;            // 1: fp32 output of the wide and pair forms also leaves through the staging buffers
 
 // How many CTAs share a tile: of products of up to 256 rows, whose `tiles` tiles per 128 rows leave most SMs idle (1: none; every
-// CTA keeps at least four k blocks).  The number, and with it the order of a result's sum, does not depend on the rows below that
-// line, so that a short chunk and its halves give the same rows.
+// CTA keeps at least four k blocks).  What that does to a row's bits: the number does not depend on the rows below that line, so
+// that a short chunk and its halves give the same rows, and above it every form adds k in one chain, so that they do there as well; the two
+// sides differ by the rounding of the sum (a few 1e-6 of the result's size; the split sum is the nearer one to 64 bits).
 constexpr int TC_KS_ROWS = 256;
 static int ksplit_of(int T, long long tiles, int kblocks) {
     int ks = 1;
@@ -779,12 +780,33 @@ static int launch_ksplit(int ks, const CUtensorMap &mA, const CUtensorMap &mW, G
     return launch_ksplit_of<8>(mA, mW, a, s);
 }
 
+// The form of a plain product.  Few tiles are split over clusters (ksplit_of).  Otherwise the form with the least time by what its tiles
+// cost per 64 k values, measured in us: a 256 x 256 tile of a pair of SMs 0.45 (waves over 74 pairs), a 128 x 256 tile of an SM 0.55, a
+// 128 x 128 tile 0.31 (bound by the 32 KB it loads; two share an SM and take twice that).  777 x 16480 x 2560: single CTAs 100 us,
+// pairs (a quarter of their tiles' area padding) 86; 520 x 12800 x 2560: wide 44, pairs 54 (a third wave for 2 of 150 tiles).  A last
+// column tile that is mostly padding rules the wide form out.
+enum TcForm { FORM_ONE = 0, FORM_WIDE = 1, FORM_PAIR = 2, FORM_SPLIT = 3 };
+static TcForm form_of(int T, int N, int K, bool mix, bool peers) {
+    auto tiles = [&](int bm, int bn) { return (long long)((T + bm - 1) / bm) * ((N + bn - 1) / bn); };
+    auto waves = [](long long n, int at_once) { return (double)((n + at_once - 1) / at_once); };
+    if (!peers && !mix && ksplit_of(T, (N + TC_BN - 1) / TC_BN, (K + TC_BK - 1) / TC_BK) > 1) return FORM_SPLIT;
+    const long long n_wide = tiles(TC_BM, TC_WIDE_BN);
+    const double c_one = 0.31 * waves(tiles(TC_BM, TC_BN), NUM_SMS), c_wide = 0.55 * waves(n_wide, NUM_SMS);
+    const double c_pair = 0.45 * waves(tiles(TC_PAIR_BM, TC_PAIR_BN), NUM_SMS / 2);
+    const bool wide_ok = g_wide_min_n > 0 && N >= g_wide_min_n && (N % TC_WIDE_BN == 0 || N % TC_WIDE_BN > TC_BN);
+    const bool pair_ok = g_pair_min_n && N >= abs(g_pair_min_n) && T > TC_BM && !mix;
+    if (pair_ok && (g_pair_min_n < 0 || (c_pair < c_one && (!wide_ok || c_pair < c_wide)))) return FORM_PAIR;
+    return wide_ok && n_wide >= NUM_SMS / 2 && c_wide < c_one ? FORM_WIDE : FORM_ONE;
+}
+
 static int gemm_plain(GemmTcArgs &a, const void *A, const void *W, void *C, int T, int N, int K, int lda, int ldw, int ldc,
                       int out_bf16, cudaStream_t s) {
     if ((K & 7) || (lda & 7) || (ldw & 7) || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return -1;
     const int tiles_t = (T + TC_BM - 1) / TC_BM;
-    const int ks = a.epi.mode == 0 && !a.wait.flags && !a.mix_xn && T <= TC_KS_ROWS ? ksplit_of(T, (N + TC_BN - 1) / TC_BN, (K + TC_BK - 1) / TC_BK) : 1;
-    if (ks > 1) {
+    const TcForm form = form_of(T, N, K, a.mix_xn != nullptr, a.epi.mode != 0 || a.wait.flags);
+    const bool wide = form == FORM_WIDE;
+    if (form == FORM_SPLIT) {
+        const int ks = ksplit_of(T, (N + TC_BN - 1) / TC_BN, (K + TC_BK - 1) / TC_BK);
         CUtensorMap mA, mW;
         if (!make_map(&mA, A, T, K, lda, TC_BM) || !make_map(&mW, W, N, K, ldw, TC_BN)) return -3;
         a.C32 = out_bf16 ? nullptr : (float *)C;
@@ -794,18 +816,7 @@ static int gemm_plain(GemmTcArgs &a, const void *A, const void *W, void *C, int 
         a.ksplit = 1; a.kb_per = 0; a.c_split = 0;
         return launch_ksplit(ks, mA, mW, a, s);
     }
-    // The form with the least time by what its tiles cost per 64 k values, measured in us: a 256 x 256 tile of a pair of SMs 0.45 (waves
-    // over 74 pairs), a 128 x 256 tile of an SM 0.55, a 128 x 128 tile 0.31 (bound by the 32 KB it loads; two share an SM and
-    // take twice that).  777 x 16480 x 2560: single CTAs 86 us, pairs (a third of their tiles' area padding) 73; 520 x 12800 x
-    // 2560: wide 44, pairs 54 (a third wave for 2 of 150 tiles).  A last column tile that is mostly padding rules the wide form out.
-    auto waves = [](long long tiles, int at_once) { return (double)((tiles + at_once - 1) / at_once); };
-    const long long n_one = (long long)tiles_t * ((N + TC_BN - 1) / TC_BN), n_wide = (long long)tiles_t * ((N + TC_WIDE_BN - 1) / TC_WIDE_BN);
-    const long long n_pair = (long long)((T + TC_PAIR_BM - 1) / TC_PAIR_BM) * ((N + TC_PAIR_BN - 1) / TC_PAIR_BN);
-    const double c_one = 0.31 * waves(n_one, NUM_SMS), c_wide = 0.55 * waves(n_wide, NUM_SMS), c_pair = 0.45 * waves(n_pair, NUM_SMS / 2);
-    const bool wide_ok = g_wide_min_n > 0 && N >= g_wide_min_n && (N % TC_WIDE_BN == 0 || N % TC_WIDE_BN > TC_BN);
-    const bool pair = g_pair_min_n > 0 && N >= g_pair_min_n && T > TC_BM && !a.mix_xn && c_pair < c_one && (!wide_ok || c_pair < c_wide);
-    const bool wide = !pair && wide_ok && n_wide >= NUM_SMS / 2 && c_wide < c_one;
-    if (pair) {
+    if (form == FORM_PAIR) {
         CUtensorMap mA, mW;
         if (!make_map(&mA, A, T, K, lda, TC_BM) || !make_map(&mW, W, N, K, ldw, TC_PAIR_BN / 2)) return -3;
         a.C32 = out_bf16 ? nullptr : (float *)C;
@@ -845,7 +856,7 @@ static int gemm_plain(GemmTcArgs &a, const void *A, const void *W, void *C, int 
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-// Products at least `min_n` columns wide use the 128 x 256 tile form (0 switches it off; measurements and tests).
+// Products at least `min_n` columns wide may use the 128 x 256 tile form (0 switches it off; measurements and tests).
 QW_API int qwk_gemm_tc_wide_min_n(int min_n) {
     const int old = g_wide_min_n;
     g_wide_min_n = min_n;
@@ -859,12 +870,17 @@ QW_API int qwk_gemm_tc_stage_local(int on) {
     return old;
 }
 
-// Products at least `min_n` columns wide (and 256 rows tall) use the CTA-pair form (0 switches it off).
+// Products at least `min_n` columns wide and of more than 128 rows may use the CTA-pair form (0 switches it off; a negative number makes
+// all of them that are at least -min_n wide and not split use it, whatever it costs: measurements and tests).
 QW_API int qwk_gemm_tc_pair_min_n(int min_n) {
     const int old = g_pair_min_n;
     g_pair_min_n = min_n;
     return old;
 }
+
+// The form that qwk_gemm_bf16_tc (mix = 0) or qwk_gemm_mix_tc (mix = 1, N = 4 SH) takes: 0 128 x 128 tiles, 1 128 x 256, 2 CTA pairs, 3 tiles
+// split over a cluster.
+QW_API int qwk_gemm_tc_form(int T, int N, int K, int mix) { return form_of(T, N, K, mix != 0, false); }
 
 // C = A . W^T.  A bf16 [T][lda], W bf16 [N][ldw], C fp32 (out_bf16 = 0) or bf16 [T][ldc].
 // Base addresses 16-byte aligned, lda/ldw multiples of 8 elements, K a multiple of 8.
