@@ -244,7 +244,6 @@ struct GdnFusedArgs {
     float *S, *save;
     bf16 *o;
     float eps;
-    PfArgs pf;
 };
 
 __global__ void __launch_bounds__(512) gdn_fused_kernel(GdnFusedArgs a) {
@@ -267,7 +266,6 @@ __global__ void __launch_bounds__(512) gdn_fused_kernel(GdnFusedArgs a) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) tap[k] = a.cw[ch * 4 + k];
     }
-    pf_issue(a.pf);
     // The row table was written before the step began and the recurrent state only by this kernel in the previous step:
     // neither depends on the predecessor, so the state (64 KB per head, from HBM) is fetched before waiting for it.
     if (a.rows.run_start[m0] != m0) return;
@@ -419,7 +417,7 @@ QW_API int qwk_gdn_step(const float *proj, int ld_proj, float *ring, const float
         GdnFusedArgs a;
         a.proj = proj; a.ld_proj = ld_proj; a.ring = ring; a.cw = cw; a.A_log = A_log; a.dt_bias = dt_bias;
         a.norm_w = norm_w; a.KL = KL; a.VL = VL; a.rows = Rows{M, slot, pos, run_start, run_len};
-        a.S = S; a.save = save; a.o = (bf16 *)o; a.eps = eps; a.pf = take_pf();
+        a.S = S; a.save = save; a.o = (bf16 *)o; a.eps = eps;
         cudaError_t e = launch_pdl(gdn_fused_kernel, dim3(M, VL), dim3(512), 0, s, a);
         return e == cudaSuccess ? 0 : -2;
     }

@@ -70,7 +70,7 @@ QW_API int qwk_gemv_bf16(const void *W, const void *x, float *y, void *y_bf16, i
         // the streaming kernel: bulk-async weight pipeline, one block per SM
         SGemvArgs g;
         g.W = (const bf16 *)W; g.x = (const bf16 *)x; g.y = y; g.y_bf16 = (bf16 *)y_bf16;
-        g.N = N; g.K = K; g.M = M; g.ldw = ldw; g.ldx = ldx; g.ldy = ldy; g.accumulate = accumulate; g.nsplit = 1; g.w_split = 0; g.err = g_err_ptr; g.pf = take_pf();
+        g.N = N; g.K = K; g.M = M; g.ldw = ldw; g.ldx = ldx; g.ldy = ldy; g.accumulate = accumulate; g.nsplit = 1; g.w_split = 0; g.err = g_err_ptr;
         g.fi = take_fi(); g.fo = take_fo();
         const cudaError_t e = launch_sgemv(g, s);
         return e == cudaSuccess ? 0 : -2;

@@ -80,7 +80,7 @@ template <bool FUSED, int UPR>
 __global__ void __launch_bounds__(256, 3) hc_up_mix_kernel(const float *red, int ld_red, const bf16 *Wu /* [SH][hc][R] */,
                                                         const float *X, const float *w1, int SH, int hc, int R, int hc_down,
                                                         float inv_H, float eps, int M, float *inj, int ld_inj, bf16 *bin,
-                                                        int ld_bin, int bin_col0, PfArgs pf, FuseIn fi, FuseOut fo) {
+                                                        int ld_bin, int bin_col0, FuseIn fi, FuseOut fo) {
     extern __shared__ float sm[];
     float *u = sm;                         // [UPR][R]
     float *rs = sm + UPR * R;          // [UPR][hc]
@@ -98,7 +98,6 @@ __global__ void __launch_bounds__(256, 3) hc_up_mix_kernel(const float *red, int
         for (int i = 0; i < UP_MAXI; ++i)
             if (li + 8 * i < nch) w[i] = ld_stream(wp + li + 8 * i);
     }
-    pf_issue(pf);
     pdl_wait();
     pdl_trigger();
     // this lane's residual values times the norm weight: needed only at the very end, fetched now so that their L2
@@ -215,7 +214,6 @@ struct HcDownArgs {
     const bf16 *Wd;         // [down][hc][SH]
     float *send;            // [M][ld_send]
     int ld_send, SH, hc, down, M, wpr;
-    PfArgs pf;
     FuseIn fi;              // fused reduce-scatter: `pend` is the sum of the ranks' slots
     FuseOut fo;             // fused all-reduce of `send`
 };
@@ -244,7 +242,6 @@ __global__ void __launch_bounds__(256, 3) hc_down_kernel(HcDownArgs a) {
             if (c < nchunk) w0[u] = ld_stream(reinterpret_cast<const uint4 *>(wrow) + c);
         }
     }
-    pf_issue(a.pf);
     pdl_wait();
     pdl_trigger();
     const bool scattered = FUSED && a.fi.active;
@@ -681,7 +678,7 @@ QW_API int qwk_hc_up_mix(const float *red, int ld_red, const void *Wu, const flo
     const size_t smem = sizeof(float) * ((size_t)UP_ROWS * R + UP_ROWS * hc + (size_t)UP_ROWS * ld_red);
     if (smem > 48 * 1024) return -1;
     return launch_pdl(fi.active ? hc_up_mix_kernel<true, UP_ROWS> : hc_up_mix_kernel<false, UP_ROWS>, grid, dim3(256), smem, s, red, ld_red, (const bf16 *)Wu, X, w1, SH, hc, R, R + n_inj,
-                      1.f / float(H), eps, M, inj, ld_inj, (bf16 *)bin, ld_bin, bin_col0, take_pf(), fi, fo) == cudaSuccess ? 0 : -2;
+                      1.f / float(H), eps, M, inj, ld_inj, (bf16 *)bin, ld_bin, bin_col0, fi, fo) == cudaSuccess ? 0 : -2;
 }
 
 // Fused combine + sum of squares + down projection (see hc_down_kernel).  Xout == null keeps X in place.
@@ -691,7 +688,7 @@ QW_API int qwk_hc_down(const float *Xin, float *Xout, const float *pend, int ld_
     if ((SH & 7) || (pend && !Xout)) return -1;
     HcDownArgs a;
     a.Xin = Xin; a.Xout = Xout; a.pend = pend; a.ld_pend = ld_pend; a.inj_prev = inj_prev; a.w1 = w1;
-    a.Wd = (const bf16 *)Wd; a.send = send; a.ld_send = ld_send; a.SH = SH; a.hc = hc; a.down = down; a.M = M; a.pf = take_pf();
+    a.Wd = (const bf16 *)Wd; a.send = send; a.ld_send = ld_send; a.SH = SH; a.hc = hc; a.down = down; a.M = M;
     a.fi = take_fi(); a.fo = take_fo();
     if (a.fi.active && !a.fo.mode) return -1;          // a fused down projection always sends its all-reduce
     hc_configure();

@@ -199,9 +199,7 @@ constexpr int DN_T = 8;      // pieces per lane over top_k down rows: top_k * F/
 
 // h[p][f] = silu(gate_e[f] . x_m) * (up_e[f] . x_m) for pair p = (m, j).  grid (ceil(F/8), pairs).
 __global__ void __launch_bounds__(256) moe_gate_up_pair_kernel(const uint32_t *w13, const bf16 *s13, const bf16 *x, int ldx,
-                                                               const int *pair_expert, int top_k, int F, int K, bf16 *h, PfArgs pf,
-                                                               SharedAct sa, int npairs) {
-    pf_issue(pf);
+                                                               const int *pair_expert, int top_k, int F, int K, bf16 *h, SharedAct sa, int npairs) {
     pdl_wait();
     pdl_trigger();
     if ((int)blockIdx.y >= npairs) {          // the extra rows of the grid: the shared expert's activation
@@ -254,9 +252,7 @@ template <bool FUSED>
 __global__ void __launch_bounds__(256) moe_down_combine_kernel(const uint32_t *w2, const bf16 *s2, const bf16 *h,
                                                                const int *pair_expert, const float *pair_w, int top_k,
                                                                int F, int H, const bf16 *shared_down, int ld_sd,
-                                                               const bf16 *sh_h, int SF, float *out, int ldo, PfArgs pf,
-                                                               FuseOut fo) {
-    pf_issue(pf);
+                                                               const bf16 *sh_h, int SF, float *out, int ldo, FuseOut fo) {
     const int m = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = blockIdx.x * 8 + warp;
@@ -360,7 +356,7 @@ QW_API int qwk_moe_router(const void *Wrs, const void *x, float *rs, int nrs, in
     if (E > 1024 || top_k > 32 || (K & 15) || (ldx & 7)) return -1;
     SGemvArgs a;
     a.W = (const bf16 *)Wrs; a.x = (const bf16 *)x; a.y = rs; a.y_bf16 = nullptr;
-    a.N = nrs; a.K = K; a.M = M; a.ldw = K; a.ldx = ldx; a.ldy = nrs; a.accumulate = 0; a.nsplit = 1; a.w_split = 0; a.err = g_err_ptr; a.pf = take_pf();
+    a.N = nrs; a.K = K; a.M = M; a.ldw = K; a.ldx = ldx; a.ldy = nrs; a.accumulate = 0; a.nsplit = 1; a.w_split = 0; a.err = g_err_ptr;
     a.fi = take_fi();
     RouteArgs r = make_route(E, top_k, F, e_first, e_local, pair_expert, pair_w, sh_h, ticket);
     r.w13 = (const char *)w13; r.w2 = (const char *)w2; r.w13_bytes = w13_bytes; r.w2_bytes = w2_bytes;
@@ -411,13 +407,13 @@ QW_API int qwk_moe_gate_up_pair(const void *w13, const void *s13, const void *x,
         // tensor-core form: 16 rows of gate and of up per block
         const size_t smem = (size_t)K * 2 + MM_WARPS * 2 * 16 * sizeof(float);
         cudaError_t e = launch_pdl(moe_gate_up_mma_kernel, dim3(F / 16, M * top_k + extra), dim3(128), smem, s, (const uint32_t *)w13,
-                                   (const bf16 *)s13, (const bf16 *)x, ldx, pair_expert, top_k, F, K, (bf16 *)h, take_pf(), sa, M * top_k);
+                                   (const bf16 *)s13, (const bf16 *)x, ldx, pair_expert, top_k, F, K, (bf16 *)h, sa, M * top_k);
         return e == cudaSuccess ? 0 : -2;
     }
     if (2 * (K >> 5) > 32 * GU_T) return -1;
     dim3 grid((F + 7) / 8, M * top_k + extra);
     cudaError_t e = launch_pdl(moe_gate_up_pair_kernel, grid, dim3(256), 0, s, (const uint32_t *)w13, (const bf16 *)s13,
-                               (const bf16 *)x, ldx, pair_expert, top_k, F, K, (bf16 *)h, take_pf(), sa, M * top_k);
+                               (const bf16 *)x, ldx, pair_expert, top_k, F, K, (bf16 *)h, sa, M * top_k);
     return e == cudaSuccess ? 0 : -2;
 }
 
@@ -454,10 +450,10 @@ QW_API int qwk_moe_down_combine(const void *w2, const void *s2, const void *h, c
             const dim3 g2(H / 16, M);
             cudaError_t e = fo.mode ? launch_pdl(moe_down_mma_kernel<true>, g2, dim3(128), smem, s, (const uint32_t *)w2, (const bf16 *)s2,
                                                  (const bf16 *)h, pair_expert, pair_w, top_k, F, H, (const bf16 *)shared_down, ld_sd,
-                                                 (const bf16 *)sh_h, SF, out, ldo, take_pf(), fo)
+                                                 (const bf16 *)sh_h, SF, out, ldo, fo)
                                     : launch_pdl(moe_down_mma_kernel<false>, g2, dim3(128), smem, s, (const uint32_t *)w2, (const bf16 *)s2,
                                                  (const bf16 *)h, pair_expert, pair_w, top_k, F, H, (const bf16 *)shared_down, ld_sd,
-                                                 (const bf16 *)sh_h, SF, out, ldo, take_pf(), fo);
+                                                 (const bf16 *)sh_h, SF, out, ldo, fo);
             return e == cudaSuccess ? 0 : -2;
         }
     }
@@ -465,10 +461,10 @@ QW_API int qwk_moe_down_combine(const void *w2, const void *s2, const void *h, c
     dim3 grid((H + 7) / 8, M);
     cudaError_t e = fo.mode ? launch_pdl(moe_down_combine_kernel<true>, grid, dim3(256), 0, s, (const uint32_t *)w2, (const bf16 *)s2,
                                          (const bf16 *)h, pair_expert, pair_w, top_k, F, H, (const bf16 *)shared_down, ld_sd,
-                                         (const bf16 *)sh_h, SF, out, ldo, take_pf(), fo)
+                                         (const bf16 *)sh_h, SF, out, ldo, fo)
                             : launch_pdl(moe_down_combine_kernel<false>, grid, dim3(256), 0, s, (const uint32_t *)w2, (const bf16 *)s2,
                                          (const bf16 *)h, pair_expert, pair_w, top_k, F, H, (const bf16 *)shared_down, ld_sd,
-                                         (const bf16 *)sh_h, SF, out, ldo, take_pf(), fo);
+                                         (const bf16 *)sh_h, SF, out, ldo, fo);
     return e == cudaSuccess ? 0 : -2;
 }
 
@@ -512,7 +508,7 @@ extern "C" __attribute__((visibility("default"))) int qwk_moe_router_static(cons
     if (cudaMemsetAsync(ticket, 0, sizeof(unsigned int), s) != cudaSuccess) return -2;
     SGemvArgs a;
     a.W = (const bf16 *)Wrs; a.x = (const bf16 *)x; a.y = rs; a.y_bf16 = nullptr;
-    a.N = nrs; a.K = K; a.M = M; a.ldw = K; a.ldx = ldx; a.ldy = nrs; a.accumulate = 0; a.nsplit = 1; a.w_split = 0; a.err = g_err_ptr; a.pf = take_pf();
+    a.N = nrs; a.K = K; a.M = M; a.ldw = K; a.ldx = ldx; a.ldy = nrs; a.accumulate = 0; a.nsplit = 1; a.w_split = 0; a.err = g_err_ptr;
     RouteArgs r = make_route(E, top_k, F, e_first, e_local, pair_expert, pair_w, sh_h, ticket);
     r.w13 = nullptr; r.w2 = nullptr; r.w13_bytes = 0; r.w2_bytes = 0; r.prefetch_rows = 0;
     const cudaError_t e = launch_router(a, r, s);

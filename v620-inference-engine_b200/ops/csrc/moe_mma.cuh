@@ -76,12 +76,10 @@ constexpr int DN_NS = 5;             // quad-steps of the shared expert per warp
 // Warp w takes the k groups g = w, w + 4, ...; every weight load of the block is issued before the first
 // one is used, and the four partial tiles are added in warp order.
 __global__ void __launch_bounds__(128) moe_gate_up_mma_kernel(const uint32_t *w13, const bf16 *s13, const bf16 *x, int ldx,
-                                                              const int *pair_expert, int top_k, int F, int K, bf16 *h, PfArgs pf,
-                                                              SharedAct sa, int npairs) {
+                                                              const int *pair_expert, int top_k, int F, int K, bf16 *h, SharedAct sa, int npairs) {
     extern __shared__ __align__(16) unsigned char mm_smem[];
     uint4 *xs = reinterpret_cast<uint4 *>(mm_smem);                       // [K / 8] activation words
     float *red = reinterpret_cast<float *>(mm_smem + (size_t)K * 2);     // [4 warps][2][16]
-    pf_issue(pf);
     pdl_wait();
     pdl_trigger();
     if ((int)blockIdx.y >= npairs) {          // the extra rows of the grid: the shared expert's activation
@@ -164,12 +162,11 @@ __global__ void __launch_bounds__(128) moe_gate_up_mma_kernel(const uint32_t *w1
 template <bool FUSED>
 __global__ void __launch_bounds__(128) moe_down_mma_kernel(const uint32_t *w2, const bf16 *s2, const bf16 *h, const int *pair_expert,
                                                            const float *pair_w, int top_k, int F, int H, const bf16 *shared_down,
-                                                           int ld_sd, const bf16 *sh_h, int SF, float *out, int ldo, PfArgs pf, FuseOut fo) {
+                                                           int ld_sd, const bf16 *sh_h, int SF, float *out, int ldo, FuseOut fo) {
     extern __shared__ __align__(16) unsigned char mm_smem[];
     uint4 *hs = reinterpret_cast<uint4 *>(mm_smem);                                       // [top_k][F / 8]
     uint4 *ss = hs + (size_t)top_k * (F >> 3);                                            // [SF / 8]
     float *red = reinterpret_cast<float *>(ss + (SF >> 3));                               // [4][16]
-    pf_issue(pf);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int r = lane >> 2, q = lane & 3;
     const int m = blockIdx.y, c0 = blockIdx.x * 16;

@@ -18,7 +18,6 @@
 
 namespace qw {
 ErrorWord *g_err_ptr = nullptr;
-PfArgs g_pf = {};
 int *g_moe_stats = nullptr;
 SharedAct g_shared_act = {nullptr, 0, 0, 0, nullptr};
 FuseOut g_fo = {};

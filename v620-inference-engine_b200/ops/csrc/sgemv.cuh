@@ -33,7 +33,6 @@ struct SGemvArgs {
     int P;              // k parts per row tile
     int nstage;
     ErrorWord *err;
-    PfArgs pf;          // weights of later kernels to pull into L2
     FuseIn fi = {};     // fused all-gather: the activation rows are built from the ranks' words
     FuseOut fo = {};    // fused reduce-scatter: y goes to the ranks that own its columns instead of memory
 };
@@ -168,7 +167,6 @@ __device__ __forceinline__ void sgemv_core(const SGemvArgs &a, unsigned char *sm
         }
         return;
     }
-    pf_issue(a.pf);
     pdl_wait();
     pdl_trigger();
     const uint32_t xs_base = smem_u32(sm.xs), st_base = smem_u32(sm.stages);
