@@ -340,3 +340,20 @@ def test_gemm_tc_rows_keep_their_bits_on_each_side_of_the_split_line(N, K):
         assert torch.equal(head, whole[:256])
     else:
         assert float((head - whole[:256]).double().norm() / head.double().norm()) < 2e-5
+
+
+@pytest.mark.parametrize("T,N,K,form", [(100, 256, 1024, 3), (300, 512, 64, 0), (520, 12800, 64, 1), (777, 4352, 64, 2)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("off", [1, 2, 4])
+def test_gemm_tc_output_at_any_address(T, N, K, form, out_dtype, off):
+    """Rows whose stride allows 16-byte stores but whose first element does not lie on 16 bytes: the same bits, nothing beside them."""
+    from qwb200.ops import kernels as K_, lib as qlib
+    assert qlib.load(True).qwk_gemm_tc_form(T, N, K, 0) == form
+    g = torch.Generator(device="cuda").manual_seed(T + off)
+    A = torch.randn(T, K, generator=g, device="cuda").to(torch.bfloat16)
+    W = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    flat = torch.full((T * (N + 8) + 16,), 768.0, dtype=out_dtype, device="cuda")
+    out = flat[off:off + T * (N + 8)].view(T, N + 8)
+    K_.gemm_bf16_tc(A, W, out=out[:, :N])
+    assert torch.equal(out[:, :N], K_.gemm_bf16_tc(A, W, out_dtype=out_dtype))
+    assert torch.all(out[:, N:].float() == 768.0) and torch.all(flat[:off].float() == 768.0) and torch.all(flat[off + T * (N + 8):].float() == 768.0)

@@ -65,6 +65,7 @@ struct GemmTcArgs {
     // input C16[row][c] = mean over s of sigmoid(logit) * mix_xn[row][s][c] (rows of 4 * mix_cols) and no logit is stored
     const bf16 *mix_xn;
     int mix_cols;
+    bool vec;            // every row and part of C starts on 16 bytes: whole pieces leave as 16-byte stores
 };
 
 struct TileAt {
@@ -149,7 +150,7 @@ __device__ __forceinline__ void store_piece(const GemmTcArgs &a, long long c_off
     }
     if (a.C32) {
         float *o = a.C32 + c_off + (long long)row * a.ldc + col0;
-        if (nmax >= 32 && ((a.ldc | col0) & 3) == 0) {
+        if (nmax >= 32 && a.vec) {
 #pragma unroll
             for (int j = 0; j < 32; j += 4)
                 *reinterpret_cast<float4 *>(o + j) = make_float4(__uint_as_float(v[j]), __uint_as_float(v[j + 1]),
@@ -159,7 +160,7 @@ __device__ __forceinline__ void store_piece(const GemmTcArgs &a, long long c_off
         }
     } else {
         bf16 *o = a.C16 + (long long)row * a.ldc + col0;
-        if (nmax >= 32 && ((a.ldc | col0) & 7) == 0) {
+        if (nmax >= 32 && a.vec) {
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
                 uint4 pk;
@@ -192,7 +193,7 @@ __device__ __forceinline__ void send_piece(const GemmTcArgs &a, float *stg, int 
     const int col = col0 + ch * 4;                                   // first of this lane's four columns
     if constexpr (LOCAL) {
         // the same transposition for this GPU's own fp32 output: whole lines instead of 16-byte pieces of 32 rows
-        const bool vec = ((a.ldc | col0) & 3) == 0 && col + 4 <= a.N;
+        const bool vec = a.vec && col + 4 <= a.N;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int r = 4 * i + rsub;
@@ -493,7 +494,7 @@ __global__ void __launch_bounds__(320, 1) gemm_tc_ksplit_kernel(const __grid_con
             const int col = t.n0 + rank * QC + x;
             if (row >= a.T || col >= a.N) continue;
             const long long at = t.c_off + (long long)row * a.ldc + col;
-            if (a.C32 && col + 16 <= a.N && ((a.ldc | col) & 3) == 0 && (t.c_off & 3) == 0) {
+            if (a.C32 && col + 16 <= a.N && a.vec) {
 #pragma unroll
                 for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4 *>(a.C32 + at + j) = make_float4(sum[j], sum[j + 1], sum[j + 2], sum[j + 3]);
             } else {
@@ -736,6 +737,16 @@ static bool configure_once(int which) {          // 0 dense 128-wide, 2 dense 25
     return true;
 }
 
+// C [T][ldc] in fp32 or bf16; parts of a split-K product `c_split` elements apart.
+static void set_output(GemmTcArgs &a, void *C, int out_bf16, int ldc, long long c_split = 0) {
+    a.C32 = out_bf16 ? nullptr : (float *)C;
+    a.C16 = out_bf16 ? (bf16 *)C : nullptr;
+    a.ldc = ldc;
+    a.c_split = c_split;
+    const int n = out_bf16 ? 8 : 4;
+    a.vec = aligned16((char *)C) && ldc % n == 0 && c_split % n == 0;
+}
+
 static int g_wide_min_n = 1024;          // products at least this wide may use the 128 x 256 tile form (0: never)
 static int g_pair_min_n = 1024;          // products at least this wide and of more than 128 rows may use CTA pairs (0: never, negative: always)
 static int g_stage_local = 1;            // 1: fp32 output of the wide and pair forms also leaves through the staging buffers
@@ -809,21 +820,19 @@ static int gemm_plain(GemmTcArgs &a, const void *A, const void *W, void *C, int 
         const int ks = ksplit_of(T, (N + TC_BN - 1) / TC_BN, (K + TC_BK - 1) / TC_BK);
         CUtensorMap mA, mW;
         if (!make_map(&mA, A, T, K, lda, TC_BM) || !make_map(&mW, W, N, K, ldw, TC_BN)) return -3;
-        a.C32 = out_bf16 ? nullptr : (float *)C;
-        a.C16 = out_bf16 ? (bf16 *)C : nullptr;
-        a.T = T; a.N = N; a.K = K; a.ldc = ldc; a.err = g_err_ptr; a.tiles = nullptr;
+        set_output(a, C, out_bf16, ldc);
+        a.T = T; a.N = N; a.K = K; a.err = g_err_ptr; a.tiles = nullptr;
         a.tiles_t = tiles_t; a.tiles_n = (N + TC_BN - 1) / TC_BN; a.total = a.tiles_t * a.tiles_n;
-        a.ksplit = 1; a.kb_per = 0; a.c_split = 0;
+        a.ksplit = 1; a.kb_per = 0;
         return launch_ksplit(ks, mA, mW, a, s);
     }
     if (form == FORM_PAIR) {
         CUtensorMap mA, mW;
         if (!make_map(&mA, A, T, K, lda, TC_BM) || !make_map(&mW, W, N, K, ldw, TC_PAIR_BN / 2)) return -3;
-        a.C32 = out_bf16 ? nullptr : (float *)C;
-        a.C16 = out_bf16 ? (bf16 *)C : nullptr;
-        a.T = T; a.N = N; a.K = K; a.ldc = ldc; a.err = g_err_ptr; a.tiles = nullptr;
+        set_output(a, C, out_bf16, ldc);
+        a.T = T; a.N = N; a.K = K; a.err = g_err_ptr; a.tiles = nullptr;
         a.tiles_t = (T + TC_PAIR_BM - 1) / TC_PAIR_BM; a.tiles_n = (N + TC_PAIR_BN - 1) / TC_PAIR_BN; a.total = a.tiles_t * a.tiles_n;
-        a.ksplit = 1; a.kb_per = 0; a.c_split = 0;
+        a.ksplit = 1; a.kb_per = 0;
         const bool staged = a.epi.mode != 0 || (g_stage_local && !out_bf16);
         if (!configure_once(staged ? 6 : 5)) return -3;
         const unsigned sm_pairs = persistent_grid(1 << 30, 1) / 2;          // SMs / 2
@@ -837,11 +846,10 @@ static int gemm_plain(GemmTcArgs &a, const void *A, const void *W, void *C, int 
     const int BN = wide ? TC_WIDE_BN : TC_BN;
     CUtensorMap mA, mW;
     if (!make_map(&mA, A, T, K, lda, TC_BM) || !make_map(&mW, W, N, K, ldw, BN)) return -3;
-    a.C32 = out_bf16 ? nullptr : (float *)C;
-    a.C16 = out_bf16 ? (bf16 *)C : nullptr;
-    a.T = T; a.N = N; a.K = K; a.ldc = ldc; a.err = g_err_ptr; a.tiles = nullptr;
+    set_output(a, C, out_bf16, ldc);
+    a.T = T; a.N = N; a.K = K; a.err = g_err_ptr; a.tiles = nullptr;
     a.tiles_t = tiles_t; a.tiles_n = (N + BN - 1) / BN; a.total = a.tiles_t * a.tiles_n;
-    a.ksplit = 1; a.kb_per = 0; a.c_split = 0;
+    a.ksplit = 1; a.kb_per = 0;
     // tiles that leave for other ranks go out as whole 128-byte lines (optionally this GPU's own fp32 tiles of the wide form too)
     const bool staged = a.epi.mode != 0 || (g_stage_local && wide && !out_bf16);
     if (!configure_once(staged ? (wide ? 4 : 3) : (wide ? 2 : 0))) return -3;
@@ -957,11 +965,10 @@ QW_API int qwk_gemm_bf16_tc_grouped(const void *A, const void *W, void *C, const
     CUtensorMap mA, mW;
     if (!make_map(&mA, A, rows, K, lda, TC_BM) || !make_map(&mW, W, w_rows, K, ldw, TC_BN)) return -3;
     GemmTcArgs a{};
-    a.C32 = out_bf16 ? nullptr : (float *)C;
-    a.C16 = out_bf16 ? (bf16 *)C : nullptr;
-    a.T = rows; a.N = Nw; a.K = K; a.ldc = ldc; a.err = g_err_ptr; a.tiles = (const int4 *)tiles;
+    set_output(a, C, out_bf16, ldc);
+    a.T = rows; a.N = Nw; a.K = K; a.err = g_err_ptr; a.tiles = (const int4 *)tiles;
     a.tiles_t = max_tiles; a.tiles_n = (Nw + TC_BN - 1) / TC_BN; a.total = a.tiles_t * a.tiles_n;
-    a.ksplit = 1; a.kb_per = 0; a.c_split = 0;
+    a.ksplit = 1; a.kb_per = 0;
     if (!configure_once(0)) return -3;
     gemm_tc_kernel<TC_BN, TC_STAGES><<<persistent_grid(a.total), 320, TC_SMEM, s>>>(mA, mW, a);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
@@ -978,13 +985,12 @@ QW_API int qwk_gemm_bf16_tc_splitk(const void *A, const void *W, float *C, int T
     CUtensorMap mA, mW;
     if (!make_map(&mA, A, T, K, lda, TC_BM) || !make_map(&mW, W, N, K, ldw, TC_BN)) return -3;
     GemmTcArgs a{};
-    a.C32 = C; a.C16 = nullptr;
-    a.T = T; a.N = N; a.K = K; a.ldc = ldc; a.err = g_err_ptr; a.tiles = nullptr;
+    set_output(a, C, 0, ldc, c_split);
+    a.T = T; a.N = N; a.K = K; a.err = g_err_ptr; a.tiles = nullptr;
     a.tiles_t = (T + TC_BM - 1) / TC_BM; a.tiles_n = (N + TC_BN - 1) / TC_BN;
     a.kb_per = (kblocks + ksplit - 1) / ksplit;
     a.ksplit = (kblocks + a.kb_per - 1) / a.kb_per;          // every share holds at least one k block
     if (a.ksplit != ksplit) return -1;
-    a.c_split = c_split;
     a.total = a.tiles_t * a.tiles_n * a.ksplit;
     const int ks = ksplit_of(T, (long long)a.tiles_n * a.ksplit, a.kb_per);
     if (ks > 1) return launch_ksplit(ks, mA, mW, a, s);
