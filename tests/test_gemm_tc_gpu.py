@@ -271,7 +271,7 @@ def test_gemm_tc_wide_tiles_match_64_bits(T, N, K, out_dtype, stage):
     """128 x 256 tiles, with the fp32 output through the staging buffers and straight from registers, ragged rows and columns."""
     from qwb200.ops import lib as qlib
     L = qlib.load(True)
-    assert L.qwk_gemm_tc_form(T, N, K, 0) == 1
+    assert L.qwk_gemm_tc_form(T, N, K) == 1
     old = L.qwk_gemm_tc_stage_local(stage)
     try:
         _against_64_bits(T, N, K, out_dtype)
@@ -279,10 +279,9 @@ def test_gemm_tc_wide_tiles_match_64_bits(T, N, K, out_dtype, stage):
         L.qwk_gemm_tc_stage_local(old)
 
 
-@pytest.mark.parametrize("T,SH,R,form", [(300, 2560, 320, 1), (3001, 2560, 320, 1), (520, 3200, 40, 1), (1021, 2560, 320, 0)])
-def test_mixer_up_projection_in_both_tile_forms(T, SH, R, form):
-    from qwb200.ops import lib as qlib
-    assert qlib.load(True).qwk_gemm_tc_form(T, 4 * SH, R, 1) == form
+@pytest.mark.parametrize("T,SH,R", [(300, 2560, 320), (3001, 2560, 320), (520, 3200, 40), (4096, 512, 64)])
+def test_mixer_up_projection_of_many_tiles(T, SH, R):
+    """Several tiles per block, ragged rows, and a width whose last column tile is not whole."""
     test_mixer_up_projection_with_the_mean_in_its_epilogue(T, SH, R)
 
 
@@ -305,7 +304,7 @@ def only_pairs():
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
 def test_gemm_tc_pairs_of_small_and_ragged_products_match_64_bits(only_pairs, T, N, K, out_dtype):
     from qwb200.ops import lib as qlib
-    assert qlib.load(True).qwk_gemm_tc_form(T, N, K, 0) == 2
+    assert qlib.load(True).qwk_gemm_tc_form(T, N, K) == 2
     _against_64_bits(T, N, K, out_dtype)
     assert only_pairs.tolist() == [0, 0]
 
@@ -317,7 +316,7 @@ def test_gemm_tc_pair_form_reduce_scatter_with_ragged_rows(only_pairs, T, N, K):
 
 def test_gemm_tc_wide_form_reduce_scatter():
     from qwb200.ops import lib as qlib
-    assert qlib.load(True).qwk_gemm_tc_form(520, 12800, 64, 0) == 1
+    assert qlib.load(True).qwk_gemm_tc_form(520, 12800, 64) == 1
     test_gemm_tc_reduce_scatter_epilogue_on_emulated_ranks(520, 12800, 64)
 
 
@@ -336,7 +335,7 @@ def test_gemm_tc_rows_keep_their_bits_on_each_side_of_the_split_line(N, K):
         assert torch.equal(K_.gemm_bf16_tc(A[:T], W), head[:T]) and torch.equal(K_.gemm_bf16_tc(A[4096 - T:], W), tail[256 - T:]), T
     for T in (257, 520, 777, 1021, 2048):
         assert torch.equal(K_.gemm_bf16_tc(A[:T], W), whole[:T]) and torch.equal(K_.gemm_bf16_tc(A[4096 - T:], W), whole[4096 - T:]), T
-    if L.qwk_gemm_tc_form(256, N, K, 0) != 3:
+    if L.qwk_gemm_tc_form(256, N, K) != 3:
         assert torch.equal(head, whole[:256])
     else:
         assert float((head - whole[:256]).double().norm() / head.double().norm()) < 2e-5
@@ -348,7 +347,7 @@ def test_gemm_tc_rows_keep_their_bits_on_each_side_of_the_split_line(N, K):
 def test_gemm_tc_output_at_any_address(T, N, K, form, out_dtype, off):
     """Rows whose stride allows 16-byte stores but whose first element does not lie on 16 bytes: the same bits, nothing beside them."""
     from qwb200.ops import kernels as K_, lib as qlib
-    assert qlib.load(True).qwk_gemm_tc_form(T, N, K, 0) == form
+    assert qlib.load(True).qwk_gemm_tc_form(T, N, K) == form
     g = torch.Generator(device="cuda").manual_seed(T + off)
     A = torch.randn(T, K, generator=g, device="cuda").to(torch.bfloat16)
     W = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)

@@ -793,19 +793,19 @@ static int launch_ksplit(int ks, const CUtensorMap &mA, const CUtensorMap &mW, G
 
 // The form of a plain product.  Few tiles are split over clusters (ksplit_of).  Otherwise the form with the least time by what its tiles
 // cost per 64 k values, measured in us: a 256 x 256 tile of a pair of SMs 0.45 (waves over 74 pairs), a 128 x 256 tile of an SM 0.55, a
-// 128 x 128 tile 0.31 (bound by the 32 KB it loads; two share an SM and take twice that).  777 x 16480 x 2560: single CTAs 100 us,
-// pairs (a quarter of their tiles' area padding) 86; 520 x 12800 x 2560: wide 44, pairs 54 (a third wave for 2 of 150 tiles).  A last
+// 128 x 128 tile 0.31 (bound by the 32 KB it loads; two share an SM and take twice that).  777 x 16480 x 2560: single CTAs 86 us,
+// pairs (a quarter of their tiles' area padding) 76; 520 x 12800 x 2560: wide 49, pairs 57 (a third wave for 2 of 150 tiles).  A last
 // column tile that is mostly padding rules the wide form out.
 enum TcForm { FORM_ONE = 0, FORM_WIDE = 1, FORM_PAIR = 2, FORM_SPLIT = 3 };
-static TcForm form_of(int T, int N, int K, bool mix, bool peers) {
+static TcForm form_of(int T, int N, int K, bool peers) {
     auto tiles = [&](int bm, int bn) { return (long long)((T + bm - 1) / bm) * ((N + bn - 1) / bn); };
     auto waves = [](long long n, int at_once) { return (double)((n + at_once - 1) / at_once); };
-    if (!peers && !mix && ksplit_of(T, (N + TC_BN - 1) / TC_BN, (K + TC_BK - 1) / TC_BK) > 1) return FORM_SPLIT;
+    if (!peers && ksplit_of(T, (N + TC_BN - 1) / TC_BN, (K + TC_BK - 1) / TC_BK) > 1) return FORM_SPLIT;
     const long long n_wide = tiles(TC_BM, TC_WIDE_BN);
     const double c_one = 0.31 * waves(tiles(TC_BM, TC_BN), NUM_SMS), c_wide = 0.55 * waves(n_wide, NUM_SMS);
     const double c_pair = 0.45 * waves(tiles(TC_PAIR_BM, TC_PAIR_BN), NUM_SMS / 2);
     const bool wide_ok = g_wide_min_n > 0 && N >= g_wide_min_n && (N % TC_WIDE_BN == 0 || N % TC_WIDE_BN > TC_BN);
-    const bool pair_ok = g_pair_min_n && N >= abs(g_pair_min_n) && T > TC_BM && !mix;
+    const bool pair_ok = g_pair_min_n && N >= abs(g_pair_min_n) && T > TC_BM;
     if (pair_ok && (g_pair_min_n < 0 || (c_pair < c_one && (!wide_ok || c_pair < c_wide)))) return FORM_PAIR;
     return wide_ok && n_wide >= NUM_SMS / 2 && c_wide < c_one ? FORM_WIDE : FORM_ONE;
 }
@@ -814,7 +814,7 @@ static int gemm_plain(GemmTcArgs &a, const void *A, const void *W, void *C, int 
                       int out_bf16, cudaStream_t s) {
     if ((K & 7) || (lda & 7) || (ldw & 7) || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return -1;
     const int tiles_t = (T + TC_BM - 1) / TC_BM;
-    const TcForm form = form_of(T, N, K, a.mix_xn != nullptr, a.epi.mode != 0 || a.wait.flags);
+    const TcForm form = a.mix_xn ? FORM_ONE : form_of(T, N, K, a.epi.mode != 0 || a.wait.flags);
     const bool wide = form == FORM_WIDE;
     if (form == FORM_SPLIT) {
         const int ks = ksplit_of(T, (N + TC_BN - 1) / TC_BN, (K + TC_BK - 1) / TC_BK);
@@ -886,9 +886,8 @@ QW_API int qwk_gemm_tc_pair_min_n(int min_n) {
     return old;
 }
 
-// The form that qwk_gemm_bf16_tc (mix = 0) or qwk_gemm_mix_tc (mix = 1, N = 4 SH) takes: 0 128 x 128 tiles, 1 128 x 256, 2 CTA pairs, 3 tiles
-// split over a cluster.
-QW_API int qwk_gemm_tc_form(int T, int N, int K, int mix) { return form_of(T, N, K, mix != 0, false); }
+// The form that qwk_gemm_bf16_tc takes: 0 128 x 128 tiles, 1 128 x 256, 2 CTA pairs, 3 tiles split over a cluster.
+QW_API int qwk_gemm_tc_form(int T, int N, int K) { return form_of(T, N, K, false); }
 
 // C = A . W^T.  A bf16 [T][lda], W bf16 [N][ldw], C fp32 (out_bf16 = 0) or bf16 [T][ldc].
 // Base addresses 16-byte aligned, lda/ldw multiples of 8 elements, K a multiple of 8.

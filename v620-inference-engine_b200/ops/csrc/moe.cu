@@ -164,7 +164,7 @@ static cudaError_t launch_router(SGemvArgs &a, const RouteArgs &r, cudaStream_t 
 
 // Stand-alone routing (prefill, and callers that computed the logits elsewhere).  Eight rows per column of blocks: blockIdx.y == 0
 // routes them (a warp per row), the others share the activation of the shared expert, which as the tail of the routing block was
-// most of its time (20 rounds of loads one behind the other: 27 us at 6 rows, 35 at 100; now 6 and 8).
+// most of its time (20 rounds of loads one behind the other: 27 us at 6 rows, 35 at 100; now 8 and 8).
 constexpr int ROUTE_ROWS = 8, ROUTE_ACT_BLOCKS = 5;
 __global__ void __launch_bounds__(256) moe_route_kernel(const float *rs, int ld_rs, int M, RouteArgs r) {
     pdl_wait();

@@ -27,7 +27,7 @@ namespace qw {
 // bf16 pair (exact integers -8..7) of nibble pair j of a q4 word in engine order
 __device__ __forceinline__ uint32_t q4_frag(uint32_t w, int j) {
     uint32_t p;
-    // one three-input instruction: written as & and | with both constants known it becomes two
+    // one three-input operation: gate/up and down of 8 rows take 35 and 28 us with it, 41 and 31 with (w & mask) | magic written out
     asm("{\n\t.reg .b32 m;\n\tmov.b32 m, 0x000F000F;\n\tlop3.b32 %0, %1, m, 0x43004300, 0xEA;\n\t}" : "=r"(p) : "r"(w >> (4 * j)));
     bf162 v = *reinterpret_cast<bf162 *>(&p);
     const bf162 off = __floats2bfloat162_rn(136.f, 136.f);
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(128) moe_down_mma_kernel(const uint32_t *w2, c
 // whole lines and need no register while in flight.  Direct 8-byte loads touch one 32-byte sector of sixteen rows per request,
 // and bulk copies of single rows (1,280 and 320 bytes) were bound by their number.  In a chain of their own, us for gate/up and
 // down with bulk copies and now: 1 row 10.4, 8.6 -> 8.4, 7.7; 8 rows 59, 38 -> 35, 28; 24 rows 172, 106 -> 96, 72.  What bounds
-// them now: the instructions of the conversion (three per two weights, beside 7 idle columns of every MMA) and, with few rows,
+// them now: the conversion (shift, merge and subtraction for two weights, beside 7 idle columns of every MMA) and, with few rows,
 // the chain routing -> weights -> sums.
 // Every column of the narrow operand holds the token: the result's column 0 is read, the others cost nothing.
 // ---------------------------------------------------------------------------------------------------------------

@@ -19,11 +19,10 @@
 // TMEM: columns 0-255 hold D (two slots of 2 x 64 columns for experts of up to 64 rows, else one of 2 x 128), 256-511 the
 // four converted stages of two tiles.  One CTA per SM walks the units round-robin.
 //
-// What bounds it: the conversion (about three instructions per weight with its waits; without the MMAs a unit takes 93 % of its
-// time), beside MMAs of at least 39 cycles each; above 64 rows also the epilogue, which then shares its one D slot.  One layer,
+// What bounds it: the conversion (without the MMAs a unit takes 93 % of its time), beside MMAs of at least 39 cycles each; above 64 rows also the epilogue, which then shares its one D slot.  One layer,
 // 512 experts x (1280 x 2560 + 2560 x 640), random routing, us for gate/up with the activation and for down, before (W converted
 // into swizzled shared memory by 8 warps, 128-row token tiles as A, activation in a kernel of its own) and now:
-//   100 tokens  434 + 5, 245 -> 227, 131     1021  520 + 26, 290 -> 274, 152     4096  695 + 96, 447 -> 439, 231
+//   100 tokens  434 + 5, 245 -> 221, 118     1021  520 + 26, 290 -> 273, 143     4096  695 + 96, 447 -> 443, 217
 #include "tc.cuh"
 
 namespace qw {
@@ -44,8 +43,7 @@ struct MoeTcArgs {
     bf16 *C16;
     int ldc;
     ErrorWord *err;
-    // 0x000F000F and 0x43004300, from the parameters so that (w & mask) | magic stays one three-input instruction: with both
-    // known at compile time it became two, each with its own immediate
+    // 0x000F000F and 0x43004300.  As parameters gate/up and down of 100 tokens take 221 and 118 us, as literals 250 and 134
     uint32_t mask, magic;
 };
 
@@ -92,8 +90,7 @@ struct MgWalk {
         tl = tl1;
         if (id < a.total) fetch(a);
     }
-    // For the roles that issue as whole warps: the compiler sees that the unit is the same in every lane, and keeps stage
-    // addresses and descriptors in uniform registers.
+    // For the roles that issue as whole warps: one unit for all lanes, said to the compiler.
     __device__ __forceinline__ void uniform() {
         id = __shfl_sync(0xffffffffu, id, 0);
         tl.x = __shfl_sync(0xffffffffu, tl.x, 0);

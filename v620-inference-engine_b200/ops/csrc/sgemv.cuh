@@ -1,5 +1,5 @@
 // Streaming skinny matrix product core: D[n][m] = sum_k W[n][k] x[m][k] for bf16 weights and up to
-// 16 activation rows per pass, with caller-supplied functors that build the activation rows in
+// 24 activation rows per pass (tiles of eight), with caller-supplied functors that build the activation rows in
 // shared memory and consume each finished 16-row tile.
 //
 // One persistent block per SM, 8 consumer warps + 1 producer warp.  The producer warp copies weight
@@ -8,12 +8,10 @@
 // the predecessor kernel because weights do not depend on it (programmatic dependent launch lets it
 // start during the predecessor's tail).  The consumer warps split a stage's k range and feed the
 // tensor core (ldmatrix + m16n8k16, fp32 accumulate) with the activation rows as the narrow operand,
-// so 16 activation rows cost the same instructions as one; the warps' partial sums are added in warp
+// so eight activation rows cost the same instructions as one; the warps' partial sums are added in warp
 // order, so a row's result does not depend on how many other rows share the step.
 //
-// Used by: the bf16 GEMV (projections, lm_head, PLE), the MoE router (+ routing epilogue), the
-// hyper-connection down projection (column splits, fused combine/norm prologue) and up projection
-// (fused gate/mean epilogue).
+// Used by: the bf16 GEMV (projections, lm_head, PLE) and the MoE router (+ routing epilogue).
 #pragma once
 #include "mma.cuh"
 #include "fuse.cuh"

@@ -35,10 +35,8 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// Roles that issue TMA loads and MMAs run as whole warps and elect the issuing lane at each group of instructions: tcgen05.mma
-// takes its descriptors from uniform registers, which the compiler can only keep across the loop when the branch is uniform for
-// the warp.  From a branch on one thread an MMA took 106 cycles to issue (83 with A in tensor memory) whatever its width;
-// elected, a 128 x 128 x 16 one takes 85 (68).
+// Roles that issue TMA loads and MMAs run as whole warps and elect the issuing lane at each group of instructions.  From a branch on one
+// thread an MMA took 106 cycles to issue (83 with A in tensor memory) whatever its width; elected, a 128 x 128 x 16 one takes 85 (68).
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;
     asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
