@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(128) gdn_conv_kernel(GdnConvArgs a) {
 
 // The same for a prefill chunk (more than MAX_ROWS rows; long runs, though nothing depends on it): a warp per head and 8 rows, four
 // channels per lane, so a head's norm is five shuffles instead of two meetings of a block per row and four rows' loads are in
-// flight.  4096 rows, 80 heads: 180 us with the kernel above, 95 here.  The last row of blocks forms decay
+// flight.  4096 rows, 80 heads, ring included: 179 us with the kernel above, 84 here.  The last row of blocks forms decay
 // and beta.  grid (ceil(M / 8), ceil((2 KL + VL) / 4) + 1), 128 threads.
 constexpr int CONVP_ROWS = 8;
 __global__ void __launch_bounds__(128) gdn_conv_prefill_kernel(GdnConvArgs a) {

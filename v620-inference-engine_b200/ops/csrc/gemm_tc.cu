@@ -941,7 +941,8 @@ QW_API int qwk_gemm_bf16_tc_tp(void *tp_, const void *A, const void *W, void *C,
 // The mixer's up projection with the block input formed in the epilogue: A bf16 [T][lda] (the activated low-rank vector), W bf16
 // [4 SH][ldw] (row 4 c + s: gate of stream s, column c), xn bf16 [T][4][SH]; out bf16 [T][ld_out]: mean over the streams of
 // sigmoid(A . W^T) * xn.  The logits (fp32, 4 SH a row) are never stored: as a product and a kernel that read them back
-// 118 us at 4096 x 2560 and 41 at 1021, here 76 and 28 (wide tiles; in pairs 79 and 29).  SH a multiple of 8.
+// 118 us at 4096 x 2560 and 41 at 1021, here 105 and 29.  Always 128 x 128 tiles: the epilogue bounds it, and two CTAs on an SM have twice
+// the warps for it (with 128 x 256 tiles 8 to 10 % more from 300 rows on).  SH a multiple of 8.
 QW_API int qwk_gemm_mix_tc(const void *A, const void *W, const void *xn, int SH, void *out, int ld_out, int T, int K, int lda, int ldw,
                            cudaStream_t s) {
     if (T <= 0) return 0;

@@ -472,8 +472,9 @@ constexpr int HU_PAD = HM_PAD, HU_COLS = 16, HU_BATCH = 4, HU_CLUSTER_MIN = 3;
 // vector u (fp32) goes through the MMAs as three bf16 parts (24 bits of mantissa: the products and sums are those of fp32
 // operands).  A block forms u itself from the down projection's parts (CLUSTER: eight blocks form every eighth row each and
 // write it into all eight shared memories), once per 16 rows.  y[s][c] = bf16(X[s][c] * w1[s][c]) as hc_down_mma_kernel has it.
-// In a chain of its own, us per launch, scalar products before and now: 1 row 5.4, 6.3 (with hc_down: 12.0, 10.0); 2 rows 8.0, 6.6;
-// 8 rows 21.2, 8.5 (lone form 9.3); 24 rows 49.6, 18.4 (lone 21.2).
+// In a chain of its own, us per launch, scalar products before and now: 1 row 5.4, 6.2 (with hc_down: 12.0, 9.9); 2 rows 8.0, 6.5;
+// 8 rows 21.2, 8.3 (lone form 9.3); 24 rows 49.6, 17.9 (lone 21.2).  One row takes it as well, although the scalar kernel would be faster
+// there: a row has to come out with the same bits alone and among others, or drafts that equal the model's choice are not accepted.
 // grid ceil(SH / 16), rounded up to clusters, 512 threads; hc must be 4; dynamic smem (3 x 16 + 64) x (R rounded up to 32, + 32) bf16.
 template <bool CLUSTER>
 __global__ void __launch_bounds__(HM_THREADS, 2) hc_up_mma_kernel(const float *red, int ld_red, const bf16 *Wu /* [SH][hc][R] */, const float *X,

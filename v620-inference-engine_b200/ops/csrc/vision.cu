@@ -151,7 +151,7 @@ __device__ __forceinline__ float vit_gelu(float v, int tanh_form) {
 }
 constexpr int VG_ROWS = 8;
 // Eight columns per thread (their bias in registers) down eight rows: 16-byte accesses.  At 3520 x 4304 53 us with two-byte
-// accesses, a division per value for its column; 19 now.
+// accesses, a division per value for its column; 21 now.
 __global__ void __launch_bounds__(128) vit_bias_gelu8_kernel(bf16 *y, const float *bias, int L, int D, int tanh_form) {
     const int c = (blockIdx.y * 128 + threadIdx.x) * 8;
     if (c >= D) return;
