@@ -8,14 +8,15 @@
 //   warp 0       TMA: Q once per unit, K and V tiles of 128 rows, three stages each
 //   warp 1       MMAs: S0, S1, then per key tile PV0, next S0, PV1, next S1
 //   warps 4-11   softmax, one warp group per query tile
-// O is rescaled only when a row's maximum rises by more than 8 (in log2 units) above the reference the sums use: the probabilities
-// then stay below 256, which costs nothing in bf16 or fp32, and the rescaling pass over O is rare after the first tile.
+// The reference is the row's running maximum, so that its largest weight is exactly 1: left up to 8 (in log2 units) below it, O needs rescaling
+// rarely and the kernel takes 111 us at 3520 patches, but the largest weights are rounded to bf16 as well, and the error against 64 bits
+// is up to 25 % above that of the kernel this one replaces (scores of size 3; 3 % at size 1).  With the maximum it is the same.
 // Head dim 72 = 64 + 8: a row's first 64 values are a 128B-swizzled panel, the last 8 a panel of 16-byte rows whose partner (the
 // other 8 of an MMA's k = 16) is a zeroed block.  V is read as it lies (key-major): 64 + 64 columns, of which the second panel's
 // first 8 count; the rest belongs to other heads and lands in columns of O that nobody reads.
 // What bounds it: the exponentials (128 x 128 per tile at 16 a cycle and SM: 1024 cycles; MMAs 780), and 224 units on 148 SMs for
 // 3520 patches and 16 heads.  It replaces a flash kernel on mma.sync (16 queries a warp, each warp reading every K and V fragment
-// from shared memory), which took 444 us there; this one takes 111.
+// from shared memory), which took 444 us there; this one takes 128.
 #include "tc.cuh"
 
 namespace qw {
@@ -180,7 +181,7 @@ __global__ void __launch_bounds__(VT_THREADS, 1) vit_attn_tc_kernel(const __grid
                 const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * a.scale;
                 if (j == 0) {
                     ref = fmaxf(mx, -1e30f);      // a row whose first scores are all -inf keeps a finite reference
-                } else if (__any_sync(0xffffffffu, mx > ref + 8.f)) {
+                } else if (__any_sync(0xffffffffu, mx > ref)) {
                     // every product issued before these scores is complete, this tile's last O among them
                     const float nref = fmaxf(ref, mx), f = exp2f(ref - nref);
                     ref = nref;
