@@ -427,3 +427,22 @@ def test_row_reduce_many_short_rows():
         val, idx, mx, sm = K_.row_reduce(x)
         assert torch.equal(val, x.max(1).values) and torch.equal(idx.long(), x.argmax(1)) and torch.equal(mx, val)
         assert torch.allclose(torch.log(sm.double()) + mx.double(), torch.logsumexp(x.double(), 1), atol=1e-5)
+
+
+def test_mixer_down_projection_is_as_exact_as_scalar_sums():
+    """2,560 exact products per stream: a tree of fp32 roundings leaves about 8e-8 of the sums' size (chains inside the tensor core, which
+    cut off instead of rounding, leave 1.1e-7)."""
+    import ctypes as C
+    from qwb200.ops import lib as qlib
+    L = qlib.load(True)
+    SH, hc, down, M, dev = 2560, 4, 324, 24, _dev()
+    ld = hc + hc * down
+    g = torch.Generator(device="cuda").manual_seed(11)
+    rn = lambda *s: torch.randn(*s, generator=g, device=dev)
+    X, w1, Wd, send = rn(M, hc, SH), 1 + 0.1 * rn(hc, SH), (rn(down, hc, SH) * 0.02).to(torch.bfloat16), torch.zeros(M, ld, device=dev)
+    P = lambda t: C.c_void_p(t.data_ptr())
+    assert L.qwk_hc_down(P(X), None, None, SH, P(X), P(w1), P(Wd), P(send), ld, SH, hc, down, M, C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    part = torch.einsum("msc,jsc->msj", (X * w1).to(torch.bfloat16).double(), Wd.double())
+    assert float((send[:, hc:].view(M, hc, down).double() - part).norm() / part.norm()) < 9e-8
+    ss = X.double().pow(2).sum(-1)
+    assert float((send[:, :hc].double() - ss).norm() / ss.norm()) < 9e-8

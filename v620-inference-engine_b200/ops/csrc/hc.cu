@@ -355,6 +355,19 @@ __device__ __forceinline__ void mma_rows(float (&c)[2][4], const uint4 &r, const
     mma_bf16(c[1], r.z, r8.z, r.w, r8.w, w.z, w.w);
 }
 
+// Sum of N values in pairs: log2 N roundings on the way of each instead of up to N - 1.
+template <int N, class F>
+__device__ __forceinline__ float pair_sum(const F &at) {
+    float v[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) v[k] = at(k);
+#pragma unroll
+    for (int o = N / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < o; ++k) v[k] += v[k + o];
+    return v[0];
+}
+
 constexpr int HM_THREADS = 512, HM_PAD = 32;      // padding of shared rows: their stride is 64 bytes off a multiple of 128
 constexpr int HD_CL = 8, HD_J = 8, HD_W = HM_THREADS / 32, HD_ROWS = 8, HD_CLUSTER_MIN = 4;
 // A CTA owns eight outputs j of one stream over all columns (its sixteen warps take every sixteenth chunk of 32).  The weights go
@@ -364,8 +377,10 @@ constexpr int HD_CL = 8, HD_J = 8, HD_W = HM_THREADS / 32, HD_ROWS = 8, HD_CLUST
 //   CLUSTER  eight CTAs build two slices each and write them into all eight shared memories; otherwise every CTA would rebuild every
 //            row, which at 24 rows was most of the kernel's time
 //   else     every CTA builds all slices, a warp each: fewer rows cost less than the cluster's two meetings
-// In a chain of its own, us per launch, scalar products before and now: 1 row 6.5, 3.9; 2 rows 8.0, 5.0; 8 rows 19.2, 6.9; 24 rows 44, 19.
-// The line between the forms: at 3 rows 6.0 (lone), at 4 rows 5.7 (cluster).
+// In a chain of its own, us per launch, scalar products before and now: 1 row 6.5, 4.1; 2 rows 8.0, 5.4; 8 rows 19.2, 7.2; 24 rows 44, 20.
+// The line between the forms: at 3 rows 6.4 (lone), at 4 rows 5.8 (cluster).
+// Error of the sums against 64 bits: 7.8e-8 of their size, as the scalar products had it (running sums kept in the tensor core 1.1e-7,
+// and 0.2 us less).
 // grid (ceil(down / 8), rounded up to clusters, hc), 512 threads, dynamic smem (8 + min(M, 8)) x (SH + 32) bf16.
 template <bool CLUSTER>
 __global__ void __launch_bounds__(HM_THREADS, 2) hc_down_mma_kernel(HcDownArgs a) {
@@ -441,26 +456,24 @@ __global__ void __launch_bounds__(HM_THREADS, 2) hc_down_mma_kernel(HcDownArgs a
         if (CLUSTER) cl.sync();
         else __syncthreads();
         if (blockIdx.x == 0 && tid < n) {
-            float ss = 0.f;
-#pragma unroll
-            for (int k = 0; k < HD_W; ++k) ss += sspart[k][tid];
-            a.send[(long long)(m0 + tid) * a.ld_send + s] = ss;
+            a.send[(long long)(m0 + tid) * a.ld_send + s] = pair_sum<HD_W>([&](int k) { return sspart[k][tid]; });
         }
         // operand rows past the last repeat it (and rows 8-15 the first eight): a result row depends on its own operand row alone
-        float c[2][4] = {};
+        float s0 = 0.f, s1 = 0.f;          // chunks are added with rounding: the tensor core's own running sum cuts off
         const bf16 *ya = y + min(g, n - 1) * ys + q * 8, *wa = ws + g * ys + q * 8;
 #pragma unroll 5
         for (int chunk = warp; chunk < nch; chunk += HD_W) {
             const uint4 r = *reinterpret_cast<const uint4 *>(ya + chunk * 32);
+            float c[2][4] = {};
             mma_rows(c, r, r, *reinterpret_cast<const uint4 *>(wa + chunk * 32));
+            s0 += c[0][0] + c[1][0];
+            s1 += c[0][1] + c[1][1];
         }
-        *reinterpret_cast<float2 *>(&red[warp][g][2 * q]) = make_float2(c[0][0] + c[1][0], c[0][1] + c[1][1]);
+        *reinterpret_cast<float2 *>(&red[warp][g][2 * q]) = make_float2(s0, s1);
         __syncthreads();
         if (tid < HD_ROWS * HD_J && (tid >> 3) < n && j0 + (tid & 7) < a.down) {
-            float v = 0.f;
-#pragma unroll
-            for (int k = 0; k < HD_W; ++k) v += red[k][tid >> 3][tid & 7];
-            a.send[(long long)(m0 + (tid >> 3)) * a.ld_send + a.hc + s * a.down + j0 + (tid & 7)] = v;
+            a.send[(long long)(m0 + (tid >> 3)) * a.ld_send + a.hc + s * a.down + j0 + (tid & 7)] =
+                pair_sum<HD_W>([&](int k) { return red[k][tid >> 3][tid & 7]; });
         }
         __syncthreads();
     }
@@ -472,7 +485,7 @@ constexpr int HU_PAD = HM_PAD, HU_COLS = 16, HU_BATCH = 4, HU_CLUSTER_MIN = 3;
 // vector u (fp32) goes through the MMAs as three bf16 parts (24 bits of mantissa: the products and sums are those of fp32
 // operands).  A block forms u itself from the down projection's parts (CLUSTER: eight blocks form every eighth row each and
 // write it into all eight shared memories), once per 16 rows.  y[s][c] = bf16(X[s][c] * w1[s][c]) as hc_down_mma_kernel has it.
-// In a chain of its own, us per launch, scalar products before and now: 1 row 5.4, 6.2 (with hc_down: 12.0, 9.9); 2 rows 8.0, 6.5;
+// In a chain of its own, us per launch, scalar products before and now: 1 row 5.4, 6.2 (with hc_down: 12.0, 10.1); 2 rows 8.0, 6.5;
 // 8 rows 21.2, 8.3 (lone form 9.3); 24 rows 49.6, 17.9 (lone 21.2).  One row takes it as well, although the scalar kernel would be faster
 // there: a row has to come out with the same bits alone and among others, or drafts that equal the model's choice are not accepted.
 // grid ceil(SH / 16), rounded up to clusters, 512 threads; hc must be 4; dynamic smem (3 x 16 + 64) x (R rounded up to 32, + 32) bf16.
