@@ -10,13 +10,14 @@
 //   warps 4-11   softmax, one warp group per query tile
 // The reference is the row's running maximum, so that its largest weight is exactly 1: left up to 8 (in log2 units) below it, O needs rescaling
 // rarely and the kernel takes 111 us at 3520 patches, but the largest weights are rounded to bf16 as well, and the error against 64 bits
-// is up to 25 % above that of the kernel this one replaces (scores of size 3; 3 % at size 1).  With the maximum it is the same.
+// is up to 25 % above that of the kernel this one replaces (scores of size 3; 3 % at size 1).  With the maximum it is the same.  O is rescaled
+// behind the probabilities, all 80 columns in flight at once (in front of them, 16 at a time, 128 us).
 // Head dim 72 = 64 + 8: a row's first 64 values are a 128B-swizzled panel, the last 8 a panel of 16-byte rows whose partner (the
 // other 8 of an MMA's k = 16) is a zeroed block.  V is read as it lies (key-major): 64 + 64 columns, of which the second panel's
 // first 8 count; the rest belongs to other heads and lands in columns of O that nobody reads.
 // What bounds it: the exponentials (128 x 128 per tile at 16 a cycle and SM: 1024 cycles; MMAs 780), and 224 units on 148 SMs for
 // 3520 patches and 16 heads.  It replaces a flash kernel on mma.sync (16 queries a warp, each warp reading every K and V fragment
-// from shared memory), which took 444 us there; this one takes 128.
+// from shared memory), which took 444 us there; this one takes 119.
 #include "tc.cuh"
 
 namespace qw {
@@ -179,23 +180,11 @@ __global__ void __launch_bounds__(VT_THREADS, 1) vit_attn_tc_kernel(const __grid
 #pragma unroll
                     for (int c = 0; c < 4; ++c) m4[c] = fmaxf(m4[c], __uint_as_float(s[c][i]));
                 const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * a.scale;
-                if (j == 0) {
-                    ref = fmaxf(mx, -1e30f);      // a row whose first scores are all -inf keeps a finite reference
-                } else if (__any_sync(0xffffffffu, mx > ref)) {
-                    // every product issued before these scores is complete, this tile's last O among them
-                    const float nref = fmaxf(ref, mx), f = exp2f(ref - nref);
-                    ref = nref;
-                    sum *= f;
-#pragma unroll 1
-                    for (int c = 0; c < 80; c += 16) {
-                        uint32_t o[16];
-                        tmem_ld16(obase + c, o);
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
-                        tmem_st16(obase + c, o);
-                    }
-                }
+                // a row whose first scores are all -inf keeps a finite reference
+                const float nref = j ? fmaxf(ref, mx) : fmaxf(mx, -1e30f), f = j ? exp2f(ref - nref) : 1.f;
+                const bool risen = __any_sync(0xffffffffu, f != 1.f) != 0;
+                ref = nref;
+                sum *= f;
                 float sum4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
@@ -209,6 +198,20 @@ __global__ void __launch_bounds__(VT_THREADS, 1) vit_attn_tc_kernel(const __grid
                     tmem_st16(sbase + c * 16, p);
                 }
                 sum += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+                if (risen) {
+                    // every product issued before these scores is complete, this tile's last O among them.  Behind the probabilities the
+                    // scores' registers are free: the whole row of O is on its way at once
+                    uint32_t o[5][16];
+#pragma unroll
+                    for (int c = 0; c < 5; ++c) tmem_ld16(obase + c * 16, o[c]);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int c = 0; c < 5; ++c) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) o[c][i] = __float_as_uint(__uint_as_float(o[c][i]) * f);
+                        tmem_st16(obase + c * 16, o[c]);
+                    }
+                }
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 __syncwarp();
