@@ -68,7 +68,7 @@ def host_kv_bytes(cfg: ModelConfig, ranks: int, host_pages: int) -> int:
 
 def buffer_bytes(cfg: ModelConfig, ranks: int, max_rows: int, prefill_chunk: int) -> int:
     """Step buffers and the prefill chunk's scratch: a generous allowance rather than a sum of shapes (the token-major
-    path keeps about 1.4 MB per token of the chunk on one rank: activations of the widest projection in fp32 and bf16,
+    path gets 1.4 MB per token of the chunk on one rank, of which it uses a little less: activations of the widest projection in fp32 and bf16,
     the expert pairs' inputs and outputs, the scoring tile), plus the CUDA context, graphs and allocator slack."""
     per_token = int(1.4e6 * cfg.hidden / 2560 / max(1, ranks) ** 0.5)
     return prefill_chunk * per_token + max_rows * 4 * (cfg.vocab // ranks + 64 * cfg.hidden) + (3 << 30)

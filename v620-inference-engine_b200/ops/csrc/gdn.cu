@@ -389,7 +389,7 @@ QW_API int qwk_gdn_conv(const float *proj, int ld_proj, float *ring, const float
         gdn_conv_kernel<<<grid, 128, 0, s>>>(a);
     }
     const int qkv_l = (2 * KL + VL) * GD;
-    // A batch of more than MAX_ROWS rows is one run of one slot (a prefill chunk): only its last GDN_RING rows stay in the ring.
+    // The ring counts on a batch of more than MAX_ROWS rows being one run of one slot (a prefill chunk): only its last GDN_RING rows stay.
     const int m_first = M > MAX_ROWS ? M - GDN_RING : 0;
     dim3 g2(M - m_first, (qkv_l + 255) / 256);
     gdn_ring_kernel<<<g2, 256, 0, s>>>(proj, ld_proj, ring, qkv_l, a.rows, m_first);
