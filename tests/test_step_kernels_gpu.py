@@ -1,0 +1,84 @@
+"""Kernels of a decode or verification step at the edges of their forms: streamed products, the delta-net step, flash-decode (GPU only)."""
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _lib():
+    from qwb200.ops import lib as qlib
+    return qlib.load(True)
+
+
+def P(t):
+    return None if t is None else C.c_void_p(t.data_ptr())
+
+
+def S():
+    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def i32(v):
+    return torch.tensor(v, dtype=torch.int32, device=DEV)
+
+
+def gen(seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return lambda *s: torch.randn(*s, generator=g, device=DEV)
+
+
+@pytest.mark.parametrize("runs", [[1], [6, 6, 6, 6], [12], [13], [32], [3, 17, 1, 8]])
+def test_delta_net_step_of_runs_equals_row_by_row(runs):
+    """A run's rows in one launch - eight at a time, runs that end inside eight, runs longer than what the kernel stores into the ring itself
+    - give what as many launches of single rows give: outputs, states, saved states and ring, bit for bit."""
+    KL, VL, ring_rows, eps = 2, 6, 16, 1e-6
+    D, slots = 128, len(runs)
+    qkv_l = (2 * KL + VL) * D
+    ld = qkv_l + VL * D + 2 * VL
+    rn = gen(sum(runs))
+    M = sum(runs)
+    proj, cw = rn(M, ld), rn(qkv_l, 4) * 0.5
+    a_log, dt, nw = rn(VL) * 0.1, rn(VL) * 0.1, 1 + 0.1 * rn(D)
+    ring0, S0 = rn(slots, ring_rows, qkv_l), rn(slots, VL, D, D) * 0.1
+    base = [0, 2, 40, 7][:slots]
+    rows = [(s, base[s] + i, sum(runs[:s])) for s in range(slots) for i in range(runs[s])]
+
+    def step(m0, n, starts, lens, ring, St, save, o):
+        scratch = torch.empty(n * (qkv_l + 2 * VL), device=DEV)
+        t = [i32([r[0] for r in rows[m0:m0 + n]]), i32([r[1] for r in rows[m0:m0 + n]]), i32(starts), i32(lens)]
+        assert _lib().qwk_gdn_step(P(proj[m0:]), ld, P(ring), P(cw), P(a_log), P(dt), P(nw), KL, VL, n, *map(P, t), P(St), P(save), P(scratch),
+                                   P(scratch[n * qkv_l:]), P(scratch[n * (qkv_l + VL):]), P(o), C.c_float(eps), S()) == 0
+        torch.cuda.synchronize()
+
+    outs = []
+    for whole in (True, False):
+        ring, St, o, save = ring0.clone(), S0.clone(), torch.zeros(M, VL * D, dtype=torch.bfloat16, device=DEV), torch.zeros(M, VL, D, D, device=DEV)
+        if whole:
+            lens = [0] * M
+            for s in range(slots):
+                lens[sum(runs[:s])] = runs[s]
+            step(0, M, [r[2] for r in rows], lens, ring, St, save, o)
+        else:
+            for m in range(M):
+                step(m, 1, [0], [1], ring, St, save[m:], o[m:])
+        outs.append((ring, St, save, o))
+    for a, b in zip(*outs):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("pairs,layers,state", [([[0, 2], [2, 0], [1, -1]], 3, 48 * 128 * 128), ([[1, 1]], 1, 4), ([[0, 1], [1, 3]], 2, 4096 * 3 + 8)])
+def test_accepted_states_are_copied_whole(pairs, layers, state):
+    """Every value of an accepted row's state, whatever its size (pieces of 16 KB, a last one that is not whole); rejected slots stay."""
+    rn = gen(state)
+    rows, slots = 4, 3
+    save, St = rn(layers, rows, state), rn(layers, slots, state)
+    want = St.clone()
+    for s, r in pairs:
+        if r >= 0:
+            want[:, s] = save[:, r]
+    ptrs = torch.tensor([St[i].data_ptr() for i in range(layers)], dtype=torch.int64, device=DEV)
+    assert _lib().qwk_gdn_accept(P(ptrs), P(save), layers, rows, C.c_longlong(state), P(i32(pairs)), len(pairs), S()) == 0
+    assert torch.equal(St, want)

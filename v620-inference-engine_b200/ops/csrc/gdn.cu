@@ -138,16 +138,18 @@ __global__ void __launch_bounds__(128) gdn_conv_prefill_kernel(GdnConvArgs a) {
     }
 }
 
-// Stores the batch's pre-conv rows into the ring (after gdn_conv has read the old entries).
+// Stores the pre-conv rows of runs longer than `min_run` into the ring (after the convolution has read the old entries).
 // grid (M, ceil(qkv_l/256)).
-__global__ void gdn_ring_kernel(const float *proj, int ld_proj, float *ring, int qkv_l, Rows rows, int m_first) {
+__global__ void gdn_ring_kernel(const float *proj, int ld_proj, float *ring, int qkv_l, Rows rows, int m_first, int min_run) {
+    pdl_wait();
+    pdl_trigger();
     const int m = m_first + blockIdx.x;
     const int c = blockIdx.y * 256 + threadIdx.x;
     if (c >= qkv_l) return;
     const int slot = rows.slot[m], pos = rows.pos[m];
     // a run longer than the ring keeps only its last GDN_RING rows
     const int rs = rows.run_start[m], len = rows.run_len[rs];
-    if (m - rs < len - GDN_RING) return;
+    if (len <= min_run || m - rs < len - GDN_RING) return;
     ring[((long long)slot * GDN_RING + (pos % GDN_RING)) * qkv_l + c] = proj[(long long)m * ld_proj + c];
 }
 
@@ -228,11 +230,13 @@ __global__ void __launch_bounds__(512) gdn_scan_kernel(GdnScanArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------
-// Fused decode step for short runs (M <= GDN_RING - 4): conv + gating + L2 norm + delta-rule update +
-// gated norm in one kernel, and the ring store.  grid (M, VL), 512 threads; the block of (run start,
-// head h) walks the run.  q/k of the head's key head are recomputed by each of the value heads that
-// share it.  Ring entries written here (positions of the run) never alias the entries read
-// (positions before the run) because the run is shorter than the ring minus the conv window.
+// Fused step: conv + gating + L2 norm + delta-rule update + gated norm in one kernel, and the ring store of runs of up to
+// RUN_INLINE rows.  grid (M, VL), 512 threads; the block of (run start, head h) walks the run, FR = 8 rows at a time: what does not
+// depend on the state - the loads, conv, norms and gates of all these rows - first, then the state's rows one behind the other with one
+// meeting each, then their outputs' norms, a warp per row.  (With a row's loads, norms and seven meetings on the chain of every row 24
+// rows of four runs took 70 us; they take 36, and one row 9.)  q/k of the head's key head are recomputed by each of the value heads that share it.
+// The ring entries of a run's first 13 rows are not those that conv reads (three positions before the run); a longer run's are stored
+// by gdn_ring_kernel behind this kernel, because the blocks of a run do not wait for one another.
 // ------------------------------------------------------------------------------------------
 struct GdnFusedArgs {
     const float *proj;
@@ -245,15 +249,19 @@ struct GdnFusedArgs {
     bf16 *o;
     float eps;
 };
+constexpr int RUN_INLINE = GDN_RING - 4;
 
-__global__ void __launch_bounds__(512) gdn_fused_kernel(GdnFusedArgs a) {
-    __shared__ float kq[2][GD];
-    __shared__ float vv[GD];
-    __shared__ float red[4][GD];
-    __shared__ float scratch[32];
-    __shared__ float s_gate[2];
+// FR = 1: a step of one row, which has nothing to gather rows for.
+template <int FR>
+__global__ void __launch_bounds__(512, FR == 1 ? 1 : 2) gdn_fused_kernel(GdnFusedArgs a) {
+    __shared__ __align__(16) float qkv[FR][3][GD];       // conv output: q (normed, scaled), k (normed), v
+    __shared__ float red[2][4][GD];                      // S k, by quarter of the keys; row r in buffer r & 1
+    __shared__ float part[FR][4][GD];                    // S q, the same
+    __shared__ float ssq[FR][8];                         // sums of squares: warps 0-3 q, 4-7 k
+    __shared__ float gate[FR][2];                        // decay, beta
+    __shared__ float zs[FR][GD];                         // output gates
     const int m0 = blockIdx.x, h = blockIdx.y;
-    const int tid = threadIdx.x, c = tid & 127, kg = tid >> 7;
+    const int tid = threadIdx.x, c = tid & 127, kg = tid >> 7, warp = tid >> 5, lane = tid & 31;
     const int qkv_l = (2 * a.KL + a.VL) * GD;
     const int rep = a.VL / a.KL, kh = h / rep;
     // conv taps of this thread's channel (weights: independent of the predecessor)
@@ -269,7 +277,7 @@ __global__ void __launch_bounds__(512) gdn_fused_kernel(GdnFusedArgs a) {
     // The row table was written before the step began and the recurrent state only by this kernel in the previous step:
     // neither depends on the predecessor, so the state (64 KB per head, from HBM) is fetched before waiting for it.
     if (a.rows.run_start[m0] != m0) return;
-    const int len = a.rows.run_len[m0], slot = a.rows.slot[m0];
+    const int len = a.rows.run_len[m0], slot = a.rows.slot[m0], pos0 = a.rows.pos[m0];
     float *ring = a.ring + (long long)slot * GDN_RING * qkv_l;
     float *Sg = a.S + ((long long)slot * a.VL + h) * GD * GD;
     float S[32];
@@ -277,80 +285,108 @@ __global__ void __launch_bounds__(512) gdn_fused_kernel(GdnFusedArgs a) {
     for (int i = 0; i < 32; ++i) S[i] = Sg[(kg * 32 + i) * GD + c];
     pdl_wait();
     pdl_trigger();
-    for (int r = 0; r < len; ++r) {
-        const int m = m0 + r, pos = a.rows.pos[m];
-        // conv + silu for q / k / v channels
-        float val = 0.f;
+    const bool stores = ch >= 0 && len <= RUN_INLINE && (kg == 2 || h % rep == 0);      // v channels by every head, q/k by the group's first
+    float w[3] = {0.f, 0.f, 0.f};                        // pre-conv values 3, 2, 1 rows back
+    if (ch >= 0) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int q = pos0 - 3 + k;
+            if (q >= 0) w[k] = ring[(q % GDN_RING) * qkv_l + ch];
+        }
+    }
+    for (int r0 = 0; r0 < len; r0 += FR) {
+        const int n = min(FR, len - r0);
+        const float *prow = a.proj + (long long)(m0 + r0) * a.ld_proj;
+        // ---- conv + silu, norms and gates of these rows
+        float x[FR];
         if (ch >= 0) {
-            float acc = 0.f;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int back = 3 - k, q = pos - back;
-                float x;
-                if (r - back >= 0) x = a.proj[(long long)(m - back) * a.ld_proj + ch];
-                else if (q >= 0) x = ring[(q % GDN_RING) * qkv_l + ch];
-                else x = 0.f;
-                acc = fmaf(tap[k], x, acc);
-            }
-            val = siluf_(acc);
-        }
-        // L2 norms of q (warps 0-3) and k (warps 4-7)
-        const float ssw = warp_sum(kg < 2 ? val * val : 0.f);
-        __syncthreads();
-        if ((tid & 31) == 0) scratch[tid >> 5] = ssw;
-        if (tid == 0) {
-            const float *row = a.proj + (long long)m * a.ld_proj + qkv_l + a.VL * GD;
+            for (int i = 0; i < FR; ++i) x[i] = i < n ? prow[(long long)i * a.ld_proj + ch] : 0.f;
+        } else if (c < n) {
+            const float *row = prow + (long long)c * a.ld_proj + qkv_l + a.VL * GD;
             const float g = -__expf(a.A_log[h]) * softplusf_(row[a.VL + h] + a.dt_bias[h]);
-            s_gate[0] = __expf(g);
-            s_gate[1] = sigmoidf_(row[h]);
+            gate[c][0] = __expf(g);
+            gate[c][1] = sigmoidf_(row[h]);
         }
-        __syncthreads();
-        if (kg == 0) {
-            const float ss = scratch[0] + scratch[1] + scratch[2] + scratch[3];
-            kq[1][c] = val / sqrtf(ss + a.eps) * 0.08838834764831845f;
-        } else if (kg == 1) {
-            const float ss = scratch[4] + scratch[5] + scratch[6] + scratch[7];
-            kq[0][c] = val / sqrtf(ss + a.eps);
-        } else if (kg == 2) {
-            vv[c] = val;
-        }
-        __syncthreads();
-        const float dec = s_gate[0], be = s_gate[1];
-        float p = 0.f;
+        if (ch >= 0) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            S[i] *= dec;
-            p = fmaf(S[i], kq[0][kg * 32 + i], p);
-        }
-        red[kg][c] = p;
-        __syncthreads();
-        const float stk = red[0][c] + red[1][c] + red[2][c] + red[3][c];
-        const float u = (vv[c] - stk) * be;
-        float oq = 0.f;
+            for (int i = 0; i < FR; ++i) {
+                const float cur = x[i];
+                const float acc = fmaf(tap[3], cur, fmaf(tap[2], w[2], fmaf(tap[1], w[1], tap[0] * w[0])));
+                if (i < n) {
+                    if (stores) ring[((pos0 + r0 + i) % GDN_RING) * qkv_l + ch] = cur;
+                    w[0] = w[1]; w[1] = w[2]; w[2] = cur;
+                }
+                x[i] = siluf_(acc);
+            }
+            if (kg < 2) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            S[i] = fmaf(kq[0][kg * 32 + i], u, S[i]);
-            oq = fmaf(S[i], kq[1][kg * 32 + i], oq);
+                for (int i = 0; i < FR; ++i) {
+                    if (i >= n) break;
+                    const float s = warp_sum(x[i] * x[i]);
+                    if (lane == 0) ssq[i][warp] = s;
+                }
+            }
         }
-        __syncthreads();
-        red[kg][c] = oq;
-        __syncthreads();
-        if (a.save) {
-            float *sv = a.save + ((long long)m * a.VL + h) * GD * GD;
+        __syncthreads();                                 // sums and gates; the rows before these are consumed
+        for (int i = kg; i < n; i += 4) zs[i][c] = prow[(long long)i * a.ld_proj + qkv_l + h * GD + c];
+        if (ch >= 0) {
 #pragma unroll
-            for (int i = 0; i < 32; ++i) sv[(kg * 32 + i) * GD + c] = S[i];
+            for (int i = 0; i < FR; ++i) {
+                if (i >= n) break;
+                float v = x[i];
+                if (kg < 2) {
+                    const float *s = ssq[i] + kg * 4;
+                    v = v / sqrtf(s[0] + s[1] + s[2] + s[3] + a.eps);
+                    if (kg == 0) v *= 0.08838834764831845f;
+                }
+                qkv[i][kg][c] = v;
+            }
         }
-        float ov = 0.f;
-        if (kg == 0) ov = red[0][c] + red[1][c] + red[2][c] + red[3][c];
-        const float ss = block_sum<512>(ov * ov, scratch);
-        if (kg == 0) {
-            const float z = a.proj[(long long)m * a.ld_proj + qkv_l + h * GD + c];
-            const float y = ov * rsqrtf(ss / float(GD) + a.eps) * a.norm_w[c] * sigmoidf_(z);
-            a.o[(long long)m * a.VL * GD + h * GD + c] = __float2bfloat16(y);
+        __syncthreads();
+        // ---- the state's rows
+        for (int i = 0; i < n; ++i) {
+            const float dec = gate[i][0], be = gate[i][1];
+            const float *kk = qkv[i][1] + kg * 32, *qq = qkv[i][0] + kg * 32;
+            float p = 0.f;
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+                const float4 k4 = *reinterpret_cast<const float4 *>(kk + j);
+                S[j] *= dec; S[j + 1] *= dec; S[j + 2] *= dec; S[j + 3] *= dec;
+                p = fmaf(S[j], k4.x, p); p = fmaf(S[j + 1], k4.y, p); p = fmaf(S[j + 2], k4.z, p); p = fmaf(S[j + 3], k4.w, p);
+            }
+            float (*rd)[GD] = red[i & 1];
+            rd[kg][c] = p;
+            __syncthreads();
+            const float u = (qkv[i][2][c] - (rd[0][c] + rd[1][c] + rd[2][c] + rd[3][c])) * be;
+            float oq = 0.f;
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+                const float4 k4 = *reinterpret_cast<const float4 *>(kk + j), q4 = *reinterpret_cast<const float4 *>(qq + j);
+                S[j] = fmaf(k4.x, u, S[j]); S[j + 1] = fmaf(k4.y, u, S[j + 1]); S[j + 2] = fmaf(k4.z, u, S[j + 2]); S[j + 3] = fmaf(k4.w, u, S[j + 3]);
+                oq = fmaf(S[j], q4.x, oq); oq = fmaf(S[j + 1], q4.y, oq); oq = fmaf(S[j + 2], q4.z, oq); oq = fmaf(S[j + 3], q4.w, oq);
+            }
+            part[i][kg][c] = oq;
+            if (a.save) {
+                float *sv = a.save + ((long long)(m0 + r0 + i) * a.VL + h) * GD * GD;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) sv[(kg * 32 + j) * GD + c] = S[j];
+            }
         }
-        // ring store of this row's pre-conv values: v channels by every head, q/k by the first head of the group
-        if (ch >= 0 && (kg == 2 || h % rep == 0))
-            ring[(pos % GDN_RING) * qkv_l + ch] = a.proj[(long long)m * a.ld_proj + ch];
+        __syncthreads();                                 // all partial outputs
+        if (warp < n) {
+            float v[4], ss = 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int d = j * 32 + lane;
+                v[j] = part[warp][0][d] + part[warp][1][d] + part[warp][2][d] + part[warp][3][d];
+                ss += warp_sum(v[j] * v[j]);
+            }
+            const float r = rsqrtf(ss / float(GD) + a.eps);
+            bf16 *o = a.o + (long long)(m0 + r0 + warp) * a.VL * GD + h * GD;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) o[j * 32 + lane] = __float2bfloat16(v[j] * r * a.norm_w[j * 32 + lane] * sigmoidf_(zs[warp][j * 32 + lane]));
+        }
     }
 #pragma unroll
     for (int i = 0; i < 32; ++i) Sg[(kg * 32 + i) * GD + c] = S[i];
@@ -359,14 +395,23 @@ __global__ void __launch_bounds__(512) gdn_fused_kernel(GdnFusedArgs a) {
 
 // Speculative acceptance: for every (slot, row) pair and every GDN layer, the state saved after `row` of the last
 // verification step becomes the slot's state.  grid (blocks, pairs, layers); S_ptrs[layer] = [slots][state] fp32,
-// save = [layers][max_rows][state].  state % 4 == 0.
+// save = [layers][max_rows][state].  state % 4 == 0.  A thread's four loads are in flight together, and there are as many blocks as
+// the state has pieces of 16 KB (eight blocks per pair and layer, one load a thread at a time: 50 us for four pairs and three layers of 3 MB, now 13).
+constexpr int ACCEPT_VALUES = 4;
 __global__ void __launch_bounds__(256) gdn_accept_kernel(float *const *S_ptrs, const float *save, int max_rows, long long state,
                                                          const int *pairs) {
     const int layer = blockIdx.z, slot = pairs[2 * blockIdx.y], row = pairs[2 * blockIdx.y + 1];
     if (row < 0) return;
     const float4 *src = reinterpret_cast<const float4 *>(save + ((long long)layer * max_rows + row) * state);
     float4 *dst = reinterpret_cast<float4 *>(S_ptrs[layer] + (long long)slot * state);
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (state >> 2); i += (long long)gridDim.x * blockDim.x) dst[i] = src[i];
+    const long long n = state >> 2, i0 = (long long)blockIdx.x * (ACCEPT_VALUES * 256) + threadIdx.x;
+    float4 v[ACCEPT_VALUES];
+#pragma unroll
+    for (int k = 0; k < ACCEPT_VALUES; ++k)
+        if (i0 + k * 256 < n) v[k] = __ldcs(src + i0 + k * 256);
+#pragma unroll
+    for (int k = 0; k < ACCEPT_VALUES; ++k)
+        if (i0 + k * 256 < n) dst[i0 + k * 256] = v[k];
 }
 
 }  // namespace qw
@@ -392,7 +437,7 @@ QW_API int qwk_gdn_conv(const float *proj, int ld_proj, float *ring, const float
     // The ring counts on a batch of more than MAX_ROWS rows being one run of one slot (a prefill chunk): only its last GDN_RING rows stay.
     const int m_first = M > MAX_ROWS ? M - GDN_RING : 0;
     dim3 g2(M - m_first, (qkv_l + 255) / 256);
-    gdn_ring_kernel<<<g2, 256, 0, s>>>(proj, ld_proj, ring, qkv_l, a.rows, m_first);
+    launch_pdl(gdn_ring_kernel, g2, dim3(256), 0, s, proj, ld_proj, ring, qkv_l, a.rows, m_first, 0);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -408,24 +453,23 @@ QW_API int qwk_gdn_scan(const float *qkv, const float *decay, const float *beta,
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-// One GDN step for M rows: the fused kernel for short batches, else conv + ring + scan.
+// One GDN step for M rows: the fused kernel, and the ring store of long runs where there can be any.
 QW_API int qwk_gdn_step(const float *proj, int ld_proj, float *ring, const float *cw, const float *A_log,
                         const float *dt_bias, const float *norm_w, int KL, int VL, int M, const int *slot, const int *pos,
                         const int *run_start, const int *run_len, float *S, float *save, float *qkv, float *decay,
                         float *beta, void *o, float eps, cudaStream_t s) {
-    if (M <= GDN_RING - 4) {
-        GdnFusedArgs a;
-        a.proj = proj; a.ld_proj = ld_proj; a.ring = ring; a.cw = cw; a.A_log = A_log; a.dt_bias = dt_bias;
-        a.norm_w = norm_w; a.KL = KL; a.VL = VL; a.rows = Rows{M, slot, pos, run_start, run_len};
-        a.S = S; a.save = save; a.o = (bf16 *)o; a.eps = eps;
-        cudaError_t e = launch_pdl(gdn_fused_kernel, dim3(M, VL), dim3(512), 0, s, a);
-        return e == cudaSuccess ? 0 : -2;
+    (void)qkv; (void)decay; (void)beta;          // scratch of the step in three kernels
+    GdnFusedArgs a;
+    a.proj = proj; a.ld_proj = ld_proj; a.ring = ring; a.cw = cw; a.A_log = A_log; a.dt_bias = dt_bias;
+    a.norm_w = norm_w; a.KL = KL; a.VL = VL; a.rows = Rows{M, slot, pos, run_start, run_len};
+    a.S = S; a.save = save; a.o = (bf16 *)o; a.eps = eps;
+    if (launch_pdl(M == 1 ? gdn_fused_kernel<1> : gdn_fused_kernel<8>, dim3(M, VL), dim3(512), 0, s, a) != cudaSuccess) return -2;
+    if (M > RUN_INLINE) {
+        const int qkv_l = (2 * KL + VL) * GD;
+        if (launch_pdl(gdn_ring_kernel, dim3(M, (qkv_l + 255) / 256), dim3(256), 0, s, proj, ld_proj, ring, qkv_l, a.rows, 0, RUN_INLINE) != cudaSuccess)
+            return -2;
     }
-    int rc = qwk_gdn_conv(proj, ld_proj, ring, cw, A_log, dt_bias, KL, VL, M, slot, pos, run_start, run_len, qkv, decay,
-                          beta, eps, s);
-    if (rc) return rc;
-    return qwk_gdn_scan(qkv, decay, beta, proj, ld_proj, S, save, norm_w, KL, VL, M, slot, pos, run_start, run_len, o,
-                        eps, s);
+    return 0;
 }
 
 
@@ -434,6 +478,6 @@ QW_API int qwk_gdn_accept(const void *S_ptrs, const float *save, int n_layers, i
                           int n_pairs, cudaStream_t s) {
     if (n_pairs <= 0 || n_layers <= 0) return 0;
     if (state & 3) return -1;
-    gdn_accept_kernel<<<dim3(8, n_pairs, n_layers), 256, 0, s>>>((float *const *)S_ptrs, save, max_rows, state, pairs);
+    gdn_accept_kernel<<<dim3((unsigned)((state / 4 + ACCEPT_VALUES * 256 - 1) / (ACCEPT_VALUES * 256)), n_pairs, n_layers), 256, 0, s>>>((float *const *)S_ptrs, save, max_rows, state, pairs);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }

@@ -240,16 +240,9 @@ void gdn_block(Ctx &c, const QwLayer &L, int flags) {
     float *save = nullptr;
     if ((flags & QWRT_SAVE_GDN) && b.gdn_save)
         save = b.gdn_save + (size_t)gi * d.max_rows * d.VL * 128 * 128;
-    if (M <= 12) {
-        QW_OP(1, nullptr, 0, qwk_gdn_step(b.proj, d.proj_gdn, md.st.gdn_ring[gi], L.cw, L.A_log, L.dt_bias, L.gdn_norm,
-                                            d.KL, d.VL, M, r.slot, r.pos, r.run_start, r.run_len, md.st.gdn_S[gi], save,
-                                            b.qkv, b.decay, b.beta, b.o, d.eps, c.s));
-    } else {
-        QW_TRYN(3, qwk_gdn_step(b.proj, d.proj_gdn, md.st.gdn_ring[gi], L.cw, L.A_log, L.dt_bias, L.gdn_norm,
-                                            d.KL, d.VL, M, r.slot, r.pos, r.run_start, r.run_len, md.st.gdn_S[gi], save,
-                                            b.qkv, b.decay, b.beta, b.o, d.eps, c.s));
-    }
-    (void)qkv_l;
+    QW_OP((M <= 12 ? 1 : 2), nullptr, 0, qwk_gdn_step(b.proj, d.proj_gdn, md.st.gdn_ring[gi], L.cw, L.A_log, L.dt_bias, L.gdn_norm,
+                                                      d.KL, d.VL, M, r.slot, r.pos, r.run_start, r.run_len, md.st.gdn_S[gi], save,
+                                                      b.qkv, b.decay, b.beta, b.o, d.eps, c.s));
     const int K = d.VL * 128;
     send_partial(c, true);
     QW_OP(1, L.Wout, (size_t)d.H * K * 2, qwk_gemv_bf16(L.Wout, b.o, b.partial, nullptr, d.H, K, M, K, K, d.H, 0, 1, 0, 0, 0, c.s));
