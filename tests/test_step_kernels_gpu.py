@@ -30,6 +30,25 @@ def gen(seed):
     return lambda *s: torch.randn(*s, generator=g, device=DEV)
 
 
+@pytest.mark.parametrize("N,K", [(40, 6000), (2600, 6144), (4800, 2560), (17, 64), (300, 8192), (33, 1296)])
+def test_streamed_products_match_64_bits_at_every_row_count(N, K):
+    """One and several tiles per group of warps, k in one, two and four passes, boxes of a whole stage (K a multiple of 64) and of 64
+    columns with a ragged end; rows behind the weights' last, and an output with guard columns.  fp32 sums of exact products in eight
+    chains of K / 128 tensor-core sums: 4e-10 K of the result's size; a row's bits do not depend on the rows beside it."""
+    from qwb200.ops import kernels as K_
+    rn = gen(N + K)
+    W, x = (rn(N, K) * 0.05).bfloat16(), rn(32, K).bfloat16()
+    ref = x.double() @ W.double().T
+    one = None
+    for M in (1, 7, 8, 9, 16, 17, 24, 25, 32):
+        out = torch.full((M, N + 3), 777.0, device=DEV)
+        K_.gemv_bf16(W, x[:M], out=out, N=N, ldy=N + 3)
+        assert torch.all(out[:, N:] == 777.0)
+        assert float((out[:, :N].double() - ref[:M]).norm() / ref[:M].norm()) < 4e-10 * max(K, 2560), M
+        one = out[0, :N].clone() if one is None else one
+        assert torch.equal(out[0, :N], one), M
+
+
 @pytest.mark.parametrize("runs", [[1], [6, 6, 6, 6], [12], [13], [32], [3, 17, 1, 8]])
 def test_delta_net_step_of_runs_equals_row_by_row(runs):
     """A run's rows in one launch - eight at a time, runs that end inside eight, runs longer than what the kernel stores into the ring itself

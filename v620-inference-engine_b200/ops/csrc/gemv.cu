@@ -21,9 +21,9 @@ __global__ void __launch_bounds__(256) gemv_bf16_kernel(GemvArgs a) {
 }
 
 template <int NT, bool FUSED>
-__global__ void __launch_bounds__(SG_THREADS, 1) sgemv_kernel(SGemvArgs a) {
+__global__ void __launch_bounds__(SG_THREADS, 1) sgemv_kernel(const __grid_constant__ CUtensorMap map, SGemvArgs a) {
     extern __shared__ __align__(128) unsigned char sg_smem[];
-    sgemv_body<NT, FUSED>(a, sg_smem);
+    sgemv_body<NT, FUSED>(map, a, sg_smem);
 }
 
 template <int NT>
@@ -34,8 +34,10 @@ static cudaError_t launch_sgemv_nt(SGemvArgs &a, size_t smem, int grid, cudaStre
         cudaFuncSetAttribute(sgemv_kernel<NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SG_SMEM_MAX);
         configured = true;
     }
-    if (a.fi.active || a.fo.mode) return launch_pdl(sgemv_kernel<NT, true>, dim3(grid), dim3(SG_THREADS), smem, s, a);
-    return launch_pdl(sgemv_kernel<NT, false>, dim3(grid), dim3(SG_THREADS), smem, s, a);
+    CUtensorMap map;
+    if (!sgemv_map(&map, a)) return cudaErrorInvalidValue;
+    if (a.fi.active || a.fo.mode) return launch_pdl(sgemv_kernel<NT, true>, dim3(grid), dim3(SG_THREADS), smem, s, map, a);
+    return launch_pdl(sgemv_kernel<NT, false>, dim3(grid), dim3(SG_THREADS), smem, s, map, a);
 }
 
 // Up to 8 activation rows per pass, or 16 or 24 when they fit in shared memory next to the weight stages: every further pass
@@ -70,7 +72,7 @@ QW_API int qwk_gemv_bf16(const void *W, const void *x, float *y, void *y_bf16, i
         // the streaming kernel: bulk-async weight pipeline, one block per SM
         SGemvArgs g;
         g.W = (const bf16 *)W; g.x = (const bf16 *)x; g.y = y; g.y_bf16 = (bf16 *)y_bf16;
-        g.N = N; g.K = K; g.M = M; g.ldw = ldw; g.ldx = ldx; g.ldy = ldy; g.accumulate = accumulate; g.nsplit = 1; g.w_split = 0; g.err = g_err_ptr;
+        g.N = N; g.K = K; g.M = M; g.ldw = ldw; g.ldx = ldx; g.ldy = ldy; g.accumulate = accumulate; g.err = g_err_ptr;
         g.fi = take_fi(); g.fo = take_fo();
         const cudaError_t e = launch_sgemv(g, s);
         return e == cudaSuccess ? 0 : -2;

@@ -114,10 +114,10 @@ __device__ __forceinline__ void route_shared(const float *rs, int ld_rs, int M, 
 
 // Router GEMV (streaming kernel) with the routing done by the block that finishes last.
 template <int NT, bool FUSED>
-__global__ void __launch_bounds__(SG_THREADS, 1) moe_router_kernel(SGemvArgs a, RouteArgs r) {
+__global__ void __launch_bounds__(SG_THREADS, 1) moe_router_kernel(const __grid_constant__ CUtensorMap map, SGemvArgs a, RouteArgs r) {
     extern __shared__ __align__(128) unsigned char sg_smem[];
     __shared__ unsigned int s_last;
-    sgemv_body<NT, FUSED>(a, sg_smem);
+    sgemv_body<NT, FUSED>(map, a, sg_smem);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) s_last = atomicAdd(r.ticket, 1u) == gridDim.x - 1 ? 1u : 0u;
@@ -140,20 +140,26 @@ static void configure_router_nt() {          // once per device: the kernels' dy
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
     if (!configured[dev]) {
-        cudaFuncSetAttribute(moe_router_kernel<NT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
-        cudaFuncSetAttribute(moe_router_kernel<NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024);
+        cudaFuncSetAttribute(moe_router_kernel<NT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SG_SMEM_MAX);
+        cudaFuncSetAttribute(moe_router_kernel<NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SG_SMEM_MAX);
         configured[dev] = true;
     }
 }
 template <int NT>
 static cudaError_t launch_router_nt(SGemvArgs &a, const RouteArgs &r, size_t smem, int grid, cudaStream_t s) {
     configure_router_nt<NT>();
-    if (a.fi.active) return launch_pdl(moe_router_kernel<NT, true>, dim3(grid), dim3(SG_THREADS), smem, s, a, r);
-    return launch_pdl(moe_router_kernel<NT, false>, dim3(grid), dim3(SG_THREADS), smem, s, a, r);
+    CUtensorMap map;
+    if (!sgemv_map(&map, a)) return cudaErrorInvalidValue;
+    if (a.fi.active) return launch_pdl(moe_router_kernel<NT, true>, dim3(grid), dim3(SG_THREADS), smem, s, map, a, r);
+    return launch_pdl(moe_router_kernel<NT, false>, dim3(grid), dim3(SG_THREADS), smem, s, map, a, r);
 }
 
 static cudaError_t launch_router(SGemvArgs &a, const RouteArgs &r, cudaStream_t s) {
     int grid;
+    if (a.M > 16 && a.M <= 24) {
+        const size_t smem3 = sgemv_plan(a, 3, grid);
+        if (smem3) return launch_router_nt<3>(a, r, smem3, grid, s);
+    }
     if (a.M > 8) {
         const size_t smem2 = sgemv_plan(a, 2, grid);
         if (smem2) return launch_router_nt<2>(a, r, smem2, grid, s);
@@ -356,7 +362,7 @@ QW_API int qwk_moe_router(const void *Wrs, const void *x, float *rs, int nrs, in
     if (E > 1024 || top_k > 32 || (K & 15) || (ldx & 7)) return -1;
     SGemvArgs a;
     a.W = (const bf16 *)Wrs; a.x = (const bf16 *)x; a.y = rs; a.y_bf16 = nullptr;
-    a.N = nrs; a.K = K; a.M = M; a.ldw = K; a.ldx = ldx; a.ldy = nrs; a.accumulate = 0; a.nsplit = 1; a.w_split = 0; a.err = g_err_ptr;
+    a.N = nrs; a.K = K; a.M = M; a.ldw = K; a.ldx = ldx; a.ldy = nrs; a.accumulate = 0; a.err = g_err_ptr;
     a.fi = take_fi();
     RouteArgs r = make_route(E, top_k, F, e_first, e_local, pair_expert, pair_w, sh_h, ticket);
     r.w13 = (const char *)w13; r.w2 = (const char *)w2; r.w13_bytes = w13_bytes; r.w2_bytes = w2_bytes;
@@ -488,6 +494,7 @@ extern "C" __attribute__((visibility("default"))) int qwk_moe_router_static_setu
     g_router_static_ptr[dev] = p;
     configure_router_nt<1>();          // the kernels' attributes too, so that a first call inside a capture has nothing left to set up
     configure_router_nt<2>();
+    configure_router_nt<3>();
     return 0;
 }
 
@@ -508,7 +515,7 @@ extern "C" __attribute__((visibility("default"))) int qwk_moe_router_static(cons
     if (cudaMemsetAsync(ticket, 0, sizeof(unsigned int), s) != cudaSuccess) return -2;
     SGemvArgs a;
     a.W = (const bf16 *)Wrs; a.x = (const bf16 *)x; a.y = rs; a.y_bf16 = nullptr;
-    a.N = nrs; a.K = K; a.M = M; a.ldw = K; a.ldx = ldx; a.ldy = nrs; a.accumulate = 0; a.nsplit = 1; a.w_split = 0; a.err = g_err_ptr;
+    a.N = nrs; a.K = K; a.M = M; a.ldw = K; a.ldx = ldx; a.ldy = nrs; a.accumulate = 0; a.err = g_err_ptr;
     RouteArgs r = make_route(E, top_k, F, e_first, e_local, pair_expert, pair_w, sh_h, ticket);
     r.w13 = nullptr; r.w2 = nullptr; r.w13_bytes = 0; r.w2_bytes = 0; r.prefetch_rows = 0;
     const cudaError_t e = launch_router(a, r, s);

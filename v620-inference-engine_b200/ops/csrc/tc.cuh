@@ -24,6 +24,12 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
                  : "memory");
 }
 
+__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int c0, int c1, int c2, uint64_t *bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 ::"r"(smem_u32(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
+                 : "memory");
+}
+
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_c, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -138,7 +144,8 @@ static EncodeTiledFn encode_fn() {
 // 2-D row-major matrix [rows][cols] (row stride ld elements) read in boxes of box_rows rows:
 enum MapKind { MAP_BF16 = 0,        // bf16, 64 columns, 128B swizzle
                MAP_BYTES64 = 1,     // bytes, 64 columns, 64B swizzle
-               MAP_BF16_X8 = 2 };   // bf16, 8 columns (16 bytes), no swizzle
+               MAP_BF16_X8 = 2,     // bf16, 8 columns (16 bytes), no swizzle
+               MAP_BF16_3D = 3 };   // bf16, 128B swizzle, boxes of (box_rows & 255) rows x (box_rows >> 8) columns as 64 columns after 64 (cols a multiple of 64)
 // A chunk issues ~800 of these for a few dozen distinct (address, shape) pairs - weights and the engine's fixed buffers -
 // so encoded maps are kept in a small direct-mapped table (per thread: the launchers run on the caller's thread) and an
 // encode is paid only on a miss.  A map depends on nothing but the key: the same address with the same shape encodes to
@@ -170,6 +177,17 @@ static bool make_map(CUtensorMap *m, const void *base, long long rows, long long
     MapSlot &slot = table[(h >> 40) % MAP_SLOTS];
     if (slot.used && slot.key == key) {
         *m = slot.map;
+        return true;
+    }
+    if (kind == MAP_BF16_3D) {
+        const cuuint64_t dims[3] = {64, (cuuint64_t)rows, (cuuint64_t)(cols / 64)}, strides[2] = {(cuuint64_t)ld * 2, 128};
+        const cuuint32_t box[3] = {64, (cuuint32_t)(box_rows & 255), (cuuint32_t)(box_rows >> 8) / 64}, estr[3] = {1, 1, 1};
+        if (fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+            return false;
+        slot.key = key;
+        slot.map = *m;
+        slot.used = true;
         return true;
     }
     cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
