@@ -88,6 +88,54 @@ def test_delta_net_step_of_runs_equals_row_by_row(runs):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("QL,KVL,topk", [(24, 2, 512), (3, 1, 16), (32, 2, 4), (40, 2, 16)])
+def test_flash_decode_parts_match_64_bits(QL, KVL, topk):
+    """The partial softmaxes of 64 list entries against 64 bits: fp32 queries, scores and weights (three bf16 parts each), bf16 keys and values.
+    A weight's relative error is the absolute one of its exponent: scores are sums of 256 products, the argument (up to 20) is rounded twice
+    (2^-23 each) and __expf is good to two ulp: 6e-6.  More than 16 heads
+    per KV head take the scalar kernel.  The merge of the parts against 64 bits: the output is rounded to bf16 (2^-9 of a value)."""
+    ratio, page = 4, 256
+    rn = gen(QL + topk)
+    positions = [0, 1, 62, 63, 64, topk * ratio - 1, topk * ratio + 2, topk * ratio + 3, topk * ratio + 700]
+    M, pages = len(positions), (positions[-1] + page) // page
+    k, v = (rn(pages, page, KVL * 256).bfloat16() for _ in range(2))
+    table = torch.randperm(pages, generator=torch.Generator().manual_seed(3)).to(DEV, torch.int32)
+    q, ldp = rn(M, QL, 256) * 2, QL * 512 + 8
+    proj = rn(M, ldp)
+    sel, sel_n, lists = torch.zeros(M, topk, dtype=torch.int32, device=DEV), torch.full((M,), -1, dtype=torch.int32, device=DEV), []
+    for m, p in enumerate(positions):
+        nb = (p + 1) // ratio
+        toks = torch.arange(p + 1)
+        if nb > topk:
+            ch = torch.sort(torch.randperm(nb, generator=torch.Generator().manual_seed(m))[:topk]).values
+            sel[m], sel_n[m] = ch.to(DEV, torch.int32), topk
+            toks = torch.cat([(ch[:, None] * ratio + torch.arange(ratio)).reshape(-1), torch.arange(nb * ratio, p + 1)])
+        lists.append(toks.to(DEV))
+    nsplit = (topk * ratio + ratio + 63) // 64
+    pm, pl = (torch.full((M, QL, nsplit), 7.0, device=DEV) for _ in range(2))
+    pacc, o = torch.full((M, QL, nsplit, 256), float("nan"), device=DEV), torch.zeros(M, QL, 256, dtype=torch.bfloat16, device=DEV)
+    assert _lib().qwk_qsa_attend(P(q), QL, KVL, M, P(i32([0] * M)), P(i32(positions)), P(k), P(v), None, None, pages, P(table), pages, P(sel), P(sel_n),
+                                 topk, ratio, nsplit, P(pm), P(pl), P(pacc), P(proj), ldp, P(o), S()) == 0
+    torch.cuda.synchronize()
+    kf, vf = (x[table.long()].reshape(-1, KVL, 256).double() for x in (k, v))
+    for m, toks in enumerate(lists):
+        for h in range(QL):
+            kv = h // (QL // KVL)
+            s = kf[toks, kv] @ q[m, h].double() / 16
+            for sp in range(nsplit):
+                part = s[sp * 64:sp * 64 + 64]
+                if len(part) == 0:
+                    assert pm[m, h, sp] == float("-inf")
+                    continue
+                w = torch.exp(part - pm[m, h, sp].double())
+                acc = w @ vf[toks[sp * 64:sp * 64 + 64], kv]
+                assert abs(float(pm[m, h, sp]) - float(part.max())) < 1e-5
+                assert abs(float(pl[m, h, sp]) / float(w.sum()) - 1) < 6e-6
+                assert float((pacc[m, h, sp].double() - acc).norm() / acc.norm()) < 6e-6
+            want = (torch.softmax(s, 0) @ vf[toks, kv]) * torch.sigmoid(proj[m, h * 512 + 256:h * 512 + 512].double())
+            assert float((o[m, h].double() - want).norm() / want.norm()) < 2 ** -8
+
+
 @pytest.mark.parametrize("pairs,layers,state", [([[0, 2], [2, 0], [1, -1]], 3, 48 * 128 * 128), ([[1, 1]], 1, 4), ([[0, 1], [1, 3]], 2, 4096 * 3 + 8)])
 def test_accepted_states_are_copied_whole(pairs, layers, state):
     """Every value of an accepted row's state, whatever its size (pieces of 16 KB, a last one that is not whole); rejected slots stay."""

@@ -60,6 +60,162 @@ __device__ __forceinline__ void att_issue(const QsaAttendArgs &a, bf16 *dst_tile
     mbar_arrive(bar);
 }
 
+// ------------------------------------------------------------------------------------------------------------------
+// Flash-decode over the token list for the rows of a step.  A block takes 64 entries of one row's list for all query heads of one KV head (<= 16,
+// the 16 rows of the MMA tile) and leaves the partial softmax (maximum, sum, sums of V) that qsa_combine_kernel merges.  Scores and weights stay
+// what fp32 makes them: the queries and the weights go through the MMAs as three bf16 parts each (24 bits), keys and values are bf16 anyway.
+// In a scalar form (four heads a block, a warp per token) each token's rows were fetched once for every four heads and every score was five
+// shuffles: 24 rows 177 us, now 49; 8 rows 40 / 11.7; one 15 / 9.
+// grid (nsplit, M, KVL), 256 threads.
+// ------------------------------------------------------------------------------------------------------------------
+constexpr int AD_SMEM = (2 * AT * KV_LD + 3 * 16 * KV_LD + 3 * 16 * P_LD) * 2 + 2 * 8 * 16 * 4 + 16;
+
+// x as three bf16 parts, two values at a time
+__device__ __forceinline__ void split3(float x, float y, uint32_t (&p)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const bf162 h = __floats2bfloat162_rn(x, y);
+        p[i] = *reinterpret_cast<const uint32_t *>(&h);
+        x -= bf16_lo(p[i]);
+        y -= bf16_hi(p[i]);
+    }
+}
+
+__global__ void __launch_bounds__(256, 2) qsa_attend_split_kernel(QsaAttendArgs a, ErrorWord *g_err) {
+    extern __shared__ __align__(16) unsigned char att_sm[];
+    bf16 *Ks = reinterpret_cast<bf16 *>(att_sm);             // [64][KV_LD]
+    bf16 *Vs = Ks + AT * KV_LD;                              // [64][KV_LD]
+    bf16 *Qs = Vs + AT * KV_LD;                              // [3][16][KV_LD]
+    bf16 *Ps = Qs + 3 * 16 * KV_LD;                          // [3][16][P_LD]
+    float *s_max = reinterpret_cast<float *>(Ps + 3 * 16 * P_LD);    // [8][16]
+    float *s_l = s_max + 128;                                // [8][16]
+    uint64_t *kbar = reinterpret_cast<uint64_t *>(s_l + 128), *vbar = kbar + 1;
+    const int sp = blockIdx.x, m = blockIdx.y, kvh = blockIdx.z;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, g = lane >> 2, t4 = lane & 3;
+    const int per_kv = a.QL / a.KVL, h0 = kvh * per_kv;
+    if (tid == 0) {
+        mbar_init(kbar, AT);
+        mbar_init(vbar, AT);
+        mbar_fence_init();
+    }
+    const int slot = a.rows.slot[m], pos = a.rows.pos[m];    // the row table: written before the step began
+    const int nb = (pos + 1) / a.ratio;
+    __syncthreads();
+    pdl_wait();
+    pdl_trigger();
+    const int dense = a.sel_n[m] < 0;
+    const int count = dense ? pos + 1 : a.topk * a.ratio + (pos + 1 - nb * a.ratio);
+    if (sp * AT >= count) {                                  // the list ends before this block: nothing that the merge reads
+        if (tid < per_kv) a.pm[((long long)m * a.QL + h0 + tid) * a.nsplit + sp] = -INFINITY;
+        return;
+    }
+    const int *sel = a.sel + (long long)m * a.topk;
+    att_issue(a, Ks, kbar, 0, sp, count, dense, sel, nb, slot, kvh, kvh == 0);
+    att_issue(a, Vs, vbar, 1, sp, count, dense, sel, nb, slot, kvh, false);
+    for (int i = tid; i < 16 * (HD / 4); i += 256) {
+        const int r = i / (HD / 4), c = (i % (HD / 4)) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < per_kv) v = *reinterpret_cast<const float4 *>(a.q + ((long long)m * a.QL + h0 + r) * HD + c);
+        uint32_t p0[3], p1[3];
+        split3(v.x, v.y, p0);
+        split3(v.z, v.w, p1);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2 *>(Qs + (k * 16 + r) * KV_LD + c) = make_uint2(p0[k], p1[k]);
+    }
+    __syncthreads();
+    const uint32_t ks_base = (uint32_t)__cvta_generic_to_shared(Ks), vs_base = (uint32_t)__cvta_generic_to_shared(Vs);
+    const uint32_t qs_base = (uint32_t)__cvta_generic_to_shared(Qs), ps_base = (uint32_t)__cvta_generic_to_shared(Ps);
+    bool ok = mbar_wait_warp(kbar, 0u, g_err);               // bounded; after a time-out the meetings still take place
+    // ---- S = Q K^T for this warp's 8 tokens
+    float s3[3][4] = {};
+    {
+        const uint32_t brow = ks_base + (uint32_t)((w * 8 + (lane & 7)) * KV_LD * 2 + (lane >> 3) * 16);
+#pragma unroll 4
+        for (int ks = 0; ks < 16; ks += 2) {
+            uint32_t b[4];
+            ldmatrix_x4(b[0], b[1], b[2], b[3], brow + ks * 32);
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    uint32_t q0, q1, q2, q3;
+                    ldmatrix_x4(q0, q1, q2, q3, a_tile_addr(qs_base + k * 16 * KV_LD * 2, KV_LD * 2, (ks + j) * 16, lane));
+                    mma_bf16(s3[k], q0, q1, q2, q3, b[2 * j], b[2 * j + 1]);
+                }
+        }
+    }
+    float s[4], tm[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        s[i] = sp * AT + w * 8 + 2 * t4 + (i & 1) < count ? ((s3[2][i] + s3[1][i]) + s3[0][i]) * 0.0625f : -INFINITY;       // 1/sqrt(256)
+        tm[i >> 1] = fmaxf(tm[i >> 1], s[i]);
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        tm[h] = fmaxf(tm[h], __shfl_xor_sync(0xffffffffu, tm[h], 1));
+        tm[h] = fmaxf(tm[h], __shfl_xor_sync(0xffffffffu, tm[h], 2));
+        if (t4 == 0) s_max[w * 16 + g + 8 * h] = tm[h];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        float mx = s_max[g + 8 * h];                         // the list's first entry of the block exists: finite
+#pragma unroll
+        for (int k = 1; k < 8; ++k) mx = fmaxf(mx, s_max[k * 16 + g + 8 * h]);
+        const float p0 = __expf(s[2 * h] - mx), p1 = __expf(s[2 * h + 1] - mx);
+        uint32_t p[3];
+        split3(p0, p1, p);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) *reinterpret_cast<uint32_t *>(Ps + (k * 16 + g + 8 * h) * P_LD + w * 8 + 2 * t4) = p[k];
+        float l = p0 + p1;
+        l += __shfl_xor_sync(0xffffffffu, l, 1);
+        l += __shfl_xor_sync(0xffffffffu, l, 2);
+        if (t4 == 0) s_l[w * 16 + g + 8 * h] = l;
+    }
+    __syncthreads();                                         // P and the sums visible
+    if (tid < per_kv) {
+        float mx = s_max[tid], l = 0.f;
+#pragma unroll
+        for (int k = 1; k < 8; ++k) mx = fmaxf(mx, s_max[k * 16 + tid]);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) l += s_l[k * 16 + tid];
+        const long long o = ((long long)m * a.QL + h0 + tid) * a.nsplit + sp;
+        a.pm[o] = mx;
+        a.pl[o] = l;
+    }
+    ok = ok && mbar_wait_warp(vbar, 0u, g_err);
+    // ---- P V for this warp's 32 output dims
+    float acc[4][4] = {};
+    {
+        const int mid = lane >> 3;
+        const uint32_t vrow = vs_base + (uint32_t)((((mid & 1) * 8 + (lane & 7)) * KV_LD + w * 32 + (mid >> 1) * 8) * 2);
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+            uint32_t b[2][4];
+#pragma unroll
+            for (int n = 0; n < 2; ++n) ldmatrix_x4_trans(b[n][0], b[n][1], b[n][2], b[n][3], vrow + (uint32_t)(ks * 16 * KV_LD * 2 + n * 32));
+#pragma unroll
+            for (int k = 2; k >= 0; --k) {                   // the smallest part first
+                uint32_t p0, p1, p2, p3;
+                ldmatrix_x4(p0, p1, p2, p3, a_tile_addr(ps_base + k * 16 * P_LD * 2, P_LD * 2, ks * 16, lane));
+#pragma unroll
+                for (int n = 0; n < 2; ++n) {
+                    mma_bf16(acc[2 * n], p0, p1, p2, p3, b[n][0], b[n][1]);
+                    mma_bf16(acc[2 * n + 1], p0, p1, p2, p3, b[n][2], b[n][3]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int r = g + 8 * h;
+        if (r >= per_kv) continue;
+        float *o = a.pacc + (((long long)m * a.QL + h0 + r) * a.nsplit + sp) * HD + w * 32 + 2 * t4;
+#pragma unroll
+        for (int n = 0; n < 4; ++n) *reinterpret_cast<float2 *>(o + n * 8) = make_float2(acc[n][2 * h], acc[n][2 * h + 1]);
+    }
+}
+
 // grid (KVL, M), 128 threads.
 __global__ void __launch_bounds__(128, 3) qsa_attend_mma_kernel(QsaAttendArgs a, const float *proj, int ld_proj, bf16 *o,
                                                                 ErrorWord *g_err) {
