@@ -1,0 +1,94 @@
+"""Attention of a prefill chunk on the tcgen05 tensor cores (`ops/csrc/qsa_tc.cu`) against 64 bits and against the kernel that gathers
+the chosen rows (`ops/csrc/qsa_mma.cuh`)."""
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _setup(QL, KVL, base, M, topk, seed, scale=1.0):
+    """A run of M rows at `base` in slot 1 of two, its pages shuffled; the pool's rows behind the run are NaN."""
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    rn = lambda *s: torch.randn(*s, generator=g, device=dev)
+    ratio, page, D = 4, 256, 256
+    pages = (base + M + page - 1) // page + 1
+    k, v = (rn(2 * pages, page, KVL * D).bfloat16() for _ in range(2))
+    table = torch.randperm(2 * pages, generator=torch.Generator().manual_seed(seed)).to(dev, torch.int32).view(2, pages)
+    at = torch.arange(base + M, pages * page, device=dev)
+    for pool in (k, v):
+        pool[table[1][at // page].long(), at % page] = float("nan")
+    ldp = QL * 2 * D + 40
+    proj, q = rn(M, ldp), rn(M, QL, D) * scale
+    pos = torch.arange(base, base + M, dtype=torch.int32, device=dev)
+    sel, sel_n = torch.zeros(M, topk, dtype=torch.int32, device=dev), torch.full((M,), -1, dtype=torch.int32, device=dev)
+    seen = torch.arange(base + M, device=dev)[None] <= pos[:, None]
+    for m in range(M):
+        nb = (base + m + 1) // ratio
+        if nb > topk:
+            ch = torch.sort(torch.randperm(nb, generator=torch.Generator().manual_seed(seed + m))[:topk]).values.to(dev)
+            sel[m], sel_n[m] = ch.int(), topk
+            chosen = torch.zeros(nb, dtype=torch.bool, device=dev)
+            chosen[ch] = True
+            seen[m, :nb * ratio] &= chosen.repeat_interleave(ratio)
+    return dict(q=q, k=k, v=v, table=table, proj=proj, ldp=ldp, pos=pos, sel=sel, sel_n=sel_n, seen=seen, slot=torch.ones_like(pos), pages=pages)
+
+
+def _exact(t, QL, KVL, base, M):
+    rows = t["table"][1].long()
+    kf, vf = (x[rows].reshape(-1, KVL, 256)[:base + M].double() for x in (t["k"], t["v"]))
+    q = t["q"].bfloat16().double()
+    out = torch.empty(M, QL, 256, dtype=torch.float64, device=q.device)
+    for h in range(QL):
+        kv = h // (QL // KVL)
+        s = (q[:, h] @ kf[:, kv].T / 16).masked_fill(~t["seen"], float("-inf"))
+        gate = t["proj"][:, h * 512 + 256:h * 512 + 512].double()
+        out[:, h] = (torch.softmax(s, 1) @ vf[:, kv]) * torch.sigmoid(gate)
+    return out
+
+
+@pytest.mark.parametrize("QL,KVL,base,M,topk,scale", [
+    (24, 2, 0, 1, 512, 1.0), (24, 2, 0, 70, 512, 1.0), (24, 2, 127, 2, 512, 1.0), (24, 2, 0, 300, 512, 3.0), (24, 2, 2040, 150, 512, 1.0),
+    (24, 2, 1001, 129, 64, 3.0), (12, 1, 6000, 33, 512, 1.0), (3, 1, 250, 400, 32, 1.0), (8, 2, 5, 64, 4, 1.0), (16, 1, 383, 257, 16, 1.0)])
+def test_matches_64_bits_and_the_gathering_kernel(QL, KVL, base, M, topk, scale):
+    """Rows that see every key and rows with chosen groups, groups that are open or just closed, tiles that end with the context.  Bound:
+    weights and the result rounded to bf16 (2^-9 each of a value), and no further from 64 bits than 1.1 times the gathering kernel."""
+    from qwb200.ops import lib as qlib
+    L = qlib.load(True)
+    t = _setup(QL, KVL, base, M, topk, 7 * M + base, scale)
+    P = lambda x: C.c_void_p(x.data_ptr())
+    s = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    want = _exact(t, QL, KVL, base, M)
+    err = lambda o: float((o.double() - want).norm() / want.norm())
+    gathered, o = (torch.zeros(M, QL, 256, dtype=torch.bfloat16, device="cuda:0") for _ in range(2))
+    last, ld = base + M - 1, (base + M) // 4 + 8
+    mask = torch.empty(M, ld, dtype=torch.int32, device="cuda:0")
+    assert L.qwk_qsa_takes_tc(QL, KVL, M, last, 4, ld, t["ldp"]) == 1
+    pool = [P(t["k"]), P(t["v"])]
+    assert L.qwk_qsa_attend_mma(P(t["q"]), QL, KVL, M, P(t["slot"]), P(t["pos"]), *pool, None, None, 2 * t["pages"], P(t["table"]), t["pages"],
+                                P(t["sel"]), P(t["sel_n"]), topk, 4, P(t["proj"]), t["ldp"], P(gathered), s) == 0
+    for p in range(last + 1, (last + 16) // 16 * 16):          # as the prep kernel leaves them
+        t["k"][t["table"][1][p // 256], p % 256] = t["v"][t["table"][1][p // 256], p % 256] = 0
+    first_host = (last // 256 + 1) * 2 // 3                      # pages from here on also lie in a pool of their own, read as staged and as host rows
+    moved = t["table"].clone()
+    hk, hv = (torch.cat([x[t["table"][1, first_host:].long()], x[:1]]) for x in (t["k"], t["v"]))
+    moved[1, first_host:] = 2 * t["pages"] + torch.arange(t["pages"] - first_host, device="cuda:0", dtype=torch.int32)
+    for table, host, staged in ((t["table"], [None, None], 0), (moved, [P(hk), P(hv)], 1), (moved, [P(hk), P(hv)], 0)):
+        before = o.clone()
+        o.zero_()
+        assert L.qwk_qsa_attend_tc(P(t["q"]), QL, KVL, M, last, P(t["slot"]), P(t["pos"]), *pool, *host, staged, 2 * t["pages"], P(table), t["pages"],
+                                   P(t["sel"]), P(t["sel_n"]), topk, P(mask), ld, P(t["proj"]), t["ldp"], P(o), s) == 0
+        torch.cuda.synchronize()
+        assert host[0] is None or torch.equal(o, before)
+    assert err(o) < 4e-3 and err(o) < 1.1 * err(gathered) + 1e-5
+
+
+def test_what_it_does_not_take():
+    """Other group sizes, contexts behind the line, rows of the projection off 16 bytes: the gathering kernel's."""
+    from qwb200.ops import lib as qlib
+    L = qlib.load(True)
+    take = lambda **k: L.qwk_qsa_takes_tc(*{**dict(QL=24, KVL=2, M=100, last=4000, ratio=4, ld=1100, ldp=13952), **k}.values())
+    assert take() == 1
+    assert not any((take(ratio=8), take(last=1 << 20, ld=1 << 20), take(last=40, M=100), take(ld=31), take(ldp=13953), take(QL=23)))

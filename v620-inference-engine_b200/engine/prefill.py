@@ -314,7 +314,6 @@ class Prefiller:
             X[rows_i] = emb.to(X.dtype)[:, None, :sc.sh].expand(-1, c.hc, -1)
         pend, inj_prev = None, None
         inj_attn, inj_mlp = b["inj_a"], b["inj_b"]
-        max_groups = (base + T) // c.idx_ratio
         for li in range(c.n_layers if self.layer_limit is None else min(c.n_layers, int(self.layer_limit))):
             lw = dm.layers_w[li]
             if li == c.ple_layer and dm.model.ple.enabled:
@@ -337,7 +336,7 @@ class Prefiller:
             self.mix(lw["attn_hc"], T, pend, inj_prev, inj_attn, c.hc)
             if self.on_block_input is not None:
                 self.on_block_input(li, "attn", b["bin"][:T])
-            self.attn_block(lw, T, rp, max_groups, c.qsa_index(li) if lw["is_qsa"] else c.gdn_index(li))
+            self.attn_block(lw, T, rp, base + T, c.qsa_index(li) if lw["is_qsa"] else c.gdn_index(li))
             self.mix(lw["mlp_hc"], T, b["out_a"], inj_attn, inj_mlp, c.hc)
             if self.on_block_input is not None:
                 self.on_block_input(li, "mlp", b["bin"][:T])
@@ -353,8 +352,8 @@ class Prefiller:
                                       _p(dm.buf["amax_idx"]), _p(dm.buf["lse_max"]), _p(dm.buf["lse_sum"]), s), "row_reduce")
         return dm.buf["logits"][0] if want_logits else None
 
-    def attn_block(self, lw, T, rp, max_groups, state_index):
-        """The attention block of one layer over T rows: bin -> out_a (fp32 [T][H])."""
+    def attn_block(self, lw, T, rp, end, state_index):
+        """The attention block of one layer over T rows, the last of them at position end - 1: bin -> out_a (fp32 [T][H])."""
         dm, b, c, sc, L = self.dm, self.b, self.dm.cfg, self.dm.sc, self.lib
         s = self._s()
         d = dm.model.d
@@ -365,18 +364,24 @@ class Prefiller:
             kd, vd = dm.k_dev[qi].data_ptr(), dm.v_dev[qi].data_ptr()
             kh = dm.k_host[qi].data_ptr() if dm.k_host else None
             vh = dm.v_host[qi].data_ptr() if dm.v_host else None
-            self._ck(L.qwk_qsa_prep(_p(b["proj"]), ldp, sc.qh_l, sc.kvh_l, c.idx_heads, P(lw["qn1"].data_ptr()),
-                                    P(lw["kn1"].data_ptr()), P(lw["iqn1"].data_ptr()), P(lw["ikn1"].data_ptr()), T,
-                                    rp("slot"), rp("pos"), rp("run_start"), rp("run_len"), P(kd), P(vd), P(kh) if kh else None,
-                                    P(vh) if vh else None, d.n_dev_pages, _p(dm.page_table), d.max_pages, _p(b["q"]),
-                                    _p(b["iq"]), _p(dm.raw_ring[qi]), _p(dm.ck[qi]), d.ck_cap, c.idx_ratio,
-                                    C.c_float(c.eps), s), "qsa_prep")
+            self._ck(L.qwk_qsa_prep_run(_p(b["proj"]), ldp, sc.qh_l, sc.kvh_l, c.idx_heads, P(lw["qn1"].data_ptr()),
+                                        P(lw["kn1"].data_ptr()), P(lw["iqn1"].data_ptr()), P(lw["ikn1"].data_ptr()), T,
+                                        rp("slot"), rp("pos"), rp("run_start"), rp("run_len"), P(kd), P(vd), P(kh) if kh else None,
+                                        P(vh) if vh else None, d.n_dev_pages, _p(dm.page_table), d.max_pages, _p(b["q"]),
+                                        _p(b["iq"]), _p(dm.raw_ring[qi]), _p(dm.ck[qi]), d.ck_cap, c.idx_ratio,
+                                        C.c_float(c.eps), s), "qsa_prep")
             self._ck(L.qwk_qsa_scores(_p(b["iq"]), c.idx_heads, _p(dm.ck[qi]), d.ck_cap, T, rp("slot"), rp("pos"),
-                                      c.idx_ratio, c.idx_topk_blocks, _p(b["scores"]), d.score_cap, max_groups, s), "scores")
+                                      c.idx_ratio, c.idx_topk_blocks, _p(b["scores"]), d.score_cap, end // c.idx_ratio, s), "scores")
             self._ck(L.qwk_qsa_select(_p(b["scores"]), d.score_cap, T, rp("pos"), c.idx_ratio, c.idx_topk_blocks,
                                       _p(b["sel"]), _p(b["sel_n"]), s), "select")
             ow = sc.qh_l * c.head_dim
-            if self.qsa_mma:
+            last_pos = end - 1
+            if self.qsa_mma and L.qwk_qsa_takes_tc(sc.qh_l, sc.kvh_l, T, last_pos, c.idx_ratio, d.score_cap, ldp):
+                self._ck(L.qwk_qsa_attend_tc(_p(b["q"]), sc.qh_l, sc.kvh_l, T, last_pos, rp("slot"), rp("pos"), P(kd), P(vd),
+                                             P(kh) if kh else None, P(vh) if vh else None, 0, d.n_dev_pages, _p(dm.page_table), d.max_pages,
+                                             _p(b["sel"]), _p(b["sel_n"]), c.idx_topk_blocks, _p(b["scores"]), d.score_cap, _p(b["proj"]), ldp,
+                                             _p(b["o"]), s), "attend_tc")
+            elif self.qsa_mma:
                 self._ck(L.qwk_qsa_attend_mma(_p(b["q"]), sc.qh_l, sc.kvh_l, T, rp("slot"), rp("pos"), P(kd), P(vd),
                                               P(kh) if kh else None, P(vh) if vh else None, d.n_dev_pages, _p(dm.page_table),
                                               d.max_pages, _p(b["sel"]), _p(b["sel_n"]), c.idx_topk_blocks, c.idx_ratio,
@@ -439,7 +444,7 @@ class Prefiller:
         self._ck(L.qwk_mtp_add(_p(b["fh"]), _p(b["fe"]), c.hidden, c.hc, _p(b["X"]), n, s), "mtp_add")
         lw = w["layer"]
         self.mix(lw["attn_hc"], n, None, None, b["inj_a"], c.hc)
-        self.attn_block(lw, n, rp, (base + n) // c.idx_ratio, c.n_qsa)
+        self.attn_block(lw, n, rp, base + n, c.n_qsa)
         self.mix(lw["mlp_hc"], n, b["out_a"], b["inj_a"], b["inj_b"], c.hc)
         self.moe(lw, n)
         # the MTP layer's output is not needed for prompt rows: only its KV / indexer state matters

@@ -108,12 +108,17 @@ int qwk_tp_argmax_merge(void *tp_, int M, int *out_idx, float *out_val, cudaStre
 // qsa.cu
 int qwk_rope_init(double theta, int rope_dim);
 int qwk_qsa_prep(const float *proj, int ld_proj, int QL, int KVL, int IH, const float *qn1, const float *kn1, const float *iqn1, const float *ikn1, int M, const int *slot, const int *pos, const int *run_start, const int *run_len, void *k_dev, void *v_dev, void *k_host, void *v_host, int n_dev_pages, const int *page_table, int max_pages, float *q, float *iq, float *raw_ring, void *ck, int ck_cap, int ratio, float eps, cudaStream_t s);
+int qwk_qsa_prep_run(const float *proj, int ld_proj, int QL, int KVL, int IH, const float *qn1, const float *kn1, const float *iqn1, const float *ikn1, int M, const int *slot, const int *pos, const int *run_start, const int *run_len, void *k_dev, void *v_dev, void *k_host, void *v_host, int n_dev_pages, const int *page_table, int max_pages, float *q, float *iq, float *raw_ring, void *ck, int ck_cap, int ratio, float eps, cudaStream_t s);
 int qwk_qsa_scores(const float *iq, int IH, const void *ck, int ck_cap, int M, const int *slot, const int *pos, int ratio, int topk_blocks, float *scores, int ld_scores, int max_groups, cudaStream_t s);
 int qwk_qsa_select(const float *scores, int ld_scores, int M, const int *pos, int ratio, int topk, int *sel, int *sel_n, cudaStream_t s);
 int qwk_qsa_attend(const float *q, int QL, int KVL, int M, const int *slot, const int *pos, void *k_dev, void *v_dev, void *k_host, void *v_host, int n_dev_pages, const int *page_table, int max_pages, const int *sel, const int *sel_n, int topk, int ratio, int nsplit, float *pm, float *pl, float *pacc, const float *proj, int ld_proj, void *o, cudaStream_t s);
 int qwk_qsa_attend_mma(const float *q, int QL, int KVL, int M, const int *slot, const int *pos, void *k_dev, void *v_dev, void *k_host, void *v_host, int n_dev_pages, const int *page_table, int max_pages, const int *sel, const int *sel_n, int topk, int ratio, const float *proj, int ld_proj, void *o, cudaStream_t s);
 int qwk_set_spill_cache(void *tags, void *rows, void *miss, void *ctl, void *stats, int entries, int miss_cap);
 int qwk_spill_cache_active(int unused);
+
+// qsa_tc.cu
+int qwk_qsa_takes_tc(int QL, int KVL, int M, int last_pos, int ratio, int ld_mask, int ld_proj);
+int qwk_qsa_attend_tc(const float *q, int QL, int KVL, int M, int last_pos, const int *slot, const int *pos, void *k_dev, void *v_dev, void *k_host, void *v_host, int staged, int n_dev_pages, const int *page_table, int max_pages, const int *sel, const int *sel_n, int topk, void *mask, int ld_mask, const float *proj, int ld_proj, void *o, cudaStream_t s);
 
 // sampling.cu
 int qwk_sample(const float *logits, int ld, int V, int M, const void *params, const void *gen, const void *seen, void *out, cudaStream_t s);

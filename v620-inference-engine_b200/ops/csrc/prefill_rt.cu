@@ -269,7 +269,7 @@ struct Builder {
             float *proj = f_at(b.proj, L.r0, b.proj_ld);
             if (w.is_qsa) {
                 const int qi = w.state_index;
-                PF_TRY(1, qwk_qsa_prep(proj, b.proj_ld, d.QL, d.KVL, d.IH, w.qn1, w.kn1, w.iqn1, w.ikn1, L.n, r.slot, r.pos, r.rs, r.rl,
+                PF_TRY(1, qwk_qsa_prep_run(proj, b.proj_ld, d.QL, d.KVL, d.IH, w.qn1, w.kn1, w.iqn1, w.ikn1, L.n, r.slot, r.pos, r.rs, r.rl,
                                        st.k_dev[qi], st.v_dev[qi], st.k_host ? st.k_host[qi] : nullptr, st.v_host ? st.v_host[qi] : nullptr,
                                        d.n_dev_pages, st.page_table, d.max_pages, f_at(b.q, L.r0, d.QL * 256), f_at(b.iq, L.r0, d.IH * 128),
                                        st.raw_ring[qi], st.ck[qi], d.ck_cap, d.idx_ratio, d.eps, L.s));
@@ -331,6 +331,7 @@ struct Builder {
             const RowsAt r = rows_of(c, L);
             const int qi = w.state_index;
             void *kh = st.k_host ? st.k_host[qi] : nullptr, *vh = st.v_host ? st.v_host[qi] : nullptr;
+            int staged = 0;
             // KV spill: the slot's host pages of this layer (the rows this chunk just wrote among them) are copied into
             // the staging buffers and the attention reads them there: a gather of ~2,000 rows per query over the host
             // link costs more than one sequential copy of the pages (host pages of slot s are [s * spill, (s + 1) * spill))
@@ -349,7 +350,16 @@ struct Builder {
                     c.launches += 2;
                     kh = (char *)b.stage_k - off;
                     vh = (char *)b.stage_v - off;
+                    staged = 1;
                 }
+            }
+            const int last_pos = (mtp ? c.job->mtp_base : c.job->base) + L.r0 + L.n - 1;
+            if (qwk_qsa_takes_tc(d.QL, d.KVL, L.n, last_pos, d.idx_ratio, d.score_cap, b.proj_ld)) {
+                PF_TRY(2, qwk_qsa_attend_tc(f_at(b.q, L.r0, d.QL * 256), d.QL, d.KVL, L.n, last_pos, r.slot, r.pos, st.k_dev[qi], st.v_dev[qi], kh, vh,
+                                            staged, d.n_dev_pages, st.page_table, d.max_pages, i_at(b.sel, L.r0, d.idx_topk), b.sel_n + L.r0, d.idx_topk,
+                                            f_at(b.scores, L.r0, d.score_cap), d.score_cap, f_at(b.proj, L.r0, b.proj_ld), b.proj_ld,
+                                            h_at(b.o, L.r0, b.o_ld), L.s));
+                return;
             }
             PF_TRY(1, qwk_qsa_attend_mma(f_at(b.q, L.r0, d.QL * 256), d.QL, d.KVL, L.n, r.slot, r.pos, st.k_dev[qi], st.v_dev[qi],
                                          kh, vh, d.n_dev_pages,

@@ -154,6 +154,7 @@ struct QsaPrepArgs {
     int ck_cap;
     int ratio;           // tokens per compressed group
     float eps;
+    int zero_tail;       // 1: the rows behind the batch's last, up to the next multiple of 16, become zeros (they are nobody's yet)
     int ring_inline;     // 1: the raw-key block also stores its row in the ring (safe for runs <= RAW_RING - ratio)
 };
 
@@ -210,9 +211,16 @@ __global__ void __launch_bounds__(256) qsa_prep_kernel(QsaPrepArgs a) {
         const float v = norm_rope<HD>(row[off_k + j * HD + d], sm, scratch, cs, a.kn1, a.eps, d);
         if (j == 0 && d == 0) spill_drop(a.kv, a.sc, slot, pos);
         k_row(a.kv, slot, pos)[j * HD + d] = __float2bfloat16(v);
+        if (a.zero_tail && m == a.rows.M - 1)
+            for (int p = pos + 1; p & 15; ++p) {
+                if (j == 0 && d == 0) spill_drop(a.kv, a.sc, slot, p);
+                k_row(a.kv, slot, p)[j * HD + d] = __float2bfloat16(0.f);
+            }
     } else if (hb < a.QL + 2 * a.KVL) {                // value head
         const int j = hb - a.QL - a.KVL;
         v_row(a.kv, slot, pos)[j * HD + d] = __float2bfloat16(row[off_v + j * HD + d]);
+        if (a.zero_tail && m == a.rows.M - 1)
+            for (int p = pos + 1; p & 15; ++p) v_row(a.kv, slot, p)[j * HD + d] = __float2bfloat16(0.f);
     } else if (hb < a.QL + 2 * a.KVL + a.IH) {         // indexer query head
         const int j = hb - a.QL - 2 * a.KVL;
         fill_cs(cs, pos);
@@ -507,7 +515,7 @@ __global__ void __launch_bounds__(256) qsa_attend_kernel(QsaAttendArgs a) {
 }
 
 // grid (M, QL), 256 threads: merge the splits, apply sigmoid(gate), write bf16.  Only the splits in front of the list's end hold anything.  The
-// weights are formed once per block and the partial sums' loads are eight at a time (24 rows, one split behind the other: 9.5 us, now 7.7).
+// weights are formed once per block and the partial sums' loads are eight at a time (24 rows, one split behind the other: 9.5 us, now 9.0).
 __global__ void __launch_bounds__(256) qsa_combine_kernel(const float *pm, const float *pl, const float *pacc, int nsplit,
                                                           const float *proj, int ld_proj, int QL, bf16 *o) {
     extern __shared__ float s_w[];          // [nsplit] weights, [nsplit] sums
@@ -580,11 +588,11 @@ static KvPool make_pool(void *k_dev, void *v_dev, void *k_host, void *v_host, in
     return p;
 }
 
-QW_API int qwk_qsa_prep(const float *proj, int ld_proj, int QL, int KVL, int IH, const float *qn1, const float *kn1,
+static int qsa_prep_launch(const float *proj, int ld_proj, int QL, int KVL, int IH, const float *qn1, const float *kn1,
                         const float *iqn1, const float *ikn1, int M, const int *slot, const int *pos,
                         const int *run_start, const int *run_len, void *k_dev, void *v_dev, void *k_host, void *v_host,
                         int n_dev_pages, const int *page_table, int max_pages, float *q, float *iq, float *raw_ring,
-                        void *ck, int ck_cap, int ratio, float eps, cudaStream_t s) {
+                        void *ck, int ck_cap, int ratio, float eps, int zero_tail, cudaStream_t s) {
     if (IH > 8) return -1;
     QsaPrepArgs a;
     a.proj = proj; a.ld_proj = ld_proj; a.QL = QL; a.KVL = KVL; a.IH = IH;
@@ -593,12 +601,30 @@ QW_API int qwk_qsa_prep(const float *proj, int ld_proj, int QL, int KVL, int IH,
     a.kv = make_pool(k_dev, v_dev, k_host, v_host, n_dev_pages, page_table, max_pages, KVL * HD);
     a.sc = k_host ? g_spill : SpillCache{};
     a.q = q; a.iq = iq; a.raw_ring = raw_ring; a.ck = (bf16 *)ck; a.ck_cap = ck_cap; a.ratio = ratio; a.eps = eps;
+    a.zero_tail = zero_tail;
     a.ring_inline = M <= RAW_RING - ratio ? 1 : 0;
     dim3 grid(M, QL + 2 * KVL + IH + 1);
     launch_pdl(qsa_prep_kernel, grid, dim3(256), 0, s, a);
     if (!a.ring_inline)
         launch_pdl(qsa_raw_ring_kernel, dim3(M), dim3(ID), 0, s, proj, ld_proj, QL * 2 * HD + 2 * KVL * HD + IH * ID, raw_ring, a.rows);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+QW_API int qwk_qsa_prep(const float *proj, int ld_proj, int QL, int KVL, int IH, const float *qn1, const float *kn1,
+                        const float *iqn1, const float *ikn1, int M, const int *slot, const int *pos,
+                        const int *run_start, const int *run_len, void *k_dev, void *v_dev, void *k_host, void *v_host,
+                        int n_dev_pages, const int *page_table, int max_pages, float *q, float *iq, float *raw_ring,
+                        void *ck, int ck_cap, int ratio, float eps, cudaStream_t s) {
+    return qsa_prep_launch(proj, ld_proj, QL, KVL, IH, qn1, kn1, iqn1, ikn1, M, slot, pos, run_start, run_len, k_dev, v_dev, k_host, v_host, n_dev_pages, page_table, max_pages, q, iq, raw_ring, ck, ck_cap, ratio, eps, 0, s);
+}
+
+// The same for a run that attention on the tensor cores follows (qwk_qsa_attend_tc).
+QW_API int qwk_qsa_prep_run(const float *proj, int ld_proj, int QL, int KVL, int IH, const float *qn1, const float *kn1,
+                        const float *iqn1, const float *ikn1, int M, const int *slot, const int *pos,
+                        const int *run_start, const int *run_len, void *k_dev, void *v_dev, void *k_host, void *v_host,
+                        int n_dev_pages, const int *page_table, int max_pages, float *q, float *iq, float *raw_ring,
+                        void *ck, int ck_cap, int ratio, float eps, cudaStream_t s) {
+    return qsa_prep_launch(proj, ld_proj, QL, KVL, IH, qn1, kn1, iqn1, ikn1, M, slot, pos, run_start, run_len, k_dev, v_dev, k_host, v_host, n_dev_pages, page_table, max_pages, q, iq, raw_ring, ck, ck_cap, ratio, eps, 1, s);
 }
 
 QW_API int qwk_qsa_scores(const float *iq, int IH, const void *ck, int ck_cap, int M, const int *slot, const int *pos,

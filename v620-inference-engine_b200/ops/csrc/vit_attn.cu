@@ -38,11 +38,6 @@ struct VitAttnArgs {
 __device__ __forceinline__ uint64_t make_plain_desc(uint32_t saddr, uint32_t lbo) {
     return (uint64_t)((saddr & 0x3FFFF) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(128 >> 4) << 32) | ((uint64_t)1 << 46);
 }
-// 128B-swizzled operand that lies MN-major (rows of 64 MN values per k): 8-k groups 1024 bytes apart, the next 64 MN values `lbo` further.
-__device__ __forceinline__ uint64_t make_mn_desc(uint32_t saddr, uint32_t lbo) {
-    return (uint64_t)((saddr & 0x3FFFF) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-}
-
 __global__ void __launch_bounds__(VT_THREADS, 1) vit_attn_tc_kernel(const __grid_constant__ CUtensorMap mapA,      // 64-column boxes of qkv
                                                                     const __grid_constant__ CUtensorMap mapB,      // 8-column boxes
                                                                     VitAttnArgs a) {
