@@ -14,10 +14,10 @@
 //
 // Three launches per layer:
 //   1. gdn_chunk_prep_kernel   grid (chunks, VL): everything that does not depend on the state (A, Wv, Wk, P, g),
-//      all chunks in parallel.  K K^T and Q K^T on mma.sync tf32; the two triangular solves by forward
-//      substitution in fp32, one column of [Wv | Wk] per thread.
+//      all chunks in parallel.  K K^T and Q K^T on mma.sync tf32; T = (I + A)^-1 in fp32, by halves; Wv and Wk as products
+//      with T in split tf32 (three products: what is dropped is below 2^-21).
 //   2. gdn_chunk_apply_kernel  grid (2, VL): walks the chunks in order with the state of one head's 64 value
-//      columns in shared memory; three tf32 products per chunk.  The value columns of a head are independent in
+//      columns in registers; three tf32 products per chunk.  The value columns of a head are independent in
 //      every state-dependent product, so a head is split over two blocks.
 //   3. gdn_chunk_norm_kernel   grid (M, VL): gated RMS norm over the head's 128 outputs -> bf16.
 //
@@ -29,10 +29,10 @@ namespace qw {
 
 constexpr int CD = 128;          // head dim (keys and values)
 constexpr int CC = 64;           // rows per chunk
-constexpr int LDA = CD + 4;      // row stride of a [64][128] A-operand tile: 4 mod 32 words -> fragment loads hit 32 banks
-constexpr int LDT = CD + 8;      // row stride of a [64][128] tile read transposed (8 mod 32)
-constexpr int LDP = CC + 4;      // [64][64] A-operand tile
-constexpr int LDS = 64 + 8;      // [.][64] B-operand tile (state half, U)
+// Row strides of shared tiles: 4 mod 32 words, so that the eight 16-byte rows of an ldmatrix lie in different banks ...
+constexpr int LDA = CD + 4;      // [.][128]
+constexpr int LDP = CC + 4;      // [.][64]
+constexpr int LDT = CD + 8;      // ... and 8 mod 32 for the tile that is read down its columns
 
 __device__ __forceinline__ uint32_t tf32(float x) {
     uint32_t r;
@@ -44,14 +44,25 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], 
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// A fragment of a 16 x 8 tile at (r0, k0) of a row-major matrix: lane (g = lane / 4, t = lane % 4) holds
-// (r0+g, k0+t), (r0+g+8, k0+t), (r0+g, k0+t+4), (r0+g+8, k0+t+4).
-__device__ __forceinline__ void lda_frag(uint32_t (&a)[4], const float *m, int ld, int r0, int k0, int g, int t) {
-    const float *p = m + (r0 + g) * ld + k0 + t;
-    a[0] = tf32(p[0]);
-    a[1] = tf32(p[8 * ld]);
-    a[2] = tf32(p[4]);
-    a[3] = tf32(p[8 * ld + 4]);
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], const float *p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ldsm2(uint32_t &r0, uint32_t &r1, const float *p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+// A 32-bit element is two of ldmatrix's: an 8 x 8 matrix is 8 rows x 4 values, and lane (g = lane / 4, t = lane % 4) gets row g's value t.
+// This lane's row address of a 16 x 8 operand-A tile: the four matrices are (rows 0-7 | 8-15) x (k 0-3, then 4-7) ...
+__device__ __forceinline__ const float *a_row(const float *m, int ld, int r0, int lane) {
+    return m + (r0 + (lane & 7) + (lane & 8)) * ld + (lane >> 4) * 4;
+}
+// ... and of two operand-B tiles whose columns are the matrix's rows n0 .. n0 + 15: (n 0-7: k 0-3, k 4-7), (n 8-15: k 0-3, k 4-7).
+__device__ __forceinline__ const float *b_row(const float *m, int ld, int n0, int lane) {
+    return m + (n0 + (lane & 7) + (lane >> 4) * 8) * ld + ((lane >> 3) & 1) * 4;
+}
+__device__ __forceinline__ void round4(uint32_t (&r)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) r[i] = tf32(__uint_as_float(r[i]));
 }
 
 struct GdnChunkArgs {
@@ -63,46 +74,63 @@ struct GdnChunkArgs {
     const float *norm_w;         // [128]
     int KL, VL, M;
     const int *slot;             // slot[0] = the run's slot
-    float *Wk, *Wv;              // scratch [chunks][VL][64][128]
-    float *P;                    // scratch [chunks][VL][64][64]
+    float *Wk, *Wv;              // scratch [chunks][VL][64][128]; Wk rounded to tf32
+    float *P;                    // scratch [chunks][VL][64][64], rounded to tf32
     float *G;                    // scratch [chunks][VL][64]   cumulative log decay
     float *Oraw;                 // scratch [M][VL*128]
     bf16 *o;                     // [M][VL*128]
     float eps;
 };
 
-// Loads rows [m0, m0+64) x 128 floats at column offset col of the qkv rows into a shared tile of stride ld;
-// rows >= M are zero.  256 threads.
-__device__ __forceinline__ void load_tile(float *dst, int ld, const float *qkv, int qkv_l, int col, int m0, int M, int tid) {
+// 16-byte asynchronous copy global -> shared; `ok` false: the destination is zero-filled (rows past the run's end).
+__device__ __forceinline__ void cp_async16(float *dst, const float *src, bool ok) {
+    const unsigned int d = (unsigned int)__cvta_generic_to_shared(dst);
+    const int n = ok ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Rows [m0, m0+64) x 128 floats at column offset col of the qkv rows -> shared tile of stride ld, asynchronously; rows
+// >= M become zero.  256 threads.
+template <int TH = 256>
+__device__ __forceinline__ void load_tile_async(float *dst, int ld, const float *qkv, int qkv_l, int col, int m0, int M, int tid) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int idx = tid + i * 256;          // float4 index: 64 rows x 32
+    for (int i = 0; i < 2048 / TH; ++i) {
+        const int idx = tid + i * TH;           // float4 index: 64 rows x 32
         const int r = idx >> 5, c4 = idx & 31;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (m0 + r < M) v = *reinterpret_cast<const float4 *>(qkv + (long long)(m0 + r) * qkv_l + col + c4 * 4);
-        *reinterpret_cast<float4 *>(dst + r * ld + c4 * 4) = v;
+        const bool ok = m0 + r < M;
+        cp_async16(dst + r * ld + c4 * 4, qkv + (long long)(ok ? m0 + r : 0) * qkv_l + col + c4 * 4, ok);
     }
 }
 
 // ------------------------------------------------------------------------------------------------
 // 1. state-independent part of every chunk
 // ------------------------------------------------------------------------------------------------
-constexpr int PREP_SMEM = (2 * CC * LDA + 2 * CC) * 4;      // 68 KB: three blocks per SM
+// What bounded it: forward substitution of all 256 columns of [Wv | Wk], one per thread - a 16-byte shared load for four multiply-adds,
+// 512 of them per warp, and 64 rows one behind the other.  Now the 64 columns of the identity go through it in two halves of 32 rows,
+// side by side, and the rest are products.  4,096 tokens, 48 heads: 407 us, now 232 (1,021: 112, 68; 100: 49, 17).
+constexpr int HC_ = CC / 2;
+constexpr int PREP_SMEM = (CC * LDA + 2 * CC * LDP + 2 * CC) * 4;      // 69 KB
 
-__global__ void __launch_bounds__(256, 3) gdn_chunk_prep_kernel(GdnChunkArgs a) {
+// (three blocks per SM leave too few registers: both kernels at 4,096 tokens 712 us against 683, at 1,021 205 against 196)
+__global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(GdnChunkArgs a) {
     extern __shared__ __align__(16) float sm[];
     float *Ks = sm;                      // [64][LDA]
-    float *Qs = Ks + CC * LDA;           // [64][LDA]
-    float *As = Qs;                      // [64][LDP]  takes Q's place once Q K^T is done
-    float *gs = Qs + CC * LDA;           // [64] cumulative log decay
+    float *Qs = Ks + CC * LDA;           // [64][LDA]; the next two take its place once Q K^T is done
+    float *As = Qs;                      // [64][LDP]  A, then the high part of T
+    float *Ts = As + CC * LDP;           // [64][LDP]  T, then its low part
+    float *gs = Ts + CC * LDP;           // [64] cumulative log decay
     float *bs = gs + CC;                 // [64] beta
     const int ch = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int qkv_l = (2 * a.KL + a.VL) * CD;
     const int kh = h / (a.VL / a.KL);
     const int m0 = ch * CC;
-    load_tile(Ks, LDA, a.qkv, qkv_l, (a.KL + kh) * CD, m0, a.M, tid);
-    load_tile(Qs, LDA, a.qkv, qkv_l, kh * CD, m0, a.M, tid);
+    load_tile_async(Ks, LDA, a.qkv, qkv_l, (a.KL + kh) * CD, m0, a.M, tid);
+    load_tile_async(Qs, LDA, a.qkv, qkv_l, kh * CD, m0, a.M, tid);
+    cp_async_commit();
     if (w == 0) {
         const int r0 = 2 * lane, r1 = r0 + 1;
         float x0 = 0.f, x1 = 0.f, b0 = 0.f, b1 = 0.f;
@@ -125,25 +153,41 @@ __global__ void __launch_bounds__(256, 3) gdn_chunk_prep_kernel(GdnChunkArgs a) 
         bs[r0] = b0;
         bs[r1] = b1;
     }
+    // V of this warp's first 16 columns as B operands (warps 0-3: Wv, 4-7: Wk): on their way under everything before the last products
+    const bool isk = w >= 4;
+    const int n0 = (w & 3) * 32;
+    float x[8][2][2];                    // [k step][tile][k t, t + 4]
+    auto fetch_v = [&](int nb) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int r = k * 8 + t + e * 4;
+#pragma unroll
+                for (int n = 0; n < 2; ++n)
+                    x[k][n][e] = m0 + r < a.M ? a.qkv[(long long)(m0 + r) * qkv_l + (2 * a.KL + h) * CD + nb + n * 8 + g] : 0.f;
+            }
+    };
+    if (!isk) fetch_v(n0);
+    cp_async_wait<0>();
     __syncthreads();
-    // K K^T and Q K^T: warp tile 16 rows x 32 columns
+    // K K^T and Q K^T: warp tile 16 rows x 32 columns; tiles above the diagonal stay zero
     const int r0 = (w & 3) * 16, c0 = (w >> 2) * 32;
     float akk[4][4], aqk[4][4];
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
         for (int i = 0; i < 4; ++i) akk[n][i] = aqk[n][i] = 0.f;
-#pragma unroll 4
-    for (int k0 = 0; k0 < CD; k0 += 8) {
-        uint32_t fk[4], fq[4];
-        lda_frag(fk, Ks, LDA, r0, k0, g, t);
-        lda_frag(fq, Qs, LDA, r0, k0, g, t);
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-            const float *p = Ks + (c0 + n * 8 + g) * LDA + k0 + t;      // B[k][n] = K[n][k]
-            const uint32_t b0 = tf32(p[0]), b1 = tf32(p[4]);
-            mma_tf32(akk[n], fk, b0, b1);
-            mma_tf32(aqk[n], fq, b0, b1);
+    if (c0 < r0 + 16) {
+        const float *ka = a_row(Ks, LDA, r0, lane), *qa = a_row(Qs, LDA, r0, lane);
+        const float *kb0 = b_row(Ks, LDA, c0, lane), *kb1 = b_row(Ks, LDA, c0 + 16, lane);
+#pragma unroll 2
+        for (int k0 = 0; k0 < CD; k0 += 8) {
+            uint32_t fk[4], fq[4], b0[4], b1[4];
+            ldsm4(fk, ka + k0); ldsm4(fq, qa + k0); ldsm4(b0, kb0 + k0); ldsm4(b1, kb1 + k0);
+            round4(fk); round4(fq); round4(b0); round4(b1);
+            mma_tf32(akk[0], fk, b0[0], b0[1]); mma_tf32(akk[1], fk, b0[2], b0[3]); mma_tf32(akk[2], fk, b1[0], b1[1]); mma_tf32(akk[3], fk, b1[2], b1[3]);
+            mma_tf32(aqk[0], fq, b0[0], b0[1]); mma_tf32(aqk[1], fq, b0[2], b0[3]); mma_tf32(aqk[2], fq, b1[0], b1[1]); mma_tf32(aqk[3], fq, b1[2], b1[3]);
         }
     }
     __syncthreads();                     // every warp is done reading Q before A overwrites it
@@ -151,41 +195,128 @@ __global__ void __launch_bounds__(256, 3) gdn_chunk_prep_kernel(GdnChunkArgs a) 
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = r0 + g + (i >> 1) * 8, c = c0 + n * 8 + 2 * t + (i & 1);
-            const float d = __expf(gs[r] - gs[c]);
-            As[r * LDP + c] = c < r ? bs[r] * d * akk[n][i] : 0.f;
-            Pg[r * CC + c] = c <= r ? d * aqk[n][i] : 0.f;
+        for (int i = 0; i < 4; i += 2) {
+            const int r = r0 + g + (i >> 1) * 8, c = c0 + n * 8 + 2 * t;
+            const float d0 = c <= r ? __expf(gs[r] - gs[c]) : 0.f, d1 = c + 1 <= r ? __expf(gs[r] - gs[c + 1]) : 0.f;
+            *reinterpret_cast<float2 *>(As + r * LDP + c) = make_float2(c < r ? bs[r] * d0 * akk[n][i] : 0.f, c + 1 < r ? bs[r] * d1 * akk[n][i + 1] : 0.f);
+            *reinterpret_cast<float2 *>(Pg + r * CC + c) =
+                make_float2(__uint_as_float(tf32(c <= r ? d0 * aqk[n][i] : 0.f)), __uint_as_float(tf32(c + 1 <= r ? d1 * aqk[n][i + 1] : 0.f)));
         }
     if (tid < CC) a.G[((long long)ch * a.VL + h) * CC + tid] = gs[tid];
     __syncthreads();
-    // forward substitution: thread j owns column j of [Wv | Wk]
-    const int j = tid & 127;
-    const bool isk = tid >= 128;
-    float wcol[CC];
+    // T = (I + A)^-1 = [T11 0; T21 T22].  T11 and T22 by forward substitution, a column per thread of the last two warps
+    if (w >= 6) {
+        const int o = (w - 6) * HC_;
+        const float *A = As + o * LDP + o;
+        float col[HC_];
 #pragma unroll
-    for (int r = 0; r < CC; ++r) {
-        float b;
-        if (isk) b = bs[r] * __expf(gs[r]) * Ks[r * LDA + j];
-        else b = (m0 + r < a.M) ? bs[r] * a.qkv[(long long)(m0 + r) * qkv_l + (2 * a.KL + h) * CD + j] : 0.f;
-        wcol[r] = b;
-    }
+        for (int r = 0; r < HC_; ++r) col[r] = r == lane ? 1.f : 0.f;
 #pragma unroll
-    for (int r = 1; r < CC; ++r) {
-        float acc0 = 0.f, acc1 = 0.f, acc2 = 0.f, acc3 = 0.f;      // four independent chains: a row's sum is r / 4 dependent FMAs deep
+        for (int r = 1; r < HC_; ++r) {
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};          // four independent chains
 #pragma unroll
-        for (int s4 = 0; s4 < r; s4 += 4) {
-            const float4 av = *reinterpret_cast<const float4 *>(As + r * LDP + s4);     // zero at s >= r
-            acc0 = fmaf(av.x, wcol[s4], acc0);
-            if (s4 + 1 < r) acc1 = fmaf(av.y, wcol[s4 + 1], acc1);
-            if (s4 + 2 < r) acc2 = fmaf(av.z, wcol[s4 + 2], acc2);
-            if (s4 + 3 < r) acc3 = fmaf(av.w, wcol[s4 + 3], acc3);
+            for (int s4 = 0; s4 < r; s4 += 4) {
+                const float4 av = *reinterpret_cast<const float4 *>(A + r * LDP + s4);     // zero at s >= r
+                acc[0] = fmaf(av.x, col[s4], acc[0]);
+                if (s4 + 1 < r) acc[1] = fmaf(av.y, col[s4 + 1], acc[1]);
+                if (s4 + 2 < r) acc[2] = fmaf(av.z, col[s4 + 2], acc[2]);
+                if (s4 + 3 < r) acc[3] = fmaf(av.w, col[s4 + 3], acc[3]);
+            }
+            col[r] -= (acc[0] + acc[1]) + (acc[2] + acc[3]);
         }
-        wcol[r] -= (acc0 + acc1) + (acc2 + acc3);
-    }
-    float *Wg = (isk ? a.Wk : a.Wv) + ((long long)ch * a.VL + h) * CC * CD;
 #pragma unroll
-    for (int r = 0; r < CC; ++r) Wg[r * CD + j] = wcol[r];
+        for (int r = 0; r < HC_; ++r) Ts[(o + r) * LDP + o + lane] = col[r];
+    }
+    __syncthreads();
+    // T21 = -T22 (A21 T11), both products in fp32; the first goes to A's empty upper right
+    float *Es = As + HC_;                // [32][LDP]
+    const int er = tid >> 3, ec = (tid & 7) * 4;
+    auto half_product = [&](const float *A, const float *B) {
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+        for (int s = 0; s < HC_; ++s) {
+            const float f = A[er * LDP + s];
+            const float4 v = *reinterpret_cast<const float4 *>(B + s * LDP + ec);
+            acc.x = fmaf(f, v.x, acc.x); acc.y = fmaf(f, v.y, acc.y); acc.z = fmaf(f, v.z, acc.z); acc.w = fmaf(f, v.w, acc.w);
+        }
+        return acc;
+    };
+    *reinterpret_cast<float4 *>(Es + er * LDP + ec) = half_product(As + HC_ * LDP, Ts);
+    __syncthreads();
+    {
+        const float4 v = half_product(Ts + HC_ * LDP + HC_, Es);
+        *reinterpret_cast<float4 *>(Ts + (HC_ + er) * LDP + ec) = make_float4(-v.x, -v.y, -v.z, -v.w);
+    }
+    __syncthreads();
+    // T as two tf32 parts (what lies above the diagonal blocks is not read)
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const int e = tid + i * 256, at = (e >> 6) * LDP + (e & 63);
+        const float v = Ts[at];
+        const uint32_t hi = tf32(v);
+        As[at] = __uint_as_float(hi);
+        Ts[at] = __uint_as_float(tf32(v - __uint_as_float(hi)));
+    }
+    __syncthreads();
+    // Wv = T diag(beta) V, Wk = T diag(beta exp(g)) K: 32 columns per warp, 16 at a time
+    float *Wg = (isk ? a.Wk : a.Wv) + ((long long)ch * a.VL + h) * CC * CD;
+    const float *ta = a_row(As, LDP, 0, lane), *tl = a_row(Ts, LDP, 0, lane);
+#pragma unroll 1
+    for (int nb = n0; nb < n0 + 32; nb += 16) {
+        if (isk) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int r = k * 8 + t + e * 4;
+#pragma unroll
+                    for (int n = 0; n < 2; ++n) x[k][n][e] = Ks[r * LDA + nb + n * 8 + g];
+                }
+        } else if (nb != n0) {
+            fetch_v(nb);
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int r = k * 8 + t + e * 4;
+                const float f = isk ? bs[r] * __expf(gs[r]) : bs[r];
+#pragma unroll
+                for (int n = 0; n < 2; ++n) x[k][n][e] *= f;
+            }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float acc[2][4] = {};
+#pragma unroll
+            for (int k = 0; k < 2 * i + 2; ++k) {
+                uint32_t hi[4], lo[4];
+                ldsm4(hi, ta + i * 16 * LDP + k * 8);
+                ldsm4(lo, tl + i * 16 * LDP + k * 8);
+#pragma unroll
+                for (int n = 0; n < 2; ++n) {
+                    uint32_t b[2], bl[2];
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        b[e] = tf32(x[k][n][e]);
+                        bl[e] = tf32(x[k][n][e] - __uint_as_float(b[e]));
+                    }
+                    mma_tf32(acc[n], lo, b[0], b[1]);
+                    mma_tf32(acc[n], hi, bl[0], bl[1]);
+                    mma_tf32(acc[n], hi, b[0], b[1]);
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                if (isk) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc[n][c] = __uint_as_float(tf32(acc[n][c]));
+                }
+                float *o = Wg + (i * 16 + g) * CD + nb + n * 8 + 2 * t;
+                *reinterpret_cast<float2 *>(o) = make_float2(acc[n][0], acc[n][1]);
+                *reinterpret_cast<float2 *>(o + 8 * CD) = make_float2(acc[n][2], acc[n][3]);
+            }
+        }
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -196,49 +327,32 @@ __global__ void __launch_bounds__(256, 3) gdn_chunk_prep_kernel(GdnChunkArgs a) 
 // split keeps the number of blocks up.  Every output element's sum runs over k in the same order whatever NC is.
 template <int NC>
 constexpr int apply_smem() {
-    return (CD * (NC + 8) + 2 * CC * LDA + CC * LDT + 2 * CC * LDP + CC * (NC + 8) + 2 * CC) * 4;
+    return (NC * LDA + 2 * CC * LDA + 2 * CC * LDT + 2 * CC * LDP + NC * LDP + 3 * CC) * 4;
 }
 
-// 16-byte asynchronous copy global -> shared; `ok` false: the destination is zero-filled (rows past the run's end).
-__device__ __forceinline__ void cp_async16(float *dst, const float *src, bool ok) {
-    const unsigned int d = (unsigned int)__cvta_generic_to_shared(dst);
-    const int n = ok ? 16 : 0;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// Rows [m0, m0+64) x 128 floats at column offset col of the qkv rows -> shared tile of stride ld, asynchronously; rows
-// >= M become zero.  256 threads.
-__device__ __forceinline__ void load_tile_async(float *dst, int ld, const float *qkv, int qkv_l, int col, int m0, int M, int tid) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int idx = tid + i * 256;          // float4 index: 64 rows x 32
-        const int r = idx >> 5, c4 = idx & 31;
-        const bool ok = m0 + r < M;
-        cp_async16(dst + r * ld + c4 * 4, qkv + (long long)(ok ? m0 + r : 0) * qkv_l + col + c4 * 4, ok);
-    }
-}
-
-// The kernel walks the chunks in order; what a chunk needs from global memory is in shared memory before its products
-// start: Wk, Q, P and the cumulative log decays of chunk c + 1 are fetched (cp.async) into the tiles that chunk c's first
-// product has finished with, under chunk c's second and third products; K of chunk c, needed only by the third
-// product, is fetched under the first two.  The chain of 64 chunk steps of a 4,096-token run is what bounds the
-// kernel (it does not shorten with fewer heads per rank), so nothing on it waits for a global load.
+// The kernel walks the chunks in order; what a chunk needs from global memory (Wk, Q, P, K and the cumulative log decays) is fetched with
+// cp.async under the second and third product of the chunk before it.  The chain of 64 chunk steps of a 4,096-token run is what bounds the
+// kernel (it does not shorten with fewer heads per rank), so nothing on it waits for a global load, and a step has two meetings.
+// The state stays in fp32 in the accumulators of the product that updates it, transposed (value columns x keys): a warp owns
+// 8 or 16 keys.  What other warps read of it, and of U, lies rounded to tf32 in shared memory with k along the rows, so that ldmatrix
+// brings an operand in one instruction where single loads and conversions took ten.
+// 4,096 tokens, 48 heads: 400 us, now 343 (1,021: 106, 89; with 16 warps 420).
 template <int NC>
-__global__ void __launch_bounds__(256) gdn_chunk_apply_kernel(GdnChunkArgs a) {
-    constexpr int LDS = NC + 8;          // [.][NC] B-operand tile (state slice, U)
-    constexpr int NT = NC / 16;          // 8-column tiles of a warp in the row-tiled products
-    constexpr int NS = NC / 8;           // 8-column tiles of a warp in the state update
+constexpr int apply_threads() { return 256; }
+template <int NC>
+__global__ void __launch_bounds__(apply_threads<NC>()) gdn_chunk_apply_kernel(GdnChunkArgs a) {
+    constexpr int TH = apply_threads<NC>(), NW = TH / 32;
+    constexpr int NT = NC / 2 / NW;      // 8-column tiles of a warp in the row-tiled products (NW / 4 warps beside each other)
+    constexpr int MT = NC / 16, KN = 16 / NW;      // 16-row and 8-column tiles of a warp's part of the state
     extern __shared__ __align__(16) float sm[];
-    float *Ss = sm;                      // [128 k][LDS]   state, this block's NC value columns
-    float *Wks = Ss + CD * LDS;          // [64][LDA]
+    float *St = sm;                      // [NC][LDA]      state, this block's value columns x keys
+    float *Wks = St + NC * LDA;          // [64][LDA]
     float *Qs = Wks + CC * LDA;          // [64][LDA]
-    float *Ks = Qs + CC * LDA;           // [64][LDT]      read transposed in the state update
-    float *Ps = Ks + CC * LDT;           // [2][64][LDP]   chunk c in buffer c & 1
-    float *Us = Ps + 2 * CC * LDP;       // [64][LDS]
-    float *gb = Us + CC * LDS;           // [2][64]        cumulative log decay g_t of the chunk
+    float *Ks = Qs + CC * LDA;           // [2][64][LDT]   chunk c in buffer c & 1
+    float *Ps = Ks + 2 * CC * LDT;       // [2][64][LDP]
+    float *Ut = Ps + 2 * CC * LDP;       // [NC][LDP]      U, value columns x rows of the chunk
+    float *gb = Ut + NC * LDP;           // [2][64]        cumulative log decay g_t of the chunk
+    float *ek = gb + 2 * CC;             // [64]           exp(g_C - g_t)
     const int vh = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int qkv_l = (2 * a.KL + a.VL) * CD;
@@ -246,36 +360,50 @@ __global__ void __launch_bounds__(256) gdn_chunk_apply_kernel(GdnChunkArgs a) {
     const int slot = a.slot[0];
     float *Sg = a.S + ((long long)slot * a.VL + h) * CD * CD + vh * NC;
     const int nch = (a.M + CC - 1) / CC;
-    // what chunk `ch` needs before its first product: Q, Wk, P, g
-    auto fetch_front = [&](int ch) {
+    auto fetch = [&](int ch) {
         const long long cb = (long long)ch * a.VL + h;
-        load_tile_async(Qs, LDA, a.qkv, qkv_l, kh * CD, ch * CC, a.M, tid);
-        load_tile_async(Wks, LDA, a.Wk + cb * CC * CD, CD, 0, 0, CC, tid);
+        const int m0 = ch * CC;
+        load_tile_async<TH>(Qs, LDA, a.qkv, qkv_l, kh * CD, m0, a.M, tid);
+        load_tile_async<TH>(Wks, LDA, a.Wk + cb * CC * CD, CD, 0, 0, CC, tid);
+        load_tile_async<TH>(Ks + (ch & 1) * CC * LDT, LDT, a.qkv, qkv_l, (a.KL + kh) * CD, m0, a.M, tid);
         const float *Pg = a.P + cb * CC * CC;
         float *Pd = Ps + (ch & 1) * CC * LDP;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int idx = tid + i * 256;      // float4 index: 64 rows x 16
+        for (int i = 0; i < 1024 / TH; ++i) {
+            const int idx = tid + i * TH;       // float4 index: 64 rows x 16
             const int r = idx >> 4, c4 = idx & 15;
             cp_async16(Pd + r * LDP + c4 * 4, Pg + r * CC + c4 * 4, true);
         }
         if (tid < CC / 4) cp_async16(gb + (ch & 1) * CC + tid * 4, a.G + cb * CC + tid * 4, true);
+        cp_async_commit();
     };
-    fetch_front(0);
-    cp_async_commit();
-    for (int idx = tid; idx < CD * (NC / 4); idx += 256) {      // float4 index: 128 rows x NC / 4
-        const int r = idx / (NC / 4), c4 = idx % (NC / 4);
-        *reinterpret_cast<float4 *>(Ss + r * LDS + c4 * 4) = *reinterpret_cast<const float4 *>(Sg + r * CD + c4 * 4);
-    }
-    const int r0 = (w & 3) * 16, c0 = (w >> 2) * (NC / 2);
+    fetch(0);
+    // accS[i][n]: value columns 16 i + g, + 8; keys k0w + 8 n + 2 t, + 1
+    float accS[MT][KN][4];
+    const int k0w = w * 8 * KN;
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int n = 0; n < KN; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) accS[i][n][e] = Sg[(long long)(k0w + n * 8 + 2 * t + (e & 1)) * CD + i * 16 + g + (e >> 1) * 8];
+    auto publish = [&]() {               // the state as the next chunk's operand
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int n = 0; n < KN; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; e += 2)
+                    *reinterpret_cast<float2 *>(St + (i * 16 + g + e * 4) * LDA + k0w + n * 8 + 2 * t) =
+                        make_float2(__uint_as_float(tf32(accS[i][n][e])), __uint_as_float(tf32(accS[i][n][e + 1])));
+    };
+    publish();
+    const int r0 = (w & 3) * 16, c0 = (w >> 2) * (8 * NT);
+    const float *wa = a_row(Wks, LDA, r0, lane), *qa = a_row(Qs, LDA, r0, lane), *sb = b_row(St, LDA, c0, lane), *ub = b_row(Ut, LDP, c0, lane);
     for (int ch = 0; ch < nch; ++ch) {
         const int m0 = ch * CC;
         const long long cb = (long long)ch * a.VL + h;
-        const float *Pc = Ps + (ch & 1) * CC * LDP, *gc = gb + (ch & 1) * CC;
-        load_tile_async(Ks, LDT, a.qkv, qkv_l, (a.KL + kh) * CD, m0, a.M, tid);      // for the third product
-        cp_async_commit();
-        cp_async_wait<1>();              // everything but K: this chunk's Q, Wk, P, g are in
-        __syncthreads();
+        const float *gc = gb + (ch & 1) * CC;
         // Wv of this thread's U elements: issued now, used after the first product
         const float *Wvg = a.Wv + cb * CC * CD + vh * NC;
         float2 wv0[NT], wv1[NT];
@@ -285,6 +413,8 @@ __global__ void __launch_bounds__(256) gdn_chunk_apply_kernel(GdnChunkArgs a) {
             wv0[n] = *reinterpret_cast<const float2 *>(Wvg + (r0 + g) * CD + c);
             wv1[n] = *reinterpret_cast<const float2 *>(Wvg + (r0 + g + 8) * CD + c);
         }
+        cp_async_wait<0>();
+        __syncthreads();                 // this chunk's tiles and the state are there
         // U = Wv - Wk S0 and Q S0: warp tile 16 rows x NC / 2 value columns
         float accW[NT][4], accO[NT][4];
 #pragma unroll
@@ -294,93 +424,100 @@ __global__ void __launch_bounds__(256) gdn_chunk_apply_kernel(GdnChunkArgs a) {
 #pragma unroll 4
         for (int k0 = 0; k0 < CD; k0 += 8) {
             uint32_t fw[4], fq[4];
-            lda_frag(fw, Wks, LDA, r0, k0, g, t);
-            lda_frag(fq, Qs, LDA, r0, k0, g, t);
+            ldsm4(fw, wa + k0);
+            ldsm4(fq, qa + k0);
+            round4(fq);
 #pragma unroll
-            for (int n = 0; n < NT; ++n) {
-                const float *p = Ss + (k0 + t) * LDS + c0 + n * 8 + g;
-                const uint32_t b0 = tf32(p[0]), b1 = tf32(p[4 * LDS]);
-                mma_tf32(accW[n], fw, b0, b1);
-                mma_tf32(accO[n], fq, b0, b1);
+            for (int n = 0; n < NT; n += 2) {
+                uint32_t b[4];
+                if (NT > 1) ldsm4(b, sb + n * 8 * LDA + k0);
+                else ldsm2(b[0], b[1], sb + k0);
+                mma_tf32(accW[n], fw, b[0], b[1]);
+                mma_tf32(accO[n], fq, b[0], b[1]);
+                if (NT > 1) {
+                    mma_tf32(accW[n + 1 < NT ? n + 1 : n], fw, b[2], b[3]);
+                    mma_tf32(accO[n + 1 < NT ? n + 1 : n], fq, b[2], b[3]);
+                }
             }
         }
+        const float gC = gc[CC - 1];
         {
+            if (tid < CC) ek[tid] = __expf(gC - gc[tid]);
             const float e0 = __expf(gc[r0 + g]), e1 = __expf(gc[r0 + g + 8]);
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
-                const int c = c0 + n * 8 + 2 * t;
-                *reinterpret_cast<float2 *>(Us + (r0 + g) * LDS + c) = make_float2(wv0[n].x - accW[n][0], wv0[n].y - accW[n][1]);
-                *reinterpret_cast<float2 *>(Us + (r0 + g + 8) * LDS + c) = make_float2(wv1[n].x - accW[n][2], wv1[n].y - accW[n][3]);
+                float *u = Ut + (c0 + n * 8 + 2 * t) * LDP + r0 + g;
+                u[0] = __uint_as_float(tf32(wv0[n].x - accW[n][0]));
+                u[LDP] = __uint_as_float(tf32(wv0[n].y - accW[n][1]));
+                u[8] = __uint_as_float(tf32(wv1[n].x - accW[n][2]));
+                u[LDP + 8] = __uint_as_float(tf32(wv1[n].y - accW[n][3]));
                 accO[n][0] *= e0; accO[n][1] *= e0;
                 accO[n][2] *= e1; accO[n][3] *= e1;
             }
         }
-        __syncthreads();                 // U is complete; the Q and Wk tiles are free
-        const bool more = ch + 1 < nch;
-        if (more) {
-            fetch_front(ch + 1);
-            cp_async_commit();
-        }
+        __syncthreads();                 // U is complete; the Q and Wk tiles and the state's copy are free
+        if (ch + 1 < nch) fetch(ch + 1);
         // O += P U (P is zero above the diagonal: k tiles past the warp's rows are skipped)
-        for (int k0 = 0; k0 < r0 + 16; k0 += 8) {
-            uint32_t fp[4];
-            lda_frag(fp, Pc, LDP, r0, k0, g, t);
-#pragma unroll
-            for (int n = 0; n < NT; ++n) {
-                const float *p = Us + (k0 + t) * LDS + c0 + n * 8 + g;
-                mma_tf32(accO[n], fp, tf32(p[0]), tf32(p[4 * LDS]));
-            }
-        }
-#pragma unroll
-        for (int n = 0; n < NT; ++n) {
-            const int c = h * CD + vh * NC + c0 + n * 8 + 2 * t;
-            const int ra = m0 + r0 + g, rb = ra + 8;
-            if (ra < a.M) *reinterpret_cast<float2 *>(a.Oraw + (long long)ra * a.VL * CD + c) = make_float2(accO[n][0], accO[n][1]);
-            if (rb < a.M) *reinterpret_cast<float2 *>(a.Oraw + (long long)rb * a.VL * CD + c) = make_float2(accO[n][2], accO[n][3]);
-        }
-        if (more) cp_async_wait<1>();    // K of this chunk (the next chunk's front tiles may still be on their way)
-        else cp_async_wait<0>();
-        __syncthreads();
-        // S1 = exp(g_C) S0 + (diag(ek) K)^T U: warp w owns state rows 16w .. 16w+15, all NC columns
         {
-            const int i0 = w * 16;
-            const float gC = gc[CC - 1];
-            const float eC = __expf(gC);
-            float accS[NS][4];
-#pragma unroll
-            for (int n = 0; n < NS; ++n) {
-                const float2 s0 = *reinterpret_cast<const float2 *>(Ss + (i0 + g) * LDS + n * 8 + 2 * t);
-                const float2 s1 = *reinterpret_cast<const float2 *>(Ss + (i0 + g + 8) * LDS + n * 8 + 2 * t);
-                accS[n][0] = s0.x * eC; accS[n][1] = s0.y * eC;
-                accS[n][2] = s1.x * eC; accS[n][3] = s1.y * eC;
-            }
+            const float *pa = a_row(Ps + (ch & 1) * CC * LDP, LDP, r0, lane);
 #pragma unroll 2
-            for (int k0 = 0; k0 < CC; k0 += 8) {
-                const float ea = __expf(gC - gc[k0 + t]), eb = __expf(gC - gc[k0 + t + 4]);
-                const float *p = Ks + (k0 + t) * LDT + i0 + g;      // A[i][s] = K[s][i] ek[s]
-                uint32_t fa[4];
-                fa[0] = tf32(p[0] * ea);
-                fa[1] = tf32(p[8] * ea);
-                fa[2] = tf32(p[4 * LDT] * eb);
-                fa[3] = tf32(p[4 * LDT + 8] * eb);
+            for (int k0 = 0; k0 < r0 + 16; k0 += 8) {
+                uint32_t fp[4];
+                ldsm4(fp, pa + k0);
 #pragma unroll
-                for (int n = 0; n < NS; ++n) {
-                    const float *q = Us + (k0 + t) * LDS + n * 8 + g;
-                    mma_tf32(accS[n], fa, tf32(q[0]), tf32(q[4 * LDS]));
+                for (int n = 0; n < NT; n += 2) {
+                    uint32_t b[4];
+                    if (NT > 1) ldsm4(b, ub + n * 8 * LDP + k0);
+                    else ldsm2(b[0], b[1], ub + k0);
+                    mma_tf32(accO[n], fp, b[0], b[1]);
+                    if (NT > 1) mma_tf32(accO[n + 1 < NT ? n + 1 : n], fp, b[2], b[3]);
                 }
             }
 #pragma unroll
-            for (int n = 0; n < NS; ++n) {
-                *reinterpret_cast<float2 *>(Ss + (i0 + g) * LDS + n * 8 + 2 * t) = make_float2(accS[n][0], accS[n][1]);
-                *reinterpret_cast<float2 *>(Ss + (i0 + g + 8) * LDS + n * 8 + 2 * t) = make_float2(accS[n][2], accS[n][3]);
+            for (int n = 0; n < NT; ++n) {
+                const int c = h * CD + vh * NC + c0 + n * 8 + 2 * t;
+                const int ra = m0 + r0 + g, rb = ra + 8;
+                if (ra < a.M) *reinterpret_cast<float2 *>(a.Oraw + (long long)ra * a.VL * CD + c) = make_float2(accO[n][0], accO[n][1]);
+                if (rb < a.M) *reinterpret_cast<float2 *>(a.Oraw + (long long)rb * a.VL * CD + c) = make_float2(accO[n][2], accO[n][3]);
             }
         }
-        __syncthreads();
+        // S1^T = exp(g_C) S0^T + U^T diag(ek) K
+        {
+            const float eC = __expf(gC);
+#pragma unroll
+            for (int i = 0; i < MT; ++i)
+#pragma unroll
+                for (int n = 0; n < KN; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) accS[i][n][e] *= eC;
+            const float *kp = Ks + (ch & 1) * CC * LDT + t * LDT + k0w + g;
+            const float *ua = a_row(Ut, LDP, 0, lane);
+#pragma unroll 2
+            for (int s0 = 0; s0 < CC; s0 += 8) {
+                const float ea = ek[s0 + t], eb = ek[s0 + t + 4];
+                uint32_t b[KN][2];
+#pragma unroll
+                for (int n = 0; n < KN; ++n) {
+                    b[n][0] = tf32(kp[s0 * LDT + n * 8] * ea);
+                    b[n][1] = tf32(kp[(s0 + 4) * LDT + n * 8] * eb);
+                }
+#pragma unroll
+                for (int i = 0; i < MT; ++i) {
+                    uint32_t fu[4];
+                    ldsm4(fu, ua + i * 16 * LDP + s0);
+#pragma unroll
+                    for (int n = 0; n < KN; ++n) mma_tf32(accS[i][n], fu, b[n][0], b[n][1]);
+                }
+            }
+        }
+        publish();
     }
-    for (int idx = tid; idx < CD * (NC / 4); idx += 256) {
-        const int r = idx / (NC / 4), c4 = idx % (NC / 4);
-        *reinterpret_cast<float4 *>(Sg + r * CD + c4 * 4) = *reinterpret_cast<const float4 *>(Ss + r * LDS + c4 * 4);
-    }
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int n = 0; n < KN; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) Sg[(long long)(k0w + n * 8 + 2 * t + (e & 1)) * CD + i * 16 + g + (e >> 1) * 8] = accS[i][n][e];
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -442,7 +579,7 @@ QW_API int qwk_gdn_scan_chunked(const float *qkv, const float *decay, const floa
     a.Oraw = a.G + nch * VL * CC;
     gdn_chunk_prep_kernel<<<dim3((unsigned)nch, VL), 256, PREP_SMEM, s>>>(a);
     // blocks of the sequential walk: 128 / NC per head, NC chosen so that about a hundred blocks run
-    if (VL >= 32) gdn_chunk_apply_kernel<64><<<dim3(2, VL), 256, apply_smem<64>(), s>>>(a);
+    if (VL >= 32) gdn_chunk_apply_kernel<64><<<dim3(2, VL), apply_threads<64>(), apply_smem<64>(), s>>>(a);
     else if (VL >= 16) gdn_chunk_apply_kernel<32><<<dim3(4, VL), 256, apply_smem<32>(), s>>>(a);
     else gdn_chunk_apply_kernel<16><<<dim3(8, VL), 256, apply_smem<16>(), s>>>(a);
     const unsigned blocks = (unsigned)(((long long)M * VL + 7) / 8);
