@@ -10,8 +10,11 @@
 // meet in the epilogue, which writes silu(gate) * up), or two neighbouring tiles of the down projection - so the tokens of a k
 // block are fetched once for both.
 //
-//   warp 0       loads, 128 k values a stage, four stages: two 128-row x 64-byte TMA tiles of packed weights (64B swizzle) and
-//                ceil(rows / 16) x 2 boxes of 16 token rows x 64 k values
+//   warp 0       loads, 128 k values a stage: two 128-row x 64-byte TMA tiles of packed weights (64B swizzle) and ceil(rows / 16) x 2
+//                boxes of 16 token rows x 64 k values.  down: both on one ring of four stages.  gate/up: weights only, on a ring of six that
+//                the conversion alone sets free, and warp 2 brings the tokens on a ring of four: four times the k blocks, and weights that
+//                wait for the MMAs' tokens left memory idle (us, one ring and two: 100 tokens 236, 218; 1,021 288, 263; 4,096 480, 455).
+//                (For down, five k blocks a unit, two rings are slower: 154 and 159 us at 1,021 tokens, 239 and 255 at 4,096.)
 //   warps 8-23   conversion: warp group (tile, parity) owns every other stage of one tile; four TMEM stages of 64 k values
 //   warps 1, 3   issue the MMAs of one tile each (A in TMEM, B in shared memory, D in TMEM): with one warp for both, its waits and
 //                issue were the longest chain
@@ -27,10 +30,12 @@
 
 namespace qw {
 
-constexpr int MG_STAGES = 4, MG_AHEAD = 2;
-constexpr int MG_W_TILE = 128 * 64, MG_X_PANEL = 128 * 128, MG_STAGE = 2 * MG_X_PANEL + 2 * MG_W_TILE;      // tokens, then weights
+template <bool SWIGLU> constexpr int mg_wst() { return SWIGLU ? 6 : 4; }
+constexpr int MG_XST = 4, MG_AHEAD = 2;
+constexpr int MG_W_TILE = 128 * 64, MG_X_PANEL = 128 * 128;
 constexpr int MG_THREADS = 768, MG_CONV_WARP0 = 8, MG_EPI_WARP0 = 4;
-constexpr int MG_SMEM = MG_STAGES * MG_STAGE + 1024 /*alignment*/ + 512 /*barriers*/;
+template <bool SWIGLU>
+constexpr int mg_smem() { return MG_XST * 2 * MG_X_PANEL + mg_wst<SWIGLU>() * 2 * MG_W_TILE + 1024 /*alignment*/ + 512 /*barriers*/; }
 
 struct MoeTcArgs {
     const int4 *tiles;       // {first token row, rows (<= 128; 0 = unused), first weight row of the expert, -}
@@ -102,16 +107,21 @@ struct MgWalk {
 template <bool SWIGLU>
 __global__ void __launch_bounds__(MG_THREADS, 1) moe_tc_kernel(const __grid_constant__ CUtensorMap mapX,
                                                                const __grid_constant__ CUtensorMap mapW, MoeTcArgs a) {
+    constexpr int MG_WST = mg_wst<SWIGLU>();
+    constexpr bool JOINT = !SWIGLU;          // weights and tokens of a k block share a stage
     extern __shared__ unsigned char raw[];
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + MG_STAGES * MG_STAGE), *empty = full + MG_STAGES;
-    uint64_t *a_full = empty + MG_STAGES;                        // [tile][parity]: a converted 128 x 128 block
+    unsigned char *sx = smem, *sw = smem + MG_XST * 2 * MG_X_PANEL;
+    uint64_t *w_full = reinterpret_cast<uint64_t *>(sw + MG_WST * 2 * MG_W_TILE), *w_empty = w_full + MG_WST;
+    uint64_t *x_full = w_empty + MG_WST, *x_empty = x_full + MG_XST;
+    uint64_t *a_full = x_empty + MG_XST;                        // [tile][parity]: a converted 128 x 128 block
     uint64_t *a_empty = a_full + 4, *done = a_empty + 8;         // [tile][parity][half]: its halves, free again
     uint64_t *acc_empty = done + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
     if (threadIdx.x == 0) {
-        for (int s = 0; s < MG_STAGES; ++s) { mbar_init(full + s, 1); mbar_init(empty + s, 8 + 2); }      // 8 converting warps, the MMAs of two tiles
+        for (int s = 0; s < MG_WST; ++s) { mbar_init(w_full + s, 1); mbar_init(w_empty + s, JOINT ? 8 + 2 : 8); }      // 8 converting warps
+        for (int s = 0; s < MG_XST; ++s) { mbar_init(x_full + s, 1); mbar_init(x_empty + s, 2); }                      // the MMAs of two tiles
         for (int s = 0; s < 4; ++s) mbar_init(a_full + s, 4);
         for (int s = 0; s < 8; ++s) mbar_init(a_empty + s, 1);
         for (int s = 0; s < 2; ++s) { mbar_init(done + s, 2); mbar_init(acc_empty + s, 4); }
@@ -126,30 +136,36 @@ __global__ void __launch_bounds__(MG_THREADS, 1) moe_tc_kernel(const __grid_cons
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
     const int kblocks = a.K >> 7;                    // 128 k values each: one scale group
-    if (warp == 0) {
-        unsigned it = 0;
+    if (warp == 0 || (!JOINT && warp == 2)) {
+        const bool weights = warp == 0, tokens = JOINT || warp == 2;
+        const unsigned stages = weights ? MG_WST : MG_XST;
+        uint64_t *const full = weights ? w_full : x_full, *const empty = weights ? w_empty : x_empty;
+        unsigned s = 0, round = 0;
         bool ok = true;
         MgWalk w(a);
         for (w.uniform(); w.valid(a) && ok; w.next(a), w.uniform()) {
             const int row = w.tl.z + (w.id % a.units_n) * a.row_step;
-            const int boxes = (w.tl.y + 15) >> 4;
-            for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                const unsigned s = it % MG_STAGES;
-                if (it >= MG_STAGES && !mg_wait_warp(empty + s, (it / MG_STAGES - 1) & 1u, a.err)) { ok = false; break; }
+            const int boxes = tokens ? (w.tl.y + 15) >> 4 : 0;
+            for (int kb = 0; kb < kblocks; ++kb) {
+                if (round && !mg_wait_warp(empty + s, (round - 1) & 1u, a.err)) { ok = false; break; }
                 if (elect_one()) {
-                    unsigned char *st = smem + s * MG_STAGE;
-                    mbar_expect_tx(full + s, 2u * MG_W_TILE + (unsigned)boxes * 4096u);
-                    tma_load_2d(st + 2 * MG_X_PANEL, &mapW, kb * 64, row, full + s);
-                    tma_load_2d(st + 2 * MG_X_PANEL + MG_W_TILE, &mapW, kb * 64, row + a.row_second, full + s);
+                    mbar_expect_tx(full + s, (weights ? 2u * MG_W_TILE : 0u) + (unsigned)boxes * 4096u);
+                    if (weights) {
+                        unsigned char *st = sw + s * 2 * MG_W_TILE;
+                        tma_load_2d(st, &mapW, kb * 64, row, full + s);
+                        tma_load_2d(st + MG_W_TILE, &mapW, kb * 64, row + a.row_second, full + s);
+                    }
+                    unsigned char *st = sx + s * 2 * MG_X_PANEL;
                     for (int b = 0; b < boxes; ++b) {
                         tma_load_2d(st + b * 2048, &mapX, kb * 128, w.tl.x + b * 16, full + s);
                         tma_load_2d(st + MG_X_PANEL + b * 2048, &mapX, kb * 128 + 64, w.tl.x + b * 16, full + s);
                     }
                 }
+                if (++s == stages) { s = 0; ++round; }
             }
         }
     } else if (warp == 1 || warp == 3) {
-        // one wait per 128 k values: the converting warps have seen the stage's loads complete, tokens included
+        // one wait per 128 k values where the converting warps have seen the stage's loads complete, tokens included
         const int tile = warp >> 1;
         uint64_t *const a_full1 = a_full + tile * 2, *const a_empty1 = a_empty + tile * 4;
         unsigned it = 0;
@@ -170,10 +186,11 @@ __global__ void __launch_bounds__(MG_THREADS, 1) moe_tc_kernel(const __grid_cons
             const uint32_t d = tmem + (uint32_t)(s0 * 128) + (tile ? (big ? 128u : 64u) : 0u);
             for (int kb = 0; kb < kblocks; ++kb, ++it) {
                 const unsigned odd = it & 1u;
+                if (!JOINT && !mg_wait_warp(x_full + it % MG_XST, (it / MG_XST) & 1u, a.err)) { ok = false; break; }
                 if (!mg_wait_warp(a_full1 + odd, (it >> 1) & 1u, a.err)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t ta = tmem + 256u + odd * 128u + (uint32_t)(tile * 32);
-                const uint32_t xb = smem_u32(smem + (it % MG_STAGES) * MG_STAGE);
+                const uint32_t xb = smem_u32(sx + (it % MG_XST) * 2 * MG_X_PANEL);
                 if (elect_one()) {
 #pragma unroll
                     for (int half = 0; half < 2; ++half) {
@@ -182,7 +199,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) moe_tc_kernel(const __grid_cons
                             umma_bf16_ts(d, ta + half * 64 + k * 8, make_sw128_desc(xb + half * MG_X_PANEL + k * 32), idesc, (kb | half | k) ? 1u : 0u);
                         umma_commit(a_empty1 + odd * 2 + half);
                     }
-                    umma_commit(empty + it % MG_STAGES);
+                    umma_commit((JOINT ? w_empty : x_empty) + it % MG_XST);
                 }
             }
             if (ok && elect_one()) umma_commit(done + s0);
@@ -194,7 +211,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) moe_tc_kernel(const __grid_cons
         const unsigned short *scale = reinterpret_cast<const unsigned short *>(a.scale);
         const bf162 off2 = __floats2bfloat162_rn(136.f, 136.f);
         const uint32_t lane_base = tmem + ((uint32_t)(q * 32) << 16) + 256u + (uint32_t)(odd * 128 + tile * 32);
-        const unsigned char *row_base = smem + 2 * MG_X_PANEL + tile * MG_W_TILE + r * 64;
+        const unsigned char *row_base = sw + tile * MG_W_TILE + r * 64;
         const int swz = ((r >> 1) & 3) << 4;                     // row r's 64 bytes: 16-byte chunk c lies at chunk c ^ ((r >> 1) & 3)
         uint64_t *const a_full2 = a_full + tile * 2 + odd, *const a_empty2 = a_empty + tile * 4 + odd * 2;
         auto scale_row = [&](int id, int z) {
@@ -232,17 +249,17 @@ __global__ void __launch_bounds__(MG_THREADS, 1) moe_tc_kernel(const __grid_cons
                     const uint32_t sc_bits = (uint32_t)ring[i] * 0x10001u;
                     const bf162 sc2 = *reinterpret_cast<const bf162 *>(&sc_bits);
                     if (kb + 2 * MG_AHEAD < kblocks) ring[i] = __ldg(sp + kb + 2 * MG_AHEAD);
-                    if (!mg_wait_warp(full + ws, w_phase, a.err)) { ok = false; break; }
+                    if (!mg_wait_warp(w_full + ws, w_phase, a.err)) { ok = false; break; }
                     uint32_t words[16];
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
-                        const uint4 v = *reinterpret_cast<const uint4 *>(row_base + ws * MG_STAGE + ((c << 4) ^ swz));
+                        const uint4 v = *reinterpret_cast<const uint4 *>(row_base + ws * 2 * MG_W_TILE + ((c << 4) ^ swz));
                         words[4 * c] = v.x; words[4 * c + 1] = v.y; words[4 * c + 2] = v.z; words[4 * c + 3] = v.w;
                     }
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(empty + ws);
+                    if (lane == 0) mbar_arrive(w_empty + ws);
                     ws += 2;
-                    if (ws >= MG_STAGES) { ws -= MG_STAGES; w_phase ^= 1u; }
+                    if (ws >= MG_WST) { ws -= MG_WST; w_phase ^= 1u; }
 #pragma unroll
                     for (int half = 0; half < 2; ++half) {
                         uint32_t o[4][8];            // converted before the stage is free: behind the wait only the stores remain
@@ -355,7 +372,7 @@ static int moe_tc_launch(MoeTcArgs &a, const void *A, const void *Wq, int rows, 
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
     if (!done[dev]) {
-        if (cudaFuncSetAttribute(moe_tc_kernel<SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SMEM) != cudaSuccess) return -3;
+        if (cudaFuncSetAttribute(moe_tc_kernel<SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, mg_smem<SWIGLU>()) != cudaSuccess) return -3;
         done[dev] = true;
     }
     CUtensorMap mX, mW;
@@ -364,7 +381,7 @@ static int moe_tc_launch(MoeTcArgs &a, const void *A, const void *Wq, int rows, 
     a.mask = 0x000F000Fu;
     a.magic = 0x43004300u;
     a.total = max_tiles * a.units_n;
-    moe_tc_kernel<SWIGLU><<<persistent_grid(a.total, 1), MG_THREADS, MG_SMEM, s>>>(mX, mW, a);
+    moe_tc_kernel<SWIGLU><<<persistent_grid(a.total, 1), MG_THREADS, mg_smem<SWIGLU>(), s>>>(mX, mW, a);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
