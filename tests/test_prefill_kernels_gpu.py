@@ -9,6 +9,61 @@ from test_step_kernels_gpu import DEV, P, S, _lib, gen, i32
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture
+def exchange():
+    """Sets the tokens of an exchanged tile (0: by cost, negative: the operands keep their roles) and puts the rule back."""
+    L = _lib()
+    word = torch.zeros(2, dtype=torch.int32, device=DEV)           # bounded waits that run out report here
+    L.qwk_set_error_word(P(word))
+    old = L.qwk_gemm_tc_exchange_nt(0)
+    yield L.qwk_gemm_tc_exchange_nt
+    torch.cuda.synchronize()
+    L.qwk_gemm_tc_exchange_nt(old)
+    L.qwk_set_error_word(None)
+    assert word.tolist() == [0, 0]
+
+
+def _product(T, N, K, dtype, off=0):
+    from qwb200.ops import kernels as K_
+    rn = gen(T + N + K)
+    A, W = rn(T, K).bfloat16(), (rn(N, K) * 0.05).bfloat16()
+    ld = (N + 7) // 8 * 8 + 8
+    flat = torch.full((ld * (T + 2) + 8,), 768.0, dtype=dtype, device=DEV)
+    out = flat[off:off + ld * (T + 2)].view(T + 2, ld)
+    K_.gemm_bf16_tc(A, W, out=out[:T, :N])
+    torch.cuda.synchronize()
+    assert torch.all(out[:, N:].float() == 768.0) and torch.all(out[T:].float() == 768.0) and torch.all(flat[:off].float() == 768.0)
+    return A, W, out[:T, :N]
+
+
+@pytest.mark.parametrize("T,N,K,nt", [(257, 300, 72, 32), (300, 700, 192, 160), (777, 1793, 320, 208), (1021, 2560, 640, 256), (513, 257, 64, 48), (33, 40000, 64, 16),
+                                      (1500, 4304, 136, 96), (3000, 5000, 64, 240)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("off", [0, 1])
+def test_exchanged_operands_give_the_bits_of_the_other_forms(exchange, T, N, K, nt, dtype, off):
+    """Weight rows as the pair's 256 rows, tokens as its columns: tiles that end inside the tokens and the columns, an odd number of columns
+    (two of them leave in one word), outputs off 16 bytes; k is one chain in every form."""
+    exchange(nt)
+    assert _lib().qwk_gemm_tc_exchanged(T, N, K) == nt
+    A, W, got = _product(T, N, K, dtype, off)
+    exchange(-1)
+    assert _lib().qwk_gemm_tc_exchanged(T, N, K) == 0
+    assert torch.equal(got, _product(T, N, K, dtype)[2])
+    ref = A.double() @ W.double().T
+    assert float((got.double() - ref).norm() / ref.norm()) < (1e-5 if dtype == torch.float32 else 2 ** -8)
+
+
+@pytest.mark.parametrize("T,N,K,form", [(520, 12800, 320, 1), (640, 12700, 72, 1), (300, 512, 64, 0), (777, 4352, 64, 2), (1111, 16480, 128, 2)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_forms_that_keep_the_roles_match_64_bits(exchange, T, N, K, form, dtype):
+    """What peers' products, and others where exchanging does not pay, go through."""
+    exchange(-1)
+    assert _lib().qwk_gemm_tc_form(T, N, K) == form
+    A, W, got = _product(T, N, K, dtype)
+    ref = A.double() @ W.double().T
+    assert float((got.double() - ref).norm() / ref.norm()) < (1e-5 if dtype == torch.float32 else 2 ** -8)
+
+
 @pytest.mark.parametrize("M", [33, 63, 65, 129])
 @pytest.mark.parametrize("KL,VL", [(1, 2), (2, 6), (8, 16), (16, 48)])
 def test_chunked_scan_of_ragged_runs_is_as_exact_as_its_operands(M, KL, VL):

@@ -673,13 +673,149 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1) gemm_tc_pair
     tp_signal(a.epi.sig);
 }
 
+// The pair form with the operands' roles exchanged: the pair's 256 rows are weight rows and the tokens the columns, so that a
+// tile is as wide as the tokens want - any multiple of 16 up to 256 - and a prompt whose length is no multiple of 256 is not padded to one.  A
+// lane of the accumulator is an output column: the epilogue's stores are whole 128-byte lines without a staging buffer.  us,
+// roles kept / exchanged: 777 x 16,480 x 2,560 78 / 61, 1,021 x 2,560 x 6,144 45 / 35, 4,096 x 16,480 x 2,560 260 / 235, 4,096 x 2,560 x 6,144
+// 124 / 99, 300 x 2,560 x 6,144 47 / 31.
+// grid as above; a.tiles_t / a.total count tiles of nt tokens x 256 columns.
+template <bool BF16>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1) gemm_tc_exchange_kernel(const __grid_constant__ CUtensorMap mapX,
+                                                                                        const __grid_constant__ CUtensorMap mapW, GemmTcArgs a, int nt) {
+    constexpr int ST = TC_PAIR_STAGES;
+    extern __shared__ unsigned char raw[];
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_ctarank();
+    const int cluster_id = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
+    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023);
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + ST * TC_PAIR_STAGE_BYTES);
+    uint64_t *empty = full + ST, *done = empty + ST, *acc_empty = done + 2;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < ST; ++s) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(done + b, 1); mbar_init(acc_empty + b, 2 * TC_EPI_WARPS); }
+        mbar_fence_init();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_sync_all();                      // both CTAs' barriers exist before anything is sent to them
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tmem_slot;
+    const int kblocks = (a.K + TC_BK - 1) / TC_BK;
+    if (warp == 0) {
+        unsigned it = 0;
+        bool ok = true;
+        for (int id = cluster_id; id < a.total && ok; id += n_clusters) {
+            const int t0 = id % a.tiles_t * nt + (int)rank * (nt >> 1), n0 = id / a.tiles_t * 256 + (int)rank * 128;
+            for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                const unsigned s = it % ST;
+                if (it >= ST && !mbar_wait_warp(empty + s, (it / ST - 1) & 1u, a.err)) { ok = false; break; }
+                if (elect_one()) {
+                    if (rank == 0) mbar_expect_tx(full + s, 2u * (16384u + (unsigned)nt * 64u));
+                    const uint32_t bar = map_to_cta(smem_u32(full + s), 0);
+                    unsigned char *st = smem + s * TC_PAIR_STAGE_BYTES;
+                    tma_load_2d_pair(st, &mapW, kb * TC_BK, n0, bar);
+                    tma_load_2d_pair(st + 16384, &mapX, kb * TC_BK, t0, bar);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {
+            // instruction descriptor: D fp32, A/B bf16, both K-major, N = nt, M = 256 (the pair's rows)
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nt >> 3) << 17) | (16u << 24);
+            int j = 0;
+            unsigned it = 0;
+            bool ok = true;
+            for (int id = cluster_id; id < a.total && ok; id += n_clusters) {
+                const int b = j & 1;
+                if (j >= 2 && !mbar_wait_warp(acc_empty + b, (unsigned)((j >> 1) - 1) & 1u, a.err)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                    const unsigned s = it % ST;
+                    if (!mbar_wait_warp(full + s, (it / ST) & 1u, a.err)) { ok = false; break; }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t sw = smem_u32(smem + s * TC_PAIR_STAGE_BYTES), sx = sw + 16384;
+                    if (elect_one()) {
+#pragma unroll
+                        for (int k = 0; k < TC_BK / 16; ++k)
+                            umma_bf16_pair(tmem + (uint32_t)(b * 256), make_sw128_desc(sw + k * 32), make_sw128_desc(sx + k * 32), idesc, (kb | k) ? 1u : 0u);
+                        umma_commit_pair(empty + s);
+                    }
+                }
+                if (ok && elect_one()) umma_commit_pair(done + b);
+                ++j;
+            }
+        }
+    } else {
+        const int q = warp & 3;
+        const uint32_t acc_bar = map_to_cta(smem_u32(acc_empty), 0);
+        int j = 0;
+        for (int id = cluster_id; id < a.total; id += n_clusters) {
+            const int t0 = id % a.tiles_t * nt, n = id / a.tiles_t * 256 + (int)rank * 128 + q * 32 + lane, b = j & 1;
+            if (!mbar_wait_warp(done + b, (unsigned)(j >> 1) & 1u, a.err)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t acc = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 256);
+#pragma unroll 1
+            for (int c0 = warp >= 6 ? 32 : 0; c0 < nt && t0 + c0 < a.T; c0 += 64) {
+                uint32_t v[2][16];
+                tmem_ld16(acc + c0, v[0]);
+                if (c0 + 16 < nt) tmem_ld16(acc + c0 + 16, v[1]);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                const int rows = min(min(32, nt - c0), a.T - t0 - c0);
+                const long long at = (long long)(t0 + c0) * a.ldc;
+                if (BF16 && a.vec) {
+                    // a lane and its neighbour exchange a token each, so that each writes two columns of one of them
+                    const bool odd = lane & 1, ok = (n | 1) < a.N;
+                    bf16 *o = a.C16 + at + (n & ~1) + (odd ? a.ldc : 0);
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2, o += 2 * a.ldc) {
+                        const uint32_t x = v[i >> 4][i & 15], y = v[i >> 4][(i & 15) + 1], r = __shfl_xor_sync(0xffffffffu, odd ? x : y, 1);
+                        if (i + (odd ? 1 : 0) >= rows) continue;
+                        if (ok) *reinterpret_cast<uint32_t *>(o) = odd ? pack_bf16(__uint_as_float(r), __uint_as_float(y)) : pack_bf16(__uint_as_float(x), __uint_as_float(r));
+                        else if ((n & ~1) < a.N) *o = __float2bfloat16(__uint_as_float(odd ? r : x));
+                    }
+                } else if (n < a.N) {
+                    float *o = a.C32 + at + n;
+                    bf16 *h = a.C16 + at + n;
+                    if (!BF16 && rows == 32) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i, o += a.ldc) *o = __uint_as_float(v[i >> 4][i & 15]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) {
+                            if (i >= rows) break;
+                            if (BF16) h[(long long)i * a.ldc] = __float2bfloat16(__uint_as_float(v[i >> 4][i & 15]));
+                            else o[(long long)i * a.ldc] = __uint_as_float(v[i >> 4][i & 15]);
+                        }
+                    }
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(acc_bar + (uint32_t)(b * 8));
+            ++j;
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_sync_all();                      // nothing is in flight towards either CTA any more
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
 }  // namespace qw
 
 using namespace qw;
 
 // One-time (per device) opt-in to the kernels' dynamic shared memory.
-static bool configure_once(int which) {          // 0 dense 128-wide, 2 dense 256-wide, 3 / 4 the two with a staged epilogue, 5 / 6 the pair form
-    static bool done[7][64] = {};
+static bool configure_once(int which) {          // 0 dense 128-wide, 2 dense 256-wide, 3 / 4 the two with a staged epilogue, 5 / 6 the pair form, 7 / 8 exchanged
+    static bool done[9][64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
@@ -694,6 +830,7 @@ static bool configure_once(int which) {          // 0 dense 128-wide, 2 dense 25
                                                       tc_smem_bytes<TC_WIDE_BN, TC_WIDE_STAGES, true>());
         else if (which == 5) e = cudaFuncSetAttribute(gemm_tc_pair_kernel<TC_PAIR_STAGES, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                       tc_pair_smem_bytes<TC_PAIR_STAGES, false>());
+        else if (which >= 7) e = cudaFuncSetAttribute(which == 7 ? gemm_tc_exchange_kernel<false> : gemm_tc_exchange_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_pair_smem_bytes<TC_PAIR_STAGES, false>());
         else e = cudaFuncSetAttribute(gemm_tc_pair_kernel<TC_PAIR_STG_STAGES, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       tc_pair_smem_bytes<TC_PAIR_STG_STAGES, true>());
         if (e != cudaSuccess) return false;
@@ -713,7 +850,8 @@ static void set_output(GemmTcArgs &a, void *C, int out_bf16, int ldc, long long 
 }
 
 static int g_wide_min_n = 1024;          // products at least this wide may use the 128 x 256 tile form (0: never)
-static int g_pair_min_n = 1024;          // products at least this wide and of more than 128 rows may use CTA pairs (0: never, negative: always)
+constexpr int TC_PAIR_MIN_N = 1024;
+static int g_pair_min_n = TC_PAIR_MIN_N;          // products at least this wide and of more than 128 rows may use CTA pairs (0: never, negative: always)
 static int g_stage_local = 1;            // 1: fp32 output of the wide and pair forms also leaves through the staging buffers
 
 // How many CTAs share a tile: of products of up to 256 rows, whose `tiles` tiles per 128 rows leave most SMs idle (1: none; every
@@ -762,17 +900,41 @@ static int launch_ksplit(int ks, const CUtensorMap &mA, const CUtensorMap &mW, G
 // pairs (a quarter of their tiles' area padding) 76; 520 x 12800 x 2560: wide 49, pairs 57 (a third wave for 2 of 150 tiles).  A last
 // column tile that is mostly padding rules the wide form out.
 enum TcForm { FORM_ONE = 0, FORM_WIDE = 1, FORM_PAIR = 2, FORM_SPLIT = 3 };
-static TcForm form_of(int T, int N, int K, bool peers) {
+static double form_cost(TcForm form, int T, int N) {          // per 64 k values
     auto tiles = [&](int bm, int bn) { return (long long)((T + bm - 1) / bm) * ((N + bn - 1) / bn); };
     auto waves = [](long long n, int at_once) { return (double)((n + at_once - 1) / at_once); };
+    if (form == FORM_PAIR) return 0.45 * waves(tiles(TC_PAIR_BM, TC_PAIR_BN), NUM_SMS / 2);
+    if (form == FORM_WIDE) return 0.55 * waves(tiles(TC_BM, TC_WIDE_BN), NUM_SMS);
+    return 0.31 * waves(tiles(TC_BM, TC_BN), NUM_SMS);
+}
+static TcForm form_of(int T, int N, int K, bool peers) {
     if (!peers && ksplit_of(T, (N + TC_BN - 1) / TC_BN, (K + TC_BK - 1) / TC_BK) > 1) return FORM_SPLIT;
-    const long long n_wide = tiles(TC_BM, TC_WIDE_BN);
-    const double c_one = 0.31 * waves(tiles(TC_BM, TC_BN), NUM_SMS), c_wide = 0.55 * waves(n_wide, NUM_SMS);
-    const double c_pair = 0.45 * waves(tiles(TC_PAIR_BM, TC_PAIR_BN), NUM_SMS / 2);
+    const long long n_wide = (long long)((T + TC_BM - 1) / TC_BM) * ((N + TC_WIDE_BN - 1) / TC_WIDE_BN);
+    const double c_one = form_cost(FORM_ONE, T, N), c_wide = form_cost(FORM_WIDE, T, N), c_pair = form_cost(FORM_PAIR, T, N);
     const bool wide_ok = g_wide_min_n > 0 && N >= g_wide_min_n && (N % TC_WIDE_BN == 0 || N % TC_WIDE_BN > TC_BN);
     const bool pair_ok = g_pair_min_n && N >= abs(g_pair_min_n) && T > TC_BM;
     if (pair_ok && (g_pair_min_n < 0 || (c_pair < c_one && (!wide_ok || c_pair < c_wide)))) return FORM_PAIR;
     return wide_ok && n_wide >= NUM_SMS / 2 && c_wide < c_one ? FORM_WIDE : FORM_ONE;
+}
+
+// Tokens of a tile of the pair form with the operands exchanged, or 0 where that form does not pay (or cannot be: peers' products keep their
+// roles).  What a tile of nt tokens costs, by the same measure: 0.07 + 0.00127 nt us, at least 0.21 (256 tokens 0.395, 208 0.33, 160 0.26, 96
+// 0.21; 4,096 x 16,480 x 2,560 in tiles of 96 to 256 tokens: 315, 266 (128), 242 (160), 235 (208), 237 us (256), and 260 with the roles kept).  The
+// widest of equally cheap tiles is taken: it reads the least.  A caller that moves the line of the pairs measures the forms that keep the roles.
+static int g_exchange_nt = 0;            // 0: by cost; > 0: that many; < 0: never (measurements and tests)
+static int exchanged_tile(int T, int N, int K) {
+    if (g_exchange_nt < 0 || g_pair_min_n != TC_PAIR_MIN_N) return 0;
+    const TcForm form = form_of(T, N, K, false);
+    if (form == FORM_SPLIT) return 0;
+    if (g_exchange_nt > 0) return g_exchange_nt;
+    auto cost = [&](int nt) {
+        const long long n = (long long)((T + nt - 1) / nt) * ((N + 255) / 256), pairs = NUM_SMS / 2;
+        return (double)((n + pairs - 1) / pairs) * fmax(0.207, 0.07 + 0.00127 * nt);
+    };
+    int best = 256;
+    for (int nt = 240; nt >= 32; nt -= 16)
+        if (cost(nt) < cost(best)) best = nt;
+    return cost(best) < form_cost(form, T, N) ? best : 0;
 }
 
 static int gemm_plain(GemmTcArgs &a, const void *A, const void *W, void *C, int T, int N, int K, int lda, int ldw, int ldc,
@@ -790,6 +952,20 @@ static int gemm_plain(GemmTcArgs &a, const void *A, const void *W, void *C, int 
         a.tiles_t = tiles_t; a.tiles_n = (N + TC_BN - 1) / TC_BN; a.total = a.tiles_t * a.tiles_n;
         a.ksplit = 1; a.kb_per = 0;
         return launch_ksplit(ks, mA, mW, a, s);
+    }
+    if (const int nt = a.mix_xn || a.epi.mode || a.wait.flags ? 0 : exchanged_tile(T, N, K)) {
+        CUtensorMap mX, mW;
+        if (!make_map(&mX, A, T, K, lda, nt / 2) || !make_map(&mW, W, N, K, ldw, 128)) return -3;
+        set_output(a, C, out_bf16, ldc);
+        a.T = T; a.N = N; a.K = K; a.err = g_err_ptr; a.tiles = nullptr;
+        a.tiles_t = (T + nt - 1) / nt; a.tiles_n = (N + 255) / 256; a.total = a.tiles_t * a.tiles_n;
+        a.ksplit = 1; a.kb_per = 0;
+        if (!configure_once(out_bf16 ? 8 : 7)) return -3;
+        const unsigned sm_pairs = persistent_grid(1 << 30, 1) / 2, clusters = (unsigned)a.total < sm_pairs ? (unsigned)a.total : sm_pairs;
+        constexpr int smem = tc_pair_smem_bytes<TC_PAIR_STAGES, false>();
+        if (out_bf16) gemm_tc_exchange_kernel<true><<<2 * clusters, 320, smem, s>>>(mX, mW, a, nt);
+        else gemm_tc_exchange_kernel<false><<<2 * clusters, 320, smem, s>>>(mX, mW, a, nt);
+        return cudaGetLastError() == cudaSuccess ? 0 : -2;
     }
     if (form == FORM_PAIR) {
         CUtensorMap mA, mW;
@@ -851,7 +1027,16 @@ QW_API int qwk_gemm_tc_pair_min_n(int min_n) {
     return old;
 }
 
-// The form that qwk_gemm_bf16_tc takes: 0 128 x 128 tiles, 1 128 x 256, 2 CTA pairs, 3 tiles split over a cluster.
+// Tokens of an exchanged tile, a multiple of 16 up to 256 (0: by cost; negative: the form is not used; measurements and tests).
+QW_API int qwk_gemm_tc_exchange_nt(int nt) {
+    const int old = g_exchange_nt;
+    g_exchange_nt = nt;
+    return old;
+}
+// Tokens per tile where qwk_gemm_bf16_tc exchanges the operands, 0 where it keeps their roles.
+QW_API int qwk_gemm_tc_exchanged(int T, int N, int K) { return exchanged_tile(T, N, K); }
+
+// The form of a product whose operands keep their roles: 0 128 x 128 tiles, 1 128 x 256, 2 CTA pairs, 3 tiles split over a cluster.
 QW_API int qwk_gemm_tc_form(int T, int N, int K) { return form_of(T, N, K, false); }
 
 // C = A . W^T.  A bf16 [T][lda], W bf16 [N][ldw], C fp32 (out_bf16 = 0) or bf16 [T][ldc].

@@ -23,6 +23,8 @@ int qwk_gdn_scan_chunked(const float *qkv, const float *decay, const float *beta
 int qwk_gemm_tc_wide_min_n(int min_n);
 int qwk_gemm_tc_stage_local(int on);
 int qwk_gemm_tc_pair_min_n(int min_n);
+int qwk_gemm_tc_exchange_nt(int nt);
+int qwk_gemm_tc_exchanged(int T, int N, int K);
 int qwk_gemm_tc_form(int T, int N, int K);
 int qwk_gemm_bf16_tc(const void *A, const void *W, void *C, int T, int N, int K, int lda, int ldw, int ldc, int out_bf16, cudaStream_t s);
 int qwk_gemm_bf16_tc_tp(void *tp_, const void *A, const void *W, void *C, int T, int N, int K, int lda, int ldw, int ldc, int out_bf16, int wait_kind, int epi_mode, int epi_kind, int ld_epi, cudaStream_t s);
