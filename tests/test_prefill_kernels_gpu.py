@@ -64,6 +64,24 @@ def test_forms_that_keep_the_roles_match_64_bits(exchange, T, N, K, form, dtype)
     assert float((got.double() - ref).norm() / ref.norm()) < (1e-5 if dtype == torch.float32 else 2 ** -8)
 
 
+@pytest.mark.parametrize("L,heads", [(128, 1), (129, 2), (600, 16), (2100, 3), (3520, 16)])
+def test_vision_attention_with_its_keys_dealt_evenly(L, heads):
+    """Runs that begin and end inside a unit's keys, units in two and more runs, a last key tile that is not whole: against 64 bits (weights and
+    output rounded to bf16: 2^-8) and no further from them than 1.05 times what whole units give."""
+    lib = _lib()
+    rn = gen(L + heads)
+    qkv = rn(L, 3 * heads * 72).bfloat16()
+    need = lib.qwk_vit_attention_scratch(L, heads)
+    parts = torch.full((max(need, 16),), 255, dtype=torch.uint8, device=DEV)          # NaN where nothing is written
+    outs = [torch.zeros(L, heads * 72, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+    assert lib.qwk_vit_attention_split(P(qkv), L, heads, P(outs[0]), P(parts) if need else None, S()) == 0
+    assert lib.qwk_vit_attention(P(qkv), L, heads, P(outs[1]), S()) == 0
+    q, k, v = (t.view(L, heads, 72).transpose(0, 1).double() for t in qkv.split(heads * 72, 1))
+    want = torch.cat([(torch.softmax(q[h] @ k[h].T / 72 ** 0.5, -1) @ v[h]) for h in range(heads)], 1)
+    err = [float((o.double() - want).norm() / want.norm()) for o in outs]
+    assert err[0] < 2 ** -8 and err[0] < 1.05 * err[1] + 1e-6
+
+
 @pytest.mark.parametrize("M", [33, 63, 65, 129])
 @pytest.mark.parametrize("KL,VL", [(1, 2), (2, 6), (8, 16), (16, 48)])
 def test_chunked_scan_of_ragged_runs_is_as_exact_as_its_operands(M, KL, VL):

@@ -135,6 +135,8 @@ int qwk_vit_bias_gelu(void *y, const float *bias, int L, int D, int tanh_form, c
 int qwk_vit_residual_add(float *x, const float *y, const float *bias, int L, int D, int assign, cudaStream_t s);
 
 // vit_attn.cu
+int qwk_vit_attention_scratch(int L, int heads);
+int qwk_vit_attention_split(const void *qkv, int L, int heads, void *out, void *parts, cudaStream_t s);
 int qwk_vit_attention(const void *qkv, int L, int heads, void *out, cudaStream_t s);
 
 }  // extern "C"

@@ -15,8 +15,10 @@
 // Head dim 72 = 64 + 8: a row's first 64 values are a 128B-swizzled panel, the last 8 a panel of 16-byte rows whose partner (the
 // other 8 of an MMA's k = 16) is a zeroed block.  V is read as it lies (key-major): 64 + 64 columns, of which the second panel's
 // first 8 count; the rest belongs to other heads and lands in columns of O that nobody reads.
-// What bounds it: the exponentials (128 x 128 per tile at 16 a cycle and SM: 1024 cycles; MMAs 780), and 224 units on 148 SMs for
-// 3520 patches and 16 heads.  It replaces a flash kernel on mma.sync (16 queries a warp, each warp reading every K and V fragment
+// The units' key tiles are dealt to the CTAs in equal runs (VitSplit) where whole units would leave SMs idle: 3520 patches and 16 heads are 224
+// units, one and a half for each of 148 SMs.  A run that does not hold all of a unit's keys leaves its O, reference and sum, and a second kernel
+// merges them: 129 us whole, 108 + 12 dealt.
+// What bounds it: the exponentials (128 x 128 per tile at 16 a cycle and SM: 1024 cycles; MMAs 780).  It replaces a flash kernel on mma.sync (16 queries a warp, each warp reading every K and V fragment
 // from shared memory), which took 444 us there; this one takes 119.
 #include "tc.cuh"
 
@@ -27,8 +29,28 @@ constexpr int VT_KA = 128 * 128, VT_KB = 128 * 16, VT_K = VT_KA + 2 * VT_KB;    
 constexpr int VT_V = 2 * 128 * 128;
 constexpr int VT_SMEM = 2 * VT_K + VT_STAGES * (VT_K + VT_V) + 1024 + 512;
 
+constexpr int VT_PART = 76;                      // floats of a row of a part: 72 of O, reference, sum
+
+// The key tiles of all units one after another, dealt to `ctas` CTAs in equal runs; a run's piece of one unit is a segment.
+struct VitSplit {
+    int ktiles, units, ctas, whole;              // whole: runs begin and end with a unit
+    __host__ __device__ long long first(int c) const {
+        return whole ? (long long)units * c / ctas * ktiles : (long long)units * ktiles * c / ctas;
+    }
+};
+struct VitSeg {
+    int unit, k0, len;
+    __device__ __forceinline__ VitSeg(const VitSplit &s, long long at, long long end) {
+        unit = (int)(at / s.ktiles);
+        k0 = (int)(at - (long long)unit * s.ktiles);
+        len = (int)min((long long)(s.ktiles - k0), end - at);
+    }
+};
+
 struct VitAttnArgs {
     int L, heads, qtiles;
+    VitSplit split;
+    float *parts;            // [CTA][first segment | last][256][VT_PART]
     bf16 *out;
     float scale;             // log2(e) / sqrt(72)
     ErrorWord *err;
@@ -71,12 +93,15 @@ __global__ void __launch_bounds__(VT_THREADS, 1) vit_attn_tc_kernel(const __grid
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
-    const int units = a.qtiles * a.heads, ktiles = (a.L + 127) >> 7, D = a.heads * VT_D;
+    const int ktiles = a.split.ktiles, D = a.heads * VT_D;
+    const long long from = a.split.first(blockIdx.x), to = a.split.first(blockIdx.x + 1);
     if (warp == 0) {
         unsigned it = 0, u = 0;
         bool ok = true;
-        for (int id = blockIdx.x; id < units && ok; id += gridDim.x, ++u) {
-            const int h = id / a.qtiles, q0 = (id % a.qtiles) * 256, col = h * VT_D;
+        for (long long at = from; at < to && ok; ++u) {
+            const VitSeg g(a.split, at, to);
+            at += g.len;
+            const int h = g.unit / a.qtiles, q0 = (g.unit % a.qtiles) * 256, col = h * VT_D;
             if (u && !mg_wait_warp(q_empty, (u - 1) & 1u, a.err)) break;
             if (elect_one()) {
                 mbar_expect_tx(q_full, 2 * (VT_KA + VT_KB));
@@ -85,7 +110,7 @@ __global__ void __launch_bounds__(VT_THREADS, 1) vit_attn_tc_kernel(const __grid
                     tma_load_2d(sq + t * VT_K + VT_KA, &mapB, col + 64, q0 + t * 128, q_full);
                 }
             }
-            for (int j = 0; j < ktiles; ++j, ++it) {
+            for (int j = g.k0; j < g.k0 + g.len; ++j, ++it) {
                 const unsigned s = it % VT_STAGES, ph = (it / VT_STAGES - 1) & 1u;
                 if (it >= VT_STAGES && !mg_wait_warp(k_empty + s, ph, a.err)) { ok = false; break; }
                 if (elect_one()) {
@@ -117,15 +142,17 @@ __global__ void __launch_bounds__(VT_THREADS, 1) vit_attn_tc_kernel(const __grid
                 if (t) umma_commit(k_empty + st);
             }
         };
-        for (int id = blockIdx.x; id < units && ok; id += gridDim.x, ++u) {
+        for (long long at = from; at < to && ok; ++u) {
+            const int len = VitSeg(a.split, at, to).len;
+            at += len;
             if (!mg_wait_warp(q_full, u & 1u, a.err) || !mg_wait_warp(k_full + it % VT_STAGES, (it / VT_STAGES) & 1u, a.err)) break;
             // the scores of a new unit overwrite probabilities that the last products of the old one read: same pipe, in order
             issue_s(0, it % VT_STAGES);
             issue_s(1, it % VT_STAGES);
-            if (ktiles == 1 && elect_one()) umma_commit(q_empty);
-            for (int j = 0; j < ktiles && ok; ++j, ++it) {
+            if (len == 1 && elect_one()) umma_commit(q_empty);
+            for (int j = 0; j < len && ok; ++j, ++it) {
                 const unsigned s = it % VT_STAGES, sn = (it + 1) % VT_STAGES;
-                const bool more = j + 1 < ktiles;
+                const bool more = j + 1 < len;
                 if (more && !mg_wait_warp(k_full + sn, ((it + 1) / VT_STAGES) & 1u, a.err)) { ok = false; break; }
                 if (!mg_wait_warp(v_full + s, (it / VT_STAGES) & 1u, a.err)) { ok = false; break; }
                 for (int t = 0; t < 2; ++t) {
@@ -142,7 +169,7 @@ __global__ void __launch_bounds__(VT_THREADS, 1) vit_attn_tc_kernel(const __grid
                     }
                     if (more) issue_s(t, sn);
                 }
-                if (ok && j + 2 == ktiles && elect_one()) umma_commit(q_empty);      // the last scores of this unit are under way
+                if (ok && j + 2 == len && elect_one()) umma_commit(q_empty);      // the last scores of this unit are under way
             }
         }
     } else if (warp >= 4) {
@@ -151,18 +178,21 @@ __global__ void __launch_bounds__(VT_THREADS, 1) vit_attn_tc_kernel(const __grid
         const uint32_t sbase = lane_base + t * 128u, obase = lane_base + 256u + t * 80u;
         unsigned it = 0, u = 0;
         bool ok = true;
-        for (int id = blockIdx.x; id < units && ok; id += gridDim.x, ++u) {
-            const int h = id / a.qtiles, row = (id % a.qtiles) * 256 + t * 128 + q * 32 + lane;
+        for (long long at = from; at < to && ok; ++u) {
+            const VitSeg g(a.split, at, to);
+            const bool begins = at == from;
+            at += g.len;
+            const int h = g.unit / a.qtiles, r256 = t * 128 + q * 32 + lane, row = (g.unit % a.qtiles) * 256 + r256;
             float ref = 0.f, sum = 0.f;
-            for (int j = 0; j < ktiles; ++j, ++it) {
+            for (int j = 0; j < g.len; ++j, ++it) {
                 if (!mg_wait_warp(s_full + t, it & 1u, a.err)) { ok = false; break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 uint32_t s[4][32];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) tmem_ld32_nowait(sbase + c * 32, s[c]);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (j + 1 == ktiles) {
-                    const int left = a.L - j * 128;
+                if (g.k0 + j + 1 == ktiles) {
+                    const int left = a.L - (g.k0 + j) * 128;
 #pragma unroll
                     for (int c = 0; c < 128; ++c)
                         if (c >= left) s[c >> 5][c & 31] = 0xff800000u;      // -inf
@@ -214,22 +244,36 @@ __global__ void __launch_bounds__(VT_THREADS, 1) vit_attn_tc_kernel(const __grid
             }
             if (!ok || !mg_wait_warp(o_full + t, u & 1u, a.err)) { ok = false; break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const float r = 1.f / sum;
-            bf16 *o = a.out + (long long)row * D + h * VT_D;
+            if (g.len < ktiles) {                        // a part: as it is, with what the merge needs
+                float *o = a.parts + ((long long)(blockIdx.x * 2 + (begins ? 0 : 1)) * 256 + r256) * VT_PART;
 #pragma unroll
-            for (int c = 0; c < 80; c += 16) {
-                uint32_t v[16];
-                tmem_ld16(obase + c, v);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                for (int c = 0; c < 80; c += 16) {
+                    uint32_t v[16];
+                    tmem_ld16(obase + c, v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int i = 0; i < 16; i += 8) {
-                    if (c + i >= VT_D || row >= a.L) continue;
-                    uint4 pk;
-                    pk.x = pack_bf16(__uint_as_float(v[i]) * r, __uint_as_float(v[i + 1]) * r);
-                    pk.y = pack_bf16(__uint_as_float(v[i + 2]) * r, __uint_as_float(v[i + 3]) * r);
-                    pk.z = pack_bf16(__uint_as_float(v[i + 4]) * r, __uint_as_float(v[i + 5]) * r);
-                    pk.w = pack_bf16(__uint_as_float(v[i + 6]) * r, __uint_as_float(v[i + 7]) * r);
-                    *reinterpret_cast<uint4 *>(o + c + i) = pk;
+                    for (int i = 0; i < 16; i += 4)
+                        if (c + i < VT_D) *reinterpret_cast<uint4 *>(o + c + i) = make_uint4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+                }
+                *reinterpret_cast<float4 *>(o + VT_D) = make_float4(ref, sum, 0.f, 0.f);
+            } else {
+                const float r = 1.f / sum;
+                bf16 *o = a.out + (long long)row * D + h * VT_D;
+    #pragma unroll
+                for (int c = 0; c < 80; c += 16) {
+                    uint32_t v[16];
+                    tmem_ld16(obase + c, v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    #pragma unroll
+                    for (int i = 0; i < 16; i += 8) {
+                        if (c + i >= VT_D || row >= a.L) continue;
+                        uint4 pk;
+                        pk.x = pack_bf16(__uint_as_float(v[i]) * r, __uint_as_float(v[i + 1]) * r);
+                        pk.y = pack_bf16(__uint_as_float(v[i + 2]) * r, __uint_as_float(v[i + 3]) * r);
+                        pk.z = pack_bf16(__uint_as_float(v[i + 4]) * r, __uint_as_float(v[i + 5]) * r);
+                        pk.w = pack_bf16(__uint_as_float(v[i + 6]) * r, __uint_as_float(v[i + 7]) * r);
+                        *reinterpret_cast<uint4 *>(o + c + i) = pk;
+                    }
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -245,14 +289,65 @@ __global__ void __launch_bounds__(VT_THREADS, 1) vit_attn_tc_kernel(const __grid
     }
 }
 
+// Units whose keys lie in several CTAs' runs: O = sum of the parts' O, each relative to the largest reference, over the sum of their sums.
+// grid (18, units), 256 threads: a thread per row and four columns.
+__global__ void __launch_bounds__(256) vit_merge_kernel(VitAttnArgs a) {
+    const int unit = blockIdx.y, i = blockIdx.x * 256 + threadIdx.x, r = i / (VT_D / 4), c = (i - r * (VT_D / 4)) * 4;
+    // 32-bit arithmetic: the launcher checks that units x key tiles x CTAs fit
+    const int kt = a.split.ktiles, G = a.split.ctas, total = a.split.units * kt, lo = unit * kt, hi = lo + kt;
+    auto first = [&](int c) { return (int)((unsigned)total * (unsigned)c / (unsigned)G); };
+    int c0 = (int)((unsigned)lo * (unsigned)G / (unsigned)total);                 // the run that holds the unit's first key tile
+    while (first(c0 + 1) <= lo) ++c0;
+    while (first(c0) > lo) --c0;
+    int f0 = first(c0), f1 = first(c0 + 1);
+    if (f1 >= hi) return;                                // one run holds them all: done
+    const int h = unit / a.qtiles, row = (unit % a.qtiles) * 256 + r;
+    if (row >= a.L) return;
+    float m = -1e30f, sum = 0.f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int k = c0; f0 < hi; ++k, f0 = f1, f1 = first(k + 1)) {
+        const float *p = a.parts + ((long long)(k * 2 + (f0 >= lo ? 0 : 1)) * 256 + r) * VT_PART;
+        const float2 rs = *reinterpret_cast<const float2 *>(p + VT_D);
+        const float4 v = *reinterpret_cast<const float4 *>(p + c);
+        const float nm = fmaxf(m, rs.x), f = exp2f(m - nm), w = exp2f(rs.x - nm);
+        m = nm;
+        sum = sum * f + rs.y * w;
+        o.x = o.x * f + v.x * w; o.y = o.y * f + v.y * w; o.z = o.z * f + v.z * w; o.w = o.w * f + v.w * w;
+    }
+    const float inv = 1.f / sum;
+    *reinterpret_cast<uint2 *>(a.out + (long long)row * a.heads * VT_D + h * VT_D + c) =
+        make_uint2(pack_bf16(o.x * inv, o.y * inv), pack_bf16(o.z * inv, o.w * inv));
+}
+
 }  // namespace qw
 
 using namespace qw;
 
-// qkv [L][3 * heads * 72] bf16 (bias and rotary applied) -> out [L][heads * 72] bf16.  qkv and out 16-byte aligned.
-QW_API int qwk_vit_attention(const void *qkv, int L, int heads, void *out, cudaStream_t s) {
+// How the key tiles are dealt: whole units where their waves fill the SMs to nine tenths, else equal runs of at least two tiles.  (The
+// merge costs a tenth of 224 units: what two waves that are three quarters full lose is twice that.)
+static VitSplit vit_split(int L, int heads, bool parts) {
+    VitSplit s;
+    s.ktiles = (L + 127) / 128;
+    s.units = (L + 255) / 256 * heads;
+    const int sms = (int)persistent_grid(1 << 30, 1), waves = (s.units + sms - 1) / sms;
+    const long long runs = (long long)s.units * s.ktiles / 2;
+    s.whole = !parts || (long long)s.units * s.ktiles * sms >= (1LL << 32) || 10LL * s.units >= 9LL * waves * sms || runs <= s.units;
+    s.ctas = s.whole ? (s.units < sms ? s.units : sms) : (int)(runs < sms ? runs : sms);
+    return s;
+}
+
+// Bytes of scratch that let qwk_vit_attention deal a slice's keys evenly (0: it deals whole units anyway).
+QW_API int qwk_vit_attention_scratch(int L, int heads) {
+    if (L <= 0 || heads <= 0) return 0;
+    const VitSplit s = vit_split(L, heads, true);
+    return s.whole ? 0 : s.ctas * 2 * 256 * VT_PART * 4;
+}
+
+// qkv [L][3 * heads * 72] bf16 (bias and rotary applied) -> out [L][heads * 72] bf16.  qkv, out and parts 16-byte aligned; parts: scratch of
+// qwk_vit_attention_scratch bytes, or null.
+QW_API int qwk_vit_attention_split(const void *qkv, int L, int heads, void *out, void *parts, cudaStream_t s) {
     if (L <= 0) return 0;
-    if (((uintptr_t)qkv & 15) || ((uintptr_t)out & 15) || heads <= 0) return -1;
+    if (((uintptr_t)qkv & 15) || ((uintptr_t)out & 15) || ((uintptr_t)parts & 15) || heads <= 0) return -1;
     static bool done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -266,7 +361,13 @@ QW_API int qwk_vit_attention(const void *qkv, int L, int heads, void *out, cudaS
     if (!make_map(&mA, qkv, L, ld, ld, 128) || !make_map(&mB, qkv, L, ld, ld, 128, MAP_BF16_X8)) return -3;
     VitAttnArgs a{};
     a.L = L; a.heads = heads; a.qtiles = (L + 255) / 256; a.out = (bf16 *)out; a.err = g_err_ptr;
+    a.split = vit_split(L, heads, parts != nullptr);
+    a.parts = (float *)parts;
     a.scale = 1.4426950408889634f / sqrtf((float)VT_D);
-    vit_attn_tc_kernel<<<persistent_grid(a.qtiles * heads, 1), VT_THREADS, VT_SMEM, s>>>(mA, mB, a);
+    vit_attn_tc_kernel<<<a.split.ctas, VT_THREADS, VT_SMEM, s>>>(mA, mB, a);
+    if (!a.split.whole) vit_merge_kernel<<<dim3(VT_D / 4, a.split.units), 256, 0, s>>>(a);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
+
+// Without scratch.
+QW_API int qwk_vit_attention(const void *qkv, int L, int heads, void *out, cudaStream_t s) { return qwk_vit_attention_split(qkv, L, heads, out, nullptr, s); }

@@ -148,6 +148,7 @@ class VisionEncoder:
         self.m_fc1, self.m_fc1_b = mat("merger.linear_fc1.weight"), vec("merger.linear_fc1.bias")
         self.m_fc2, self.m_fc2_b = mat("merger.linear_fc2.weight"), vec("merger.linear_fc2.bias")
         self.cap = 0
+        self.parts = None
         self.bytes = sum(t.numel() * t.element_size() for b in self.blocks for t in b.values())
 
     @classmethod
@@ -193,6 +194,10 @@ class VisionEncoder:
         pos, idx, wts = slice_positions(h, w, c.merge, c.grid_side)
         pos_d, idx_d, wts_d = (torch.from_numpy(a).to(self.dev) for a in (pos, idx, wts))
         pin = torch.as_tensor(patches).to(self.dev, torch.bfloat16).contiguous()
+        need = lib.qwk_vit_attention_scratch(L, c.heads)
+        if need and (self.parts is None or self.parts.numel() < need):
+            self.parts = torch.empty(need, dtype=torch.uint8, device=self.dev)
+        parts = _p(self.parts) if need else None
         x, y, xn, qkv, att = self.x[:L], self.y[:L], self.xn[:L], self.qkv[:L], self.att[:L]
         D = c.dim
         self._gemm(pin, self.patch_w, y)
@@ -204,7 +209,7 @@ class VisionEncoder:
             self.check(lib.qwk_vit_layernorm(_p(x), *pend, _p(b["norm1.weight"]), _p(b["norm1.bias"]), L, D, C.c_float(c.eps), _p(xn), s), "vit_ln")
             self._gemm(xn, b["attn.qkv.weight"], qkv)
             self.check(lib.qwk_vit_bias_rope(_p(qkv), _p(b["attn.qkv.bias"]), _p(tab), L, c.heads, s), "vit_rope")
-            self.check(lib.qwk_vit_attention(_p(qkv), L, c.heads, _p(att), s), "vit_attention")
+            self.check(lib.qwk_vit_attention_split(_p(qkv), L, c.heads, _p(att), parts, s), "vit_attention")
             self._gemm(att, b["attn.proj.weight"], y)
             self.check(lib.qwk_vit_layernorm(_p(x), _p(y), _p(b["attn.proj.bias"]), _p(b["norm2.weight"]), _p(b["norm2.bias"]), L, D,
                                              C.c_float(c.eps), _p(xn), s), "vit_ln")
