@@ -103,3 +103,19 @@ def test_chunked_scan_of_ragged_runs_is_as_exact_as_its_operands(M, KL, VL):
         want, Sw = scan_sequential(*a)
         assert float((raw[:, h].double().cpu() - want).norm() / want.norm()) < 1.5e-3
         assert float((St[0, h].double().cpu() - Sw).norm() / Sw.norm()) < 1.5e-3
+
+
+@pytest.mark.parametrize("T,H,k,off,shared", [(3, 2560, 10, 0, True), (5, 516, 3, 0, True), (4, 510, 7, 0, False), (4, 512, 5, 1, True), (33, 8, 11, 0, False)])
+def test_combined_experts_of_any_width_and_address(T, H, k, off, shared):
+    """Four columns at a time or one, experts of other ranks left out: the sums of the same products in the same order."""
+    rn = gen(T + H)
+    flat = torch.zeros(T * k * H + 8, device=DEV)
+    y = flat[off:off + T * k * H].view(T * k, H)
+    y.copy_(rn(T * k, H))
+    inv = torch.randperm(T * k, device=DEV).int().view(T, k)
+    inv[0, 0] = -1
+    w, sh, out = rn(T, k), rn(T, H), torch.zeros(T, H, device=DEV)
+    assert _lib().qwk_moe_combine_T(P(y), H, P(inv), P(w), k, P(sh) if shared else None, H, P(out), T, S()) == 0
+    rows = torch.where((inv >= 0)[..., None], y[inv.long().clamp(min=0)], torch.zeros((), device=DEV))
+    want = (rows.double() * w[..., None].double()).sum(1) + (sh.double() if shared else 0)
+    assert float((out.double() - want).norm() / want.norm()) < 1e-6

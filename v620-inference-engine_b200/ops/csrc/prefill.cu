@@ -165,6 +165,39 @@ __global__ void swiglu_T_kernel(const bf16 *h13, int F, bf16 *h, long long total
 }
 
 // out[t][c] = sum_j w[t][j] * y[inv[t*top_k + j]][c] + shared[t][c].  inv maps a pair to its expert-sorted row (-1: none).
+// Four columns per thread, the rows of five experts on their way at once.  4,096 tokens x 2,560 x 10: one column and one row behind the other
+// 135 us, so 71.  grid (T, ceil(H / 512)), 128 threads.
+__global__ void __launch_bounds__(128) moe_combine4_T_kernel(const float *y, int ld_y, const int *inv, const float *pair_w, int top_k,
+                                                             const float *shared, int H, float *out) {
+    const long long t = blockIdx.x;
+    const int c = (blockIdx.y * 128 + threadIdx.x) * 4;
+    if (c >= H) return;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), sh = acc;
+    if (shared) sh = *reinterpret_cast<const float4 *>(shared + t * H + c);
+    for (int j0 = 0; j0 < top_k; j0 += 5) {
+        float4 v[5];
+        float w[5];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+            const int r = j0 + j < top_k ? inv[t * top_k + j0 + j] : -1;
+            w[j] = 0.f;
+            if (r >= 0) {
+                w[j] = pair_w[t * top_k + j0 + j];
+                v[j] = __ldcs(reinterpret_cast<const float4 *>(y + (long long)r * ld_y + c));
+            } else {
+                v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 5; ++j) {
+            acc.x = fmaf(w[j], v[j].x, acc.x); acc.y = fmaf(w[j], v[j].y, acc.y);
+            acc.z = fmaf(w[j], v[j].z, acc.z); acc.w = fmaf(w[j], v[j].w, acc.w);
+        }
+    }
+    if (shared) { acc.x += sh.x; acc.y += sh.y; acc.z += sh.z; acc.w += sh.w; }
+    *reinterpret_cast<float4 *>(out + t * H + c) = acc;
+}
+// Any width and address.
 __global__ void moe_combine_T_kernel(const float *y, int ld_y, const int *inv, const float *pair_w, int top_k, const float *shared,
                                      int H, float *out, long long total) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -213,7 +246,8 @@ QW_API int qwk_swiglu_T(const void *h13, int F, void *h, long long P, cudaStream
 QW_API int qwk_moe_combine_T(const float *y, int ld_y, const int *inv, const float *pair_w, int top_k, const float *shared,
                              int H, float *out, int T, cudaStream_t s) {
     const long long total = (long long)T * H;
-    moe_combine_T_kernel<<<blocks_for(total, 256), 256, 0, s>>>(y, ld_y, inv, pair_w, top_k, shared, H, out, total);
+    if (((H | ld_y) & 3) == 0 && aligned16(y, shared, out)) moe_combine4_T_kernel<<<dim3(T, (H + 511) / 512), 128, 0, s>>>(y, ld_y, inv, pair_w, top_k, shared, H, out);
+    else moe_combine_T_kernel<<<blocks_for(total, 256), 256, 0, s>>>(y, ld_y, inv, pair_w, top_k, shared, H, out, total);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
