@@ -119,3 +119,38 @@ def test_combined_experts_of_any_width_and_address(T, H, k, off, shared):
     rows = torch.where((inv >= 0)[..., None], y[inv.long().clamp(min=0)], torch.zeros((), device=DEV))
     want = (rows.double() * w[..., None].double()).sum(1) + (sh.double() if shared else 0)
     assert float((out.double() - want).norm() / want.norm()) < 1e-6
+
+
+@pytest.mark.parametrize("base,M", [(0, 64), (3, 61), (257, 70)])
+def test_attention_inputs_of_a_chunk_equal_the_step_kernels(base, M):
+    """More than 32 rows take a block per row and a warp per head: queries, keys, values, indexer queries, compressed keys and the raw-key ring
+    are those of the same rows in pieces of at most 32, bit for bit; behind the last row zeros up to the next multiple of 16."""
+    lib = _lib()
+    QL, KVL, IH, ratio, page, rope = 6, 2, 4, 4, 256, 64
+    assert lib.qwk_rope_init(C.c_double(1e6), rope) == 0
+    rn = gen(M + base)
+    ld = QL * 512 + 2 * KVL * 256 + IH * 128 + 128
+    proj = rn(M, ld)
+    w = [1 + 0.1 * rn(n) for n in (256, 256, 128, 128)]
+    pages = (base + M + page - 1) // page + 1
+    table = torch.arange(pages, dtype=torch.int32, device=DEV)
+    ring0 = rn(1, 16, 128)
+
+    def run(pieces, entry):
+        out = dict(k=torch.full((pages * page, KVL * 256), 3.0, dtype=torch.bfloat16, device=DEV), q=torch.zeros(M, QL, 256, device=DEV),
+                   iq=torch.zeros(M, IH, 128, device=DEV), ring=ring0.clone(), ck=torch.zeros(1, (base + M) // ratio + 1, 128, dtype=torch.bfloat16, device=DEV))
+        out["v"] = out["k"].clone()
+        for m0, n in pieces:
+            lens = [n] + [0] * (n - 1)
+            t = [i32([0] * n), i32([base + m0 + i for i in range(n)]), i32([0] * n), i32(lens)]
+            assert getattr(lib, entry)(P(proj[m0:]), ld, QL, KVL, IH, *map(P, w), n, *map(P, t), P(out["k"]), P(out["v"]), None, None, pages, P(table), pages,
+                                       P(out["q"][m0:]), P(out["iq"][m0:]), P(out["ring"]), P(out["ck"]), out["ck"].shape[1], ratio, C.c_float(1e-6), S()) == 0
+            torch.cuda.synchronize()
+        return out
+
+    a, b = run([(0, M)], "qwk_qsa_prep_run"), run([(m, min(32, M - m)) for m in range(0, M, 32)], "qwk_qsa_prep")
+    end, tail = base + M, (base + M + 15) // 16 * 16
+    for key in ("q", "iq", "ring", "ck"):
+        assert torch.equal(a[key], b[key]), key
+    for key in ("k", "v"):
+        assert torch.equal(a[key][:end], b[key][:end]) and torch.equal(a[key][tail:], b[key][tail:]) and torch.all(a[key][end:tail] == 0), key

@@ -10,6 +10,8 @@
 // KV pages: a page holds KV_PAGE tokens of one layer, row = KVL*256 bf16.  page ids < n_dev_pages
 // live in the device pool, the rest in the host pool (pinned, mapped: the kernels read host RAM
 // directly).  page_table[slot][i] is the page of tokens i*KV_PAGE ...
+#include <type_traits>
+
 #include "common.cuh"
 #include "mma.cuh"
 
@@ -248,6 +250,115 @@ __global__ void __launch_bounds__(256) qsa_prep_kernel(QsaPrepArgs a) {
         const float v = norm_rope<ID>(mean, sm, scratch, cs, a.ikn1, a.eps, d);
         const int g = pos / a.ratio;
         if (d < ID && g < a.ck_cap) a.ck[((long long)slot * a.ck_cap + g) * ID + d] = __float2bfloat16(v);
+    }
+}
+
+// The same for a prefill chunk (more than MAX_ROWS rows): a block per row whose warps take a head at a time, so that the rotary angles (in
+// double precision) are formed once for the 30 heads that need them and a norm is shuffles; the sums are added in the same order.
+// 4,096 rows, 24 + 2 + 4 heads: 206 us, now 86 (1,021: 54, 28).  grid M, 256 threads.
+__global__ void __launch_bounds__(256) qsa_prep_run_kernel(QsaPrepArgs a) {
+    pdl_wait();
+    pdl_trigger();
+    __shared__ float sm[8][HD];
+    __shared__ float cs[2][2 * MAX_HALF];                // of the row's position, of the first position of the group that it closes
+    const int m = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, half = c_rope_half;
+    const int slot = a.rows.slot[m], pos = a.rows.pos[m];
+    QW_DCHECK(slot >= 0 && pos >= 0 && pos / KV_PAGE < a.kv.max_pages, 0x02000000u | (unsigned)(m & 0xffffff));
+    QW_DCHECK(a.kv.page_table[(long long)slot * a.kv.max_pages + pos / KV_PAGE] >= 0, 0x03000000u | (unsigned)(m & 0xffffff));
+    const bool closes = (pos + 1) % a.ratio == 0;
+    if ((tid & (MAX_HALF - 1)) < half && tid < (closes ? 2 : 1) * MAX_HALF) {
+        const int g = tid / MAX_HALF, t = tid & (MAX_HALF - 1);
+        double sd, cd;
+        sincos(double(g ? pos + 1 - a.ratio : pos) * c_inv_freq[t], &sd, &cd);
+        cs[g][t] = float(cd);
+        cs[g][MAX_HALF + t] = float(sd);
+    }
+    __syncthreads();
+    const float *row = a.proj + (long long)m * a.ld_proj;
+    const int off_k = a.QL * 2 * HD, off_v = off_k + a.KVL * HD, off_iq = off_v + a.KVL * HD, off_raw = off_iq + a.IH * ID;
+    float *s = sm[warp];
+    // x: a lane's every 32nd value; normed, weighted and rotated in place
+    auto norm_rot = [&](float *x, auto count, const float *w1, const float *c) {
+        constexpr int n = decltype(count)::value;
+        float ss = 0.f;
+#pragma unroll
+        for (int j = 0; j < n; ++j) ss += warp_sum(x[j] * x[j]);
+        const float r = rsqrtf(ss / float(n * 32) + a.eps);
+#pragma unroll
+        for (int j = 0; j < n; ++j) s[j * 32 + lane] = x[j] * r * w1[j * 32 + lane];
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < n; ++j) {
+            const int d = j * 32 + lane;
+            if (d < half) x[j] = s[d] * c[d] - s[d + half] * c[MAX_HALF + d];
+            else if (d < 2 * half) x[j] = s[d] * c[d - half] + s[d - half] * c[MAX_HALF + d - half];
+            else x[j] = s[d];
+        }
+        __syncwarp();
+    };
+    for (int hb = warp; hb < a.QL + 2 * a.KVL + a.IH + 1; hb += 8) {
+        if (hb < a.QL + a.KVL) {                         // query and key heads
+            const bool key = hb >= a.QL;
+            const int j0 = key ? hb - a.QL : hb;
+            const float *src = key ? row + off_k + j0 * HD : row + hb * 2 * HD;
+            float x[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) x[j] = src[j * 32 + lane];
+            norm_rot(x, std::integral_constant<int, 8>{}, key ? a.kn1 : a.qn1, cs[0]);
+            if (!key) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) a.q[((long long)m * a.QL + hb) * HD + j * 32 + lane] = x[j];
+                continue;
+            }
+            if (j0 == 0 && lane == 0) spill_drop(a.kv, a.sc, slot, pos);
+            bf16 *k = k_row(a.kv, slot, pos) + j0 * HD;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) k[j * 32 + lane] = __float2bfloat16(x[j]);
+            if (a.zero_tail && m == a.rows.M - 1)
+                for (int p = pos + 1; p & 15; ++p) {
+                    if (j0 == 0 && lane == 0) spill_drop(a.kv, a.sc, slot, p);
+                    for (int j = 0; j < 8; ++j) k_row(a.kv, slot, p)[j0 * HD + j * 32 + lane] = __float2bfloat16(0.f);
+                }
+        } else if (hb < a.QL + 2 * a.KVL) {              // value head
+            const int j0 = hb - a.QL - a.KVL;
+            bf16 *v = v_row(a.kv, slot, pos) + j0 * HD;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j * 32 + lane] = __float2bfloat16(row[off_v + j0 * HD + j * 32 + lane]);
+            if (a.zero_tail && m == a.rows.M - 1)
+                for (int p = pos + 1; p & 15; ++p)
+                    for (int j = 0; j < 8; ++j) v_row(a.kv, slot, p)[j0 * HD + j * 32 + lane] = __float2bfloat16(0.f);
+        } else {
+            float x[8];
+            const bool raw = hb == a.QL + 2 * a.KVL + a.IH;
+            if (!raw) {                                  // indexer query head
+                const int j0 = hb - a.QL - 2 * a.KVL;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) x[j] = row[off_iq + j0 * ID + j * 32 + lane];
+                norm_rot(x, std::integral_constant<int, 4>{}, a.iqn1, cs[0]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) a.iq[((long long)m * a.IH + j0) * ID + j * 32 + lane] = x[j];
+                continue;
+            }
+            if (!closes) continue;                       // raw key: the compressed key of a group that is complete now
+            const int rs = a.rows.run_start[m];
+            const float *ring = a.raw_ring + (long long)slot * RAW_RING * ID;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int d = j * 32 + lane;
+                float mean = 0.f;
+                for (int r = 0; r < a.ratio; ++r) {      // positions pos-ratio+1 .. pos, oldest first
+                    const int back = a.ratio - 1 - r;
+                    if (m - back >= rs) mean += a.proj[(long long)(m - back) * a.ld_proj + off_raw + d];
+                    else mean += ring[((pos - back) % RAW_RING) * ID + d];
+                }
+                x[j] = mean / float(a.ratio);
+            }
+            norm_rot(x, std::integral_constant<int, 4>{}, a.ikn1, cs[1]);
+            const int g = pos / a.ratio;
+            if (g < a.ck_cap)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) a.ck[((long long)slot * a.ck_cap + g) * ID + j * 32 + lane] = __float2bfloat16(x[j]);
+        }
     }
 }
 
@@ -604,7 +715,8 @@ static int qsa_prep_launch(const float *proj, int ld_proj, int QL, int KVL, int 
     a.zero_tail = zero_tail;
     a.ring_inline = M <= RAW_RING - ratio ? 1 : 0;
     dim3 grid(M, QL + 2 * KVL + IH + 1);
-    launch_pdl(qsa_prep_kernel, grid, dim3(256), 0, s, a);
+    if (M > MAX_ROWS) launch_pdl(qsa_prep_run_kernel, dim3(M), dim3(256), 0, s, a);
+    else launch_pdl(qsa_prep_kernel, grid, dim3(256), 0, s, a);
     if (!a.ring_inline)
         launch_pdl(qsa_raw_ring_kernel, dim3(M), dim3(ID), 0, s, proj, ld_proj, QL * 2 * HD + 2 * KVL * HD + IH * ID, raw_ring, a.rows);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
