@@ -107,27 +107,6 @@ __device__ __forceinline__ bool tile_at(const GemmTcArgs &a, int id, TileAt &t) 
 // One 32-column piece of an accumulator row -> C.
 __device__ __forceinline__ void store_piece(const GemmTcArgs &a, long long c_off, int row, int col0, const uint32_t (&v)[32]) {
     const int nmax = a.N - col0;
-    if (a.mix_xn) {
-        if (nmax < 32) return;                          // mix_cols is a multiple of 8: pieces are whole
-        const bf16 *x = a.mix_xn + (long long)row * 4 * a.mix_cols + (col0 >> 2);
-        uint4 xv[4];
-#pragma unroll
-        for (int s = 0; s < 4; ++s) xv[s] = __ldg(reinterpret_cast<const uint4 *>(x + (long long)s * a.mix_cols));
-        uint32_t o[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {                   // columns 2 j, 2 j + 1 of the piece
-            float lo = 0.f, hi = 0.f;
-#pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                const uint32_t w = j == 0 ? xv[s].x : j == 1 ? xv[s].y : j == 2 ? xv[s].z : xv[s].w;
-                lo = fmaf(sigmoidf_(__uint_as_float(v[8 * j + s])), bf16_lo(w), lo);
-                hi = fmaf(sigmoidf_(__uint_as_float(v[8 * j + 4 + s])), bf16_hi(w), hi);
-            }
-            o[j] = pack_bf16(lo * 0.25f, hi * 0.25f);
-        }
-        *reinterpret_cast<uint4 *>(a.C16 + (long long)row * a.ldc + (col0 >> 2)) = make_uint4(o[0], o[1], o[2], o[3]);
-        return;
-    }
     if (a.epi.mode) {
         // fp32 pieces to the receive buffers: every rank's (parts of an all-reduce) or the column owner's (reduce-scatter)
         const int owner = a.epi.mode == 2 ? col0 / a.epi.cols_per_rank : 0;
@@ -282,6 +261,56 @@ __device__ __forceinline__ void epilogue_role(const GemmTcArgs &a, uint32_t tmem
     }
 }
 
+// The mixer form's epilogue: logits to gates, times the streams' values, their mean.  A warp's half of a tile is 32 rows of two pieces of 8
+// columns (of 4 streams).  The values of a piece of the next tile are on their way as soon as this tile's are used: fetched when they were needed,
+// every tile waited for memory twice.  4,096 rows x 10,240 x 320: 112 us, now 90.
+__device__ __forceinline__ void mix_role(const GemmTcArgs &a, uint32_t tmem, uint64_t *done, uint64_t *acc_empty, int warp, int lane) {
+    const int q = warp & 3, cbeg = warp >= 6 ? TC_BN / 2 : 0;
+    uint4 xv[2][4];
+    auto fetch = [&](const TileAt &t, int p) {
+        const int row = t.t0 + q * 32 + lane, col = t.n0 + cbeg + p * 32;
+        const bf16 *x = a.mix_xn + (long long)row * 4 * a.mix_cols + (col >> 2);
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+            xv[p][s] = row < a.T && col < a.N ? __ldg(reinterpret_cast<const uint4 *>(x + (long long)s * a.mix_cols)) : make_uint4(0u, 0u, 0u, 0u);
+    };
+    TileAt t;
+    int j = 0;
+    if ((int)blockIdx.x < a.total && tile_at<TC_BN>(a, blockIdx.x, t)) {
+        fetch(t, 0);
+        fetch(t, 1);
+    }
+    for (int id = blockIdx.x; id < a.total; id += gridDim.x, ++j) {          // every tile of a plain product exists
+        const int b = j & 1, row = t.t0 + q * 32 + lane, n0 = t.n0 + cbeg;
+        const bool more = id + (int)gridDim.x < a.total;
+        if (more) tile_at<TC_BN>(a, id + gridDim.x, t);
+        if (!mbar_wait_warp(done + b, (unsigned)(j >> 1) & 1u, a.err)) return;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            uint32_t v[32], o[4];
+            tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * TC_BN + cbeg + p * 32), v);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {                   // columns 2 k, 2 k + 1 of the piece
+                float lo = 0.f, hi = 0.f;
+#pragma unroll
+                for (int s = 0; s < 4; ++s) {
+                    const uint32_t w = k == 0 ? xv[p][s].x : k == 1 ? xv[p][s].y : k == 2 ? xv[p][s].z : xv[p][s].w;
+                    lo = fmaf(sigmoidf_(__uint_as_float(v[8 * k + s])), bf16_lo(w), lo);
+                    hi = fmaf(sigmoidf_(__uint_as_float(v[8 * k + 4 + s])), bf16_hi(w), hi);
+                }
+                o[k] = pack_bf16(lo * 0.25f, hi * 0.25f);
+            }
+            if (more) fetch(t, p);
+            // mix_cols is a multiple of 8: pieces are whole
+            if (row < a.T && n0 + p * 32 < a.N) *reinterpret_cast<uint4 *>(a.C16 + (long long)row * a.ldc + ((n0 + p * 32) >> 2)) = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty + b);
+    }
+}
+
 // The MMA role of both kernels (one warp).
 template <int BN = TC_BN, int ST = TC_STAGES>
 __device__ __forceinline__ void mma_role(const GemmTcArgs &a, unsigned char *smem, uint32_t tmem, uint64_t *full, uint64_t *empty,
@@ -392,7 +421,10 @@ __global__ void __launch_bounds__(320, (BN == TC_BN && !STG) ? 2 : 1) gemm_tc_ke
         float *stg = nullptr;
         if constexpr (STG)
             stg = reinterpret_cast<float *>(sh.smem + ST * tc_stage_bytes<BN>() + 256 + (warp - 2) * TC_STG_BYTES);
-        epilogue_role<BN, STG>(a, sh.tmem, sh.done, sh.acc_empty, warp, lane, 2, TC_EPI_WARPS, stg);
+        bool mixes = false;
+        if constexpr (BN == TC_BN && !STG) mixes = a.mix_xn != nullptr;
+        if (mixes) mix_role(a, sh.tmem, sh.done, sh.acc_empty, warp, lane);
+        else epilogue_role<BN, STG>(a, sh.tmem, sh.done, sh.acc_empty, warp, lane, 2, TC_EPI_WARPS, stg);
     }
     tc_teardown<BN>(sh, warp);
     tp_signal(a.epi.sig);
