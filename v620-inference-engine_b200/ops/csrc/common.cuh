@@ -118,7 +118,15 @@ __device__ __forceinline__ float block_sum(float v, float *scratch /* >= 32 floa
     return s;
 }
 
-__device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + __expf(-x)); }
+// 1 / (1 + e^-x): the hardware's reciprocal and one step of Newton's method.  (As a division the compiler adds a branch per value, which no
+// other value's instructions fill: @@SIG@@)  Error against 64 bits: @@SIGE@@.
+__device__ __forceinline__ float sigmoidf_(float x) {
+    float e, y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.4426950408889634f));
+    const float d = 1.f + e;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+    return d < 8.5e37f ? fmaf(y, fmaf(-d, y, 1.f), y) : y;          // beyond that (and for NaN) the step has nothing to correct
+}
 __device__ __forceinline__ float siluf_(float x) { return x * sigmoidf_(x); }
 __device__ __forceinline__ float softplusf_(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
 
