@@ -154,3 +154,31 @@ def test_attention_inputs_of_a_chunk_equal_the_step_kernels(base, M):
         assert torch.equal(a[key], b[key]), key
     for key in ("k", "v"):
         assert torch.equal(a[key][:end], b[key][:end]) and torch.equal(a[key][tail:], b[key][tail:]) and torch.all(a[key][end:tail] == 0), key
+
+
+@pytest.mark.parametrize("T,SH,R", [(1200, 2560, 320), (1201, 264, 40), (1407, 8, 320), (2500, 520, 72), (40000, 40, 136)])
+def test_mixer_up_projection_of_a_long_chunk_equals_its_pieces(T, SH, R):
+    """The form that keeps its weights against the one for few rows: the same products and sums, so the same bits, and nothing beside them."""
+    L, rn = _lib(), gen(T + SH)
+    u, W, xn = rn(T, R).bfloat16(), (rn(4 * SH, R) * 0.1).bfloat16(), rn(T, 4, SH).bfloat16()
+    u[T // 2, 0] = float("nan")
+    W[:, 1] = 0
+    W[4 * (SH // 2) + 1, 1] = 1.0
+    u[5, 1], u[6, 1] = 300.0, -300.0                              # gates of 1 and 0
+    word = torch.zeros(2, dtype=torch.int32, device=DEV)
+    L.qwk_set_error_word(P(word))
+    whole, parts = (torch.full((T + 2, SH + 8), 768.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    assert L.qwk_gemm_mix_tc(P(u), P(W), P(xn), SH, P(whole), SH + 8, T, R, R, R, S()) == 0
+    for r in range(0, T, 640):
+        n = min(640, T - r)
+        assert L.qwk_gemm_mix_tc(P(u[r:]), P(W), P(xn[r:]), SH, P(parts[r:]), SH + 8, n, R, R, R, S()) == 0
+    torch.cuda.synchronize()
+    L.qwk_set_error_word(None)
+    assert word.tolist() == [0, 0]
+    assert torch.equal(whole.view(torch.int16), parts.view(torch.int16))
+    assert torch.all(whole[T:].float() == 768.0) and torch.all(whole[:, SH:].float() == 768.0)
+    assert torch.all(torch.isnan(whole[T // 2, :SH])) and torch.isfinite(torch.cat([whole[:T // 2, :SH], whole[T // 2 + 1:T, :SH]])).all()
+    c = SH // 2
+    gate = torch.sigmoid((u[5:7].double() @ W.double().T).view(2, SH, 4)[:, c])
+    ref = (gate * xn[5:7, :, c].double()).mean(1)
+    assert torch.allclose(whole[5:7, c].double(), ref, rtol=2 ** -8, atol=1e-5)      # bf16 result, fp32 logits

@@ -261,9 +261,24 @@ __device__ __forceinline__ void epilogue_role(const GemmTcArgs &a, uint32_t tmem
     }
 }
 
+// 32 logits of a row (8 columns of 4 streams) and the streams' values -> 8 means of gated values.
+__device__ __forceinline__ void mix_piece(const uint32_t (&v)[32], const uint4 &x0, const uint4 &x1, const uint4 &x2, const uint4 &x3, uint32_t (&o)[4]) {
+    const uint32_t x[4][4] = {{x0.x, x0.y, x0.z, x0.w}, {x1.x, x1.y, x1.z, x1.w}, {x2.x, x2.y, x2.z, x2.w}, {x3.x, x3.y, x3.z, x3.w}};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {                           // columns 2 k, 2 k + 1 of the piece
+        float lo = 0.f, hi = 0.f;
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            lo = fmaf(sigmoidf_(__uint_as_float(v[8 * k + s])), bf16_lo(x[s][k]), lo);
+            hi = fmaf(sigmoidf_(__uint_as_float(v[8 * k + 4 + s])), bf16_hi(x[s][k]), hi);
+        }
+        o[k] = pack_bf16(lo * 0.25f, hi * 0.25f);
+    }
+}
+
 // The mixer form's epilogue: logits to gates, times the streams' values, their mean.  A warp's half of a tile is 32 rows of two pieces of 8
 // columns (of 4 streams).  The values of a piece of the next tile are on their way as soon as this tile's are used: fetched when they were needed,
-// every tile waited for memory twice.  4,096 rows x 10,240 x 320: 112 us, now 90.
+// every tile waited for memory twice.  4,096 rows x 10,240 x 320: 112 us, then 90.
 __device__ __forceinline__ void mix_role(const GemmTcArgs &a, uint32_t tmem, uint64_t *done, uint64_t *acc_empty, int warp, int lane) {
     const int q = warp & 3, cbeg = warp >= 6 ? TC_BN / 2 : 0;
     uint4 xv[2][4];
@@ -290,17 +305,7 @@ __device__ __forceinline__ void mix_role(const GemmTcArgs &a, uint32_t tmem, uin
         for (int p = 0; p < 2; ++p) {
             uint32_t v[32], o[4];
             tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * TC_BN + cbeg + p * 32), v);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {                   // columns 2 k, 2 k + 1 of the piece
-                float lo = 0.f, hi = 0.f;
-#pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    const uint32_t w = k == 0 ? xv[p][s].x : k == 1 ? xv[p][s].y : k == 2 ? xv[p][s].z : xv[p][s].w;
-                    lo = fmaf(sigmoidf_(__uint_as_float(v[8 * k + s])), bf16_lo(w), lo);
-                    hi = fmaf(sigmoidf_(__uint_as_float(v[8 * k + 4 + s])), bf16_hi(w), hi);
-                }
-                o[k] = pack_bf16(lo * 0.25f, hi * 0.25f);
-            }
+            mix_piece(v, xv[p][0], xv[p][1], xv[p][2], xv[p][3], o);
             if (more) fetch(t, p);
             // mix_cols is a multiple of 8: pieces are whole
             if (row < a.T && n0 + p * 32 < a.N) *reinterpret_cast<uint4 *>(a.C16 + (long long)row * a.ldc + ((n0 + p * 32) >> 2)) = make_uint4(o[0], o[1], o[2], o[3]);
@@ -705,6 +710,140 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1) gemm_tc_pair
     tp_signal(a.epi.sig);
 }
 
+// The mixer form of chunks: a CTA keeps 256 weight rows whole (K <= 320: 160 KB) and takes a run of row tiles, column panel by
+// column panel, so that a tile brings 80 KB of activations and nothing else.  (As 128 x 128 tiles, two CTAs an SM, each brought 160 KB for a
+// quarter of that: 420 MB out of L2 at 4,096 rows.)  Sixteen epilogue warps of 64 columns, whose 32 bytes of each stream's row are whole sectors.
+// 4,096 x 10,240 x 320: 85 us, now 70; 2,048 rows 43, 39; 1,021 rows 27 either way.
+//   warp 0 TMA, warp 1 MMA, warps 2-17 epilogue; columns 0-255 and 256-511 of tensor memory: two accumulators
+constexpr int MX_KB = 5, MX_ST = 4, MX_EPI = 16, MX_THREADS = 64 + MX_EPI * 32, MX_W_BYTES = 256 * TC_BK * 2;
+constexpr int MX_SMEM = MX_KB * MX_W_BYTES + MX_ST * TC_A_BYTES + 1024 /*alignment*/ + 256 /*barriers*/;
+
+__global__ void __launch_bounds__(MX_THREADS, 1) gemm_mix_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapW,
+                                                                    GemmTcArgs a) {
+    extern __shared__ unsigned char raw[];
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
+    unsigned char *sw = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~(uintptr_t)1023), *sa = sw + MX_KB * MX_W_BYTES;
+    uint64_t *w_full = reinterpret_cast<uint64_t *>(sa + MX_ST * TC_A_BYTES), *w_empty = w_full + MX_KB, *full = w_empty + 1, *empty = full + MX_ST,
+             *done = empty + MX_ST, *acc_empty = done + 2;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < MX_KB; ++k) mbar_init(w_full + k, 1);
+        mbar_init(w_empty, 1);
+        for (int k = 0; k < MX_ST; ++k) { mbar_init(full + k, 1); mbar_init(empty + k, 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(done + b, 1); mbar_init(acc_empty + b, MX_EPI); }
+        mbar_fence_init();
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tmem_slot;
+    const int kblocks = (a.K + TC_BK - 1) / TC_BK;
+    const int from = (int)((long long)a.total * blockIdx.x / gridDim.x), to = (int)((long long)a.total * (blockIdx.x + 1) / gridDim.x);
+    if (warp == 0) {
+        unsigned it = 0, panels = 0;
+        int at = -1;
+        bool ok = true;
+        for (int id = from; id < to && ok; ++id) {
+            const int n = id / a.tiles_t, t0 = (id - n * a.tiles_t) * TC_BM;
+            if (n != at) {                               // the next panel, once the last one's products have read theirs
+                if (panels && !mbar_wait_warp(w_empty, (panels - 1) & 1u, a.err)) break;
+                if (elect_one())
+                    for (int kb = 0; kb < kblocks; ++kb) {
+                        mbar_expect_tx(w_full + kb, MX_W_BYTES);
+                        tma_load_2d(sw + kb * MX_W_BYTES, &mapW, kb * TC_BK, n * 256, w_full + kb);
+                    }
+                at = n;
+                ++panels;
+            }
+            for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                const unsigned st = it % MX_ST;
+                if (it >= MX_ST && !mbar_wait_warp(empty + st, (it / MX_ST - 1) & 1u, a.err)) { ok = false; break; }
+                if (elect_one()) {
+                    mbar_expect_tx(full + st, TC_A_BYTES);
+                    tma_load_2d(sa + st * TC_A_BYTES, &mapA, kb * TC_BK, t0, full + st);
+                }
+            }
+        }
+    } else if (warp == 1) {
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
+        unsigned it = 0, panels = 0;
+        int at = -1;
+        bool ok = true;
+        for (int id = from, j = 0; id < to && ok; ++id, ++j) {
+            const int n = id / a.tiles_t, b = j & 1;
+            const bool fresh = n != at;
+            if (fresh) { at = n; ++panels; }
+            if (j >= 2 && !mbar_wait_warp(acc_empty + b, (unsigned)((j >> 1) - 1) & 1u, a.err)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                const unsigned st = it % MX_ST;
+                if ((fresh && !mbar_wait_warp(w_full + kb, (panels - 1) & 1u, a.err)) || !mbar_wait_warp(full + st, (it / MX_ST) & 1u, a.err)) {
+                    ok = false;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t pa = smem_u32(sa + st * TC_A_BYTES), pb = smem_u32(sw + kb * MX_W_BYTES);
+                if (elect_one()) {
+#pragma unroll
+                    for (int k = 0; k < TC_BK / 16; ++k)
+                        umma_bf16(tmem + (uint32_t)(b * 256), make_sw128_desc(pa + k * 32), make_sw128_desc(pb + k * 32), idesc, (kb | k) ? 1u : 0u);
+                    umma_commit(empty + st);
+                }
+            }
+            if (ok && elect_one()) {
+                umma_commit(done + b);
+                if (id + 1 < to && (id + 1) / a.tiles_t != n) umma_commit(w_empty);
+            }
+        }
+    } else {
+        const int q = warp & 3, c0 = ((warp - 2) >> 2) * 64;             // this warp's 32 rows and 64 columns of a tile
+        uint4 xv[4][2];
+        auto fetch = [&](int id) {                       // both halves of a sector at once (a half behind each piece: 70 us -> 87)
+            const int n = id / a.tiles_t, row = (id - n * a.tiles_t) * TC_BM + q * 32 + lane, col = n * 256 + c0;
+            const bf16 *x = a.mix_xn + (long long)row * 4 * a.mix_cols + (col >> 2);
+#pragma unroll
+            for (int s = 0; s < 4; ++s)
+#pragma unroll
+                for (int p = 0; p < 2; ++p)
+                    xv[s][p] = row < a.T && col + p * 32 < a.N ? __ldg(reinterpret_cast<const uint4 *>(x + (long long)s * a.mix_cols) + p) : make_uint4(0u, 0u, 0u, 0u);
+        };
+        if (from < to) fetch(from);
+        for (int id = from, j = 0; id < to; ++id, ++j) {
+            const int n = id / a.tiles_t, row = (id - n * a.tiles_t) * TC_BM + q * 32 + lane, col = n * 256 + c0, b = j & 1;
+            if (!mbar_wait_warp(done + b, (unsigned)(j >> 1) & 1u, a.err)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            uint32_t o[2][4];
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                uint32_t v[32];
+                tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 256 + c0 + p * 32), v);
+                if (p == 1) {                            // the accumulator is read
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(acc_empty + b);
+                }
+                mix_piece(v, xv[0][p], xv[1][p], xv[2][p], xv[3][p], o[p]);
+            }
+            if (id + 1 < to) fetch(id + 1);
+            // mix_cols is a multiple of 8: pieces are whole
+#pragma unroll
+            for (int p = 0; p < 2; ++p)
+                if (row < a.T && col + p * 32 < a.N)
+                    *reinterpret_cast<uint4 *>(a.C16 + (long long)row * a.ldc + ((col + p * 32) >> 2)) = make_uint4(o[p][0], o[p][1], o[p][2], o[p][3]);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
 // The pair form with the operands' roles exchanged: the pair's 256 rows are weight rows and the tokens the columns, so that a
 // tile is as wide as the tokens want - any multiple of 16 up to 256 - and a prompt whose length is no multiple of 256 is not padded to one.  A
 // lane of the accumulator is an output column: the epilogue's stores are whole 128-byte lines without a staging buffer.  us,
@@ -847,7 +986,7 @@ using namespace qw;
 
 // One-time (per device) opt-in to the kernels' dynamic shared memory.
 static bool configure_once(int which) {          // 0 dense 128-wide, 2 dense 256-wide, 3 / 4 the two with a staged epilogue, 5 / 6 the pair form, 7 / 8 exchanged
-    static bool done[9][64] = {};
+    static bool done[10][64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
@@ -862,6 +1001,7 @@ static bool configure_once(int which) {          // 0 dense 128-wide, 2 dense 25
                                                       tc_smem_bytes<TC_WIDE_BN, TC_WIDE_STAGES, true>());
         else if (which == 5) e = cudaFuncSetAttribute(gemm_tc_pair_kernel<TC_PAIR_STAGES, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                       tc_pair_smem_bytes<TC_PAIR_STAGES, false>());
+        else if (which == 9) e = cudaFuncSetAttribute(gemm_mix_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MX_SMEM);
         else if (which >= 7) e = cudaFuncSetAttribute(which == 7 ? gemm_tc_exchange_kernel<false> : gemm_tc_exchange_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_pair_smem_bytes<TC_PAIR_STAGES, false>());
         else e = cudaFuncSetAttribute(gemm_tc_pair_kernel<TC_PAIR_STG_STAGES, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       tc_pair_smem_bytes<TC_PAIR_STG_STAGES, true>());
@@ -1120,11 +1260,14 @@ QW_API int qwk_gemm_bf16_tc_tp(void *tp_, const void *A, const void *W, void *C,
     return gemm_plain(a, A, W, C, T, N, K, lda, ldw, ldc, out_bf16, s);
 }
 
+// From here on the form that keeps its weights: 777 rows 22.6 / 20.5 us, but 400 to 600 18.5 / 20.5 and 1,021 26.7 / 26.6 (a CTA's tiles are few and
+// the last ones lonely); 1,500 34.8 / 32.8, 2,048 43 / 39.
+constexpr int MX_MIN_T = 1200;
 // The mixer's up projection with the block input formed in the epilogue: A bf16 [T][lda] (the activated low-rank vector), W bf16
 // [4 SH][ldw] (row 4 c + s: gate of stream s, column c), xn bf16 [T][4][SH]; out bf16 [T][ld_out]: mean over the streams of
 // sigmoid(A . W^T) * xn.  The logits (fp32, 4 SH a row) are never stored: as a product and a kernel that read them back
-// 118 us at 4096 x 2560 and 41 at 1021, here 105 and 29.  Always 128 x 128 tiles: the epilogue bounds it, and two CTAs on an SM have twice
-// the warps for it (with 128 x 256 tiles 8 to 10 % more from 300 rows on).  SH a multiple of 8.
+// 118 us at 4096 x 2560 and 41 at 1021, here 70 and 27.  Below MX_MIN_T 128 x 128 tiles: two CTAs on an SM have the warps that
+// the epilogue wants (with 128 x 256 tiles 8 to 10 % more from 300 rows on).  SH a multiple of 8.
 QW_API int qwk_gemm_mix_tc(const void *A, const void *W, const void *xn, int SH, void *out, int ld_out, int T, int K, int lda, int ldw,
                            cudaStream_t s) {
     if (T <= 0) return 0;
@@ -1132,6 +1275,17 @@ QW_API int qwk_gemm_mix_tc(const void *A, const void *W, const void *xn, int SH,
     GemmTcArgs a{};
     a.mix_xn = (const bf16 *)xn;
     a.mix_cols = SH;
+    if (K <= MX_KB * TC_BK && T >= MX_MIN_T) {
+        if ((K & 7) || (lda & 7) || (ldw & 7) || ((uintptr_t)A & 15) || ((uintptr_t)W & 15)) return -1;
+        CUtensorMap mA, mW;
+        if (!make_map(&mA, A, T, K, lda, TC_BM) || !make_map(&mW, W, 4 * SH, K, ldw, 256)) return -3;
+        set_output(a, out, 1, ld_out);
+        a.T = T; a.N = 4 * SH; a.K = K; a.err = g_err_ptr;
+        a.tiles_t = (T + TC_BM - 1) / TC_BM; a.tiles_n = (4 * SH + 255) / 256; a.total = a.tiles_t * a.tiles_n;
+        if (!configure_once(9)) return -3;
+        gemm_mix_tc_kernel<<<persistent_grid(a.total, 1), MX_THREADS, MX_SMEM, s>>>(mA, mW, a);
+        return cudaGetLastError() == cudaSuccess ? 0 : -2;
+    }
     return gemm_plain(a, A, W, out, T, 4 * SH, K, lda, ldw, ld_out, 1, s);
 }
 
