@@ -65,7 +65,6 @@ def test_matches_64_bits_and_the_gathering_kernel(QL, KVL, base, M, topk, scale)
     gathered, o = (torch.zeros(M, QL, 256, dtype=torch.bfloat16, device="cuda:0") for _ in range(2))
     last, ld = base + M - 1, (base + M) // 4 + 8
     mask = torch.empty(M, ld, dtype=torch.int32, device="cuda:0")
-    assert L.qwk_qsa_takes_tc(QL, KVL, M, last, 4, ld, t["ldp"]) == 1
     pool = [P(t["k"]), P(t["v"])]
     assert L.qwk_qsa_attend_mma(P(t["q"]), QL, KVL, M, P(t["slot"]), P(t["pos"]), *pool, None, None, 2 * t["pages"], P(t["table"]), t["pages"],
                                 P(t["sel"]), P(t["sel_n"]), topk, 4, P(t["proj"]), t["ldp"], P(gathered), s) == 0
@@ -86,9 +85,13 @@ def test_matches_64_bits_and_the_gathering_kernel(QL, KVL, base, M, topk, scale)
 
 
 def test_what_it_does_not_take():
-    """Other group sizes, contexts behind the line, rows of the projection off 16 bytes: the gathering kernel's."""
+    """Other group sizes, masks that do not fit, rows of the projection off 16 bytes are refused by the kernel; contexts that are long for
+    their chunk, and chunks too small to matter, are the gathering kernel's."""
     from qwb200.ops import lib as qlib
     L = qlib.load(True)
-    take = lambda **k: L.qwk_qsa_takes_tc(*{**dict(QL=24, KVL=2, M=100, last=4000, ratio=4, ld=1100, ldp=13952), **k}.values())
-    assert take() == 1
-    assert not any((take(ratio=8), take(last=1 << 20, ld=1 << 20), take(last=40, M=100), take(ld=31), take(ldp=13953), take(QL=23)))
+    take = lambda **k: L.qwk_qsa_takes_tc(*{**dict(QL=24, KVL=2, M=100, last=4000, topk=512, ratio=4, ld=20000, ldp=13952), **k}.values())
+    assert take() == 1 and take(M=1, last=1000) == 1 and take(M=4096, last=4095) == 1 and take(M=2048, last=16384 + 2047) == 1
+    assert not any((take(ratio=8), take(last=40, M=100), take(ld=31), take(ldp=13953), take(QL=23), take(QL=0), take(KVL=0)))
+    assert not any((take(last=1 << 20), take(M=100, last=99), take(M=1, last=9000), take(M=300, last=16684), take(M=2048, last=32000)))
+    none = [None] * 4
+    assert L.qwk_qsa_attend_tc(None, 23, 2, 4, 100, None, None, *none, 0, 1, None, 1, None, None, 512, None, 4, None, 13952, None, None) == -1

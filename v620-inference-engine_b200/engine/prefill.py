@@ -376,7 +376,7 @@ class Prefiller:
                                       _p(b["sel"]), _p(b["sel_n"]), s), "select")
             ow = sc.qh_l * c.head_dim
             last_pos = end - 1
-            if self.qsa_mma and L.qwk_qsa_takes_tc(sc.qh_l, sc.kvh_l, T, last_pos, c.idx_ratio, d.score_cap, ldp):
+            if self.qsa_mma and L.qwk_qsa_takes_tc(sc.qh_l, sc.kvh_l, T, last_pos, c.idx_topk_blocks, c.idx_ratio, d.score_cap, ldp):
                 self._ck(L.qwk_qsa_attend_tc(_p(b["q"]), sc.qh_l, sc.kvh_l, T, last_pos, rp("slot"), rp("pos"), P(kd), P(vd),
                                              P(kh) if kh else None, P(vh) if vh else None, 0, d.n_dev_pages, _p(dm.page_table), d.max_pages,
                                              _p(b["sel"]), _p(b["sel_n"]), c.idx_topk_blocks, _p(b["scores"]), d.score_cap, _p(b["proj"]), ldp,

@@ -119,7 +119,7 @@ int qwk_set_spill_cache(void *tags, void *rows, void *miss, void *ctl, void *sta
 int qwk_spill_cache_active(int unused);
 
 // qsa_tc.cu
-int qwk_qsa_takes_tc(int QL, int KVL, int M, int last_pos, int ratio, int ld_mask, int ld_proj);
+int qwk_qsa_takes_tc(int QL, int KVL, int M, int last_pos, int topk, int ratio, int ld_mask, int ld_proj);
 int qwk_qsa_attend_tc(const float *q, int QL, int KVL, int M, int last_pos, const int *slot, const int *pos, void *k_dev, void *v_dev, void *k_host, void *v_host, int staged, int n_dev_pages, const int *page_table, int max_pages, const int *sel, const int *sel_n, int topk, void *mask, int ld_mask, const float *proj, int ld_proj, void *o, cudaStream_t s);
 
 // sampling.cu

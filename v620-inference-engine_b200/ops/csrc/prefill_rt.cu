@@ -353,8 +353,10 @@ struct Builder {
                     staged = 1;
                 }
             }
-            const int last_pos = (mtp ? c.job->mtp_base : c.job->base) + L.r0 + L.n - 1;
-            if (qwk_qsa_takes_tc(d.QL, d.KVL, L.n, last_pos, d.idx_ratio, d.score_cap, b.proj_ld)) {
+            // both halves of a chunk in two lanes take the kernel that the whole chunk would
+            const int base = mtp ? c.job->mtp_base : c.job->base, rows = mtp ? L.n : c.job->T;
+            const int last_pos = base + L.r0 + L.n - 1;
+            if (qwk_qsa_takes_tc(d.QL, d.KVL, rows, base + rows - 1, d.idx_topk, d.idx_ratio, d.score_cap, b.proj_ld)) {
                 PF_TRY(2, qwk_qsa_attend_tc(f_at(b.q, L.r0, d.QL * 256), d.QL, d.KVL, L.n, last_pos, r.slot, r.pos, st.k_dev[qi], st.v_dev[qi], kh, vh,
                                             staged, d.n_dev_pages, st.page_table, d.max_pages, i_at(b.sel, L.r0, d.idx_topk), b.sel_n + L.r0, d.idx_topk,
                                             f_at(b.scores, L.r0, d.score_cap), d.score_cap, f_at(b.proj, L.r0, b.proj_ld), b.proj_ld,

@@ -13,8 +13,8 @@
 //
 // Why not gather: 2,051 rows per query are 4.2 MB out of L2 for every query, and that, at 6.8 TB/s, is what the gather costs
 // (qsa_mma.cuh: 0.66 us per query, wherever it lies).  Here a tile is read once for 21 queries of 12 heads; the price is the keys nobody
-// chose, so the line lies where the context is long enough.  24 query heads over 2, us a layer, gathered /
-// here: 100 tokens 23 / 25, 1,021 226 / 57, 4,096 1941 / 336, 2,000 at position 32,768 1362 / 1009.
+// chose, so contexts that are long for their chunk stay with the gather (qwk_qsa_takes_tc).  24 query heads over 2, us a layer,
+// gathered / here: 1,021 tokens 226 / 57, 4,096 tokens 1941 / 336, 2,048 tokens at position 16,384 1362 / 1009.
 #include "tc.cuh"
 
 namespace qw {
@@ -370,13 +370,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QT_THREADS, 1) qsa_a
 
 using namespace qw;
 
-constexpr int QT_MAX_TILES = 400;
+// What qwk_qsa_attend_tc can take: groups of four, a mask that fits its buffer, offsets in 32 bits.
+static bool qsa_tc_fits(int QL, int KVL, int M, int last_pos, int ratio, int ld_mask, int ld_proj) {
+    return KVL >= 1 && QL >= KVL && QL % KVL == 0 && M >= 1 && ratio == 4 && last_pos >= M - 1 && (last_pos >> 7) < ld_mask && (ld_proj & 3) == 0 &&
+           (long long)M * ld_proj < (1LL << 31) - 65536 && (long long)M * QL * QT_D < (1LL << 31);
+}
 
-// 1: this chunk's attention (M rows of one run, the last at position last_pos) goes through qwk_qsa_attend_tc.  The line: a query costs
-// 0.66 us in the kernel that gathers, wherever it stands behind the budget, and 1.6 ns per 128 keys here (12 heads share a KV head).
-QW_API int qwk_qsa_takes_tc(int QL, int KVL, int M, int last_pos, int ratio, int ld_mask, int ld_proj) {
-    return KVL >= 1 && QL % KVL == 0 && M >= 1 && ratio == 4 && last_pos >= M - 1 && (last_pos >> 7) < QT_MAX_TILES && (last_pos >> 7) < ld_mask &&
-           (ld_proj & 3) == 0 && (long long)M * ld_proj < (1LL << 31) - 65536 && (long long)M * QL * QT_D < (1LL << 31);
+// 1: the attention of a chunk (M rows of one run, the last at position last_pos, topk groups chosen of `ratio` tokens) goes through
+// qwk_qsa_attend_tc.  Both kernels run in waves of equal blocks.  Here a pair of CTAs has 256 rows of a KV head and takes 2.3 us per
+// tile of 128 keys; the kernel that gathers has three blocks of a query and KV head on each SM and takes a wave 20 us and 112 more when
+// the lists are full.  us, gathered / here: 1 row at position 1,000 69 / 46, at 9,000 129 / 186; 300 rows at 0 50 / 34, at 9,000 267 / 190,
+// at 16,384 269 / 320; 1,021 at 16,384 683 / 641, at 24,000 688 / 922; 2,048 at 16,384 1340 / 978, at 24,000 1344 / 1385; 100 at 0 27 / 31.
+QW_API int qwk_qsa_takes_tc(int QL, int KVL, int M, int last_pos, int topk, int ratio, int ld_mask, int ld_proj) {
+    if (!qsa_tc_fits(QL, KVL, M, last_pos, ratio, ld_mask, ld_proj)) return 0;
+    const long long pairs = NUM_SMS / 2, blocks = 3 * NUM_SMS, units = ((long long)M * (QL / KVL) + 255) / 256 * KVL;
+    const long long here = (units + pairs - 1) / pairs, gathered = ((long long)M * KVL + blocks - 1) / blocks;
+    const double full = (double)ratio * topk + ratio - 1, len = last_pos + 1 - 0.5 * (M - 1);          // a row's list: all before it, until it is full
+    return 27 + 2.3 * ((last_pos >> 7) + 1) * here < gathered * (20 + 112 * (len < full ? len : full) / 2051);
 }
 
 // Attention of the rows of one run (slot[0], positions pos[0] + m, the last of them last_pos); what sel / sel_n name is what a row attends
@@ -386,7 +396,7 @@ QW_API int qwk_qsa_takes_tc(int QL, int KVL, int M, int last_pos, int ratio, int
 QW_API int qwk_qsa_attend_tc(const float *q, int QL, int KVL, int M, int last_pos, const int *slot, const int *pos, void *k_dev, void *v_dev,
                              void *k_host, void *v_host, int staged, int n_dev_pages, const int *page_table, int max_pages, const int *sel,
                              const int *sel_n, int topk, void *mask, int ld_mask, const float *proj, int ld_proj, void *o, cudaStream_t s) {
-    if (!qwk_qsa_takes_tc(QL, KVL, M, last_pos, 4, ld_mask, ld_proj) || !aligned16(q, proj, k_dev, v_dev, k_host, v_host) || ((uintptr_t)o & 7)) return -1;
+    if (!qsa_tc_fits(QL, KVL, M, last_pos, 4, ld_mask, ld_proj) || !aligned16(q, proj, k_dev, v_dev, k_host, v_host) || ((uintptr_t)o & 7)) return -1;
     static bool done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
