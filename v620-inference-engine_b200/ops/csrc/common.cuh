@@ -119,7 +119,9 @@ __device__ __forceinline__ float block_sum(float v, float *scratch /* >= 32 floa
 }
 
 // 1 / (1 + e^-x): the hardware's reciprocal and one step of Newton's method.  (As a division the compiler adds a branch per value, which no
-// other value's instructions fill: @@SIG@@)  Error against 64 bits: @@SIGE@@.
+// other value's instructions fill: the mixer's up projection at 100 rows 15.4 us, so 12.3; the experts' gate/up product at 4,096 tokens 458, so
+// 396.)  Error against 64 bits: the division's, to every digit of its largest and its mean (|x| up to 1, 4, 10, 30, 80); results below 2^-126
+// are 0.
 __device__ __forceinline__ float sigmoidf_(float x) {
     float e, y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * -1.4426950408889634f));
