@@ -136,6 +136,47 @@ def test_flash_decode_parts_match_64_bits(QL, KVL, topk):
             assert float((o[m, h].double() - want).norm() / want.norm()) < 2 ** -8
 
 
+@pytest.mark.parametrize("size", [0.3, 1.0, 4.0])
+def test_flash_decode_on_tensor_cores_is_as_exact_as_the_scalar_kernel(size):
+    """The merged parts before bf16, against 64 bits, of both kernels: 17 heads per KV head take the scalar one, 12 of the same heads the tensor
+    cores.  Bound: the scalar kernel's error and a tenth (420 rows of 256 values each: their mean error is known to a few percent)."""
+    topk, ratio, page, KVL = 64, 4, 256, 2
+    rn = gen(int(size * 10))
+    positions = [3, 62, 64, 200, 255, 258, 300, 777, 1500, 3000]
+    M, pages = len(positions), 12
+    k, v = (rn(pages, page, KVL * 256).bfloat16() for _ in range(2))
+    table, all_q = torch.arange(pages, dtype=torch.int32, device=DEV), rn(M, KVL, 17, 256) * size
+    sel, sel_n = torch.zeros(M, topk, dtype=torch.int32, device=DEV), torch.full((M,), -1, dtype=torch.int32, device=DEV)
+    lists = []
+    for m, p in enumerate(positions):
+        nb, toks = (p + 1) // ratio, torch.arange(p + 1, device=DEV)
+        if nb > topk:
+            ch = torch.sort(torch.randperm(nb, generator=torch.Generator().manual_seed(m))[:topk]).values.to(DEV)
+            sel[m], sel_n[m] = ch.int(), topk
+            toks = torch.cat([(ch[:, None] * ratio + torch.arange(ratio, device=DEV)).reshape(-1), toks[nb * ratio:]])
+        lists.append(toks)
+    nsplit, errs = (topk * ratio + ratio + 63) // 64, []
+    for heads in (12, 17):
+        QL, q = heads * KVL, all_q[:, :, :heads].contiguous()
+        pm, pl = (torch.full((M, QL, nsplit), float("-inf"), device=DEV) for _ in range(2))
+        pacc, o, proj = torch.zeros(M, QL, nsplit, 256, device=DEV), torch.zeros(M, QL, 256, dtype=torch.bfloat16, device=DEV), rn(M, QL * 512)
+        assert _lib().qwk_qsa_attend(P(q), QL, KVL, M, P(i32([0] * M)), P(i32(positions)), P(k), P(v), None, None, pages, P(table), pages, P(sel), P(sel_n),
+                                     topk, ratio, nsplit, P(pm), P(pl), P(pacc), P(proj), QL * 512, P(o), S()) == 0
+        torch.cuda.synchronize()
+        total = 0.0
+        for m, toks in enumerate(lists):
+            n = (len(toks) + 63) // 64
+            for kv in range(KVL):
+                kf, vf = (x.view(-1, KVL, 256)[toks, kv].double() for x in (k, v))
+                want = torch.softmax(all_q[m, kv, :12].double() @ kf.T / 16, 1) @ vf
+                at = slice(kv * heads, kv * heads + 12)
+                w = torch.exp(pm[m, at, :n].double() - pm[m, at, :n].double().amax(1, keepdim=True))
+                got = (w[..., None] * pacc[m, at, :n].double()).sum(1) / (w * pl[m, at, :n].double()).sum(1, keepdim=True)
+                total += float(((got - want).norm(dim=1) / want.norm(dim=1)).pow(2).sum())
+        errs.append((total / (M * KVL * 12)) ** 0.5)
+    assert errs[0] < 1.1 * errs[1], errs
+
+
 @pytest.mark.parametrize("pairs,layers,state", [([[0, 2], [2, 0], [1, -1]], 3, 48 * 128 * 128), ([[1, 1]], 1, 4), ([[0, 1], [1, 3]], 2, 4096 * 3 + 8)])
 def test_accepted_states_are_copied_whole(pairs, layers, state):
     """Every value of an accepted row's state, whatever its size (pieces of 16 KB, a last one that is not whole); rejected slots stay."""

@@ -62,10 +62,13 @@ __device__ __forceinline__ void att_issue(const QsaAttendArgs &a, bf16 *dst_tile
 
 // ------------------------------------------------------------------------------------------------------------------
 // Flash-decode over the token list for the rows of a step.  A block takes 64 entries of one row's list for all query heads of one KV head (<= 16,
-// the 16 rows of the MMA tile) and leaves the partial softmax (maximum, sum, sums of V) that qsa_combine_kernel merges.  Scores and weights stay
-// what fp32 makes them: the queries and the weights go through the MMAs as three bf16 parts each (24 bits), keys and values are bf16 anyway.
+// the 16 rows of the MMA tile) and leaves the partial softmax (maximum, sum, sums of V) that qsa_combine_kernel merges.  Operands keep what fp32
+// holds: the queries and the weights go through the MMAs as three bf16 parts each (24 bits), keys and values are bf16 anyway.  Sums are rounded
+// fp32 additions of what one MMA sums; with one running sum in the tensor core the error was three times the scalar form's.
+// Error of the merged output before bf16 against 64 bits, queries of size 0.3 / 1 / 2 / 4: scalar form 0.95, 1.34, 2.41, 3.64e-7; here 0.62, 1.18,
+// 2.36, 3.51e-7.
 // In a scalar form (four heads a block, a warp per token) each token's rows were fetched once for every four heads and every score was five
-// shuffles: 24 rows 177 us, now 49; 8 rows 40 / 11.7; one 15 / 9.
+// shuffles.  With the merge, at 4,096 tokens: 24 rows 181 us, now 55; 8 rows 69 / 25; one 17.4 / 11.
 // grid (nsplit, M, KVL), 256 threads.
 // ------------------------------------------------------------------------------------------------------------------
 constexpr int AD_SMEM = (2 * AT * KV_LD + 3 * 16 * KV_LD + 3 * 16 * P_LD) * 2 + 2 * 8 * 16 * 4 + 16;
@@ -126,8 +129,9 @@ __global__ void __launch_bounds__(256, 2) qsa_attend_split_kernel(QsaAttendArgs 
     const uint32_t ks_base = (uint32_t)__cvta_generic_to_shared(Ks), vs_base = (uint32_t)__cvta_generic_to_shared(Vs);
     const uint32_t qs_base = (uint32_t)__cvta_generic_to_shared(Qs), ps_base = (uint32_t)__cvta_generic_to_shared(Ps);
     bool ok = mbar_wait_warp(kbar, 0u, g_err);               // bounded; after a time-out the meetings still take place
-    // ---- S = Q K^T for this warp's 8 tokens
-    float s3[3][4] = {};
+    // ---- S = Q K^T for this warp's 8 tokens.  Of the queries' first parts every 16 products are summed from zero and added with rounding, in four
+    // chains (the tensor core's own running sum cuts off); the other two parts are 2^-8 and 2^-16 of them
+    float s1[4][4] = {}, s2[4] = {};
     {
         const uint32_t brow = ks_base + (uint32_t)((w * 8 + (lane & 7)) * KV_LD * 2 + (lane >> 3) * 16);
 #pragma unroll 4
@@ -135,19 +139,25 @@ __global__ void __launch_bounds__(256, 2) qsa_attend_split_kernel(QsaAttendArgs 
             uint32_t b[4];
             ldmatrix_x4(b[0], b[1], b[2], b[3], brow + ks * 32);
 #pragma unroll
-            for (int k = 0; k < 3; ++k)
+            for (int j = 0; j < 2; ++j) {
+                uint32_t q0, q1, q2, q3;
+                float c[4] = {};
+                ldmatrix_x4(q0, q1, q2, q3, a_tile_addr(qs_base, KV_LD * 2, (ks + j) * 16, lane));
+                mma_bf16(c, q0, q1, q2, q3, b[2 * j], b[2 * j + 1]);
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    uint32_t q0, q1, q2, q3;
+                for (int i = 0; i < 4; ++i) s1[(ks + j) & 3][i] += c[i];
+#pragma unroll
+                for (int k = 1; k < 3; ++k) {
                     ldmatrix_x4(q0, q1, q2, q3, a_tile_addr(qs_base + k * 16 * KV_LD * 2, KV_LD * 2, (ks + j) * 16, lane));
-                    mma_bf16(s3[k], q0, q1, q2, q3, b[2 * j], b[2 * j + 1]);
+                    mma_bf16(s2, q0, q1, q2, q3, b[2 * j], b[2 * j + 1]);
                 }
+            }
         }
     }
     float s[4], tm[2] = {-INFINITY, -INFINITY};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        s[i] = sp * AT + w * 8 + 2 * t4 + (i & 1) < count ? ((s3[2][i] + s3[1][i]) + s3[0][i]) * 0.0625f : -INFINITY;       // 1/sqrt(256)
+        s[i] = sp * AT + w * 8 + 2 * t4 + (i & 1) < count ? (s2[i] + ((s1[0][i] + s1[1][i]) + (s1[2][i] + s1[3][i]))) * 0.0625f : -INFINITY;       // 1/sqrt(256)
         tm[i >> 1] = fmaxf(tm[i >> 1], s[i]);
     }
 #pragma unroll
@@ -184,8 +194,8 @@ __global__ void __launch_bounds__(256, 2) qsa_attend_split_kernel(QsaAttendArgs 
         a.pl[o] = l;
     }
     ok = ok && mbar_wait_warp(vbar, 0u, g_err);
-    // ---- P V for this warp's 32 output dims
-    float acc[4][4] = {};
+    // ---- P V for this warp's 32 output dims, summed as the scores are
+    float acc[4][4] = {}, acc2[4][4] = {};
     {
         const int mid = lane >> 3;
         const uint32_t vrow = vs_base + (uint32_t)((((mid & 1) * 8 + (lane & 7)) * KV_LD + w * 32 + (mid >> 1) * 8) * 2);
@@ -195,17 +205,28 @@ __global__ void __launch_bounds__(256, 2) qsa_attend_split_kernel(QsaAttendArgs 
 #pragma unroll
             for (int n = 0; n < 2; ++n) ldmatrix_x4_trans(b[n][0], b[n][1], b[n][2], b[n][3], vrow + (uint32_t)(ks * 16 * KV_LD * 2 + n * 32));
 #pragma unroll
-            for (int k = 2; k >= 0; --k) {                   // the smallest part first
+            for (int k = 0; k < 3; ++k) {
                 uint32_t p0, p1, p2, p3;
                 ldmatrix_x4(p0, p1, p2, p3, a_tile_addr(ps_base + k * 16 * P_LD * 2, P_LD * 2, ks * 16, lane));
 #pragma unroll
-                for (int n = 0; n < 2; ++n) {
-                    mma_bf16(acc[2 * n], p0, p1, p2, p3, b[n][0], b[n][1]);
-                    mma_bf16(acc[2 * n + 1], p0, p1, p2, p3, b[n][2], b[n][3]);
+                for (int n = 0; n < 4; ++n) {
+                    const uint32_t b0 = b[n >> 1][(n & 1) * 2], b1 = b[n >> 1][(n & 1) * 2 + 1];
+                    if (k) {
+                        mma_bf16(acc2[n], p0, p1, p2, p3, b0, b1);
+                    } else {
+                        float c[4] = {};
+                        mma_bf16(c, p0, p1, p2, p3, b0, b1);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) acc[n][i] += c[i];
+                    }
                 }
             }
         }
     }
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[n][i] += acc2[n][i];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const int r = g + 8 * h;
