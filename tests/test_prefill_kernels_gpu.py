@@ -105,6 +105,28 @@ def test_chunked_scan_of_ragged_runs_is_as_exact_as_its_operands(M, KL, VL):
         assert float((St[0, h].double().cpu() - Sw).norm() / Sw.norm()) < 1.5e-3
 
 
+@pytest.mark.parametrize("bad", [20, 50, 63, 64 + 33, 64 + 50])
+def test_chunked_scan_keeps_a_row_that_is_not_finite_from_the_tiles_before_it(bad):
+    """Rows before the 16-row tile of a NaN row have the bits that they have without it; the row itself and the state show it."""
+    KL, VL, M, D = 2, 4, 130, 128
+    rn = gen(bad)
+    qkv, decay, beta = rn(M, (2 * KL + VL) * D) * 0.1, torch.exp(-rn(M, VL).abs() * 0.2).contiguous(), torch.sigmoid(rn(M, VL)).contiguous()
+    ld = qkv.shape[1] + VL * D + 2 * VL
+    proj, S0, nw = rn(M, ld), rn(1, VL, D, D) * 0.1, 1 + 0.1 * rn(D)
+    outs = []
+    for poison in (False, True):
+        x, St, o = qkv.clone(), S0.clone(), torch.zeros(M, VL * D, dtype=torch.bfloat16, device=DEV)
+        if poison:
+            x[bad] = float("nan")
+        scratch = torch.zeros((M + 63) // 64 * VL * (2 * 64 * 128 + 64 * 64 + 64) + M * VL * D, device=DEV)
+        assert _lib().qwk_gdn_scan_chunked(P(x), P(decay), P(beta), P(proj), ld, P(St), P(nw), KL, VL, M, P(i32([0] * M)), P(scratch), P(o), C.c_float(1e-6), S()) == 0
+        torch.cuda.synchronize()
+        outs.append((o, St))
+    first = bad // 16 * 16
+    assert torch.equal(outs[0][0][:first], outs[1][0][:first]) and torch.isfinite(outs[0][0]).all()
+    assert torch.isnan(outs[1][0][bad:]).all() and torch.isnan(outs[1][1]).all()
+
+
 @pytest.mark.parametrize("T,H,k,off,shared", [(3, 2560, 10, 0, True), (5, 516, 3, 0, True), (4, 510, 7, 0, False), (4, 512, 5, 1, True), (33, 8, 11, 0, False)])
 def test_combined_experts_of_any_width_and_address(T, H, k, off, shared):
     """Four columns at a time or one, experts of other ranks left out: the sums of the same products in the same order."""

@@ -228,23 +228,24 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(GdnChunkArgs a) 
         for (int r = 0; r < HC_; ++r) Ts[(o + r) * LDP + o + lane] = col[r];
     }
     __syncthreads();
-    // T21 = -T22 (A21 T11), both products in fp32; the first goes to A's empty upper right
+    // T21 = -T22 (A21 T11), both products in fp32; the first goes to A's empty upper right.  T22's sums end at its diagonal: a row that is not
+    // finite reaches none before it
     float *Es = As + HC_;                // [32][LDP]
     const int er = tid >> 3, ec = (tid & 7) * 4;
-    auto half_product = [&](const float *A, const float *B) {
+    auto half_product = [&](const float *A, const float *B, int n) {
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 8
-        for (int s = 0; s < HC_; ++s) {
+        for (int s = 0; s < n; ++s) {
             const float f = A[er * LDP + s];
             const float4 v = *reinterpret_cast<const float4 *>(B + s * LDP + ec);
             acc.x = fmaf(f, v.x, acc.x); acc.y = fmaf(f, v.y, acc.y); acc.z = fmaf(f, v.z, acc.z); acc.w = fmaf(f, v.w, acc.w);
         }
         return acc;
     };
-    *reinterpret_cast<float4 *>(Es + er * LDP + ec) = half_product(As + HC_ * LDP, Ts);
+    *reinterpret_cast<float4 *>(Es + er * LDP + ec) = half_product(As + HC_ * LDP, Ts, HC_);
     __syncthreads();
     {
-        const float4 v = half_product(Ts + HC_ * LDP + HC_, Es);
+        const float4 v = half_product(Ts + HC_ * LDP + HC_, Es, er + 1);
         *reinterpret_cast<float4 *>(Ts + (HC_ + er) * LDP + ec) = make_float4(-v.x, -v.y, -v.z, -v.w);
     }
     __syncthreads();
