@@ -105,6 +105,39 @@ def test_chunked_scan_of_ragged_runs_is_as_exact_as_its_operands(M, KL, VL):
         assert float((St[0, h].double().cpu() - Sw).norm() / Sw.norm()) < 1.5e-3
 
 
+@pytest.mark.parametrize("M,shared", [(64, 0), (130, 0), (130, 1)])
+def test_chunked_scan_solves_its_systems_as_exactly_as_fp32_substitution(M, shared):
+    """Keys in steps of 1/16 and a beta of 8 bits without decay: the matrix of a chunk is exact, so what is left is the solve.  Its result against 64
+    bits, beside forward substitution in fp32 (each multiply-add rounded once): no further off than 1.05 times that (16,000 values)."""
+    KL, VL, D = 1, 2, 128
+    g = torch.Generator().manual_seed(M + shared)
+    k = (torch.randint(-2, 3, (M, D), generator=g) if not shared else torch.randint(0, 3, (M, D), generator=g)).float() / 16
+    v, beta = torch.randn(M, VL, D, generator=g), torch.randint(16, 256, (M, VL), generator=g).float() / 256
+    qkv = torch.cat([k, k, v.reshape(M, -1)], 1).to(DEV).contiguous()
+    ld, nch = qkv.shape[1] + VL * D + 2 * VL, (M + 63) // 64
+    proj, St, o = torch.zeros(M, ld, device=DEV), torch.zeros(1, VL, D, D, device=DEV), torch.zeros(M, VL * D, dtype=torch.bfloat16, device=DEV)
+    scratch = torch.zeros(nch * VL * (2 * 64 * 128 + 64 * 64 + 64) + M * VL * D, device=DEV)
+    bd, dec, nw = beta.to(DEV), torch.ones(M, VL, device=DEV), torch.ones(D, device=DEV)
+    assert _lib().qwk_gdn_scan_chunked(P(qkv), P(dec), P(bd), P(proj), ld, P(St), P(nw), KL, VL, M, P(i32([0] * M)), P(scratch), P(o), C.c_float(1e-6), S()) == 0
+    got = scratch[nch * VL * 64 * D:2 * nch * VL * 64 * D].view(nch, VL, 64, D).cpu()
+    here = there = 0.0
+    for ch in range(nch):
+        n = min(64, M - ch * 64)
+        rows = slice(ch * 64, ch * 64 + n)
+        for h in range(VL):
+            A = torch.tril(beta[rows, h, None].double() * (k[rows].double() @ k[rows].double().T), -1)
+            B = (beta[rows, h, None] * v[rows, h]).float()
+            W, want = B.clone(), torch.linalg.solve_triangular(torch.eye(n).double() + A, B.double(), upper=False)
+            for r in range(1, n):
+                acc = torch.zeros(4, D)
+                for s in range(r):
+                    acc[s & 3] = (acc[s & 3].double() + A[r, s] * W[s].double()).float()
+                W[r] -= (acc[0] + acc[1]) + (acc[2] + acc[3])
+            here += float((got[ch, h, :n].double() - want).pow(2).sum())
+            there += float((W.double() - want).pow(2).sum())
+    assert here ** 0.5 < 1.05 * there ** 0.5, (here ** 0.5, there ** 0.5)
+
+
 @pytest.mark.parametrize("bad", [20, 50, 63, 64 + 33, 64 + 50])
 def test_chunked_scan_keeps_a_row_that_is_not_finite_from_the_tiles_before_it(bad):
     """Rows before the 16-row tile of a NaN row have the bits that they have without it; the row itself and the state show it."""

@@ -14,8 +14,8 @@
 //
 // Three launches per layer:
 //   1. gdn_chunk_prep_kernel   grid (chunks, VL): everything that does not depend on the state (A, Wv, Wk, P, g),
-//      all chunks in parallel.  K K^T and Q K^T on mma.sync tf32; T = (I + A)^-1 in fp32, by halves; Wv and Wk as products
-//      with T in split tf32 (three products: what is dropped is below 2^-21).
+//      all chunks in parallel.  K K^T and Q K^T on mma.sync tf32; the two triangular solves by forward substitution in
+//      fp32, a column of each per thread.
 //   2. gdn_chunk_apply_kernel  grid (2, VL): walks the chunks in order with the state of one head's 64 value
 //      columns in registers; three tf32 products per chunk.  The value columns of a head are independent in
 //      every state-dependent product, so a head is split over two blocks.
@@ -108,28 +108,28 @@ __device__ __forceinline__ void load_tile_async(float *dst, int ld, const float 
 // ------------------------------------------------------------------------------------------------
 // 1. state-independent part of every chunk
 // ------------------------------------------------------------------------------------------------
-// What bounded it: forward substitution of all 256 columns of [Wv | Wk], one per thread - a 16-byte shared load for four multiply-adds,
-// 512 of them per warp, and 64 rows one behind the other.  Now the 64 columns of the identity go through it in two halves of 32 rows,
-// side by side, and the rest are products.  4,096 tokens, 48 heads: 407 us, now 232 (1,021: 112, 68; 100: 49, 17).
-constexpr int HC_ = CC / 2;
-constexpr int PREP_SMEM = (CC * LDA + 2 * CC * LDP + 2 * CC) * 4;      // 69 KB
+// Forward substitution in fp32, a column of Wv and a column of Wk per thread: a 16-byte shared load (four cycles, although its lanes share it) serves
+// eight multiply-adds.  As products with T = (I + A)^-1 in two tf32 parts Wv was 3.3 times as far from 64 bits as by substitution, for the
+// tensor core's sums cut off.  The whole scan, 48 heads, one column a thread / those products / now: 4,096 tokens 840 / 605 / 591 us, 1,021
+// 235 / 171 / 165, 100 77 / 40 / 44.
+constexpr int PREP_THREADS = 128, HC_ = CC / 2;
+constexpr int PREP_SMEM = (2 * CC * LDA + 3 * CC) * 4;      // 68 KB: three blocks per SM
 
-// (three blocks per SM leave too few registers: both kernels at 4,096 tokens 712 us against 683, at 1,021 205 against 196)
-__global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(GdnChunkArgs a) {
+__global__ void __launch_bounds__(PREP_THREADS, 3) gdn_chunk_prep_kernel(GdnChunkArgs a) {
     extern __shared__ __align__(16) float sm[];
     float *Ks = sm;                      // [64][LDA]
-    float *Qs = Ks + CC * LDA;           // [64][LDA]; the next two take its place once Q K^T is done
-    float *As = Qs;                      // [64][LDP]  A, then the high part of T
-    float *Ts = As + CC * LDP;           // [64][LDP]  T, then its low part
-    float *gs = Ts + CC * LDP;           // [64] cumulative log decay
+    float *Qs = Ks + CC * LDA;           // [64][LDA]
+    float *As = Qs;                      // [64][LDP]  takes Q's place once Q K^T is done
+    float *gs = Qs + CC * LDA;           // [64] cumulative log decay
     float *bs = gs + CC;                 // [64] beta
+    float *be = bs + CC;                 // [64] beta exp(g)
     const int ch = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int qkv_l = (2 * a.KL + a.VL) * CD;
     const int kh = h / (a.VL / a.KL);
     const int m0 = ch * CC;
-    load_tile_async(Ks, LDA, a.qkv, qkv_l, (a.KL + kh) * CD, m0, a.M, tid);
-    load_tile_async(Qs, LDA, a.qkv, qkv_l, kh * CD, m0, a.M, tid);
+    load_tile_async<PREP_THREADS>(Ks, LDA, a.qkv, qkv_l, (a.KL + kh) * CD, m0, a.M, tid);
+    load_tile_async<PREP_THREADS>(Qs, LDA, a.qkv, qkv_l, kh * CD, m0, a.M, tid);
     cp_async_commit();
     if (w == 0) {
         const int r0 = 2 * lane, r1 = r0 + 1;
@@ -152,51 +152,51 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(GdnChunkArgs a) 
         gs[r1] = s;
         bs[r0] = b0;
         bs[r1] = b1;
+        be[r0] = b0 * __expf(s - x1);
+        be[r1] = b1 * __expf(s);
     }
-    // V of this warp's first 16 columns as B operands (warps 0-3: Wv, 4-7: Wk): on their way under everything before the last products
-    const bool isk = w >= 4;
-    const int n0 = (w & 3) * 32;
-    float x[8][2][2];                    // [k step][tile][k t, t + 4]
-    auto fetch_v = [&](int nb) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int r = k * 8 + t + e * 4;
-#pragma unroll
-                for (int n = 0; n < 2; ++n)
-                    x[k][n][e] = m0 + r < a.M ? a.qkv[(long long)(m0 + r) * qkv_l + (2 * a.KL + h) * CD + nb + n * 8 + g] : 0.f;
-            }
-    };
-    if (!isk) fetch_v(n0);
     cp_async_wait<0>();
     __syncthreads();
-    // K K^T and Q K^T: warp tile 16 rows x 32 columns; tiles above the diagonal stay zero
-    const int r0 = (w & 3) * 16, c0 = (w >> 2) * 32;
-    float akk[4][4], aqk[4][4];
+    // K K^T and Q K^T: 16 rows per warp; tiles above the diagonal stay zero
+    const int r0 = w * 16;
+    float akk[8][4], aqk[8][4];
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
+    for (int n = 0; n < 8; ++n)
 #pragma unroll
         for (int i = 0; i < 4; ++i) akk[n][i] = aqk[n][i] = 0.f;
-    if (c0 < r0 + 16) {
-        const float *ka = a_row(Ks, LDA, r0, lane), *qa = a_row(Qs, LDA, r0, lane);
-        const float *kb0 = b_row(Ks, LDA, c0, lane), *kb1 = b_row(Ks, LDA, c0 + 16, lane);
+    {
+        const float *ka = a_row(Ks, LDA, r0, lane), *qa = a_row(Qs, LDA, r0, lane), *kb = b_row(Ks, LDA, 0, lane);
 #pragma unroll 2
         for (int k0 = 0; k0 < CD; k0 += 8) {
-            uint32_t fk[4], fq[4], b0[4], b1[4];
-            ldsm4(fk, ka + k0); ldsm4(fq, qa + k0); ldsm4(b0, kb0 + k0); ldsm4(b1, kb1 + k0);
-            round4(fk); round4(fq); round4(b0); round4(b1);
-            mma_tf32(akk[0], fk, b0[0], b0[1]); mma_tf32(akk[1], fk, b0[2], b0[3]); mma_tf32(akk[2], fk, b1[0], b1[1]); mma_tf32(akk[3], fk, b1[2], b1[3]);
-            mma_tf32(aqk[0], fq, b0[0], b0[1]); mma_tf32(aqk[1], fq, b0[2], b0[3]); mma_tf32(aqk[2], fq, b1[0], b1[1]); mma_tf32(aqk[3], fq, b1[2], b1[3]);
+            uint32_t fk[4], fq[4];
+            ldsm4(fk, ka + k0); ldsm4(fq, qa + k0);
+            round4(fk); round4(fq);
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                if (n > w) break;
+                uint32_t b[4];
+                ldsm4(b, kb + n * 16 * LDA + k0);
+                round4(b);
+                mma_tf32(akk[2 * n], fk, b[0], b[1]); mma_tf32(akk[2 * n + 1], fk, b[2], b[3]);
+                mma_tf32(aqk[2 * n], fq, b[0], b[1]); mma_tf32(aqk[2 * n + 1], fq, b[2], b[3]);
+            }
         }
     }
+    // column tid of V, the first half of its rows: on their way under what follows
+    const float *v = a.qkv + (long long)m0 * qkv_l + (2 * a.KL + h) * CD + tid;
+    float wv[HC_], wk[HC_], nv[HC_];
+    auto fetch_v = [&](int o) {
+#pragma unroll
+        for (int r = 0; r < HC_; ++r) nv[r] = m0 + o + r < a.M ? v[(long long)(o + r) * qkv_l] : 0.f;
+    };
+    fetch_v(0);
     __syncthreads();                     // every warp is done reading Q before A overwrites it
     float *Pg = a.P + ((long long)ch * a.VL + h) * CC * CC;
 #pragma unroll
-    for (int n = 0; n < 4; ++n)
+    for (int n = 0; n < 8; ++n)
 #pragma unroll
         for (int i = 0; i < 4; i += 2) {
-            const int r = r0 + g + (i >> 1) * 8, c = c0 + n * 8 + 2 * t;
+            const int r = r0 + g + (i >> 1) * 8, c = n * 8 + 2 * t;
             const float d0 = c <= r ? __expf(gs[r] - gs[c]) : 0.f, d1 = c + 1 <= r ? __expf(gs[r] - gs[c + 1]) : 0.f;
             *reinterpret_cast<float2 *>(As + r * LDP + c) = make_float2(c < r ? bs[r] * d0 * akk[n][i] : 0.f, c + 1 < r ? bs[r] * d1 * akk[n][i + 1] : 0.f);
             *reinterpret_cast<float2 *>(Pg + r * CC + c) =
@@ -204,118 +204,58 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prep_kernel(GdnChunkArgs a) 
         }
     if (tid < CC) a.G[((long long)ch * a.VL + h) * CC + tid] = gs[tid];
     __syncthreads();
-    // T = (I + A)^-1 = [T11 0; T21 T22].  T11 and T22 by forward substitution, a column per thread of the last two warps
-    if (w >= 6) {
-        const int o = (w - 6) * HC_;
+    // The rows in two halves by the same code (all 64 unrolled are 80 KB of instructions, which a short run waits for: the scan of 100 tokens 62 us, so 44).
+    // What the first half's rows add to the second's sums waits in this thread's own columns of shared memory.
+    float *sv = Ks + tid, *sk = As + CC * LDP + tid;       // [32][LDA]: K's first rows are consumed by then; [32][128]: the rest of Q's place
+#pragma unroll 1
+    for (int o = 0; o < CC; o += HC_) {
         const float *A = As + o * LDP + o;
-        float col[HC_];
 #pragma unroll
-        for (int r = 0; r < HC_; ++r) col[r] = r == lane ? 1.f : 0.f;
+        for (int r = 0; r < HC_; ++r) {
+            wv[r] = bs[o + r] * nv[r];
+            wk[r] = be[o + r] * Ks[(o + r) * LDA + tid];
+        }
 #pragma unroll
-        for (int r = 1; r < HC_; ++r) {
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};          // four independent chains
+        for (int r = 0; r < HC_; ++r) {
+            // four chains each: a row's sum is r / 4 dependent multiply-adds deep
+            float av[4] = {o ? sv[r * LDA] : 0.f, 0.f, 0.f, 0.f}, ak[4] = {o ? sk[r * CD] : 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
             for (int s4 = 0; s4 < r; s4 += 4) {
-                const float4 av = *reinterpret_cast<const float4 *>(A + r * LDP + s4);     // zero at s >= r
-                acc[0] = fmaf(av.x, col[s4], acc[0]);
-                if (s4 + 1 < r) acc[1] = fmaf(av.y, col[s4 + 1], acc[1]);
-                if (s4 + 2 < r) acc[2] = fmaf(av.z, col[s4 + 2], acc[2]);
-                if (s4 + 3 < r) acc[3] = fmaf(av.w, col[s4 + 3], acc[3]);
-            }
-            col[r] -= (acc[0] + acc[1]) + (acc[2] + acc[3]);
-        }
+                const float4 f = *reinterpret_cast<const float4 *>(A + r * LDP + s4);
+                const float x[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
-        for (int r = 0; r < HC_; ++r) Ts[(o + r) * LDP + o + lane] = col[r];
-    }
-    __syncthreads();
-    // T21 = -T22 (A21 T11), both products in fp32; the first goes to A's empty upper right.  T22's sums end at its diagonal: a row that is not
-    // finite reaches none before it
-    float *Es = As + HC_;                // [32][LDP]
-    const int er = tid >> 3, ec = (tid & 7) * 4;
-    auto half_product = [&](const float *A, const float *B, int n) {
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-        for (int s = 0; s < n; ++s) {
-            const float f = A[er * LDP + s];
-            const float4 v = *reinterpret_cast<const float4 *>(B + s * LDP + ec);
-            acc.x = fmaf(f, v.x, acc.x); acc.y = fmaf(f, v.y, acc.y); acc.z = fmaf(f, v.z, acc.z); acc.w = fmaf(f, v.w, acc.w);
-        }
-        return acc;
-    };
-    *reinterpret_cast<float4 *>(Es + er * LDP + ec) = half_product(As + HC_ * LDP, Ts, HC_);
-    __syncthreads();
-    {
-        const float4 v = half_product(Ts + HC_ * LDP + HC_, Es, er + 1);
-        *reinterpret_cast<float4 *>(Ts + (HC_ + er) * LDP + ec) = make_float4(-v.x, -v.y, -v.z, -v.w);
-    }
-    __syncthreads();
-    // T as two tf32 parts (what lies above the diagonal blocks is not read)
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const int e = tid + i * 256, at = (e >> 6) * LDP + (e & 63);
-        const float v = Ts[at];
-        const uint32_t hi = tf32(v);
-        As[at] = __uint_as_float(hi);
-        Ts[at] = __uint_as_float(tf32(v - __uint_as_float(hi)));
-    }
-    __syncthreads();
-    // Wv = T diag(beta) V, Wk = T diag(beta exp(g)) K: 32 columns per warp, 16 at a time
-    float *Wg = (isk ? a.Wk : a.Wv) + ((long long)ch * a.VL + h) * CC * CD;
-    const float *ta = a_row(As, LDP, 0, lane), *tl = a_row(Ts, LDP, 0, lane);
-#pragma unroll 1
-    for (int nb = n0; nb < n0 + 32; nb += 16) {
-        if (isk) {
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int r = k * 8 + t + e * 4;
-#pragma unroll
-                    for (int n = 0; n < 2; ++n) x[k][n][e] = Ks[r * LDA + nb + n * 8 + g];
-                }
-        } else if (nb != n0) {
-            fetch_v(nb);
-        }
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int r = k * 8 + t + e * 4;
-                const float f = isk ? bs[r] * __expf(gs[r]) : bs[r];
-#pragma unroll
-                for (int n = 0; n < 2; ++n) x[k][n][e] *= f;
-            }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float acc[2][4] = {};
-#pragma unroll
-            for (int k = 0; k < 2 * i + 2; ++k) {
-                uint32_t hi[4], lo[4];
-                ldsm4(hi, ta + i * 16 * LDP + k * 8);
-                ldsm4(lo, tl + i * 16 * LDP + k * 8);
-#pragma unroll
-                for (int n = 0; n < 2; ++n) {
-                    uint32_t b[2], bl[2];
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        b[e] = tf32(x[k][n][e]);
-                        bl[e] = tf32(x[k][n][e] - __uint_as_float(b[e]));
+                for (int e = 0; e < 4; ++e)
+                    if (s4 + e < r) {
+                        av[e] = fmaf(x[e], wv[s4 + e], av[e]);
+                        ak[e] = fmaf(x[e], wk[s4 + e], ak[e]);
                     }
-                    mma_tf32(acc[n], lo, b[0], b[1]);
-                    mma_tf32(acc[n], hi, bl[0], bl[1]);
-                    mma_tf32(acc[n], hi, b[0], b[1]);
+            }
+            wv[r] -= (av[0] + av[1]) + (av[2] + av[3]);
+            wk[r] -= (ak[0] + ak[1]) + (ak[2] + ak[3]);
+        }
+        const long long at = (((long long)ch * a.VL + h) * CC + o) * CD + tid;
+#pragma unroll
+        for (int r = 0; r < HC_; ++r) {
+            a.Wv[at + r * CD] = wv[r];
+            a.Wk[at + r * CD] = __uint_as_float(tf32(wk[r]));
+        }
+        if (o) break;
+        fetch_v(HC_);
+#pragma unroll 2
+        for (int r = 0; r < HC_; ++r) {
+            float av[4] = {0.f, 0.f, 0.f, 0.f}, ak[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int s4 = 0; s4 < HC_; s4 += 4) {
+                const float4 f = *reinterpret_cast<const float4 *>(As + (HC_ + r) * LDP + s4);
+                const float x[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    av[e] = fmaf(x[e], wv[s4 + e], av[e]);
+                    ak[e] = fmaf(x[e], wk[s4 + e], ak[e]);
                 }
             }
-#pragma unroll
-            for (int n = 0; n < 2; ++n) {
-                if (isk) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) acc[n][c] = __uint_as_float(tf32(acc[n][c]));
-                }
-                float *o = Wg + (i * 16 + g) * CD + nb + n * 8 + 2 * t;
-                *reinterpret_cast<float2 *>(o) = make_float2(acc[n][0], acc[n][1]);
-                *reinterpret_cast<float2 *>(o + 8 * CD) = make_float2(acc[n][2], acc[n][3]);
-            }
+            sv[r * LDA] = (av[0] + av[1]) + (av[2] + av[3]);
+            sk[r * CD] = (ak[0] + ak[1]) + (ak[2] + ak[3]);
         }
     }
 }
@@ -578,7 +518,7 @@ QW_API int qwk_gdn_scan_chunked(const float *qkv, const float *decay, const floa
     a.P = a.Wv + nch * VL * CC * CD;
     a.G = a.P + nch * VL * CC * CC;
     a.Oraw = a.G + nch * VL * CC;
-    gdn_chunk_prep_kernel<<<dim3((unsigned)nch, VL), 256, PREP_SMEM, s>>>(a);
+    gdn_chunk_prep_kernel<<<dim3((unsigned)nch, VL), PREP_THREADS, PREP_SMEM, s>>>(a);
     // blocks of the sequential walk: 128 / NC per head, NC chosen so that about a hundred blocks run
     if (VL >= 32) gdn_chunk_apply_kernel<64><<<dim3(2, VL), apply_threads<64>(), apply_smem<64>(), s>>>(a);
     else if (VL >= 16) gdn_chunk_apply_kernel<32><<<dim3(4, VL), 256, apply_smem<32>(), s>>>(a);
