@@ -190,3 +190,30 @@ def test_accepted_states_are_copied_whole(pairs, layers, state):
     ptrs = torch.tensor([St[i].data_ptr() for i in range(layers)], dtype=torch.int64, device=DEV)
     assert _lib().qwk_gdn_accept(P(ptrs), P(save), layers, rows, C.c_longlong(state), P(i32(pairs)), len(pairs), S()) == 0
     assert torch.equal(St, want)
+
+
+def test_logistic_function_against_64_bits():
+    """The gates of a delta-net chunk, over all of fp32's range and most densely around 0.  e^-x: the rounding of x log2(e) and of that constant, |x| 2^-23
+    together, and two units of the exponential, of which 1 / (1 + e^-x) keeps the share e^-x / (1 + e^-x); one rounding of the sum and one unit of the
+    reciprocal.  Results below 2^-126 are values of their own, in steps of 2^-149; where e^-x is infinite (x < -88.7) the result is 0."""
+    KL, VL, D = 1, 48, 128
+    edges = torch.tensor([0.0, -0.0, 1e-30, -1e-30, -87.0, -87.3, -87.4, -88.0, -88.5, -88.7, -88.8, -104.0, 88.0, 104.0, 3e38, -3e38, float("inf"), float("-inf"), float("nan")])
+    x = torch.cat([torch.linspace(-104, 104, 40001), torch.linspace(-4, 4, 20001), torch.linspace(-89, -86, 3001), edges])
+    M = (len(x) + VL - 1) // VL
+    x = torch.cat([x, torch.zeros(M * VL - len(x))]).to(DEV)
+    qkv_l = (2 * KL + VL) * D
+    ld = qkv_l + VL * D + 2 * VL
+    proj = torch.zeros(M, ld, device=DEV)
+    proj[:, qkv_l + VL * D:qkv_l + VL * D + VL] = x.view(M, VL)
+    ring, cw, al, dt = torch.zeros(1, 16, qkv_l, device=DEV), torch.zeros(qkv_l, 4, device=DEV), torch.zeros(VL, device=DEV), torch.zeros(VL, device=DEV)
+    qkv, decay, beta = torch.zeros(M, qkv_l, device=DEV), torch.zeros(M, VL, device=DEV), torch.zeros(M, VL, device=DEV)
+    run_len = i32([M] + [0] * (M - 1))
+    assert _lib().qwk_gdn_conv(P(proj), ld, P(ring), P(cw), P(al), P(dt), KL, VL, M, P(i32([0] * M)), P(i32(range(M))), P(i32([0] * M)), P(run_len), P(qkv),
+                               P(decay), P(beta), C.c_float(1e-6), S()) == 0
+    got, xd = beta.view(-1).double(), x.double()
+    want = torch.sigmoid(xd)
+    share = torch.sigmoid(-xd)
+    tol = want * (share * (xd.abs().clamp(max=104) * 2 ** -23 + 2 ** -22) + 2 ** -24 + 2 ** -23) + 2 ** -149
+    tol = torch.where(xd < -88.7, want + 2 ** -149, tol)
+    ok = torch.where(torch.isnan(xd), torch.isnan(got), (got - want).abs() <= tol)
+    assert bool(ok.all()), (x[~ok][:8].tolist(), got[~ok][:8].tolist())
