@@ -88,6 +88,36 @@ def test_delta_net_step_of_runs_equals_row_by_row(runs):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("runs", [[2], [1, 1], [3], [1, 2], [4], [5], [1, 1, 1, 1], [9, 3], [12], [13], [4, 4, 5]])
+def test_delta_net_step_gives_the_same_with_and_without_saved_states(runs):
+    """Few rows, and few rows whose states are kept, take a form of their own (four rows at a time): the bits of the form for many runs."""
+    KL, VL, D, slots, M = 2, 6, 128, len(runs), sum(runs)
+    qkv_l = (2 * KL + VL) * D
+    ld = qkv_l + VL * D + 2 * VL
+    rn = gen(M)
+    proj, cw = rn(M + 2 * 8, ld), rn(qkv_l, 4) * 0.5
+    a_log, dt, nw, ring0, S0 = rn(VL) * 0.1, rn(VL) * 0.1, 1 + 0.1 * rn(D), rn(slots + 2, 16, qkv_l), rn(slots + 2, VL, D, D) * 0.1
+    outs = []
+    for extra, saves in ((0, True), (0, False), (2, False)):          # two runs of eight rows more: always the form for many
+        lens = list(runs) + [8] * extra
+        n, starts = sum(lens), [sum(lens[:s]) for s in range(len(lens))]
+        tables = [i32([s for s, k in enumerate(lens) for _ in range(k)]), i32([7 * s + i for s, k in enumerate(lens) for i in range(k)]),
+                  i32([starts[s] for s, k in enumerate(lens) for _ in range(k)]), i32([k if i == 0 else 0 for k in lens for i in range(k)])]
+        ring, St, o = ring0.clone(), S0.clone(), torch.zeros(n, VL * D, dtype=torch.bfloat16, device=DEV)
+        save = torch.zeros(n, VL, D, D, device=DEV) if saves else None
+        scratch = torch.empty(n * (qkv_l + 2 * VL), device=DEV)
+        assert _lib().qwk_gdn_step(P(proj), ld, P(ring), P(cw), P(a_log), P(dt), P(nw), KL, VL, n, *map(P, tables), P(St), P(save), P(scratch),
+                                   P(scratch[n * qkv_l:]), P(scratch[n * (qkv_l + VL):]), P(o), C.c_float(1e-6), S()) == 0
+        torch.cuda.synchronize()
+        if saves:
+            for s in range(slots):
+                assert torch.equal(save[starts[s] + runs[s] - 1], St[s])
+        outs.append((ring[:slots], St[:slots], o[:M]))
+    for other in outs[1:]:
+        for a, b in zip(outs[0], other):
+            assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("QL,KVL,topk", [(24, 2, 512), (3, 1, 16), (32, 2, 4), (40, 2, 16)])
 def test_flash_decode_parts_match_64_bits(QL, KVL, topk):
     """The partial softmaxes of 64 list entries against 64 bits: fp32 queries, scores and weights (three bf16 parts each), bf16 keys and values.

@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(512) gdn_scan_kernel(GdnScanArgs a) {
 
 // ------------------------------------------------------------------------------------------
 // Fused step: conv + gating + L2 norm + delta-rule update + gated norm in one kernel, and the ring store of runs of up to
-// RUN_INLINE rows.  grid (M, VL), 512 threads; the block of (run start, head h) walks the run, FR = 8 rows at a time: what does not
+// RUN_INLINE rows.  grid (M, VL), 512 threads; the block of (run start, head h) walks the run, FR rows at a time: what does not
 // depend on the state - the loads, conv, norms and gates of all these rows - first, then the state's rows one behind the other with one
 // meeting each, then their outputs' norms, a warp per row.  (With a row's loads, norms and seven meetings on the chain of every row 24
 // rows of four runs took 70 us; they take 36, and one row 9.)  q/k of the head's key head are recomputed by each of the value heads that share it.
@@ -251,9 +251,11 @@ struct GdnFusedArgs {
 };
 constexpr int RUN_INLINE = GDN_RING - 4;
 
-// FR = 1: a step of one row, which has nothing to gather rows for.
-template <int FR>
-__global__ void __launch_bounds__(512, FR == 1 ? 1 : 2) gdn_fused_kernel(GdnFusedArgs a) {
+// FR rows at a time, BLOCKS on an SM.  <8, 2>, at 64 registers, where there may be many runs.  <4, 1>, whose rows have the registers to fetch their
+// operands ahead, where runs are few: then an SM has one block anyway, and the chain of its rows is what is waited for.  <1, 1>: a step of one row,
+// which has nothing to gather rows for.
+template <int FR, int BLOCKS>
+__global__ void __launch_bounds__(512, BLOCKS) gdn_fused_kernel(GdnFusedArgs a) {
     __shared__ __align__(16) float qkv[FR][3][GD];       // conv output: q (normed, scaled), k (normed), v
     __shared__ float red[2][4][GD];                      // S k, by quarter of the keys; row r in buffer r & 1
     __shared__ float part[FR][4][GD];                    // S q, the same
@@ -463,7 +465,12 @@ QW_API int qwk_gdn_step(const float *proj, int ld_proj, float *ring, const float
     a.proj = proj; a.ld_proj = ld_proj; a.ring = ring; a.cw = cw; a.A_log = A_log; a.dt_bias = dt_bias;
     a.norm_w = norm_w; a.KL = KL; a.VL = VL; a.rows = Rows{M, slot, pos, run_start, run_len};
     a.S = S; a.save = save; a.o = (bf16 *)o; a.eps = eps;
-    if (launch_pdl(M == 1 ? gdn_fused_kernel<1> : gdn_fused_kernel<8>, dim3(M, VL), dim3(512), 0, s, a) != cudaSuccess) return -2;
+    // Up to three runs of 48 heads are one block an SM.  Which rows are runs is known on the device alone: up to three rows cannot be more, and the rows
+    // of a verification step (they save their states) are long runs, so that up to RUN_INLINE of them are taken for few.  us, <8, 2> / <4, 1>, 48 heads:
+    // 2 rows 7.3 / 5.8; saved, one run of 6 rows 25.3 / 15.4, two of 6 26.0 / 17.1, three of 3 16.3 / 12.4; but four of 2 13.6 / 16.5, four of 6 32.6 /
+    // 40, and 8 rows of 8 streams 17.0 / 18.2.
+    const auto kernel = M == 1 ? gdn_fused_kernel<1, 1> : M <= 3 || (save && M <= RUN_INLINE) ? gdn_fused_kernel<4, 1> : gdn_fused_kernel<8, 2>;
+    if (launch_pdl(kernel, dim3(M, VL), dim3(512), 0, s, a) != cudaSuccess) return -2;
     if (M > RUN_INLINE) {
         const int qkv_l = (2 * KL + VL) * GD;
         if (launch_pdl(gdn_ring_kernel, dim3(M, (qkv_l + 255) / 256), dim3(256), 0, s, proj, ld_proj, ring, qkv_l, a.rows, 0, RUN_INLINE) != cudaSuccess)
