@@ -1199,10 +1199,11 @@ QW_API int qwk_gemm_tc_pair_min_n(int min_n) {
     return old;
 }
 
-// Tokens of an exchanged tile, a multiple of 16 up to 256 (0: by cost; negative: the form is not used; measurements and tests).
+// Tokens of an exchanged tile, a multiple of 16 up to 256 (0: by cost; negative: the form is not used; measurements and tests).  Any other number leaves
+// the setting as it is: a wider tile would not fit its stage nor its accumulator, and there is no such shape between the multiples.
 QW_API int qwk_gemm_tc_exchange_nt(int nt) {
     const int old = g_exchange_nt;
-    g_exchange_nt = nt;
+    if (nt <= 0 || (nt <= 256 && nt % 16 == 0)) g_exchange_nt = nt;
     return old;
 }
 // Tokens per tile where qwk_gemm_bf16_tc exchanges the operands, 0 where it keeps their roles.
