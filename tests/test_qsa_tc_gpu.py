@@ -84,6 +84,46 @@ def test_matches_64_bits_and_the_gathering_kernel(QL, KVL, base, M, topk, scale)
     assert err(o) < 4e-3 and err(o) < 1.1 * err(gathered) + 1e-5
 
 
+def _launch(L, t, QL, KVL, M, last, o, dev, host, staged, n_dev, topk, proj=None, q=None):
+    P = lambda x: None if x is None else C.c_void_p(x.data_ptr())
+    ld = last // 4 + 9
+    mask = torch.empty(M, ld, dtype=torch.int32, device="cuda:0")
+    rc = L.qwk_qsa_attend_tc(P(t["q"] if q is None else q), QL, KVL, M, last, P(t["slot"]), P(t["pos"]), *map(P, dev), *map(P, host), staged, n_dev, P(t["table"]),
+                             t["pages"], P(t["sel"]), P(t["sel_n"]), topk, P(mask), ld, P(t["proj"] if proj is None else proj), t["ldp"], P(o),
+                             C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    return rc
+
+
+def _gather(L, t, QL, KVL, M, o, topk, proj=None, q=None):
+    P = lambda x: C.c_void_p(x.data_ptr())
+    rc = L.qwk_qsa_attend_mma(P(t["q"] if q is None else q), QL, KVL, M, P(t["slot"]), P(t["pos"]), P(t["k"]), P(t["v"]), None, None, 2 * t["pages"], P(t["table"]),
+                              t["pages"], P(t["sel"]), P(t["sel_n"]), topk, 4, P(t["proj"] if proj is None else proj), t["ldp"], P(o),
+                              C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    return rc
+
+
+def _zero_tail(t, last):
+    """The rows behind the last as the kernel before this one leaves them."""
+    for p in range(last + 1, (last + 16) // 16 * 16):
+        t["k"][t["table"][1][p // 256], p % 256] = t["v"][t["table"][1][p // 256], p % 256] = 0
+
+
+@pytest.mark.parametrize("base,M,topk", [(0, 70, 512), (700, 130, 32)])
+def test_a_pool_without_device_pages(base, M, topk):
+    """Every page in the other pool, read as a staged copy and in place: the bits of the same pages in the first pool."""
+    from qwb200.ops import lib as qlib
+    L, QL, KVL, last = qlib.load(True), 12, 1, base + M - 1
+    t = _setup(QL, KVL, base, M, topk, 11)
+    _zero_tail(t, last)
+    outs = [torch.zeros(M, QL, 256, dtype=torch.bfloat16, device="cuda:0") for _ in range(3)]
+    assert _launch(L, t, QL, KVL, M, last, outs[0], [t["k"], t["v"]], [None, None], 0, 2 * t["pages"], topk) == 0
+    for staged in (1, 0):
+        assert _launch(L, t, QL, KVL, M, last, outs[1 + staged], [None, None], [t["k"], t["v"]], staged, 0, topk) == 0
+        assert torch.equal(outs[0], outs[1 + staged])
+
+
 def test_what_it_does_not_take():
     """Other group sizes, masks that do not fit, rows of the projection off 16 bytes are refused by the kernel; contexts that are long for
     their chunk, and chunks too small to matter, are the gathering kernel's."""

@@ -409,15 +409,11 @@ QW_API int qwk_qsa_attend_tc(const float *q, int QL, int KVL, int M, int last_po
     auto maps = [row](CUtensorMap *k, CUtensorMap *v, const void *kp, const void *vp, long long rows) {
         return make_map(k, kp, rows, row, row, 64) && make_map(v, vp, rows, row, row, 128);
     };
-    CUtensorMap mK, mV, hK, hV;
-    if (!maps(&mK, &mV, k_dev, v_dev, (long long)n_dev_pages * KV_PAGE)) return -3;
+    // a pool that has no pages has no map: no page id leads to it
+    CUtensorMap mK{}, mV{}, hK{}, hV{};
+    if (n_dev_pages > 0 && !maps(&mK, &mV, k_dev, v_dev, (long long)n_dev_pages * KV_PAGE)) return -3;
     staged = staged && k_host;
-    if (staged) {
-        if (!maps(&hK, &hV, k_host, v_host, 1LL << 30)) return -3;
-    } else {
-        hK = mK;
-        hV = mV;
-    }
+    if (staged && !maps(&hK, &hV, k_host, v_host, 1LL << 30)) return -3;
     qsa_mask_kernel<<<M, 128, ((size_t)(last_pos >> 7) + 1) * 4, s>>>(pos, sel, sel_n, topk, (uint32_t *)mask, ld_mask);
     QsaTcArgs a{};
     a.q = q; a.QL = QL; a.KVL = KVL; a.M = M; a.slot = slot; a.pos = pos; a.page_table = page_table; a.max_pages = max_pages;
