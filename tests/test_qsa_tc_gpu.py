@@ -124,6 +124,22 @@ def test_a_pool_without_device_pages(base, M, topk):
         assert torch.equal(outs[0], outs[1 + staged])
 
 
+@pytest.mark.parametrize("off_q,off_proj,off_o", [(2, 0, 0), (0, 2, 0), (0, 0, 2), (2, 2, 6)])
+def test_addresses_off_16_bytes_are_gathered(off_q, off_proj, off_o):
+    """Queries and gates on 8 bytes and an output on 4: what the rule accepts is served, by the kernel whose loads are that narrow."""
+    from qwb200.ops import lib as qlib
+    L, QL, KVL, base, M, topk = qlib.load(True), 12, 1, 300, 70, 32
+    t, last = _setup(QL, KVL, base, M, topk, 5), base + M - 1
+    _zero_tail(t, last)
+    at = lambda x, off: torch.cat([x.new_zeros(off), x.reshape(-1)])[off:].view(x.shape)
+    q, proj = at(t["q"], off_q), at(t["proj"], off_proj)
+    got, want = (at(torch.zeros(M, QL, 256, dtype=torch.bfloat16, device="cuda:0"), off_o) for _ in range(2))
+    assert q.data_ptr() % 16 == off_q * 4 and proj.data_ptr() % 16 == off_proj * 4 and got.data_ptr() % 16 == off_o * 2 % 16
+    assert _launch(L, t, QL, KVL, M, last, got, [t["k"], t["v"]], [None, None], 0, 2 * t["pages"], topk, proj=proj, q=q) == 0
+    assert _gather(L, t, QL, KVL, M, want, topk, proj=proj, q=q) == 0
+    assert torch.equal(got, want)
+
+
 def test_what_it_does_not_take():
     """Other group sizes, masks that do not fit, rows of the projection off 16 bytes are refused by the kernel; contexts that are long for
     their chunk, and chunks too small to matter, are the gathering kernel's."""

@@ -15,6 +15,7 @@
 // (qsa_mma.cuh: 0.66 us per query, wherever it lies).  Here a tile is read once for 21 queries of 12 heads; the price is the keys nobody
 // chose, so contexts that are long for their chunk stay with the gather (qwk_qsa_takes_tc).  24 query heads over 2, us a layer,
 // gathered / here: 1,021 tokens 226 / 57, 4,096 tokens 1941 / 336, 2,048 tokens at position 16,384 1362 / 1009.
+#include "kernels.h"
 #include "tc.cuh"
 
 namespace qw {
@@ -392,11 +393,14 @@ QW_API int qwk_qsa_takes_tc(int QL, int KVL, int M, int last_pos, int topk, int 
 // Attention of the rows of one run (slot[0], positions pos[0] + m, the last of them last_pos); what sel / sel_n name is what a row attends
 // to (see qsa_select_kernel; groups of four).  Pages from n_dev_pages on lie at k_host / v_host (null: there are none), in device memory if
 // `staged`.  mask: [M][ld_mask] words of scratch, one bit per group.  The pool's rows behind last_pos, up to the next multiple of 16, have to
-// be finite (qwk_qsa_prep_run zeroes them): the products read V in steps of 16 keys, and they meet weights of zero there.
+// be finite (qwk_qsa_prep_run zeroes them): the products read V in steps of 16 keys, and they meet weights of zero there.  Where q or proj do not lie on
+// 16 bytes, or o not on 8, the rows are gathered instead: that kernel's loads and stores are narrower.
 QW_API int qwk_qsa_attend_tc(const float *q, int QL, int KVL, int M, int last_pos, const int *slot, const int *pos, void *k_dev, void *v_dev,
                              void *k_host, void *v_host, int staged, int n_dev_pages, const int *page_table, int max_pages, const int *sel,
                              const int *sel_n, int topk, void *mask, int ld_mask, const float *proj, int ld_proj, void *o, cudaStream_t s) {
-    if (!qsa_tc_fits(QL, KVL, M, last_pos, 4, ld_mask, ld_proj) || !aligned16(q, proj, k_dev, v_dev, k_host, v_host) || ((uintptr_t)o & 7)) return -1;
+    if (!qsa_tc_fits(QL, KVL, M, last_pos, 4, ld_mask, ld_proj) || !aligned16(k_dev, v_dev, k_host, v_host)) return -1;
+    if (!aligned16(q, proj) || ((uintptr_t)o & 7))
+        return qwk_qsa_attend_mma(q, QL, KVL, M, slot, pos, k_dev, v_dev, k_host, v_host, n_dev_pages, page_table, max_pages, sel, sel_n, topk, 4, proj, ld_proj, o, s);
     static bool done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
