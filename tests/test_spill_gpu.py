@@ -127,6 +127,28 @@ def test_token_major_prefill_into_spilled_pages_equals_resident(stage):
     assert torch.equal(lw, lg) and sw == sg
 
 
+def test_staged_pages_of_several_layers_and_slots_equal_resident():
+    """Every attention layer's spilled pages are staged in the same buffer, slot after slot: a row that the cache in front of the host pages keeps is a row
+    of host memory, never one of the buffer.  Three attention layers, two slots, chunks that gather their keys."""
+    from qwb200.engine.engine import Engine, EngineOptions
+    from qwb200.models.config import ModelConfig
+    prompts = [[(i * 13 + 7) % 900 + 5 for i in range(700)], [(i * 29 + 3) % 900 + 5 for i in range(690)]]
+
+    def run(**spill):
+        cfg = ModelConfig.tiny(layer_types=("qsa", "gdn", "qsa", "qsa"))
+        eng = Engine.synthetic(cfg, EngineOptions(slots=2, slot_tokens=1024, use_graphs=False, prefill_chunk=128, **spill), device="cuda:0", exact=True,
+                               ple_rows=4096, seed=3)
+        logits = [eng.prefill(s, prompts[s]).clone() for s in range(2)]
+        steps = [eng.decode([0, 1], [5 + i, 9 + i]) for i in range(4)]
+        torch.cuda.synchronize()
+        eng.dm.check_error()
+        return eng, logits, steps
+    _, want, steps = run()
+    eng, got, spilled_steps = run(dev_pages=2, host_pages=6)
+    assert eng.dm.spill_cache is not None and "stage_k" in eng.prefiller.b
+    assert torch.equal(want[0], got[0]) and torch.equal(want[1], got[1]) and steps == spilled_steps
+
+
 def test_spill_pool_reports_its_numa_placement():
     """The host pages come either from the NUMA-placed arena (policy bind / preferred / interleave; the node they landed on
     is read back) or from the CUDA allocator (policy process); both are pinned and hold zeros before first use."""

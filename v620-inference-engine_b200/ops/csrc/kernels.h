@@ -115,6 +115,7 @@ int qwk_qsa_scores(const float *iq, int IH, const void *ck, int ck_cap, int M, c
 int qwk_qsa_select(const float *scores, int ld_scores, int M, const int *pos, int ratio, int topk, int *sel, int *sel_n, cudaStream_t s);
 int qwk_qsa_attend(const float *q, int QL, int KVL, int M, const int *slot, const int *pos, void *k_dev, void *v_dev, void *k_host, void *v_host, int n_dev_pages, const int *page_table, int max_pages, const int *sel, const int *sel_n, int topk, int ratio, int nsplit, float *pm, float *pl, float *pacc, const float *proj, int ld_proj, void *o, cudaStream_t s);
 int qwk_qsa_attend_mma(const float *q, int QL, int KVL, int M, const int *slot, const int *pos, void *k_dev, void *v_dev, void *k_host, void *v_host, int n_dev_pages, const int *page_table, int max_pages, const int *sel, const int *sel_n, int topk, int ratio, const float *proj, int ld_proj, void *o, cudaStream_t s);
+int qwk_qsa_attend_mma_staged(const float *q, int QL, int KVL, int M, const int *slot, const int *pos, void *k_dev, void *v_dev, void *k_host, void *v_host, int n_dev_pages, const int *page_table, int max_pages, const int *sel, const int *sel_n, int topk, int ratio, const float *proj, int ld_proj, void *o, cudaStream_t s);
 int qwk_set_spill_cache(void *tags, void *rows, void *miss, void *ctl, void *stats, int entries, int miss_cap);
 int qwk_spill_cache_active(int unused);
 

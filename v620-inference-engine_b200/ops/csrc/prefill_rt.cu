@@ -363,10 +363,10 @@ struct Builder {
                                             h_at(b.o, L.r0, b.o_ld), L.s));
                 return;
             }
-            PF_TRY(1, qwk_qsa_attend_mma(f_at(b.q, L.r0, d.QL * 256), d.QL, d.KVL, L.n, r.slot, r.pos, st.k_dev[qi], st.v_dev[qi],
-                                         kh, vh, d.n_dev_pages,
-                                         st.page_table, d.max_pages, i_at(b.sel, L.r0, d.idx_topk), b.sel_n + L.r0, d.idx_topk, d.idx_ratio,
-                                         f_at(b.proj, L.r0, b.proj_ld), b.proj_ld, h_at(b.o, L.r0, b.o_ld), L.s));
+            PF_TRY(1, (staged ? qwk_qsa_attend_mma_staged : qwk_qsa_attend_mma)(
+                          f_at(b.q, L.r0, d.QL * 256), d.QL, d.KVL, L.n, r.slot, r.pos, st.k_dev[qi], st.v_dev[qi], kh, vh, d.n_dev_pages,
+                          st.page_table, d.max_pages, i_at(b.sel, L.r0, d.idx_topk), b.sel_n + L.r0, d.idx_topk, d.idx_ratio,
+                          f_at(b.proj, L.r0, b.proj_ld), b.proj_ld, h_at(b.o, L.r0, b.o_ld), L.s));
         });
         // out projection (K depends on the layer kind, which every rank knows alike: resolve when run)
         cur_cat = CAT_OUT;

@@ -795,12 +795,10 @@ QW_API int qwk_qsa_attend(const float *q, int QL, int KVL, int M, const int *slo
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-// The same attention for the rows of a token-major prefill chunk, on the tensor cores: one launch for all M rows, no
-// partial buffers.  Needs QL / KVL <= 16 query heads per KV head.
-QW_API int qwk_qsa_attend_mma(const float *q, int QL, int KVL, int M, const int *slot, const int *pos, void *k_dev,
-                              void *v_dev, void *k_host, void *v_host, int n_dev_pages, const int *page_table,
-                              int max_pages, const int *sel, const int *sel_n, int topk, int ratio, const float *proj,
-                              int ld_proj, void *o, cudaStream_t s) {
+// `cache`: the host pages' rows may come from the cache in front of them.
+static int attend_mma_launch(const float *q, int QL, int KVL, int M, const int *slot, const int *pos, void *k_dev, void *v_dev, void *k_host, void *v_host,
+                             int n_dev_pages, const int *page_table, int max_pages, const int *sel, const int *sel_n, int topk, int ratio, const float *proj,
+                             int ld_proj, void *o, bool cache, cudaStream_t s) {
     if (KVL < 1 || QL % KVL != 0 || QL / KVL > 16 || M < 1 || M > 65535) return -1;
     static bool attr_done = false;
     if (!attr_done) {
@@ -811,12 +809,30 @@ QW_API int qwk_qsa_attend_mma(const float *q, int QL, int KVL, int M, const int 
     QsaAttendArgs a;
     a.q = q; a.QL = QL; a.KVL = KVL; a.rows = Rows{M, slot, pos, nullptr, nullptr};
     a.kv = make_pool(k_dev, v_dev, k_host, v_host, n_dev_pages, page_table, max_pages, KVL * HD);
-    a.sc = k_host ? g_spill : SpillCache{};
+    a.sc = k_host && cache ? g_spill : SpillCache{};
     a.sel = sel; a.sel_n = sel_n; a.topk = topk; a.ratio = ratio; a.nsplit = 0;
     a.pm = nullptr; a.pl = nullptr; a.pacc = nullptr;
     qsa_attend_mma_kernel<<<dim3(KVL, M), 128, ATT_SMEM, s>>>(a, proj, ld_proj, (bf16 *)o, g_err_ptr);
     if (a.sc.tags) spill_cache_fill_kernel<<<64, 256, 0, s>>>(a.sc, (const bf16 *)k_host, (const bf16 *)v_host, KVL * HD);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+// The same attention for the rows of a token-major prefill chunk, on the tensor cores: one launch for all M rows, no
+// partial buffers.  Needs QL / KVL <= 16 query heads per KV head.
+QW_API int qwk_qsa_attend_mma(const float *q, int QL, int KVL, int M, const int *slot, const int *pos, void *k_dev,
+                              void *v_dev, void *k_host, void *v_host, int n_dev_pages, const int *page_table,
+                              int max_pages, const int *sel, const int *sel_n, int topk, int ratio, const float *proj,
+                              int ld_proj, void *o, cudaStream_t s) {
+    return attend_mma_launch(q, QL, KVL, M, slot, pos, k_dev, v_dev, k_host, v_host, n_dev_pages, page_table, max_pages, sel, sel_n, topk, ratio, proj, ld_proj, o, true, s);
+}
+
+// The same where k_host / v_host are copies of the slot's host pages in device memory.  The cache is left alone: it knows a row by its address, and at an
+// address of the copies lies another row with every layer and slot.
+QW_API int qwk_qsa_attend_mma_staged(const float *q, int QL, int KVL, int M, const int *slot, const int *pos, void *k_dev,
+                              void *v_dev, void *k_host, void *v_host, int n_dev_pages, const int *page_table,
+                              int max_pages, const int *sel, const int *sel_n, int topk, int ratio, const float *proj,
+                              int ld_proj, void *o, cudaStream_t s) {
+    return attend_mma_launch(q, QL, KVL, M, slot, pos, k_dev, v_dev, k_host, v_host, n_dev_pages, page_table, max_pages, sel, sel_n, topk, ratio, proj, ld_proj, o, false, s);
 }
 
 // Installs (entries > 0, a power of two) or removes (entries == 0) the cache of host KV rows.  tags: entries x u64,

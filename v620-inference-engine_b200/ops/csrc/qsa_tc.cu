@@ -400,7 +400,7 @@ QW_API int qwk_qsa_attend_tc(const float *q, int QL, int KVL, int M, int last_po
                              const int *sel_n, int topk, void *mask, int ld_mask, const float *proj, int ld_proj, void *o, cudaStream_t s) {
     if (!qsa_tc_fits(QL, KVL, M, last_pos, 4, ld_mask, ld_proj) || !aligned16(k_dev, v_dev, k_host, v_host)) return -1;
     if (!aligned16(q, proj) || ((uintptr_t)o & 7))
-        return qwk_qsa_attend_mma(q, QL, KVL, M, slot, pos, k_dev, v_dev, k_host, v_host, n_dev_pages, page_table, max_pages, sel, sel_n, topk, 4, proj, ld_proj, o, s);
+        return (staged ? qwk_qsa_attend_mma_staged : qwk_qsa_attend_mma)(q, QL, KVL, M, slot, pos, k_dev, v_dev, k_host, v_host, n_dev_pages, page_table, max_pages, sel, sel_n, topk, 4, proj, ld_proj, o, s);
     static bool done[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
