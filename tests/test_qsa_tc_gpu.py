@@ -140,6 +140,35 @@ def test_addresses_off_16_bytes_are_gathered(off_q, off_proj, off_o):
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("base,M,topk,host", [(0, 70, 512, False), (600, 90, 32, False), (600, 90, 32, True), (1500, 300, 64, False)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+def test_values_that_are_not_finite_reach_only_rows_that_attend_to_them(base, M, topk, host, bad):
+    """Single values of V that are not finite, at a key that some rows chose and at positions inside the chunk: the rows that attend to them show what the
+    gathering kernel shows, every other row of the same tiles is as close to 64 bits as without them (weights and result rounded to bf16)."""
+    from qwb200.ops import lib as qlib
+    L, QL, KVL, last = qlib.load(True), 24, 2, base + M - 1
+    t = _setup(QL, KVL, base, M, topk, base + M)
+    _zero_tail(t, last)
+    want = _exact(t, QL, KVL, base, M)
+    cols = {base // 3: 5, base + M // 2: 256 + 77, last: 130}          # of K/V head 0, 1 and 0
+    hit = torch.zeros(M, QL, 256, dtype=torch.bool, device="cuda:0")
+    for at, c in cols.items():
+        t["v"][t["table"][1][at // 256], at % 256, c] = bad
+        hit[:, c // 256 * 12:c // 256 * 12 + 12, c % 256] |= t["seen"][:, at, None]
+    got, gathered = (torch.zeros(M, QL, 256, dtype=torch.bfloat16, device="cuda:0") for _ in range(2))
+    n_dev = 2 * t["pages"]
+    assert _gather(L, t, QL, KVL, M, gathered, topk) == 0
+    if host:
+        pools, n_dev = ([None, None], [t["k"], t["v"]]), 0
+    else:
+        pools = ([t["k"], t["v"]], [None, None])
+    assert _launch(L, t, QL, KVL, M, last, got, *pools, 0, n_dev, topk) == 0
+    assert bool(hit.any()) and not bool(hit.all())
+    assert torch.equal(torch.isfinite(gathered), ~hit) and torch.equal(torch.isfinite(got), ~hit)
+    assert torch.equal(torch.isnan(got), torch.isnan(gathered))
+    assert float((got.double() - want)[~hit].norm() / want[~hit].norm()) < 4e-3
+
+
 def test_what_it_does_not_take():
     """Other group sizes, masks that do not fit, rows of the projection off 16 bytes are refused by the kernel; contexts that are long for
     their chunk, and chunks too small to matter, are the gathering kernel's."""

@@ -10,6 +10,8 @@
 //   warps 4-11   softmax: two threads per row, 64 keys each; the maxima meet in shared memory, O is rescaled by 128 columns each
 // A row's set of keys is one bit per group of four (qsa_mask_kernel); only tiles that reach past a row's position compare positions.
 // The reference of the exponentials is the row's running maximum, as in the kernel that gathers.
+// A masked key's weight is 0, and 0 times a value that is not finite is NaN: a row that such a key of other rows, or of a later position, has
+// spoiled is formed again from its own keys (qt_row_alone).
 //
 // Why not gather: 2,051 rows per query are 4.2 MB out of L2 for every query, and that, at 6.8 TB/s, is what the gather costs
 // (qsa_mma.cuh: 0.66 us per query, wherever it lies).  Here a tile is read once for 21 queries of 12 heads; the price is the keys nobody
@@ -22,12 +24,14 @@ namespace qw {
 
 constexpr int QT_D = 256;                        // head dim
 constexpr int QT_ST = 5, QT_STAGE = 32768, QT_Q = 65536, QT_THREADS = 384;
+constexpr float QT_SCALE = 1.4426950408889634f / 16.f;          // log2(e) / sqrt(256)
 constexpr int QT_STG_LD = 36;                    // floats between the rows of an epilogue piece
 constexpr int QT_SMEM = QT_Q + QT_ST * QT_STAGE + 1024 /*alignment*/ + 128 /*barriers*/ + 2 * 128 * 4 /*maxima, sums*/;
 
 struct QsaTcArgs {
     const float *q;          // [M][QL][256]
     int QL, KVL, M, n_dev_pages, staged;
+    const bf16 *k_dev, *v_dev;       // the pages that the first pair of maps covers
     const bf16 *k_host, *v_host;     // pages from n_dev_pages on; staged: copies of them in device memory, which the second pair of maps covers
     const int *slot, *pos;   // one run of one slot: pos[m] = pos[0] + m
     const int *page_table;
@@ -93,10 +97,51 @@ __device__ __forceinline__ void qt_copy(unsigned char *d, const bf16 *src, int r
     }
 }
 
+// Row (m, h) from the keys that it attends to and no others, by one warp: eight of the 256 dims a lane, a key at a time, with the roundings of the tiles.
+__device__ __noinline__ void qt_row_alone(const QsaTcArgs &a, int m, int h, int lane) {
+    const int pos = a.pos[0] + m, row = a.KVL * QT_D, col = h / (a.QL / a.KVL) * QT_D + lane * 8;
+    const int *pages = a.page_table + (long long)a.slot[0] * a.max_pages;
+    const uint32_t *mask = a.mask + (long long)m * a.ld_mask;
+    const float *qr = a.q + ((long long)m * a.QL + h) * QT_D + lane * 8;
+    float q[8], acc[8], ref = -1e30f, sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        q[i] = __bfloat162float(__float2bfloat16(qr[i]));
+        acc[i] = 0.f;
+    }
+    for (int t = 0; t <= pos; ++t) {
+        if (!(mask[t >> 7] >> ((t >> 2) & 31) & 1u)) {
+            t |= 3;                              // none of the group's four
+            continue;
+        }
+        const int page = pages[t / KV_PAGE];
+        const bool host = page >= a.n_dev_pages;
+        const long long at = ((long long)(host ? page - a.n_dev_pages : page) * KV_PAGE + t % KV_PAGE) * row + col;
+        const uint4 k = *reinterpret_cast<const uint4 *>((host ? a.k_host : a.k_dev) + at), v = *reinterpret_cast<const uint4 *>((host ? a.v_host : a.v_dev) + at);
+        const uint32_t kw[4] = {k.x, k.y, k.z, k.w}, vw[4] = {v.x, v.y, v.z, v.w};
+        float s = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s = fmaf(q[i], i & 1 ? bf16_hi(kw[i >> 1]) : bf16_lo(kw[i >> 1]), s);
+        s = warp_sum(s) * QT_SCALE;
+        const float nref = fmaxf(ref, s), f = ex2(ref - nref), x = ex2(s - nref), w = __bfloat162float(__float2bfloat16(x));
+        ref = nref;
+        sum = fmaf(sum, f, x);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) acc[i] = fmaf(acc[i], f, w * (i & 1 ? bf16_hi(vw[i >> 1]) : bf16_lo(vw[i >> 1])));
+    }
+    const float inv = 1.f / sum, *gate = a.proj + (long long)m * a.ld_proj + h * 2 * QT_D + QT_D + lane * 8;
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[i] = pack_bf16(acc[2 * i] * inv * sigmoidf_(gate[2 * i]), acc[2 * i + 1] * inv * sigmoidf_(gate[2 * i + 1]));
+    uint2 *out = reinterpret_cast<uint2 *>(a.o + ((long long)m * a.QL + h) * QT_D + lane * 8);
+    out[0] = make_uint2(o[0], o[1]);
+    out[1] = make_uint2(o[2], o[3]);
+}
+
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QT_THREADS, 1) qsa_attend_tc_kernel(const __grid_constant__ CUtensorMap mapK,
                                                                                                const __grid_constant__ CUtensorMap mapV,
                                                                                                const __grid_constant__ CUtensorMap hostK,
-                                                                                               const __grid_constant__ CUtensorMap hostV, QsaTcArgs a) {
+                                                                                               const __grid_constant__ CUtensorMap hostV, const __grid_constant__ QsaTcArgs a) {
     extern __shared__ unsigned char raw[];
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
@@ -236,7 +281,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QT_THREADS, 1) qsa_a
         const uint32_t p_bar = map_to_cta(smem_u32(p_full), 0);
         const int m = R < rows ? R / per_kv : 0, pos = R < rows ? pos0 + m : -1;
         const uint32_t *mask = a.mask + (long long)m * a.ld_mask;
-        constexpr float scale = 1.4426950408889634f / 16.f;          // log2(e) / sqrt(256)
+        constexpr float scale = QT_SCALE;
         float ref = -1e30f, sum = 0.f;
         bool ok = true;                      // after a wait that ran out: no further waits, but every meeting
         uint32_t next = pos >= 0 ? __ldg(mask) : 0u;
@@ -334,13 +379,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QT_THREADS, 1) qsa_a
         asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");
         s_max[half * 128 + r] = sum;
         asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");
+        const float total = s_max[r] + s_max[128 + r];
+        float z[4] = {0.f, 0.f, 0.f, 0.f};   // NaN behind a value that is not finite
         if (ok) {
-            const float inv = 1.f / (s_max[r] + s_max[128 + r]);
+            const float inv = 1.f / total;
             float *stg = reinterpret_cast<float *>(st) + (warp - 4) * 32 * QT_STG_LD;
 #pragma unroll 1
             for (int c0 = 0; c0 < 128; c0 += 32) {
                 uint32_t v[32];
                 tmem_ld32(obase + c0, v);
+#pragma unroll
+                for (int c = 0; c < 32; ++c) z[c & 3] = fmaf(__uint_as_float(v[c]), 0.f, z[c & 3]);
 #pragma unroll
                 for (int c = 0; c < 32; c += 4)
                     *reinterpret_cast<float4 *>(stg + lane * QT_STG_LD + c) =
@@ -356,6 +405,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(QT_THREADS, 1) qsa_a
                 if (c0 + 32 < 128) fetch_gates(c0 + 32);
                 __syncwarp();
             }
+        }
+        // A row whose own scores are finite has a finite sum.  The two warps share what they found and take every other row of it
+        const float zs = (z[0] + z[1]) + (z[2] + z[3]);
+        const unsigned mine = __ballot_sync(0xffffffffu, zs != zs && total > 0.f && total < INFINITY);
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");
+        if (lane == 0) s_max[half * 128 + q * 32] = __uint_as_float(mine);
+        asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");
+        for (unsigned left = (__float_as_uint(s_max[q * 32]) | __float_as_uint(s_max[128 + q * 32])) & (half ? 0xaaaaaaaau : 0x55555555u); left; left &= left - 1) {
+            const int RR = R0 + (int)rank * 128 + q * 32 + __ffs(left) - 1, mm = RR / per_kv;
+            qt_row_alone(a, mm, kvh * per_kv + RR - mm * per_kv, lane);
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -421,6 +480,7 @@ QW_API int qwk_qsa_attend_tc(const float *q, int QL, int KVL, int M, int last_po
     qsa_mask_kernel<<<M, 128, ((size_t)(last_pos >> 7) + 1) * 4, s>>>(pos, sel, sel_n, topk, (uint32_t *)mask, ld_mask);
     QsaTcArgs a{};
     a.q = q; a.QL = QL; a.KVL = KVL; a.M = M; a.slot = slot; a.pos = pos; a.page_table = page_table; a.max_pages = max_pages;
+    a.k_dev = (const bf16 *)k_dev; a.v_dev = (const bf16 *)v_dev;
     a.n_dev_pages = k_host ? n_dev_pages : 0x7fffffff; a.staged = staged; a.k_host = (const bf16 *)k_host; a.v_host = (const bf16 *)v_host;
     a.mask = (const uint32_t *)mask; a.ld_mask = ld_mask; a.proj = proj; a.ld_proj = ld_proj; a.o = (bf16 *)o; a.err = g_err_ptr;
     const long long rows = (long long)M * (QL / KVL);
