@@ -64,6 +64,26 @@ def test_forms_that_keep_the_roles_match_64_bits(exchange, T, N, K, form, dtype)
     assert float((got.double() - ref).norm() / ref.norm()) < (1e-5 if dtype == torch.float32 else 2 ** -8)
 
 
+@pytest.mark.parametrize("T,N,K,form", [(100, 256, 1024, 3), (300, 512, 64, 0), (520, 12800, 64, 1), (777, 10200, 320, 1), (777, 4352, 64, 2), (300, 10190, 136, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("off", [0, 1, 2, 4])
+@pytest.mark.parametrize("stage", [1, 0])
+def test_forms_that_keep_the_roles_at_any_address_with_and_without_staging(exchange, T, N, K, form, dtype, off, stage):
+    """Each form that products between ranks take, told to run (none of these is exchanged): fp32 output through the staging buffers and straight from
+    registers, outputs off 16 bytes, nothing beside them.  k is one chain in every form but the split one: the bits of an aligned output."""
+    lib = _lib()
+    exchange(-1)
+    assert lib.qwk_gemm_tc_form(T, N, K) == form and lib.qwk_gemm_tc_exchanged(T, N, K) == 0
+    old = lib.qwk_gemm_tc_stage_local(stage)
+    try:
+        A, W, got = _product(T, N, K, dtype, off)
+    finally:
+        lib.qwk_gemm_tc_stage_local(old)
+    assert torch.equal(got, _product(T, N, K, dtype)[2])
+    ref = A.double() @ W.double().T
+    assert float((got.double() - ref).norm() / ref.norm()) < (1e-5 if dtype == torch.float32 else 2 ** -8)
+
+
 @pytest.mark.parametrize("L,heads", [(128, 1), (129, 2), (600, 16), (2100, 3), (3520, 16)])
 def test_vision_attention_with_its_keys_dealt_evenly(L, heads):
     """Runs that begin and end inside a unit's keys, units in two and more runs, a last key tile that is not whole: against 64 bits (weights and
