@@ -1,11 +1,13 @@
 """Throughput of the tcgen05 GEMM on the prefill shapes against cuBLAS (torch.matmul), CUDA-event
 timed with operands rotated through a set larger than L2:
 
-    python -m qwb200.tools.gemm_bench [--tokens 4096] [--fp32] [--wide MIN_N] [--pair MIN_N] [--stage-local]
+    python -m qwb200.tools.gemm_bench [--tokens 4096] [--fp32] [--wide MIN_N] [--pair MIN_N] [--stage-local {0,1}] [--exchange NT]
 
 ``--wide`` / ``--pair`` set from which width on the 128 x 256 tile form / the CTA-pair form (256 x 256 tiles,
-tcgen05.mma.cta_group::2) is used (0 = never); ``--stage-local`` writes fp32 output through the epilogue's staging
-buffers; ``--fp32`` measures fp32 output instead of bf16."""
+tcgen05.mma.cta_group::2) is used (0 = never); ``--stage-local 1`` / ``0`` writes fp32 output through the epilogue's staging
+buffers / straight from registers.  With any of the three the operands keep their roles; without them most shapes take
+the exchanged form (weight rows as the pair's 256 rows), whose tokens a tile ``--exchange`` sets (0 = by cost, -1 =
+never).  ``--fp32`` measures fp32 output instead of bf16."""
 import argparse
 import json
 import os
@@ -37,7 +39,8 @@ def main():
     ap.add_argument("--fp32", action="store_true")
     ap.add_argument("--wide", type=int, default=-1)
     ap.add_argument("--pair", type=int, default=-1)
-    ap.add_argument("--stage-local", action="store_true")
+    ap.add_argument("--stage-local", type=int, choices=(0, 1), nargs="?", const=1)
+    ap.add_argument("--exchange", type=int)
     a = ap.parse_args()
     from ..ops import lib as qlib
     L = qlib.load(True)
@@ -45,8 +48,12 @@ def main():
         L.qwk_gemm_tc_wide_min_n(a.wide)
     if a.pair >= 0:
         L.qwk_gemm_tc_pair_min_n(a.pair)
-    if a.stage_local:
-        L.qwk_gemm_tc_stage_local(1)
+    if a.stage_local is not None:
+        L.qwk_gemm_tc_stage_local(a.stage_local)
+    if a.exchange is not None:
+        L.qwk_gemm_tc_exchange_nt(a.exchange)
+    elif a.wide >= 0 or a.pair >= 0 or a.stage_local is not None:
+        L.qwk_gemm_tc_exchange_nt(-1)          # what is asked for is a form that keeps the roles
     T = a.tokens
     peak = 1600.0
     p = os.path.join(os.path.dirname(__file__), "..", "..", "MEASURED_PEAKS.json")
@@ -71,7 +78,9 @@ def main():
                 torch.matmul(As[i[0]], Ws[i[0]].T, out=out)
         t1, t2 = time_fn(ours), time_fn(cublas)
         fl = 2.0 * T * N * Kd / 1e9
-        print(f"{name:14s} T={T} N={N:6d} K={Kd:5d}: tcgen05 {t1 * 1e3:8.1f} us {fl / t1:7.1f} TFLOP/s ({100 * fl / t1 / peak:4.1f}% of measured cuBLAS peak) | "
+        tokens = L.qwk_gemm_tc_exchanged(T, N, Kd)
+        form = f"exchanged, {tokens} tokens" if tokens else ("128x128", "128x256", "pairs", "split")[L.qwk_gemm_tc_form(T, N, Kd)]
+        print(f"{name:14s} [{form}] T={T} N={N:6d} K={Kd:5d}: tcgen05 {t1 * 1e3:8.1f} us {fl / t1:7.1f} TFLOP/s ({100 * fl / t1 / peak:4.1f}% of measured cuBLAS peak) | "
               f"cuBLAS {t2 * 1e3:8.1f} us {fl / t2:7.1f} TFLOP/s", flush=True)
 
 
