@@ -47,7 +47,7 @@ constexpr int SG_THREADS = SG_CONSUMERS + 32;      // + the producer warp
 constexpr int SG_TILE = 16;              // weight rows per tile
 constexpr int SG_PN = 20;                // floats between the activation rows of a partial tile (16 used): its stores hit 32 banks
 constexpr int SG_STEPS = 6;              // k steps of a warp in a stage of 768 columns
-constexpr int SG_MIN_STAGES = 4;          // two for each group
+constexpr int SG_STAGES = 6, SG_MIN_STAGES = 4;      // three for each group, or at least two
 constexpr size_t SG_SMEM_MAX = 226 * 1024;
 
 struct SGemvSmem {
@@ -279,19 +279,23 @@ static inline size_t sgemv_plan(SGemvArgs &a, int NT, int &grid) {
             // the sums wait in registers between the passes: at most one tile per group
             if (a.KH > 1 && (nitems > SG_GROUPS * grid || a.fi.active)) break;
             const int most = (a.K + 127) / 128;
-            for (int P = ((most + SG_STEPS - 1) / SG_STEPS + a.KH - 1) / a.KH * a.KH; P <= most; P += a.KH) {
-                const int Kc = (most + P - 1) / P * 128;
-                if ((a.K + Kc - 1) / Kc != P || (Kc < least * 128 && P > 1)) continue;
-                const size_t xbytes = (size_t)xrows * ((a.KH == 1 ? a.K : P / a.KH * Kc) * 2 + ROW_PAD), stage = (size_t)SG_TILE * Kc * 2;
-                if (fixed + xbytes + SG_MIN_STAGES * stage > SG_SMEM_MAX) continue;
-                const long long ns = ((long long)SG_SMEM_MAX - (long long)(fixed + xbytes)) / (long long)stage;
-                a.P = P;
-                a.Kc = Kc;
-                a.box3 = a.K % 64 == 0;
-                a.nstage = (int)(ns > 8 ? 8 : ns);
-                a.groups = SG_GROUPS;
-                return fixed + xbytes + (size_t)a.nstage * stage;
-            }
+            // Three stages for each group, where shorter parts make room for them, before two of longer parts: at 16 rows of 2,560 (four parts with two
+            // stages / five with three) 16,480 weight rows take 20.7 / 19.5 us and 248,320 227 / 217.  In passes over k the longer parts are better (2,560 x
+            // 6,144 at 24 rows 18.7 us, shorter 19.7).
+            for (int stages = a.KH == 1 ? SG_STAGES : SG_MIN_STAGES; stages >= SG_MIN_STAGES; stages -= SG_GROUPS)
+                for (int P = ((most + SG_STEPS - 1) / SG_STEPS + a.KH - 1) / a.KH * a.KH; P <= most; P += a.KH) {
+                    const int Kc = (most + P - 1) / P * 128;
+                    if ((a.K + Kc - 1) / Kc != P || (Kc < least * 128 && P > 1)) continue;
+                    const size_t xbytes = (size_t)xrows * ((a.KH == 1 ? a.K : P / a.KH * Kc) * 2 + ROW_PAD), stage = (size_t)SG_TILE * Kc * 2;
+                    if (fixed + xbytes + stages * stage > SG_SMEM_MAX) continue;
+                    const long long ns = ((long long)SG_SMEM_MAX - (long long)(fixed + xbytes)) / (long long)stage;
+                    a.P = P;
+                    a.Kc = Kc;
+                    a.box3 = a.K % 64 == 0;
+                    a.nstage = (int)(ns > 8 ? 8 : ns);
+                    a.groups = SG_GROUPS;
+                    return fixed + xbytes + (size_t)a.nstage * stage;
+                }
         }
     return 0;
 }
