@@ -166,6 +166,44 @@ def test_flash_decode_parts_match_64_bits(QL, KVL, topk):
             assert float((o[m, h].double() - want).norm() / want.norm()) < 2 ** -8
 
 
+@pytest.mark.parametrize("heads", [12, 17])
+def test_flash_decode_with_infinite_keys_and_values(heads):
+    """Against 64 bits.  A key with one infinite value has a score of -inf for the queries of the other sign there: no weight, and no part of the list
+    that holds nothing else counts.  A row that gives such a key a score of +inf is NaN; an infinite value is an infinite output where the key has weight.
+    (The scalar kernel, which takes 17 heads a KV head, makes a part NaN whose warp meets such a key first: its lists have them later.)"""
+    topk, ratio, page, KVL = 64, 4, 256, 2
+    rn = gen(heads)
+    lists = {70: [5], 65: [64], 64: list(range(64)), 200: list(range(64, 128)), 130: list(range(128, 131))} if heads == 12 else {70: [13], 200: [13, 100, 200]}
+    positions = list(lists)
+    M, QL = len(positions), heads * KVL
+    k, v = (rn(M, page, KVL, 256).bfloat16() for _ in range(2))
+    q = rn(M, KVL, heads, 256)
+    for m, p in enumerate(positions):
+        k[m, lists[p], :, 3] = float("inf")
+        q[m, :, 1:, 3] = -q[m, :, 1:, 3].abs()
+        q[m, 0, 0, 3] = 1.0                                # one head that the infinite keys win
+        at = 64 if p == 64 else 35                          # a key with weight
+        v[m, at, 1, 7], v[m, at, 0, 9] = float("inf"), float("-inf")
+    table, sel, sel_n = torch.arange(M, dtype=torch.int32, device=DEV), torch.zeros(M, topk, dtype=torch.int32, device=DEV), torch.full((M,), -1, dtype=torch.int32, device=DEV)
+    nsplit = (topk * ratio + ratio + 63) // 64
+    pm, pl, pacc = torch.full((M, QL, nsplit), 7.0, device=DEV), torch.full((M, QL, nsplit), float("nan"), device=DEV), torch.full((M, QL, nsplit, 256), float("nan"), device=DEV)
+    o, proj = torch.zeros(M, QL, 256, dtype=torch.bfloat16, device=DEV), torch.full((M, QL * 512), 30.0, device=DEV)          # gates of 1
+    assert _lib().qwk_qsa_attend(P(q), QL, KVL, M, P(i32(range(M))), P(i32(positions)), P(k), P(v), None, None, M, P(table), 1, P(sel), P(sel_n),
+                                 topk, ratio, nsplit, P(pm), P(pl), P(pacc), P(proj), QL * 512, P(o), S()) == 0
+    torch.cuda.synchronize()
+    got = o.view(M, KVL, heads, 256).double()
+    for m, p in enumerate(positions):
+        w = torch.softmax(torch.einsum("khd,tkd->kht", q[m].double(), k[m, :p + 1].double()) / 16, 2)
+        # keys without weight have no part in the output, whatever their values are
+        want = torch.where(w[..., None] > 0, w[..., None] * v[m, :p + 1].double().permute(1, 0, 2)[:, None], torch.where(w[..., None].isnan(), w[..., None], 0.0)).sum(2)
+        assert bool(torch.isnan(want[0, 0]).all()) and bool(torch.isfinite(want).any())
+        assert torch.equal(torch.isnan(got[m]), torch.isnan(want)), p
+        inf = torch.isinf(want)
+        assert torch.equal(got[m][inf], want[inf]) and torch.equal(torch.isinf(got[m]), inf)
+        ok = torch.isfinite(want)
+        assert float((got[m] - want)[ok].norm() / want[ok].norm()) < 2 ** -8
+
+
 @pytest.mark.parametrize("size", [0.3, 1.0, 4.0])
 def test_flash_decode_on_tensor_cores_is_as_exact_as_the_scalar_kernel(size):
     """The merged parts before bf16, against 64 bits, of both kernels: 17 heads per KV head take the scalar one, 12 of the same heads the tensor

@@ -10,6 +10,7 @@
 // KV pages: a page holds KV_PAGE tokens of one layer, row = KVL*256 bf16.  page ids < n_dev_pages
 // live in the device pool, the rest in the host pool (pinned, mapped: the kernels read host RAM
 // directly).  page_table[slot][i] is the page of tokens i*KV_PAGE ...
+#include <cfloat>
 #include <type_traits>
 
 #include "common.cuh"
@@ -621,12 +622,13 @@ __global__ void __launch_bounds__(256) qsa_attend_kernel(QsaAttendArgs a) {
         }
         const long long o = ((long long)m * a.QL + h0 + j) * a.nsplit + sp;
         a.pacc[o * HD + d] = A;
-        if (d == 0) { a.pm[o] = M; a.pl[o] = L; }
+        if (d == 0) { a.pm[o] = M == -INFINITY && sp * 64 < count ? -FLT_MAX : M; a.pl[o] = L; }
     }
 }
 
-// grid (M, QL), 256 threads: merge the splits, apply sigmoid(gate), write bf16.  Only the splits in front of the list's end hold anything.  The
-// weights are formed once per block and the partial sums' loads are eight at a time (24 rows, one split behind the other: 9.5 us, now 9.0).
+// grid (M, QL), 256 threads: merge the splits, apply sigmoid(gate), write bf16.  The splits behind the list's end have a maximum of -inf and hold
+// nothing (one in front of it whose scores are all -inf, for keys that are infinite, has the lowest number instead, and sums of 0).  The weights are
+// formed once per block and the partial sums' loads are eight at a time (24 rows, sums out of memory: one split behind the other 22 us, now 15).
 __global__ void __launch_bounds__(256) qsa_combine_kernel(const float *pm, const float *pl, const float *pacc, int nsplit,
                                                           const float *proj, int ld_proj, int QL, bf16 *o) {
     extern __shared__ float s_w[];          // [nsplit] weights, [nsplit] sums

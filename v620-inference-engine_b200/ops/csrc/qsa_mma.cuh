@@ -68,7 +68,7 @@ __device__ __forceinline__ void att_issue(const QsaAttendArgs &a, bf16 *dst_tile
 // Error of the merged output before bf16 against 64 bits, queries of size 0.3 / 1 / 2 / 4: scalar form 0.95, 1.34, 2.41, 3.64e-7; here 0.62, 1.18,
 // 2.36, 3.51e-7.
 // In a scalar form (four heads a block, a warp per token) each token's rows were fetched once for every four heads and every score was five
-// shuffles.  With the merge, at 4,096 tokens: 24 rows 181 us, now 55; 8 rows 69 / 25; one 17.4 / 11.
+// shuffles.  With the merge, at 4,096 tokens: 24 rows 197 us, now 57; 8 rows 67 / 21.6; one 17.2 / 11.1.
 // grid (nsplit, M, KVL), 256 threads.
 // ------------------------------------------------------------------------------------------------------------------
 constexpr int AD_SMEM = (2 * AT * KV_LD + 3 * 16 * KV_LD + 3 * 16 * P_LD) * 2 + 2 * 8 * 16 * 4 + 16;
@@ -83,6 +83,10 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t (&p)[3]) {
         y -= bf16_hi(p[i]);
     }
 }
+
+// Sum over first parts + sum over the others.  An infinity of K or V has its sign from the first part alone: the others may be zero or of the other sign, and
+// their products with it would make the sum NaN.
+__device__ __forceinline__ float split_sum(float first, float rest) { return fabsf(first) == INFINITY ? first : rest + first; }
 
 __global__ void __launch_bounds__(256, 2) qsa_attend_split_kernel(QsaAttendArgs a, ErrorWord *g_err) {
     extern __shared__ __align__(16) unsigned char att_sm[];
@@ -157,7 +161,8 @@ __global__ void __launch_bounds__(256, 2) qsa_attend_split_kernel(QsaAttendArgs 
     float s[4], tm[2] = {-INFINITY, -INFINITY};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        s[i] = sp * AT + w * 8 + 2 * t4 + (i & 1) < count ? (s2[i] + ((s1[0][i] + s1[1][i]) + (s1[2][i] + s1[3][i]))) * 0.0625f : -INFINITY;       // 1/sqrt(256)
+        const float first = (s1[0][i] + s1[1][i]) + (s1[2][i] + s1[3][i]);
+        s[i] = sp * AT + w * 8 + 2 * t4 + (i & 1) < count ? split_sum(first, s2[i]) * 0.0625f : -INFINITY;       // 1/sqrt(256)
         tm[i >> 1] = fmaxf(tm[i >> 1], s[i]);
     }
 #pragma unroll
@@ -167,11 +172,13 @@ __global__ void __launch_bounds__(256, 2) qsa_attend_split_kernel(QsaAttendArgs 
         if (t4 == 0) s_max[w * 16 + g + 8 * h] = tm[h];
     }
     __syncthreads();
+    bool none[2];                                            // every score is -inf (keys that are infinite): the block adds nothing to this row
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-        float mx = s_max[g + 8 * h];                         // the list's first entry of the block exists: finite
+        float mx = s_max[g + 8 * h];
 #pragma unroll
         for (int k = 1; k < 8; ++k) mx = fmaxf(mx, s_max[k * 16 + g + 8 * h]);
+        none[h] = mx == -INFINITY;
         const float p0 = __expf(s[2 * h] - mx), p1 = __expf(s[2 * h + 1] - mx);
         uint32_t p[3];
         split3(p0, p1, p);
@@ -190,8 +197,8 @@ __global__ void __launch_bounds__(256, 2) qsa_attend_split_kernel(QsaAttendArgs 
 #pragma unroll
         for (int k = 0; k < 8; ++k) l += s_l[k * 16 + tid];
         const long long o = ((long long)m * a.QL + h0 + tid) * a.nsplit + sp;
-        a.pm[o] = mx;
-        a.pl[o] = l;
+        a.pm[o] = fmaxf(mx, -FLT_MAX);
+        a.pl[o] = mx == -INFINITY ? 0.f : l;
     }
     ok = ok && mbar_wait_warp(vbar, 0u, g_err);
     // ---- P V for this warp's 32 output dims, summed as the scores are
@@ -226,7 +233,7 @@ __global__ void __launch_bounds__(256, 2) qsa_attend_split_kernel(QsaAttendArgs 
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) acc[n][i] += acc2[n][i];
+        for (int i = 0; i < 4; ++i) acc[n][i] = none[i >> 1] ? 0.f : split_sum(acc[n][i], acc2[n][i]);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         const int r = g + 8 * h;
