@@ -204,6 +204,16 @@ def test_flash_decode_with_infinite_keys_and_values(heads):
         assert float((got[m] - want)[ok].norm() / want[ok].norm()) < 2 ** -8
 
 
+def test_router_rows_without_room_are_refused():
+    """Rows so long that shared memory has no room for them in any plan: an error of the launcher, and nothing runs."""
+    K_, nrs, M = 65536, 16, 8
+    W, x = torch.zeros(nrs, K_, dtype=torch.bfloat16, device=DEV), torch.zeros(M, K_, dtype=torch.bfloat16, device=DEV)
+    rs, pe, pw, ticket = torch.full((M, nrs), 7.0, device=DEV), torch.full((M, 2), -7, dtype=torch.int32, device=DEV), torch.full((M, 2), 7.0, device=DEV), i32([0])
+    assert _lib().qwk_moe_router(P(W), P(x), P(rs), nrs, K_, M, K_, nrs, 2, 640, 0, nrs, P(pe), P(pw), None, P(ticket), None, None, 0, 0, S()) == -2
+    torch.cuda.synchronize()
+    assert bool((rs == 7.0).all()) and bool((pe == -7).all()) and bool((pw == 7.0).all()) and int(ticket) == 0
+
+
 @pytest.mark.parametrize("size", [0.3, 1.0, 4.0])
 def test_flash_decode_on_tensor_cores_is_as_exact_as_the_scalar_kernel(size):
     """The merged parts before bf16, against 64 bits, of both kernels: 17 heads per KV head take the scalar one, 12 of the same heads the tensor

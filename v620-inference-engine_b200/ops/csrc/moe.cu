@@ -165,6 +165,7 @@ static cudaError_t launch_router(SGemvArgs &a, const RouteArgs &r, cudaStream_t 
         if (smem2) return launch_router_nt<2>(a, r, smem2, grid, s);
     }
     const size_t smem1 = sgemv_plan(a, 1, grid);
+    if (!smem1) return cudaErrorInvalidValue;          // rows that shared memory has no room for
     return launch_router_nt<1>(a, r, smem1, grid, s);
 }
 
