@@ -253,7 +253,6 @@ class DeviceModel:
             "proj": ((R, max(sc.gdn_proj_l, sc.qsa_proj_l)), f32), "inj_a": ((R, c.hc), f32), "inj_b": ((R, c.hc), f32),
             "partial": ((R, c.hidden), f32), "out_a": ((R, sc.sh), f32), "out_b": ((R, sc.sh), f32),
             "o": ((R, max(sc.gdn_vl * c.gdn_dim, sc.qh_l * c.head_dim)), bf),
-            "qkv": ((R, sc.gdn_qkv_l), f32), "decay": ((R, sc.gdn_vl), f32), "beta": ((R, sc.gdn_vl), f32),
             "q": ((R, sc.qh_l, c.head_dim), f32), "iq": ((R, c.idx_heads, c.idx_dim), f32),
             "scores": ((R, d.score_cap), f32), "sel": ((R, c.idx_topk_blocks), i32), "sel_n": ((R,), i32),
             "pm": ((R, sc.qh_l, d.nsplit), f32), "pl": ((R, sc.qh_l, d.nsplit), f32),

@@ -460,7 +460,7 @@ QW_API int qwk_gdn_step(const float *proj, int ld_proj, float *ring, const float
                         const float *dt_bias, const float *norm_w, int KL, int VL, int M, const int *slot, const int *pos,
                         const int *run_start, const int *run_len, float *S, float *save, float *qkv, float *decay,
                         float *beta, void *o, float eps, cudaStream_t s) {
-    (void)qkv; (void)decay; (void)beta;          // scratch of the step in three kernels
+    (void)qkv; (void)decay; (void)beta;          // not read: null will do
     GdnFusedArgs a;
     a.proj = proj; a.ld_proj = ld_proj; a.ring = ring; a.cw = cw; a.A_log = A_log; a.dt_bias = dt_bias;
     a.norm_w = norm_w; a.KL = KL; a.VL = VL; a.rows = Rows{M, slot, pos, run_start, run_len};

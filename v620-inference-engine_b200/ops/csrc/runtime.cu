@@ -233,7 +233,6 @@ void gdn_block(Ctx &c, const QwLayer &L, int flags) {
     const QwBuffers &b = md.b;
     const QwRows &r = *c.rows;
     const int M = r.M, gi = L.state_index;
-    const int qkv_l = (2 * d.KL + d.VL) * 128;
     await_bin(c);
     QW_OP(1, L.Wproj, (size_t)d.proj_gdn * d.H * 2,
           qwk_gemv_bf16(L.Wproj, b.bin, b.proj, nullptr, d.proj_gdn, d.H, M, d.H, d.H, d.proj_gdn, 0, 1, 0, 0, 0, c.s));
@@ -242,7 +241,7 @@ void gdn_block(Ctx &c, const QwLayer &L, int flags) {
         save = b.gdn_save + (size_t)gi * d.max_rows * d.VL * 128 * 128;
     QW_OP((M <= 12 ? 1 : 2), nullptr, 0, qwk_gdn_step(b.proj, d.proj_gdn, md.st.gdn_ring[gi], L.cw, L.A_log, L.dt_bias, L.gdn_norm,
                                                       d.KL, d.VL, M, r.slot, r.pos, r.run_start, r.run_len, md.st.gdn_S[gi], save,
-                                                      b.qkv, b.decay, b.beta, b.o, d.eps, c.s));
+                                                      nullptr, nullptr, nullptr, b.o, d.eps, c.s));
     const int K = d.VL * 128;
     send_partial(c, true);
     QW_OP(1, L.Wout, (size_t)d.H * K * 2, qwk_gemv_bf16(L.Wout, b.o, b.partial, nullptr, d.H, K, M, K, K, d.H, 0, 1, 0, 0, 0, c.s));

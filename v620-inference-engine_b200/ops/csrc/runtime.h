@@ -96,7 +96,6 @@ typedef struct QwBuffers {
     float *partial;      // [rows][H] block output before the reduce-scatter
     float *out_a, *out_b;// [rows][SH] block outputs after it
     void *o;             // bf16 [rows][max(VL*128, QL*256)]
-    float *qkv, *decay, *beta;        // GDN
     float *q, *iq, *scores;           // QSA
     int *sel, *sel_n;
     float *pm, *pl, *pacc;
