@@ -204,6 +204,28 @@ def test_flash_decode_with_infinite_keys_and_values(heads):
         assert float((got[m] - want)[ok].norm() / want[ok].norm()) < 2 ** -8
 
 
+@pytest.mark.parametrize("off,nsplit", [(1, 6)])
+def test_flash_decode_with_scratch_at_any_address_and_many_splits(off, nsplit):
+    """Sums that lie on 4 bytes, and more splits than a list needs (behind its end they hold nothing): what plain scratch gives, to the fp32 sums'
+    order (the scalar kernel takes the first: 6e-6, and one rounding to bf16)."""
+    QL, KVL, topk, positions = 4, 2, 64, [5, 200]
+    rn, M = gen(3), len(positions)
+    k, v = (rn(M, 256, KVL * 256).bfloat16() for _ in range(2))
+    q, proj, table = rn(M, QL, 256), rn(M, QL * 512), i32(range(M))
+    sel, sel_n = torch.zeros(M, topk, dtype=torch.int32, device=DEV), i32([-1] * M)
+    outs = []
+    for o_, n in ((0, 6), (off, nsplit)):
+        pm, pl = (torch.full((M, QL, n), float("nan"), device=DEV) for _ in range(2))
+        pacc = torch.full((M * QL * n * 256 + o_,), float("nan"), device=DEV)[o_:]
+        o = torch.zeros(M, QL, 256, dtype=torch.bfloat16, device=DEV)
+        assert _lib().qwk_qsa_attend(P(q), QL, KVL, M, P(i32(range(M))), P(i32(positions)), P(k), P(v), None, None, M, P(table), 1, P(sel), P(sel_n), topk, 4, n,
+                                     P(pm), P(pl), P(pacc), P(proj), QL * 512, P(o), S()) == 0
+        torch.cuda.synchronize()
+        outs.append(o.float())
+    assert bool(torch.isfinite(outs[0]).all())
+    assert bool(((outs[1] - outs[0]).abs() <= outs[0].abs() * 2 ** -7 + 1e-5).all())
+
+
 def test_router_rows_without_room_are_refused():
     """Rows so long that shared memory has no room for them in any plan: an error of the launcher, and nothing runs."""
     K_, nrs, M = 65536, 16, 8

@@ -785,7 +785,8 @@ QW_API int qwk_qsa_attend(const float *q, int QL, int KVL, int M, const int *slo
     }
     int ht = per_kv % 4 == 0 ? 4 : (per_kv % 3 == 0 ? 3 : (per_kv % 2 == 0 ? 2 : 1));
     dim3 grid(nsplit, M, QL / ht);
-    if (QL % KVL == 0 && per_kv <= 16) launch_pdl(qsa_attend_split_kernel, dim3(nsplit, M, KVL), dim3(256), AD_SMEM, s, a, g_err_ptr);
+    // the tensor-core form stores sums two at a time
+    if (QL % KVL == 0 && per_kv <= 16 && ((uintptr_t)pacc & 7) == 0) launch_pdl(qsa_attend_split_kernel, dim3(nsplit, M, KVL), dim3(256), AD_SMEM, s, a, g_err_ptr);
     else if (ht == 4) launch_pdl(qsa_attend_kernel<4>, grid, dim3(256), 0, s, a);
     else if (ht == 3) launch_pdl(qsa_attend_kernel<3>, grid, dim3(256), 0, s, a);
     else if (ht == 2) launch_pdl(qsa_attend_kernel<2>, grid, dim3(256), 0, s, a);
