@@ -204,7 +204,7 @@ def test_flash_decode_with_infinite_keys_and_values(heads):
         assert float((got[m] - want)[ok].norm() / want[ok].norm()) < 2 ** -8
 
 
-@pytest.mark.parametrize("off,nsplit", [(1, 6)])
+@pytest.mark.parametrize("off,nsplit", [(1, 6), (0, 6200)])
 def test_flash_decode_with_scratch_at_any_address_and_many_splits(off, nsplit):
     """Sums that lie on 4 bytes, and more splits than a list needs (behind its end they hold nothing): what plain scratch gives, to the fp32 sums'
     order (the scalar kernel takes the first: 6e-6, and one rounding to bf16)."""

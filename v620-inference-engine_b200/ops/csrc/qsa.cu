@@ -629,6 +629,7 @@ __global__ void __launch_bounds__(256) qsa_attend_kernel(QsaAttendArgs a) {
 // grid (M, QL), 256 threads: merge the splits, apply sigmoid(gate), write bf16.  The splits behind the list's end have a maximum of -inf and hold
 // nothing (one in front of it whose scores are all -inf, for keys that are infinite, has the lowest number instead, and sums of 0).  The weights are
 // formed once per block and the partial sums' loads are eight at a time (24 rows, sums out of memory: one split behind the other 22 us, now 15).
+constexpr int COMBINE_SPLITS = 28000;          // as many as shared memory holds weights and sums of: lists of 1.8 million tokens
 __global__ void __launch_bounds__(256) qsa_combine_kernel(const float *pm, const float *pl, const float *pacc, int nsplit,
                                                           const float *proj, int ld_proj, int QL, bf16 *o) {
     extern __shared__ float s_w[];          // [nsplit] weights, [nsplit] sums
@@ -780,7 +781,8 @@ QW_API int qwk_qsa_attend(const float *q, int QL, int KVL, int M, const int *slo
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
     if (!attr_done[dev]) {
-        if (cudaFuncSetAttribute(qsa_attend_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AD_SMEM) != cudaSuccess) return -3;
+        if (cudaFuncSetAttribute(qsa_attend_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AD_SMEM) != cudaSuccess ||
+            cudaFuncSetAttribute(qsa_combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, COMBINE_SPLITS * 8) != cudaSuccess) return -3;
         attr_done[dev] = true;
     }
     int ht = per_kv % 4 == 0 ? 4 : (per_kv % 3 == 0 ? 3 : (per_kv % 2 == 0 ? 2 : 1));
