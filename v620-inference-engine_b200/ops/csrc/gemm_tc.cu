@@ -1093,6 +1093,7 @@ static TcForm form_of(int T, int N, int K, bool peers) {
 // roles).  What a tile of nt tokens costs, by the same measure: 0.07 + 0.00127 nt us, at least 0.21 (256 tokens 0.395, 208 0.33, 160 0.26, 96
 // 0.21; 4,096 x 16,480 x 2,560 in tiles of 96 to 256 tokens: 315, 266 (128), 242 (160), 235 (208), 237 us (256), and 260 with the roles kept).  The
 // widest of equally cheap tiles is taken: it reads the least.  A caller that moves the line of the pairs measures the forms that keep the roles.
+// By these figures an exchanged tile of 256 tokens costs less than a pair's tile that keeps the roles, so that form is left to products between ranks.
 static int g_exchange_nt = 0;            // 0: by cost; > 0: that many; < 0: never (measurements and tests)
 static int exchanged_tile(int T, int N, int K) {
     if (g_exchange_nt < 0 || g_pair_min_n != TC_PAIR_MIN_N) return 0;

@@ -41,7 +41,8 @@ static cudaError_t launch_sgemv_nt(SGemvArgs &a, size_t smem, int grid, cudaStre
 }
 
 // Up to 8 activation rows per pass, or 16 or 24 when they fit in shared memory next to the weight stages: every further pass
-// streams the weights again (the head over 24 rows of a verification step: 442 us in two passes, 230 in one).
+// streams the weights again (the head over 24 rows of a verification step: 422 us in two passes, 268 in one; 25 to 32 rows
+// take two of 16).
 static cudaError_t launch_sgemv(SGemvArgs &a, cudaStream_t s) {
     int grid;
     if (a.M > 16 && a.M <= 24) {

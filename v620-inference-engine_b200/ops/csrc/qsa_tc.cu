@@ -16,7 +16,7 @@
 // Why not gather: 2,051 rows per query are 4.2 MB out of L2 for every query, and that, at 6.8 TB/s, is what the gather costs
 // (qsa_mma.cuh: 0.66 us per query, wherever it lies).  Here a tile is read once for 21 queries of 12 heads; the price is the keys nobody
 // chose, so contexts that are long for their chunk stay with the gather (qwk_qsa_takes_tc).  24 query heads over 2, us a layer,
-// gathered / here: 1,021 tokens 226 / 57, 4,096 tokens 1941 / 336, 2,048 tokens at position 16,384 1362 / 1009.
+// gathered / here: 1,021 tokens 220 / 58, 4,096 tokens 1897 / 314, 2,048 tokens at position 16,384 1340 / 991.
 #include "kernels.h"
 #include "tc.cuh"
 
@@ -441,6 +441,9 @@ static bool qsa_tc_fits(int QL, int KVL, int M, int last_pos, int ratio, int ld_
 // tile of 128 keys; the kernel that gathers has three blocks of a query and KV head on each SM and takes a wave 20 us and 112 more when
 // the lists are full.  us, gathered / here: 1 row at position 1,000 69 / 46, at 9,000 129 / 186; 300 rows at 0 50 / 34, at 9,000 267 / 190,
 // at 16,384 269 / 320; 1,021 at 16,384 683 / 641, at 24,000 688 / 922; 2,048 at 16,384 1340 / 978, at 24,000 1344 / 1385; 100 at 0 27 / 31.
+// Where the keys lie makes no difference to the line: over host pages that are not staged the dense tiles cost 4 to 35 times less still (each row
+// crosses the host link once per pair of CTAs, not once per query), ms: 300 rows at 0 7.4 / 0.44, at 4,000 49 / 2.6; 1,021 at 0 51 / 3.3, at 9,000
+// 184 / 18; 4,096 at 0 571 / 16.  (Only where the cache of host rows holds all that a small chunk chose would the gather be the faster one.)
 QW_API int qwk_qsa_takes_tc(int QL, int KVL, int M, int last_pos, int topk, int ratio, int ld_mask, int ld_proj) {
     if (!qsa_tc_fits(QL, KVL, M, last_pos, ratio, ld_mask, ld_proj)) return 0;
     const long long pairs = NUM_SMS / 2, blocks = 3 * NUM_SMS, units = ((long long)M * (QL / KVL) + 255) / 256 * KVL;

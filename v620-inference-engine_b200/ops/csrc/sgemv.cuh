@@ -12,10 +12,10 @@
 // order, so a row's result does not depend on how many other rows share the step.
 //
 // What bounds it: the weights, and beside them the work per stage that does not shrink with the rows.  Boxes of 16 rows (single rows as bulk
-// copies cost 85 cycles each), two groups that take every other tile (one converts its sums while the other multiplies) and all of the
-// rows in one pass (x in parts of K where it has no room).  us, one group and 16 rows a pass / now: 248,320 x 2,560 at 1 row 215 / 187, at 8
-// 215 / 194, at 16 225 / 227, at 24 421 / 267; 16,480 x 2,560 at 1 15.9 / 14.3, at 24 33 / 24; 2,560 x 6,144 at 1 10.8 / 9.8, at 16 28 / 17,
-// at 24 41 / 18.7, at 32 54 / 30.
+// copies cost 85 cycles each), two groups that take every other tile (one converts its sums while the other multiplies) and up to
+// 24 rows in one pass (x in parts of K where it has no room).  us, one group and 16 rows a pass / now: 248,320 x 2,560 at 1 row 215 / 187, at 8
+// 216 / 195, at 16 226 / 217, at 24 422 / 268, at 32 (two passes) 447 / 430; 16,480 x 2,560 at 1 15.9 / 14.3, at 16 19.2 / 19.4, at 24 33 / 24;
+// 2,560 x 6,144 at 1 10.7 / 9.8, at 16 28 / 17, at 24 41 / 18.7, at 32 54 / 30.
 // Used by: the bf16 GEMV (projections, lm_head, PLE) and the MoE router (+ routing epilogue).
 #pragma once
 #include "fuse.cuh"

@@ -19,7 +19,7 @@
 // units, one and a half for each of 148 SMs.  A run that does not hold all of a unit's keys leaves its O, reference and sum, and a second kernel
 // merges them: 129 us whole, 108 + 12 dealt.
 // What bounds it: the exponentials (128 x 128 per tile at 16 a cycle and SM: 1024 cycles; MMAs 780).  It replaces a flash kernel on mma.sync (16 queries a warp, each warp reading every K and V fragment
-// from shared memory), which took 444 us there; this one takes 119.
+// from shared memory), which took 444 us there.
 #include "tc.cuh"
 
 namespace qw {
