@@ -14,7 +14,11 @@ def _lib():
 
 
 def P(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
+    if t is None:
+        return None
+    p = C.c_void_p(t.data_ptr())
+    p.tensor = t          # a tensor made inside a call lives until the launch: freed at once, its memory would be the next argument's
+    return p
 
 
 def S():
